@@ -1,15 +1,323 @@
 // Matrix product on the FMA units: Y[M,N] = X[M,K] * W[N,K]^T with float32
 // accumulation and no reduced-precision mode of any kind.  It is the matrix
-// product of the true 32-bit path, and the fallback of the bfloat16 path for
-// shapes the tensor-core kernel refuses (K not a multiple of 8) and for
-// weights that the checkpoint stores in 32-bit.
+// product of the true 32-bit path (gemm_f32_kernel), and the fallback of the
+// bfloat16 path for shapes the tensor-core kernel refuses (K not a multiple of
+// 8) and for weights that the checkpoint stores in 32-bit (gemm_fma_kernel).
 //
 // y[t,o] = sum_i W[o,i] x[t,i], W row-major [out, in]
 // (crates/model/src/ops.rs:83-101).  Every output element is accumulated by
-// one thread in the order i = 0..K-1, so a row's result does not depend on M,
-// on the tile it falls into or on what else is in the batch.
+// one thread in an order that K alone decides, so a row's result does not
+// depend on M, on the tile it falls into or on what else is in the batch.
 #include "common.cuh"
 
+// ---------------------------------------------------------------------------
+// float32 x float32 -> float32.  K is cut into segments of F32_SEG.  Within a segment an element has two chains, one
+// over the even and one over the odd k, each from the segment's first k up and added at its end: the two halves of one
+// packed multiply-add (fma.rn.f32x2), whose operands are neighbouring k as they lie in memory, so nothing is transposed or
+// duplicated on the way.  The segments' sums are added in their order.  Both kernels follow that order.
+// ---------------------------------------------------------------------------
+#define F32_SEG 512
+
+// BYTES from global to shared memory; where not valid nothing is read and zeros are written
+template <int BYTES>
+__device__ __forceinline__ void copy_async(uint32_t dst, const float* src, bool valid) {
+  const int n = valid ? BYTES : 0;
+  if (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float both(unsigned long long v) {          // the even chain plus the odd one
+  return __fadd_rn(__uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32)));
+}
+// One thread's share of the copies of a [ROWS x BK] block of a row-major matrix into rows BK + 4 floats apart, VEC floats a
+// copy: the thread keeps its columns, walks down the rows, and moves on by whole k blocks, so that a copy costs an
+// addition.  Rows past the matrix and columns past K read nothing and give zeros.
+template <int ROWS, int BK, int VEC>
+struct BlockCopy {
+  static constexpr int PER_ROW = BK / VEC, STEP = PER_ROW < 128 ? 128 / PER_ROW : 1, N = (ROWS + STEP - 1) / STEP;
+  static_assert(128 % PER_ROW == 0, "a thread keeps its columns");
+  const float* src;            // this thread's first element of the block at k = 0
+  long long row_step;
+  uint32_t to;                 // its place in the block, bytes
+  int k, live;                 // its column; how many of its rows exist
+  __device__ __forceinline__ BlockCopy(const float* matrix, long long ld, int row0, int rows) {
+    const int r = (int)threadIdx.x / PER_ROW;
+    k = ((int)threadIdx.x % PER_ROW) * VEC;
+    live = row0 + r < rows && r < ROWS ? (min(rows - row0, ROWS) - r + STEP - 1) / STEP : 0;
+    src = matrix + (live ? (size_t)(row0 + r) * ld + k : 0);
+    row_step = live > 1 ? STEP * ld : 0;
+    to = (uint32_t)(r * (BK + 4) + k) * 4u;
+  }
+  __device__ __forceinline__ void operator()(uint32_t block, int k0, int K) const {
+    const int n = k0 + k < K ? live : 0;
+    const float* p = n ? src + k0 : src;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      if (ROWS % STEP && (int)threadIdx.x / PER_ROW + i * STEP >= ROWS) break;
+      copy_async<VEC * 4>(block + to + (uint32_t)(i * STEP * (BK + 4) * 4), p, i < n);
+      if (i + 1 < n) p += row_step;
+    }
+  }
+};
+
+// Prompts: 128 threads as 8 (tokens) x 16 (features), TM x TN elements each.  Rows in shared memory are 20 floats apart,
+// so eight rows read at the same k lie in different banks; 8 x 8 elements take 16 shared-memory reads per 128 packed
+// multiply-adds.  The sums of earlier segments wait in shared memory.  Bound by the FMA units and the reads that feed
+// them (4 x 4: fmaheavy 66 %, shared-memory wavefronts 72 % of the cycles).  970 tokens, N = K = 2048: 231 us (35 TFLOP/s;
+// the one-chain 64 x 64 kernel that this replaced: 16 TFLOP/s); 2500 tokens, N = 4096: 971 us (43 TFLOP/s).
+template <int TM, int TN>
+struct F32Tile {
+  static constexpr int BM = 8 * TM, BN = 16 * TN, BK = 16, STAGES = 4, PITCH = BK + 4;
+  static constexpr int STAGE = (BM + BN) * PITCH;                      // floats
+  static constexpr int TOTAL_PITCH = BN + 8;
+  static constexpr size_t SMEM = ((size_t)STAGES * STAGE + (size_t)BM * TOTAL_PITCH) * sizeof(float);
+};
+
+template <int TM, int TN, int VEC>
+__global__ void __launch_bounds__(128, TM * TN >= 64 ? 2 : 4)
+gemm_f32_tile_kernel(const float* __restrict__ X, const float* __restrict__ W, float* __restrict__ Y, int M, int N, int K,
+                     long long ldx, long long ldw, long long ldy, int n_tiles) {
+  using Tile = F32Tile<TM, TN>;
+  constexpr int BM = Tile::BM, BN = Tile::BN, BK = Tile::BK, STAGES = Tile::STAGES, PITCH = Tile::PITCH, STAGE = Tile::STAGE;
+  extern __shared__ __align__(16) float tiles[];                      // per stage: W [BN][PITCH], X [BM][PITCH]; totals
+  float* totals = tiles + STAGES * STAGE;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(tiles);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tn = (warp & 1) * 8 + (lane & 7), tm = (warp >> 1) * 4 + (lane >> 3);      // 16 x 8
+  const int n0 = (blockIdx.x % n_tiles) * BN, m0 = (blockIdx.x / n_tiles) * BM;
+  const int n_kb = (K + BK - 1) / BK;
+  const BlockCopy<BN, BK, VEC> copy_w(W, ldw, n0, N);
+  const BlockCopy<BM, BK, VEC> copy_x(X, ldx, m0, M);
+  auto load = [&](int kb) {
+    const uint32_t dst = base + (uint32_t)((kb % STAGES) * STAGE) * 4u;
+    copy_w(dst, kb * BK, K);
+    copy_x(dst + (uint32_t)(BN * PITCH) * 4u, kb * BK, K);
+  };
+  pdl_launch_dependents();
+  pdl_wait();
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (s < n_kb) load(s);
+    copy_commit();
+  }
+  unsigned long long acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+
+  for (int kb = 0; kb < n_kb; ++kb) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();                           // tile kb is there, and everyone is done with the stage that is filled next
+    if (kb + STAGES - 1 < n_kb) load(kb + STAGES - 1);
+    copy_commit();
+    const float* ws = tiles + (kb % STAGES) * STAGE + tn * PITCH;
+    const float* xs = tiles + (kb % STAGES) * STAGE + BN * PITCH + tm * PITCH;
+    constexpr int UNROLL = TM * TN >= 64 ? 1 : BK / 4;        // (8 x 8: the next reads' registers would be spilled)
+#pragma unroll UNROLL
+    for (int k = 0; k < BK; k += 4) {
+      ulonglong2 a[TM];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + i * 8 * PITCH + k);
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(ws + j * 16 * PITCH + k);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) fma2(acc[i][j], a[i].x, b.x);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) fma2(acc[i][j], a[i].y, b.y);
+      }
+    }
+    if ((kb + 1) % (F32_SEG / BK) == 0 && kb + 1 < n_kb) {           // a segment ends and another follows
+      const bool first = kb + 1 == F32_SEG / BK;
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+          float* t = totals + (i * 8 + tm) * Tile::TOTAL_PITCH + j * 16 + tn;          // this thread's own word
+          *t = first ? both(acc[i][j]) : __fadd_rn(*t, both(acc[i][j]));
+          acc[i][j] = 0ull;
+        }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + i * 8 + tm;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int n = n0 + j * 16 + tn;
+      const float v = both(acc[i][j]);
+      if (n < N)
+        Y[(size_t)m * ldy + n] = K > F32_SEG ? __fadd_rn(totals[(i * 8 + tm) * Tile::TOTAL_PITCH + j * 16 + tn], v) : v;
+    }
+  }
+}
+
+// Few tokens (up to 2 MT a CTA): 16 features, four segments of K at a time.  Thread (feature f, segment g, token half h)
+// follows its feature's chain over segment g for MT tokens, so a value of W is read from shared memory once per token
+// half and the tokens' values are broadcasts; a quarter of the chain's length and four streams of each row are what a
+// row costs.  The first stages of W are asked for before the kernel before has ended.  Three tokens, K = 2048: 10 us at
+// N = 2048 (the 64 x 64 kernel, 32 CTAs with one chain of 2048 steps: 184 us a product), 65 us at N = 32768 (4.1 TB/s);
+// bound by the latency of a CTA's first tiles at the former, by HBM and the reads of X at the latter.
+template <int MT>
+struct F32Rows {
+  static constexpr int BM = 2 * MT, BN = 16, GROUPS = 4, BK = 32, PITCH = BK + 4;
+  static constexpr int STAGES = 6;
+  static constexpr int STAGE = GROUPS * (BN + BM) * PITCH;             // floats
+  static constexpr size_t SMEM = ((size_t)STAGES * STAGE + GROUPS * BN * BM) * sizeof(float);
+};
+
+template <int MT, int VEC>
+__global__ void __launch_bounds__(128)
+gemm_f32_rows_kernel(const float* __restrict__ X, const float* __restrict__ W, float* __restrict__ Y, int M, int N, int K,
+                     long long ldx, long long ldw, long long ldy, int n_tiles) {
+  using Rows = F32Rows<MT>;
+  constexpr int BM = Rows::BM, BN = Rows::BN, G = Rows::GROUPS, BK = Rows::BK, PITCH = Rows::PITCH, STAGES = Rows::STAGES;
+  constexpr int STAGE = Rows::STAGE, PER_SEG = F32_SEG / BK;
+  extern __shared__ __align__(16) float tiles[];           // per stage: W [G][BN][PITCH], X [G][BM][PITCH]; segment sums
+  float* sums = tiles + STAGES * STAGE;                    // [G][BM][BN]
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(tiles);
+  const int f = threadIdx.x & 15, g = (threadIdx.x >> 4) & 3, h = threadIdx.x >> 6;
+  const int n0 = (blockIdx.x % n_tiles) * BN, m0 = (blockIdx.x / n_tiles) * BM;
+  const int n_seg = (K + F32_SEG - 1) / F32_SEG, n_rounds = (n_seg + G - 1) / G;
+  const int n_steps = n_rounds * PER_SEG;                  // step i: k block i % PER_SEG of the segments of round i / PER_SEG
+  const BlockCopy<BN, BK, VEC> copy_w(W, ldw, n0, N);
+  const BlockCopy<BM, BK, VEC> copy_x(X, ldx, m0, M);
+  auto load_w = [&](int i) {
+#pragma unroll
+    for (int q = 0; q < G; ++q)
+      copy_w(base + (uint32_t)((i % STAGES) * STAGE + q * BN * PITCH) * 4u,
+             ((i / PER_SEG) * G + q) * F32_SEG + (i % PER_SEG) * BK, K);
+  };
+  auto load_x = [&](int i) {
+#pragma unroll
+    for (int q = 0; q < G; ++q)
+      copy_x(base + (uint32_t)((i % STAGES) * STAGE + (G * BN + q * BM) * PITCH) * 4u,
+             ((i / PER_SEG) * G + q) * F32_SEG + (i % PER_SEG) * BK, K);
+  };
+  pdl_launch_dependents();
+  for (int s = 0; s < STAGES - 1 && s < n_steps; ++s) load_w(s);     // the weights do not wait for the kernel before
+  pdl_wait();
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (s < n_steps) load_x(s);
+    copy_commit();
+  }
+  unsigned long long acc[MT];
+  float total[MT];                                         // (group 0 keeps the totals of its feature)
+#pragma unroll
+  for (int i = 0; i < MT; ++i) acc[i] = 0ull, total[i] = 0.f;
+  for (int step = 0; step < n_steps; ++step) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();
+    if (step + STAGES - 1 < n_steps) load_w(step + STAGES - 1), load_x(step + STAGES - 1);
+    copy_commit();
+    const float* ws = tiles + (step % STAGES) * STAGE + (g * BN + f) * PITCH;
+    const float* xs = tiles + (step % STAGES) * STAGE + (G * BN + g * BM + h) * PITCH;   // token i of this thread: row 2 i + h
+#pragma unroll
+    for (int k = 0; k < BK; k += 4) {
+      const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(ws + k);
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(xs + 2 * i * PITCH + k);
+        fma2(acc[i], a.x, b.x), fma2(acc[i], a.y, b.y);
+      }
+    }
+    if ((step + 1) % PER_SEG == 0) {                       // the round's segments join the totals in their order
+      const int round = step / PER_SEG;
+#pragma unroll
+      for (int i = 0; i < MT; ++i) sums[(g * BM + 2 * i + h) * BN + f] = both(acc[i]), acc[i] = 0ull;
+      __syncthreads();
+      if (g == 0) {
+#pragma unroll
+        for (int i = 0; i < MT; ++i) {
+          const float* t = sums + (2 * i + h) * BN + f;
+          total[i] = round == 0 ? *t : __fadd_rn(total[i], *t);
+          for (int q = 1; q < G && round * G + q < n_seg; ++q) total[i] = __fadd_rn(total[i], t[q * BM * BN]);
+        }
+      }
+      __syncthreads();
+    }
+  }
+  if (g == 0 && n0 + f < N) {
+#pragma unroll
+    for (int i = 0; i < MT; ++i) {
+      const int m = m0 + 2 * i + h;
+      if (m < M) Y[(size_t)m * ldy + n0 + f] = total[i];
+    }
+  }
+}
+
+// One launch of a kernel whose CTAs own BM tokens x BN features.
+template <typename Shape, typename Kernel>
+static int launch_f32(Kernel kernel, bool& attr_set, const float* X, const float* W, float* Y, int M, int N, int K,
+                      long long ldx, long long ldw, long long ldy, cudaStream_t stream) {
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape::SMEM);
+    if (e != cudaSuccess) return (int)e;
+    attr_set = true;
+  }
+  const long long n_tiles = (N + Shape::BN - 1) / Shape::BN, m_tiles = (M + Shape::BM - 1) / Shape::BM;
+  if (n_tiles * m_tiles > 0x7fffffff) return LLMX_REFUSED(3);
+  launch_pdl(kernel, dim3((unsigned)(n_tiles * m_tiles)), dim3(128), Shape::SMEM, stream, X, W, Y, M, N, K, ldx, ldw, ldy,
+             (int)n_tiles);
+  return LLMX_LAUNCH_STATUS();
+}
+
+// The float32 product by a launch of the caller's choice (tests: every one gives the same bits); -1: by the rule.
+// 0..3: rows kernel with 2, 4, 8, 16 tokens a CTA; 4: tiles of 32 x 64; 5: tiles of 64 x 128.
+#define F32_N_FORMS 6
+LLMX_API int llmx_gemm_f32_form(int form, const float* X, const float* W, float* Y, int M, int N, int K, long long ldx,
+                                long long ldw, long long ldy, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0 || ldx < K || ldw < K || ldy < N || form >= F32_N_FORMS) return LLMX_REFUSED(1);
+  if ((M + 63) / 64 > 65535) return LLMX_REFUSED(3);
+  if (form < 0) {
+    // Rule: up to 16 tokens in one CTA's rows.  Beyond that the cheapest of what was measured at K = 2048 (us; all three
+    // grow with K alike): a round of 296 CTAs of 16 x 16 elements takes 19, 148 tiles of 32 x 64 take 33 (52 at least,
+    // for one alone cannot hide its waits), 148 tiles of 64 x 128 take 112 (150 at least).
+    const auto rounds = [](long long n, int m) { return (n + m - 1) / m; };
+    const auto tiles = [&](int bm, int bn) { return rounds(M, bm) * rounds(N, bn); };
+    if (M <= 16) {
+      form = M <= 2 ? 0 : M <= 4 ? 1 : M <= 8 ? 2 : 3;
+    } else {
+      const long long rows = 19 * rounds(tiles(16, 16), 296);
+      long long small = 33 * rounds(tiles(32, 64), 148), large = 112 * rounds(tiles(64, 128), 148);
+      if (small < 52) small = 52;
+      if (large < 150) large = 150;
+      form = rows <= small && rows <= large ? 3 : small <= large ? 4 : 5;
+    }
+  }
+  // 16-byte copies where every row starts on a 16-byte boundary and K ends on one, else 4-byte copies
+  const bool wide = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && !((uintptr_t)X & 15) && !((uintptr_t)W & 15);
+#define GO(SHAPE, KERNEL, ...)                                                                                      \
+  {                                                                                                                 \
+    static bool set4 = false, set1 = false;                                                                         \
+    return wide ? launch_f32<SHAPE>(KERNEL<__VA_ARGS__, 4>, set4, X, W, Y, M, N, K, ldx, ldw, ldy, stream)           \
+                : launch_f32<SHAPE>(KERNEL<__VA_ARGS__, 1>, set1, X, W, Y, M, N, K, ldx, ldw, ldy, stream);          \
+  }
+#define TILE(TM, TN) \
+  { using S = F32Tile<TM, TN>; GO(S, gemm_f32_tile_kernel, TM, TN) }
+  switch (form) {
+    case 0: GO(F32Rows<1>, gemm_f32_rows_kernel, 1)
+    case 1: GO(F32Rows<2>, gemm_f32_rows_kernel, 2)
+    case 2: GO(F32Rows<4>, gemm_f32_rows_kernel, 4)
+    case 3: GO(F32Rows<8>, gemm_f32_rows_kernel, 8)
+    case 4: TILE(4, 4)
+    case 5: TILE(8, 8)
+  }
+#undef TILE
+#undef GO
+  return LLMX_REFUSED(1);
+}
+
+// ---------------------------------------------------------------------------
+// The other types: one chain per element, k = 0..K-1.
+// ---------------------------------------------------------------------------
 #define FMA_BM 64
 #define FMA_BN 64
 #define FMA_BK 16
@@ -80,7 +388,7 @@ LLMX_API int llmx_gemm_fma(const void* X, int x_dtype, const void* W, int w_dtyp
   launch_pdl(gemm_fma_kernel<TX, TW, TY>, grid, dim3(256), 0, stream, (const TX*)X, (const TW*)W, (TY*)Y, M, N, K, ldx, ldw, ldy)
   const int key = x_dtype * 4 + w_dtype * 2 + y_dtype;
   switch (key) {
-    case 0: CASE(float, float, float); break;
+    case 0: return llmx_gemm_f32_form(-1, (const float*)X, (const float*)W, (float*)Y, M, N, K, ldx, ldw, ldy, stream);
     case 1: CASE(float, float, bf16); break;
     case 2: CASE(float, bf16, float); break;
     case 3: CASE(float, bf16, bf16); break;
