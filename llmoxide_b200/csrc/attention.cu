@@ -128,17 +128,398 @@ __global__ void attention_paged_kernel(const TA* __restrict__ q, TA* __restrict_
   }
 }
 
+// ---------------------------------------------------------------------------
+// The same in float32, by tiles.  The kernel above takes a warp per (token, head), reads every key row once per head and
+// query, and follows one chain of loads; this one shares a tile of 64 keys (one page) among the query rows of a CTA.
+//
+// A query row's keys are cut at multiples of 64 positions.  Within a tile: scores from two chains over the even and the
+// odd dims (packed multiply-adds), the tile's maximum, exponentials against it, their sum (four keys a lane, then a
+// butterfly over 16 lanes) and the weighted values key by key.  The tiles' (maximum, sum, values) then join a running
+// state in the order of the tiles.  That order depends on the query's position and mask alone, and both forms below
+// follow it step by step, so a position's result does not depend on how tokens were cut into steps or batched.
+//   prompts (SPLIT false)   a CTA owns 8 TR query rows (tokens x the heads that share a kv head) and walks the tiles
+//   few tokens (SPLIT true) a cluster of 8 CTAs owns one token's rows; CTA r takes tiles r, r + 8, ..., and after every
+//                           round of 8 tiles each CTA joins a slice of the dims out of the eight partial results
+// A key that a row must not see is left out, not multiplied by zero (its value may be anything).
+// 16 heads of 128 over 4 kv heads, a window of 1024: three prompts of 517, 323 and 130 tokens 235 us (the kernel above:
+// 2060), one more token each 27 us (656).  A few tokens are bound by the latency of a round of tiles (copy, scores,
+// values, join, one after the other), prompts by the shared-memory reads.
+// ---------------------------------------------------------------------------
+#define AF_KEYS 64             // keys per tile = LLMX_PAGE
+#define AF_THREADS 128         // 8 (rows) x 16 (keys, then dims)
+#define AF_SPLIT 8             // CTAs of a cluster
+static_assert(AF_KEYS == LLMX_PAGE, "a tile is a page");
+
+struct AfArgs {
+  const float *q, *k_cache, *v_cache, *gate, *sinks, *score_bias;
+  float* out;
+  const int *block_table, *token_seq, *token_pos;
+  size_t q_stride, gate_stride;
+  int table_width, n_tokens, H, G, D, Dv, window, keep_first, chunk, bias_len;
+  int heads_per_cta, tokens_per_cta, head_blocks;
+  float scale, sink, softcap;
+};
+
+__device__ __forceinline__ void af_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long af_pair(float x, float y) {
+  return (unsigned long long)__float_as_uint(x) | ((unsigned long long)__float_as_uint(y) << 32);
+}
+__device__ __forceinline__ float af_lo(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float af_hi(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
+// rows x d floats (d a multiple of 4), 16 bytes a copy, a warp per row
+__device__ __forceinline__ void af_copy_rows(float* dst, int pitch, const float* src, size_t ld, int rows, int d) {
+  for (int r = threadIdx.x >> 5; r < rows; r += AF_THREADS / 32)
+    for (int c = (threadIdx.x & 31) * 4; c < d; c += 128)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                       (uint32_t)__cvta_generic_to_shared(dst + r * pitch + c)), "l"(src + r * ld + c) : "memory");
+}
+// A partial result joins a running one: the maximum, and the factors of both.
+__device__ __forceinline__ float af_join(float m, float pm, float& c1, float& c2) {
+  const float mn = fmaxf(m, pm);
+  c1 = expf(m - mn), c2 = expf(pm - mn);
+  return mn;
+}
+__device__ __forceinline__ float af_remote(const float* local, unsigned rank) {      // the same word of another CTA of the cluster
+  uint32_t a = (uint32_t)__cvta_generic_to_shared(local), b;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(a), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(b) : "memory");
+  return v;
+}
+__device__ __forceinline__ void af_cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// shared memory (floats): Q [8 TR][D + 4], K [64][D + 4], V [64][64 NC], P [8 TR][68], row facts, and for SPLIT two
+// buffers of partial results [8][64 NC + 2]
+template <int TR, int NC>
+__host__ __device__ constexpr size_t af_smem(int D, bool split) {
+  return 4 * ((size_t)8 * TR * (D + 4) + AF_KEYS * (D + 4) + AF_KEYS * 64 * NC + 8 * TR * (AF_KEYS + 4) + 3 * 8 * TR +
+              (split ? 2 * 8 * (64 * NC + 2) : 0));
+}
+
+template <int TR, int NC, bool SPLIT>
+__global__ void __launch_bounds__(AF_THREADS) attention_f32_kernel(const AfArgs a) {
+  constexpr int BR = 8 * TR, VP = 64 * NC, PP = AF_KEYS + 4, PART = VP + 2;
+  extern __shared__ __align__(16) float af_buf[];
+  const int D = a.D, DP = D + 4, Dv = a.Dv;
+  float* Qs = af_buf;
+  float* Ks = Qs + BR * DP;
+  float* Vs = Ks + AF_KEYS * DP;
+  float* Ps = Vs + AF_KEYS * VP;
+  int* row_pos = reinterpret_cast<int*>(Ps + BR * PP);       // position, first key of the window, sequence (-1: no row)
+  int* row_first = row_pos + BR;
+  int* row_seq = row_first + BR;
+  float* part = reinterpret_cast<float*>(row_seq + BR);      // SPLIT: [2][8][PART] = maximum, sum (-1: no key), values
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tn = lane & 15, tm = warp * 2 + (lane >> 4);     // a row's 16 threads are half a warp
+  const int rank = SPLIT ? (int)(blockIdx.x % AF_SPLIT) : 0;
+  const int R = a.H / a.G, g = blockIdx.y / a.head_blocks, h0 = (blockIdx.y % a.head_blocks) * a.heads_per_cta;
+  // prompts: the last tokens, which see most keys, start first
+  const int t0 = SPLIT ? (int)(blockIdx.x / AF_SPLIT) : ((int)gridDim.x - 1 - (int)blockIdx.x) * a.tokens_per_cta;
+  const int n_tok = SPLIT ? 1 : min(a.tokens_per_cta, a.n_tokens - t0);
+
+  for (int r = threadIdx.x; r < BR; r += AF_THREADS) {
+    const int tok = r / a.heads_per_cta, h = h0 + r % a.heads_per_cta;
+    const bool here = tok < n_tok && h < R;
+    const int p = here ? a.token_pos[t0 + tok] : 0;
+    int first = (a.window > 0 && p - (a.window - 1) > 0) ? p - (a.window - 1) : 0;
+    if (a.chunk > 0) first = max(first, p - p % a.chunk);
+    row_pos[r] = p, row_first[r] = first, row_seq[r] = here ? a.token_seq[t0 + tok] : -1;
+  }
+  for (int i = threadIdx.x; i < AF_KEYS * VP; i += AF_THREADS) Vs[i] = 0.f;       // (dims past Dv)
+  for (int r = 0; r < BR; ++r) {
+    const int tok = r / a.heads_per_cta, h = h0 + r % a.heads_per_cta;
+    if (tok >= n_tok || h >= R) {
+      for (int i = threadIdx.x; i < D; i += AF_THREADS) Qs[r * DP + i] = 0.f;
+    } else {
+      const float* src = a.q + (size_t)(t0 + tok) * a.q_stride + (size_t)(g * R + h) * D;
+      for (int i = threadIdx.x; i < D; i += AF_THREADS) Qs[r * DP + i] = src[i];
+    }
+  }
+  __syncthreads();
+
+  int pos[TR], first[TR], seq[TR];
+  float m[TR], l[TR];
+  unsigned long long acc[TR][2 * NC];
+#pragma unroll
+  for (int i = 0; i < TR; ++i) {
+    pos[i] = row_pos[i * 8 + tm], first[i] = row_first[i * 8 + tm], seq[i] = row_seq[i * 8 + tm];
+    m[i] = -INFINITY, l[i] = 0.f;
+#pragma unroll
+    for (int c = 0; c < 2 * NC; ++c) acc[i][c] = 0ull;
+  }
+  // SPLIT: this thread's elements of the CTA's slice of the dims, and their running state
+  const int slice = (Dv + AF_SPLIT - 1) / AF_SPLIT;
+  constexpr int OWN = SPLIT ? (8 * 8 * NC + AF_THREADS - 1) / AF_THREADS : 1;
+  float om[OWN], ol[OWN], oa[OWN];
+#pragma unroll
+  for (int e = 0; e < OWN; ++e) om[e] = -INFINITY, ol[e] = 0.f, oa[e] = 0.f;
+
+  // tokens of one sequence that follow one another share its tiles
+  for (int run = 0; run < n_tok;) {
+    const int s = row_seq[run * a.heads_per_cta];
+    int lo = row_first[run * a.heads_per_cta], hi = row_pos[run * a.heads_per_cta], end = run + 1;
+    for (; end < n_tok && row_seq[end * a.heads_per_cta] == s; ++end) {
+      lo = min(lo, row_first[end * a.heads_per_cta]);
+      hi = max(hi, row_pos[end * a.heads_per_cta]);
+    }
+    const int tok_lo = run, tok_hi = end;
+    run = end;
+    const int tile_first = lo / AF_KEYS, tile_last = hi / AF_KEYS;
+    const int n_kept = a.window > 0 && a.keep_first > 0 ? min(tile_first, (a.keep_first + AF_KEYS - 1) / AF_KEYS) : 0;
+    const int n_tiles = n_kept + tile_last - tile_first + 1;
+    const int* pages = a.block_table + (size_t)s * a.table_width;
+    bool mine[TR];              // whether the row belongs to this run
+#pragma unroll
+    for (int i = 0; i < TR; ++i) {
+      const int tok = (i * 8 + tm) / a.heads_per_cta;
+      mine[i] = seq[i] >= 0 && tok >= tok_lo && tok < tok_hi;
+    }
+    auto tile_at = [&](int j) { return j < n_kept ? j : tile_first + (j - n_kept); };
+    auto load_k = [&](int j) {
+      if (j < n_tiles)
+        af_copy_rows(Ks, DP, a.k_cache + cache_row_offset(pages[tile_at(j)], g, 0, a.G, D), D, AF_KEYS, D);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto load_v = [&](int j) {
+      if (j < n_tiles)
+        af_copy_rows(Vs, VP, a.v_cache + cache_row_offset(pages[tile_at(j)], g, 0, a.G, Dv), Dv, AF_KEYS, Dv);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    constexpr int STEP = SPLIT ? AF_SPLIT : 1;
+    __syncthreads();                            // (a run before is done with K and V)
+    load_k(rank), load_v(rank);
+    for (int j = rank, round = 0; j - rank < n_tiles; j += STEP, ++round) {
+      unsigned long long pacc[TR][2 * NC];
+      float pm[TR], pl[TR];
+      bool any[TR];
+      if (j < n_tiles) {
+        const int k0 = tile_at(j) * AF_KEYS;
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        // ---- scores: TR rows x keys tn, tn + 16, tn + 32, tn + 48 ----
+        unsigned long long sc[TR][4];
+#pragma unroll
+        for (int i = 0; i < TR; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) sc[i][c] = 0ull;
+        const float* qs = Qs + tm * DP;
+        const float* ks = Ks + tn * DP;
+#pragma unroll 4
+        for (int d = 0; d < D; d += 4) {
+          ulonglong2 x[TR];
+#pragma unroll
+          for (int i = 0; i < TR; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(qs + i * 8 * DP + d);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(ks + c * 16 * DP + d);
+#pragma unroll
+            for (int i = 0; i < TR; ++i) af_fma2(sc[i][c], x[i].x, y.x);
+#pragma unroll
+            for (int i = 0; i < TR; ++i) af_fma2(sc[i][c], x[i].y, y.y);
+          }
+        }
+        __syncthreads();                        // everyone has read K
+        load_k(j + STEP);
+        // ---- the tile's maximum, exponentials and their sum; P to shared memory, -1 where the row does not see the key
+#pragma unroll
+        for (int i = 0; i < TR; ++i) {
+          const int p = pos[i], f = first[i];
+          any[i] = mine[i] && k0 <= p && (k0 + AF_KEYS - 1 >= f || k0 < a.keep_first);
+          float sv[4];
+          bool live[4];
+          pm[i] = -INFINITY;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int key = k0 + tn + 16 * c;
+            live[c] = any[i] && key <= p && (key >= f || key < a.keep_first);
+            float v = __fmul_rn(__fadd_rn(af_lo(sc[i][c]), af_hi(sc[i][c])), a.scale);
+            if (a.softcap > 0.f) v = a.softcap * tanhf(v / a.softcap);
+            if (a.score_bias && live[c])
+              v = __fadd_rn(v, a.score_bias[(size_t)(g * R + h0 + (i * 8 + tm) % a.heads_per_cta) * a.bias_len +
+                                            min(p - key, a.bias_len - 1)]);
+            sv[c] = v;
+            if (live[c]) pm[i] = fmaxf(pm[i], v);
+          }
+#pragma unroll
+          for (int o = 8; o > 0; o >>= 1) pm[i] = fmaxf(pm[i], __shfl_xor_sync(0xffffffffu, pm[i], o));
+          pl[i] = 0.f;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const float e = live[c] ? expf(sv[c] - pm[i]) : -1.f;
+            if (live[c]) pl[i] = __fadd_rn(pl[i], e);
+            Ps[(i * 8 + tm) * PP + tn + 16 * c] = e;
+          }
+#pragma unroll
+          for (int o = 8; o > 0; o >>= 1) pl[i] = __fadd_rn(pl[i], __shfl_xor_sync(0xffffffffu, pl[i], o));
+        }
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();                        // V is there (and P)
+        // ---- weighted values: TR rows x dims 4 tn .. 4 tn + 3 of every 64 ----
+#pragma unroll
+        for (int i = 0; i < TR; ++i)
+#pragma unroll
+          for (int c = 0; c < 2 * NC; ++c) pacc[i][c] = 0ull;
+        const float* vs = Vs + tn * 4;
+#pragma unroll 1
+        for (int key = 0; key < AF_KEYS; key += 4) {
+          float4 w[TR];
+#pragma unroll
+          for (int i = 0; i < TR; ++i) w[i] = *reinterpret_cast<const float4*>(Ps + (i * 8 + tm) * PP + key);
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) {
+            ulonglong2 v[NC];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) v[c] = *reinterpret_cast<const ulonglong2*>(vs + (key + kk) * VP + 64 * c);
+#pragma unroll
+            for (int i = 0; i < TR; ++i) {
+              const float e = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
+              if (!(e < 0.f)) {
+                const unsigned long long ee = af_pair(e, e);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) af_fma2(pacc[i][2 * c], ee, v[c].x), af_fma2(pacc[i][2 * c + 1], ee, v[c].y);
+              }
+            }
+          }
+        }
+        __syncthreads();                        // everyone has read V and P
+        load_v(j + STEP);
+      }
+      if (!SPLIT) {
+#pragma unroll
+        for (int i = 0; i < TR; ++i) {
+          if (!any[i]) continue;
+          float c1, c2;
+          m[i] = af_join(m[i], pm[i], c1, c2);
+          l[i] = __fmaf_rn(pl[i], c2, __fmul_rn(l[i], c1));
+#pragma unroll
+          for (int c = 0; c < 2 * NC; ++c)
+            acc[i][c] = af_pair(__fmaf_rn(af_lo(pacc[i][c]), c2, __fmul_rn(af_lo(acc[i][c]), c1)),
+                                __fmaf_rn(af_hi(pacc[i][c]), c2, __fmul_rn(af_hi(acc[i][c]), c1)));
+        }
+      } else {
+        float* mine_part = part + ((size_t)(round & 1) * 8 + tm) * PART;
+        if (j < n_tiles) {
+          if (tn == 0) mine_part[0] = pm[0], mine_part[1] = any[0] ? pl[0] : -1.f;
+#pragma unroll
+          for (int c = 0; c < 2 * NC; ++c) {
+            const int d = (c >> 1) * 64 + tn * 4 + (c & 1) * 2;
+            mine_part[2 + d] = af_lo(pacc[0][c]), mine_part[3 + d] = af_hi(pacc[0][c]);
+          }
+        }
+        af_cluster_sync();                      // (a buffer is written again two rounds on, behind the next barrier)
+        const int here = min(AF_SPLIT, n_tiles - round * AF_SPLIT);
+#pragma unroll
+        for (int e = 0; e < OWN; ++e) {
+          const int idx = e * AF_THREADS + threadIdx.x, row = idx / slice, d = rank * slice + idx % slice;
+          if (row >= 8 || d >= Dv) continue;
+          const float* src = part + ((size_t)(round & 1) * 8 + row) * PART;
+          for (int k = 0; k < here; ++k) {
+            const float km = af_remote(src, k), kl = af_remote(src + 1, k), ka = af_remote(src + 2 + d, k);
+            if (kl < 0.f) continue;
+            float c1, c2;
+            om[e] = af_join(om[e], km, c1, c2);
+            ol[e] = __fmaf_rn(kl, c2, __fmul_rn(ol[e], c1));
+            oa[e] = __fmaf_rn(ka, c2, __fmul_rn(oa[e], c1));
+          }
+        }
+      }
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+
+  // ---- sinks, the output's gate, the division ----
+  auto inverse = [&](float mm, float ll, int tok, int h) {
+    if (a.sink > 0.f) ll = __fadd_rn(ll, __fmul_rn(a.sink, expf(-mm)));
+    if (a.sinks) ll = __fadd_rn(ll, expf(a.sinks[h] - mm));
+    float inv = __fdiv_rn(1.0f, ll);
+    if (a.gate) inv = __fmul_rn(inv, __fdiv_rn(1.0f, 1.0f + expf(-a.gate[(size_t)tok * a.gate_stride + h])));
+    return inv;
+  };
+  if (SPLIT) {
+#pragma unroll
+    for (int e = 0; e < OWN; ++e) {
+      const int idx = e * AF_THREADS + threadIdx.x, row = idx / slice, d = rank * slice + idx % slice;
+      if (row >= 8 || d >= Dv || row_seq[row] < 0) continue;
+      const int h = g * R + h0 + row;
+      a.out[((size_t)t0 * a.H + h) * Dv + d] = __fmul_rn(oa[e], inverse(om[e], ol[e], t0, h));
+    }
+    af_cluster_sync();                          // nobody leaves while its partial results may be read
+  } else {
+#pragma unroll
+    for (int i = 0; i < TR; ++i) {
+      if (seq[i] < 0) continue;
+      const int r = i * 8 + tm, tok = t0 + r / a.heads_per_cta, h = g * R + h0 + r % a.heads_per_cta;
+      const float inv = inverse(m[i], l[i], tok, h);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const int d = c * 64 + tn * 4;
+        if (d < Dv)
+          *reinterpret_cast<float4*>(a.out + ((size_t)tok * a.H + h) * Dv + d) =
+              make_float4(__fmul_rn(af_lo(acc[i][2 * c]), inv), __fmul_rn(af_hi(acc[i][2 * c]), inv),
+                          __fmul_rn(af_lo(acc[i][2 * c + 1]), inv), __fmul_rn(af_hi(acc[i][2 * c + 1]), inv));
+      }
+    }
+  }
+}
+
+template <int TR, int NC, bool SPLIT>
+static int launch_f32(AfArgs a, cudaStream_t stream) {
+  const int R = a.H / a.G, rows = 8 * TR;
+  a.heads_per_cta = R < rows ? R : rows;
+  a.tokens_per_cta = SPLIT ? 1 : rows / a.heads_per_cta;
+  a.head_blocks = (R + a.heads_per_cta - 1) / a.heads_per_cta;
+  auto kernel = attention_f32_kernel<TR, NC, SPLIT>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)af_smem<TR, NC>(ATT_MAX_D, SPLIT));
+    if (e != cudaSuccess) return (int)e;
+    attr_set = true;
+  }
+  const size_t smem = af_smem<TR, NC>(a.D, SPLIT);
+  if (SPLIT)
+    launch_pdl_cluster(kernel, dim3((unsigned)a.n_tokens * AF_SPLIT, a.G * a.head_blocks), dim3(AF_THREADS), smem, stream,
+                       AF_SPLIT, a);
+  else
+    launch_pdl(kernel, dim3((a.n_tokens + a.tokens_per_cta - 1) / a.tokens_per_cta, a.G * a.head_blocks), dim3(AF_THREADS),
+               smem, stream, a);
+  return LLMX_LAUNCH_STATUS();
+}
+
+// Rule: a step of single tokens (each of a sequence of its own), or one of so few tokens that tiles of rows would leave
+// most SMs idle, gives every token a cluster; other steps share tiles among rows.
+static int attention_f32(const AfArgs& a, bool single_tokens, cudaStream_t stream) {
+  const bool split = single_tokens || a.n_tokens <= 32;
+#define GO(NC) return split ? launch_f32<1, NC, true>(a, stream) : launch_f32<4, NC, false>(a, stream)
+  switch ((a.Dv + 63) / 64) {
+    case 1: GO(1);
+    case 2: GO(2);
+    case 3: GO(3);
+    default: GO(4);
+  }
+#undef GO
+}
+
 // pool > 0: pool_k / pool_v hold one row per block of `pool` positions, paged like the cache, with the block table
 // pool_table (as wide as block_table); needs a window and no kept first keys.  gate: null, or float32 with
 // gate[t * gate_stride + head] the logit of head's output gate.
 // softcap <= 0: scores are not capped; sinks: null, or float32 [H]; score_bias: null, or float32 [H, bias_len].
+// single_tokens: every token is a sequence's only one in this step (a hint: it picks the launch, not the result).
 LLMX_API int llmx_attention_paged_biased(const void* q, void* out, int act_dtype, const void* k_cache,
                                   const void* v_cache, int cache_dtype, const int* block_table, int table_width,
                                   const int* token_seq, const int* token_pos, int n_tokens, int H, int G, int D,
                                   int Dv, long long q_stride, int window, int keep_first, float scale, float sink,
                                   int chunk, int pool, const void* pool_k, const void* pool_v, const int* pool_table,
                                   const float* gate, long long gate_stride, float softcap, const float* sinks,
-                                  const float* score_bias, int bias_len, cudaStream_t stream) {
+                                  const float* score_bias, int bias_len, int single_tokens, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (score_bias && (bias_len <= 0 || pool > 0 || softcap > 0.f)) return LLMX_REFUSED(1);
   if (chunk < 0 || (chunk > 0 && keep_first > 0)) return LLMX_REFUSED(1);
@@ -147,6 +528,18 @@ LLMX_API int llmx_attention_paged_biased(const void* q, void* out, int act_dtype
   if (gate && gate_stride < H) return LLMX_REFUSED(1);
   if (H <= 0 || G <= 0 || H % G != 0 || D <= 0 || D > ATT_MAX_D || window < 0) return LLMX_REFUSED(1);
   if (Dv <= 0 || Dv > ATT_MAX_D || keep_first < 0 || q_stride < (long long)H * D) return LLMX_REFUSED(1);
+  // float32 by tiles: whole 16-byte rows (a layer's sizes and strides, the same for every step), no pooled blocks
+  const auto aligned = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
+  if (act_dtype == LLMX_F32 && cache_dtype == LLMX_F32 && pool == 0 && D % 4 == 0 && Dv % 4 == 0 && aligned(k_cache) &&
+      aligned(v_cache) && aligned(out) && n_tokens <= 0x7fffffff / AF_SPLIT && (long long)H <= 65535) {
+    AfArgs a = {};
+    a.q = (const float*)q, a.k_cache = (const float*)k_cache, a.v_cache = (const float*)v_cache, a.gate = gate;
+    a.sinks = sinks, a.score_bias = score_bias, a.out = (float*)out, a.block_table = block_table;
+    a.token_seq = token_seq, a.token_pos = token_pos, a.q_stride = (size_t)q_stride, a.gate_stride = (size_t)gate_stride;
+    a.table_width = table_width, a.n_tokens = n_tokens, a.H = H, a.G = G, a.D = D, a.Dv = Dv, a.window = window;
+    a.keep_first = keep_first, a.chunk = chunk, a.bias_len = bias_len, a.scale = scale, a.sink = sink, a.softcap = softcap;
+    return attention_f32(a, single_tokens != 0, stream);
+  }
   dim3 grid(n_tokens, (H + ATT_WARPS - 1) / ATT_WARPS);
   const size_t smem = (size_t)ATT_WARPS * D * sizeof(float);
 #define CASE(TA, TC)                                                                                      \
@@ -173,7 +566,7 @@ LLMX_API int llmx_attention_paged_capped(const void* q, void* out, int act_dtype
   return llmx_attention_paged_biased(q, out, act_dtype, k_cache, v_cache, cache_dtype, block_table, table_width,
                                      token_seq, token_pos, n_tokens, H, G, D, Dv, q_stride, window, keep_first, scale,
                                      sink, chunk, pool, pool_k, pool_v, pool_table, gate, gate_stride, softcap, sinks,
-                                     nullptr, 0, stream);
+                                     nullptr, 0, 0, stream);
 }
 
 LLMX_API int llmx_attention_paged_pooled(const void* q, void* out, int act_dtype, const void* k_cache,

@@ -246,7 +246,8 @@ class LatentAttention:
                                       ctx.n_seqs, ctx.max_new, H, H, E, self.window, self.scale, sinks=self.sinks)
         else:
             kernels.attention_paged(q, out, view.k, view.v, block_table, ctx.token_seq, ctx.token_pos,
-                                    H, H, E, self.window, self.scale, v_head_dim=self.Dv, gate=gate, sinks=self.sinks)
+                                    H, H, E, self.window, self.scale, v_head_dim=self.Dv, gate=gate, sinks=self.sinks,
+                                    single_tokens=ctx.is_decode)
             return
         if gate is not None:
             kernels.head_gate(out, gate, H, self.Dv)
