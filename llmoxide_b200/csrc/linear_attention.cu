@@ -10,9 +10,9 @@
 // angle from float32 tables), a scale on k.  All of it, the state and the sums are float32.
 //
 // The recurrence is independent for every column of v, so a CTA owns `cols` columns of one (sequence, head)
-// and walks that sequence's tokens of the step in order.  Within a CTA a warp owns 4 columns; the 8 lanes of
-// a column split D among them in blocks of 4 dims (lane r owns dims 4 (r + 8 i) + 0..3), update their part of
-// S and add up q . S with three shuffles.  The order of every addition is fixed by (d, column) alone, and a
+// and walks that sequence's tokens of the step in order.  Within a CTA a warp owns 4 or 8 columns; the 8 lanes of
+// a column (or of two neighbouring ones) split D among them in blocks of 4 dims (lane r owns dims 4 (r + 8 i) + 0..3),
+// update their part of S and add up q . S by shuffles.  The order of every addition is fixed by (d, column) alone, and a
 // token's update is the same arithmetic whether it arrives in a prompt, in a later portion of one or alone, so
 // a position's result does not depend on how tokens were cut into steps or batched, to the last bit.
 //
@@ -123,7 +123,27 @@ __device__ __forceinline__ void la_cp_async_wait() {
 // GATED: decay and input weight per token from `gates` [T, H, 4] = (a, b, exp(-m), product of a over the segment
 // up to and including the token) instead of the head's fixed decay.  head_stride: floats from one head's state to
 // the next (a design may keep more than S there).
-template <int DPT, int PASS, bool GATED>
+// C: neighbouring columns a thread owns.  Prompts take two: q and k then cost half as many shared-memory reads a
+// multiply-add, which is what one column a thread waits for (the multiply-adds are packed in pairs of dims), and the
+// shares of a chunk's eight tokens are added so that each of the eight lanes ends with one token's sum (7 shuffles a
+// column instead of 24).  Steps of few tokens stream the state and want the threads: one column.  Both, and a chunk cut
+// short, make the same additions in the same order.  Prompts of 700 to 1300 tokens, 16 heads of 128 x 128: the first pass
+// 383 -> 292 us, the second 339 -> 293.
+__device__ __forceinline__ void la_fma2(unsigned long long& d, unsigned long long a, unsigned long long b, unsigned long long c) {
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+}
+__device__ __forceinline__ unsigned long long la_mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long la_pair(float x, float y) {
+  return (unsigned long long)__float_as_uint(x) | ((unsigned long long)__float_as_uint(y) << 32);
+}
+__device__ __forceinline__ float la_lo(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float la_hi(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
+template <int DPT, int PASS, bool GATED, int C>
 __global__ void __launch_bounds__(256)
 decay_scan_kernel(const float* __restrict__ prep, float* __restrict__ out, float* __restrict__ state,
                   float* __restrict__ partial, const int* __restrict__ seq_start, const int* __restrict__ seq_slot,
@@ -137,9 +157,9 @@ decay_scan_kernel(const float* __restrict__ prep, float* __restrict__ out, float
   const int b = blockIdx.z, h = blockIdx.y;
   const int seg = blockIdx.x / col_blocks, c0 = (blockIdx.x - seg * col_blocks) * cols;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int col = c0 + warp * 4 + (lane >> 3);    // this thread's column of v
+  const int cw = (warp * 4 + (lane >> 3)) * C;    // this thread's first column of the CTA's
+  const int col = c0 + cw;                        // and of v
   const int r = lane & 7;                         // its share of D
-  const bool col_live = col < Dv;
   const int seq_t0 = seq_start[b], seq_new = seq_start[b + 1] - seq_t0;
   const int n_seg = (seq_new + seg_len - 1) / seg_len;        // this sequence's segments
   const float g = GATED ? 1.f : decay[h];
@@ -151,23 +171,38 @@ decay_scan_kernel(const float* __restrict__ prep, float* __restrict__ out, float
   pdl_wait();
 
   auto own = [&](int i) { return 4 * (r + 8 * (i >> 2)) + (i & 3); };        // dim of this thread's i-th state value
-  float s_reg[DPT];
+  unsigned long long s2[C][DPT / 2];                                         // its values in pairs of neighbouring dims
   if (PASS == 1) {
 #pragma unroll
-    for (int i = 0; i < DPT; ++i) s_reg[i] = (seg == 0 && col_live && own(i) < D) ? S[(size_t)own(i) * Dv + col] : 0.f;
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+      for (int i = 0; i < DPT; i += 2) {
+        const bool live = seg == 0 && col + c < Dv;
+        s2[c][i >> 1] = la_pair(live && own(i) < D ? S[(size_t)own(i) * Dv + col + c] : 0.f,
+                                live && own(i + 1) < D ? S[(size_t)own(i + 1) * Dv + col + c] : 0.f);
+      }
   } else {
     // E_(seg-1): what the segments before left, each decayed over the segments after it
     float g_seg = 1.f;
     if (!GATED)
       for (int i = 0; i < seg_len; ++i) g_seg *= g;
 #pragma unroll
-    for (int i = 0; i < DPT; ++i) s_reg[i] = 0.f;
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+      for (int i = 0; i < DPT / 2; ++i) s2[c][i] = 0ull;
     for (int sp = 0; sp < seg; ++sp) {
       const float* ps = part_seq + (size_t)sp * D * Dv;
       if (GATED) g_seg = __ldcg(gates + ((size_t)(seq_t0 + (sp + 1) * seg_len - 1) * H + h) * 4 + 3);   // over all of segment sp
+      const unsigned long long gg = la_pair(g_seg, g_seg);
 #pragma unroll
-      for (int i = 0; i < DPT; ++i)
-        if (col_live && own(i) < D) s_reg[i] = fmaf(g_seg, s_reg[i], __ldcg(ps + (size_t)own(i) * Dv + col));
+      for (int i = 0; i < DPT; i += 2)
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const bool live = col + c < Dv;
+          la_fma2(s2[c][i >> 1], gg, s2[c][i >> 1],
+                  la_pair(live && own(i) < D ? __ldcg(ps + (size_t)own(i) * Dv + col + c) : 0.f,
+                          live && own(i + 1) < D ? __ldcg(ps + (size_t)own(i + 1) * Dv + col + c) : 0.f));
+        }
     }
   }
 
@@ -214,73 +249,109 @@ decay_scan_kernel(const float* __restrict__ prep, float* __restrict__ out, float
     // one token.  PASS 1: S = g S + k v, then this thread's share of q . S.  PASS 2: its share of q . E.  The
     // shares are added and stored afterwards, so that in a full chunk (the loop below unrolls) one token's
     // shuffles overlap the next token's arithmetic.
-    auto one_token = [&](int tt) {
+    auto one_token = [&](int tt, float (&share)[C]) {
       const float* qrow = buf + tt * tok_len;
       const float* krow = qrow + Dp;
-      float v = (PASS == 1 && col_live) ? qrow[2 * Dp + warp * 4 + (lane >> 3)] : 0.f;
-      float gt = g;
-      if (GATED && PASS == 1) gt = qrow[2 * Dp + cols], v *= qrow[2 * Dp + cols + 1];      // a_t; b_t rides on v
-      float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f, acc3 = 0.f;
+      unsigned long long vv[C], acc01[C], acc23[C];
+      const float gt = GATED && PASS == 1 ? qrow[2 * Dp + cols] : g;              // a_t
+      const unsigned long long gg = la_pair(gt, gt);
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        float v = (PASS == 1 && col + c < Dv) ? qrow[2 * Dp + cw + c] : 0.f;
+        if (GATED && PASS == 1) v *= qrow[2 * Dp + cols + 1];                       // b_t rides on v
+        vv[c] = la_pair(v, v);
+        acc01[c] = acc23[c] = 0ull;
+      }
 #pragma unroll
       for (int i4 = 0; i4 < DPT / 4; ++i4) {
         const int d = 4 * (r + 8 * i4);
         if (d < Dp) {
-          const float4 q4 = *reinterpret_cast<const float4*>(qrow + d);
-          float* s4 = s_reg + 4 * i4;
+          const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(qrow + d);
           if (PASS == 1) {
-            const float4 k4 = *reinterpret_cast<const float4*>(krow + d);
-            s4[0] = fmaf(gt, s4[0], k4.x * v);
-            s4[1] = fmaf(gt, s4[1], k4.y * v);
-            s4[2] = fmaf(gt, s4[2], k4.z * v);
-            s4[3] = fmaf(gt, s4[3], k4.w * v);
+            const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(krow + d);
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+              la_fma2(s2[c][2 * i4], gg, s2[c][2 * i4], la_mul2(k4.x, vv[c]));
+              la_fma2(s2[c][2 * i4 + 1], gg, s2[c][2 * i4 + 1], la_mul2(k4.y, vv[c]));
+            }
           }
-          acc0 = fmaf(s4[0], q4.x, acc0);
-          acc1 = fmaf(s4[1], q4.y, acc1);
-          acc2 = fmaf(s4[2], q4.z, acc2);
-          acc3 = fmaf(s4[3], q4.w, acc3);
+#pragma unroll
+          for (int c = 0; c < C; ++c) {
+            la_fma2(acc01[c], s2[c][2 * i4], q4.x, acc01[c]);
+            la_fma2(acc23[c], s2[c][2 * i4 + 1], q4.y, acc23[c]);
+          }
         }
       }
-      return (acc0 + acc1) + (acc2 + acc3);
+#pragma unroll
+      for (int c = 0; c < C; ++c) share[c] = (la_lo(acc01[c]) + la_hi(acc01[c])) + (la_lo(acc23[c]) + la_hi(acc23[c]));
     };
-    const bool writer = r == 0 && col_live;
     float* out_chunk = out_col + (size_t)base * out_stride;
-    auto out_at = [&](int tt) { return out_chunk + (size_t)tt * out_stride; };
-    auto finish = [&](int tt, float acc, float before) {       // before: PASS 2, what the first pass left there
-      acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-      acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-      acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-      if (PASS == 1) {
-        if (writer) *out_at(tt) = acc;
-      } else if (GATED) {
-        if (writer) *out_at(tt) = before + buf[tt * tok_len + 2 * Dp + cols + 3] * acc;
-      } else {
-        if (writer) *out_at(tt) = before + g_pow * acc;
-        g_pow *= g;
-      }
+    // what token tt's sum is worth (PASS 2: added to what the first pass left there)
+    auto result = [&](int tt, float acc, float before, float pow) {
+      if (PASS == 1) return acc;
+      return GATED ? before + buf[tt * tok_len + 2 * Dp + cols + 3] * acc : before + pow * acc;
     };
     if (n_tok == LA_CHUNK) {
-      float part[LA_CHUNK], before[LA_CHUNK];
-      if (PASS == 2) {                       // the chunk's outputs of the first pass, fetched together
+      static_assert(LA_CHUNK == 8, "a token for each of a column's lanes");
+      float part[LA_CHUNK][C], before[C], pow = 0.f;
+      float* mine = out_chunk + (size_t)r * out_stride;        // lane r finishes token r
 #pragma unroll
-        for (int tt = 0; tt < LA_CHUNK; ++tt) before[tt] = writer ? __ldcg(out_at(tt)) : 0.f;
+      for (int c = 0; c < C; ++c) before[c] = (PASS == 2 && col + c < Dv) ? __ldcg(mine + c) : 0.f;
+#pragma unroll
+      for (int tt = 0; tt < LA_CHUNK; ++tt) one_token(tt, part[tt]);
+      if (PASS == 2 && !GATED) {
+#pragma unroll
+        for (int tt = 0; tt < LA_CHUNK; ++tt) {
+          if (tt == r) pow = g_pow;
+          g_pow *= g;
+        }
       }
+      // lanes r and r ^ 1 add their shares and keep every other token, then r ^ 2, then r ^ 4
 #pragma unroll
-      for (int tt = 0; tt < LA_CHUNK; ++tt) part[tt] = one_token(tt);
+      for (int c = 0; c < C; ++c) {
+        float a4[4], a2[2];
 #pragma unroll
-      for (int tt = 0; tt < LA_CHUNK; ++tt) finish(tt, part[tt], PASS == 2 ? before[tt] : 0.f);
+        for (int j = 0; j < 4; ++j) {               // tokens 2 j (even lanes) and 2 j + 1 (odd lanes)
+          const float give = (r & 1) ? part[2 * j][c] : part[2 * j + 1][c], keep = (r & 1) ? part[2 * j + 1][c] : part[2 * j][c];
+          a4[j] = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float give = (r & 2) ? a4[2 * j] : a4[2 * j + 1], keep = (r & 2) ? a4[2 * j + 1] : a4[2 * j];
+          a2[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+        }
+        const float give = (r & 4) ? a2[0] : a2[1], keep = (r & 4) ? a2[1] : a2[0];
+        const float acc = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+        if (col + c < Dv) mine[c] = result(r, acc, before[c], pow);
+      }
     } else {
       for (int tt = 0; tt < n_tok; ++tt) {
-        const float before = (PASS == 2 && writer) ? __ldcg(out_at(tt)) : 0.f;
-        finish(tt, one_token(tt), before);
+        float* at = out_chunk + (size_t)tt * out_stride;
+        float share[C];
+        one_token(tt, share);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const bool writer = r == 0 && col + c < Dv;
+          const float before = (PASS == 2 && writer) ? __ldcg(at + c) : 0.f;
+          float acc = share[c];
+          acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+          acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+          acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+          if (writer) at[c] = result(tt, acc, before, g_pow);
+        }
+        if (PASS == 2 && !GATED) g_pow *= g;
       }
     }
     __syncthreads();                              // the buffer is refilled by the next round's copies
   }
+  auto value = [&](int c, int i) { return (i & 1) ? la_hi(s2[c][i >> 1]) : la_lo(s2[c][i >> 1]); };
   if (PASS == 1) {
     float* dst = n_seg == 1 ? S : part_seq + (size_t)seg * D * Dv;
 #pragma unroll
     for (int i = 0; i < DPT; ++i)
-      if (col_live && own(i) < D) dst[(size_t)own(i) * Dv + col] = s_reg[i];
+#pragma unroll
+      for (int c = 0; c < C; ++c)
+        if (col + c < Dv && own(i) < D) dst[(size_t)own(i) * Dv + col + c] = value(c, i);
   } else if (seg == n_seg - 1) {
     // the sequence's new state: E_(n_seg-1) = decay^(its length) E_(n_seg-2) + partial_(n_seg-1)
     float g_len = 1.f;
@@ -290,8 +361,10 @@ decay_scan_kernel(const float* __restrict__ prep, float* __restrict__ out, float
     const float* ps = part_seq + (size_t)seg * D * Dv;
 #pragma unroll
     for (int i = 0; i < DPT; ++i)
-      if (col_live && own(i) < D)
-        S[(size_t)own(i) * Dv + col] = fmaf(g_len, s_reg[i], __ldcg(ps + (size_t)own(i) * Dv + col));
+#pragma unroll
+      for (int c = 0; c < C; ++c)
+        if (col + c < Dv && own(i) < D)
+          S[(size_t)own(i) * Dv + col + c] = fmaf(g_len, value(c, i), __ldcg(ps + (size_t)own(i) * Dv + col + c));
   }
 }
 
@@ -419,30 +492,34 @@ LLMX_API int llmx_decay_scan(const void* proj, int in_dtype, int n_split, long l
   if (e != cudaSuccess) return (int)e;
   Dv = Dva;                                        // from here on the extra column is a column like the others
   // columns per CTA: as many as still give every SM a CTA or two (a CTA with more columns stages q and k fewer times)
-  int cols = 32;
-  while (cols > 8 && (long long)n_seqs * H * n_seg * ((Dv + cols - 1) / cols) < 2LL * n_sm) cols >>= 1;
-  while (cols > 4 && cols / 2 >= Dv) cols >>= 1;
+  // and two a thread in prompts
+  const int C = max_new >= 2 * LA_CHUNK ? 2 : 1;
+  int cols = 32 * C;
+  while (cols > 8 * C && (long long)n_seqs * H * n_seg * ((Dv + cols - 1) / cols) < 2LL * n_sm) cols >>= 1;
+  while (cols > 4 * C && cols / 2 >= Dv) cols >>= 1;
   const int Dp = (D + 3) & ~3;
   const int col_blocks = (Dv + cols - 1) / cols;
   if ((long long)col_blocks * n_seg > 0x7fffffff) return LLMX_REFUSED(3);
-  dim3 grid(col_blocks * n_seg, H, n_seqs), block(cols * 8);
+  dim3 grid(col_blocks * n_seg, H, n_seqs), block(cols * 8 / C);
   const size_t smem = (size_t)LA_STAGES * LA_CHUNK * (2 * Dp + cols + (gates ? 4 : 0)) * sizeof(float);
-#define GO2(DPT, PASS, GATED)                                                                                          \
+#define GO2(DPT, PASS, GATED, C)                                                                                       \
   do {                                                                                                                 \
     static bool attr_set = false;                                                                                      \
     if (!attr_set && smem > 48 * 1024) {                                                                               \
-      e = cudaFuncSetAttribute(decay_scan_kernel<DPT, PASS, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
+      e = cudaFuncSetAttribute(decay_scan_kernel<DPT, PASS, GATED, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
                                100 * 1024);                                                                            \
       if (e != cudaSuccess) return (int)e;                                                                             \
       attr_set = true;                                                                                                 \
     }                                                                                                                  \
-    launch_pdl(decay_scan_kernel<DPT, PASS, GATED>, grid, block, smem, stream, (const float*)prep, out, state, partial, \
+    launch_pdl(decay_scan_kernel<DPT, PASS, GATED, C>, grid, block, smem, stream, (const float*)prep, out, state, partial, \
                seq_start, seq_slot, decay, gates, (size_t)head_stride, H, D, Dv, cols, col_blocks, seg_len, n_seg);    \
   } while (0)
 #define GO1(DPT, PASS)              \
   do {                              \
-    if (gates) GO2(DPT, PASS, true); \
-    else GO2(DPT, PASS, false);     \
+    if (gates && C == 2) GO2(DPT, PASS, true, 2);       \
+    else if (gates) GO2(DPT, PASS, true, 1);            \
+    else if (C == 2) GO2(DPT, PASS, false, 2);          \
+    else GO2(DPT, PASS, false, 1);                      \
   } while (0)
 #define GO(DPT)                    \
   do {                             \
