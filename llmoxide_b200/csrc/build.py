@@ -67,7 +67,7 @@ LIBRARIES = {
     # host code only (no CUDA): the cache's bookkeeping and the step plan
     "host_runtime": (["host_runtime.cpp"], []),
 }
-HEADERS = ["common.cuh", "attention_decode_noalloc.h", "tc_ptx.cuh"]
+HEADERS = ["common.cuh", "attention_decode_noalloc.h", "tc_ptx.cuh", "chunk_products.cuh"]
 
 _loaded: dict = {}
 _lock = threading.Lock()

@@ -31,7 +31,18 @@
 // Work per token and head is 3 D Dv float32 operations (a multiply for k v, one fused multiply-add for the
 // state, one for the output), which is what the FMA units are for; the state is read and written once per
 // step, which is what bounds a decode step.
-#include "common.cuh"
+//
+// A sequence that brings a long prompt under a fixed decay, with a state worth it, is walked in chunks of 64 tokens
+// instead.  With E the state a chunk starts from,
+//   o_i = decay^(i+1) E^T q_i + sum_(j<=i) decay^(i-j) (q_i . k_j) v_j,   E' = decay^n E + sum_j decay^(n-1-j) k_j v_j^T
+// which is the recurrence written out as products of small matrices (chunk_products.cuh, as the state-space layers walk
+// theirs): as many multiply-adds, but 8 x 8 results a thread share what they read from shared memory.
+//   decay_chunk   per (chunk, head): the chunk's own part of E', and the 64 x 64 products q_i . k_j
+//   decay_pass    walks a sequence's chunks in order: leaves every chunk its E and the sequence its new state
+//   decay_out     per (chunk, head, 64 columns): the outputs
+// Four prompts of 700 to 1300 tokens, 16 heads of 128 x 128: 291 us, where the recurrence in segments took 586 (two
+// passes); off the 64-bit result by 2.7e-7 (3.4e-7).
+#include "chunk_products.cuh"
 
 #define LA_CHUNK 8           // tokens per staged chunk
 #define LA_STAGES 3          // chunks in flight or in use
@@ -128,7 +139,7 @@ __device__ __forceinline__ void la_cp_async_wait() {
 // shares of a chunk's eight tokens are added so that each of the eight lanes ends with one token's sum (7 shuffles a
 // column instead of 24).  Steps of few tokens stream the state and want the threads: one column.  Both, and a chunk cut
 // short, make the same additions in the same order.  Prompts of 700 to 1300 tokens, 16 heads of 128 x 128: the first pass
-// 383 -> 292 us, the second 339 -> 293.
+// took 383 us with one column, 292 with two.
 __device__ __forceinline__ void la_fma2(unsigned long long& d, unsigned long long a, unsigned long long b, unsigned long long c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
 }
@@ -148,7 +159,7 @@ __global__ void __launch_bounds__(256)
 decay_scan_kernel(const float* __restrict__ prep, float* __restrict__ out, float* __restrict__ state,
                   float* __restrict__ partial, const int* __restrict__ seq_start, const int* __restrict__ seq_slot,
                   const float* __restrict__ decay, const float* __restrict__ gates, size_t head_stride, int H, int D,
-                  int Dv, int cols, int col_blocks, int seg_len, int n_seg_max) {
+                  int Dv, int cols, int col_blocks, int seg_len, int n_seg_max, int by_chunks) {
   extern __shared__ __align__(16) float la_smem[];
   const int Dp = (D + 3) & ~3, Dvp = (Dv + 3) & ~3;
   const int row_len = 2 * Dp + Dvp;               // floats per (token, head) of prep
@@ -164,7 +175,10 @@ decay_scan_kernel(const float* __restrict__ prep, float* __restrict__ out, float
   const int n_seg = (seq_new + seg_len - 1) / seg_len;        // this sequence's segments
   const float g = GATED ? 1.f : decay[h];
   float* S = state + ((size_t)seq_slot[b] * H + h) * head_stride;
-  if (seg >= n_seg || (PASS == 2 && (n_seg == 1 || seg == 0))) return;       // (uniform over the CTA)
+  if (seg >= n_seg || (PASS == 2 && (n_seg == 1 || seg == 0)) || (by_chunks && n_seg > 1)) {       // (uniform over the CTA)
+    pdl_wait();                        // (a kernel whose CTAs all leave must not end before the one ahead of it)
+    return;
+  }
   const int t0 = seq_t0 + seg * seg_len;                                      // the segment's first token
   const int n_new = min(seg_len, seq_new - seg * seg_len);
   float* part_seq = partial ? partial + ((size_t)b * H + h) * (size_t)n_seg_max * D * Dv : nullptr;
@@ -368,6 +382,322 @@ decay_scan_kernel(const float* __restrict__ prep, float* __restrict__ out, float
   }
 }
 
+// ---------------------------------------------------------------------------
+// Long prompts under a fixed decay, by chunks.  prep as above; chunks of sequences with more than short_new tokens.
+// st [slots][H][D][Dvp]: the chunk's own part of its last state, then (decay_pass) the state it starts from; at [slots][H]:
+// decay to the power of its tokens; cb [slots][H][64][64]: q_i . k_j at row j, column i.
+// Powers of the decay are taken in 64 bits: a product of equal float32 factors errs the same way every time, and the
+// recurrence applies the decay itself, which is exact.  `at` keeps what its rounding to float32 left out beside it, for it
+// is applied chunk after chunk.
+// ---------------------------------------------------------------------------
+struct LaDims {
+  int H, D, Dv, short_new;
+  size_t head_stride;                                   // of the state
+  __host__ __device__ int Dp() const { return (D + 3) & ~3; }
+  __host__ __device__ int Dvp() const { return (Dv + 3) & ~3; }
+  __host__ __device__ int row() const { return 2 * Dp() + Dvp(); }
+};
+
+#define LA_FOLD 128              // dims whose products are added in one chain; more are added in two
+__device__ __forceinline__ double la_power(double g, int n) {       // g^n, 0 <= n <= 64
+  double p = 1.0;
+#pragma unroll
+  for (int bit = 0; bit < 7; ++bit) {
+    if (n >> bit & 1) p *= g;
+    g *= g;
+  }
+  return p;
+}
+
+__global__ void __launch_bounds__(SS_THREADS)
+decay_chunk_kernel(const float* __restrict__ prep, const float* __restrict__ decay, float* __restrict__ st,
+                   float2* __restrict__ at, float* __restrict__ cb, const int* __restrict__ seq_start, int n_seqs,
+                   int n_tokens, const LaDims dm) {
+  __shared__ __align__(16) float As[64 * 64];
+  __shared__ __align__(16) float Bs[64 * 64];
+  __shared__ float ws[SS_CHUNK];
+  pdl_launch_dependents();
+  const int Dp = dm.Dp(), Dvp = dm.Dvp();
+  const size_t step = (size_t)dm.H * dm.row();          // from token to token
+  const int p_tiles = (Dvp + 63) >> 6, tiles = ((dm.D + 63) >> 6) * p_tiles;
+  const int tid = threadIdx.x, slot = blockIdx.x / (dm.H * (tiles + 1)), job = blockIdx.x - slot * dm.H * (tiles + 1);
+  const SsChunk ck = ss_chunk_of(seq_start, n_seqs, n_tokens, slot, dm.short_new);
+  pdl_wait();                                          // (ahead of any leaving: a kernel whose CTAs all leave must not end
+  if (ck.n <= 0) return;                               // before the one ahead of it)
+  float acc[8][8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[r][c] = 0.f;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int i0 = ss_row0(), j0 = ss_col0();
+  if (job < dm.H * tiles) {
+    const int h = job / tiles, tl = job - h * tiles;
+    const int n0 = (tl / p_tiles) * 64, c0 = (tl % p_tiles) * 64;
+    const float g = decay[h];
+    // 16 lanes a row: v goes straight to shared memory, k through registers, where it takes its token's weight
+    const int lr = tid >> 4, lc = (tid & 15) * 4;
+    const float* krow = prep + (size_t)ck.t0 * step + (size_t)h * dm.row() + Dp + n0 + lc;
+    const float* vrow = prep + (size_t)ck.t0 * step + (size_t)h * dm.row() + 2 * Dp + c0 + lc;
+    const bool k_live = n0 + lc < Dp, v_live = c0 + lc < Dvp;
+#pragma unroll
+    for (int m = 0; m < 16; ++m) {
+      const int j = lr + 4 * m;
+      const bool live = v_live && j < ck.n;
+      ss_copy16(Bs + j * 64 + lc, live ? vrow + (size_t)j * step : prep, live);
+    }
+    ss_copy_commit();
+    float4 kv[16];
+#pragma unroll
+    for (int m = 0; m < 16; ++m) {
+      const int j = lr + 4 * m;
+      kv[m] = k_live && j < ck.n ? ss_load4(krow + (size_t)j * step) : zero;
+    }
+    ws[tid] = (float)la_power(g, max(ck.n - 1 - tid, 0));        // (k past the chunk's tokens is zero)
+    if (tid == 0 && tl == 0) {
+      const double all = la_power(g, ck.n);
+      at[(size_t)slot * dm.H + h] = make_float2((float)all, (float)(all - (double)(float)all));
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 16; ++m) {
+      const int j = lr + 4 * m;
+      const float w = ws[j];
+      ss_store4(As + j * 64 + lc, make_float4(kv[m].x * w, kv[m].y * w, kv[m].z * w, kv[m].w * w));
+    }
+    ss_copy_wait<0>();
+    __syncthreads();
+    ss_product<4>(acc, As, 64, Bs, 64, (ck.n + 3) & ~3);   // (rows past the chunk's tokens are zero)
+    float* dst = st + ((size_t)slot * dm.H + h) * dm.D * Dvp + c0 + j0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const int n = n0 + ss_row(i0, r);
+      if (n >= dm.D) continue;
+      if (c0 + j0 < Dvp) ss_store4(dst + (size_t)n * Dvp, make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]));
+      if (c0 + j0 + 32 < Dvp) ss_store4(dst + (size_t)n * Dvp + 32, make_float4(acc[r][4], acc[r][5], acc[r][6], acc[r][7]));
+    }
+    return;
+  }
+  // ---- q_i . k_j: both operands are turned so that a row of shared memory holds one dim of all tokens
+  const int h = job - dm.H * tiles;
+  const float* qrow = prep + (size_t)(ck.t0 + tid) * step + (size_t)h * dm.row();
+  const bool live = tid < ck.n;
+  for (int kb = 0; kb < Dp; kb += 32) {
+    float4 qv[8], kv[8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      qv[m] = live && kb + 4 * m < Dp ? ss_load4(qrow + kb + 4 * m) : zero;
+      kv[m] = live && kb + 4 * m < Dp ? ss_load4(qrow + Dp + kb + 4 * m) : zero;
+    }
+    __syncthreads();                                   // (the tiles of the block before have been read)
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      float* ap = As + 4 * m * 64 + tid;
+      float* bp = Bs + 4 * m * 64 + tid;
+      ap[0] = qv[m].x, ap[64] = qv[m].y, ap[128] = qv[m].z, ap[192] = qv[m].w;
+      bp[0] = kv[m].x, bp[64] = kv[m].y, bp[128] = kv[m].z, bp[192] = kv[m].w;
+    }
+    __syncthreads();
+    ss_product<4>(acc, As, 64, Bs, 64, min(32, Dp - kb));
+    if (kb + 32 == LA_FOLD || kb + 32 >= Dp) {         // the first LA_FOLD dims' sums wait where the result goes
+      float* dst = cb + ((size_t)slot * dm.H + h) * 4096;
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          float* row = dst + ss_row(j0, c) * 64 + i0 + 32 * half;
+          float4 v = make_float4(acc[4 * half][c], acc[4 * half + 1][c], acc[4 * half + 2][c], acc[4 * half + 3][c]);
+          if (kb >= LA_FOLD) {
+            const float4 w = ss_load4(row);
+            v = make_float4(w.x + v.x, w.y + v.y, w.z + v.z, w.w + v.w);
+          }
+          ss_store4(row, v);
+          acc[4 * half][c] = acc[4 * half + 1][c] = acc[4 * half + 2][c] = acc[4 * half + 3][c] = 0.f;
+        }
+    }
+  }
+}
+
+// Every four elements of a sequence's state, one thread: E_0 is the stored state, E_(c+1) = at_c E_c + st_c; st_c becomes
+// E_c, the stored state the last E.
+__global__ void __launch_bounds__(256)
+decay_pass_kernel(float* __restrict__ st, const float2* __restrict__ at, float* __restrict__ state,
+                  const int* __restrict__ seq_start, const int* __restrict__ seq_slot, const LaDims dm) {
+  pdl_launch_dependents();
+  const int b = blockIdx.y, row0 = seq_start[b], n_new = seq_start[b + 1] - row0;
+  pdl_wait();
+  if (n_new <= dm.short_new) return;
+  const int Dvp = dm.Dvp(), p4 = Dvp >> 2;
+  const size_t per_head = (size_t)dm.D * p4, idx = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (idx >= per_head * dm.H) return;
+  const int h = (int)(idx / per_head), d = (int)((idx - h * per_head) / p4), p = (int)(idx % p4) * 4;
+  const int chunks = (n_new + SS_CHUNK - 1) / SS_CHUNK, slot0 = row0 / SS_CHUNK + b;
+  float* sp = state + ((size_t)seq_slot[b] * dm.H + h) * dm.head_stride + (size_t)d * dm.Dv + p;
+  const bool vec = (dm.Dv & 3) == 0 && (dm.head_stride & 3) == 0 && ((uintptr_t)state & 15) == 0;
+  float4 e;
+  if (vec) e = ss_load4(sp);
+  else e = make_float4(sp[0], p + 1 < dm.Dv ? sp[1] : 0.f, p + 2 < dm.Dv ? sp[2] : 0.f, p + 3 < dm.Dv ? sp[3] : 0.f);
+  const size_t step = (size_t)dm.H * dm.D * Dvp;
+  float* cp = st + (size_t)slot0 * step + ((size_t)h * dm.D + d) * Dvp + p;
+  const float2* ap = at + (size_t)slot0 * dm.H + h;
+  for (int c0 = 0; c0 < chunks; c0 += 4) {              // four chunks' parts in flight
+    float4 s[4];
+    float2 a[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (c0 + u < chunks) s[u] = ss_load4(cp + (size_t)(c0 + u) * step), a[u] = ap[(size_t)(c0 + u) * dm.H];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (c0 + u < chunks) {
+        ss_store4(cp + (size_t)(c0 + u) * step, e);
+        e = make_float4(fmaf(a[u].x, e.x, fmaf(a[u].y, e.x, s[u].x)), fmaf(a[u].x, e.y, fmaf(a[u].y, e.y, s[u].y)),
+                        fmaf(a[u].x, e.z, fmaf(a[u].y, e.z, s[u].z)), fmaf(a[u].x, e.w, fmaf(a[u].y, e.w, s[u].w)));
+      }
+  }
+  if (vec) {
+    ss_store4(sp, e);
+  } else {
+    sp[0] = e.x;
+    if (p + 1 < dm.Dv) sp[1] = e.y;
+    if (p + 2 < dm.Dv) sp[2] = e.z;
+    if (p + 3 < dm.Dv) sp[3] = e.w;
+  }
+}
+
+#define LA_LDM 68                // row stride of the masked 64 x 64 matrix in shared memory: 16-byte stores meet no bank twice
+__global__ void __launch_bounds__(SS_THREADS)
+decay_out_kernel(const float* __restrict__ prep, const float* __restrict__ decay, const float* __restrict__ st,
+                 const float* __restrict__ cb, float* __restrict__ out, const int* __restrict__ seq_start, int n_seqs,
+                 int n_tokens, const LaDims dm) {
+  __shared__ __align__(16) float Ms[64 * LA_LDM];      // row j: decay^(i-j) (q_i . k_j) over i; before that the turned q
+  __shared__ __align__(16) float Bs[2][32 * 64];       // rows of E, then of v
+  __shared__ float power[SS_CHUNK + 1];                // of the decay
+  pdl_launch_dependents();
+  const int Dp = dm.Dp(), Dvp = dm.Dvp(), p_tiles = (Dvp + 63) >> 6;
+  const int tid = threadIdx.x, slot = blockIdx.x / (dm.H * p_tiles), job = blockIdx.x - slot * dm.H * p_tiles;
+  const SsChunk ck = ss_chunk_of(seq_start, n_seqs, n_tokens, slot, dm.short_new);
+  pdl_wait();
+  if (ck.n <= 0) return;                               // (uniform)
+  const int h = job / p_tiles, c0 = (job - h * p_tiles) * 64;
+  const size_t step = (size_t)dm.H * dm.row();
+  const float g = decay[h];
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int lr = tid >> 4, lc = (tid & 15) * 4;        // a row of E or v: 16 lanes
+  const bool col_live = c0 + lc < Dvp;
+  const float* e_base = st + ((size_t)slot * dm.H + h) * dm.D * Dvp + c0 + lc;
+  const float* v_base = prep + (size_t)ck.t0 * step + (size_t)h * dm.row() + 2 * Dp + c0 + lc;
+  const float* qrow = prep + (size_t)(ck.t0 + tid) * step + (size_t)h * dm.row();
+  const int e_steps = (dm.D + 31) >> 5, steps = e_steps + ((ck.n + 31) >> 5);
+  auto copy_rows = [&](int k0) {                        // step k0: 32 rows of E, then of v, into one of two buffers
+    float* dst = Bs[k0 & 1] + lc;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const int r = lr + 4 * m, k = (k0 < e_steps ? k0 : k0 - e_steps) * 32 + r;
+      const bool live = col_live && (k0 < e_steps ? k < dm.D : k < ck.n);
+      const float* src = k0 < e_steps ? e_base + (size_t)k * Dvp : v_base + (size_t)k * step;
+      ss_copy16(dst + r * 64, live ? src : prep, live);
+    }
+    ss_copy_commit();
+  };
+  float4 qv[8];
+  auto fetch_q = [&](int kb) {
+#pragma unroll
+    for (int m = 0; m < 8; ++m) qv[m] = tid < ck.n && kb + 4 * m < Dp ? ss_load4(qrow + kb + 4 * m) : zero;
+  };
+  copy_rows(0);
+  fetch_q(0);
+  power[tid] = (float)la_power(g, tid);
+  if (tid == 0) power[SS_CHUNK] = (float)la_power(g, SS_CHUNK);
+  float acc[8][8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[r][c] = 0.f;
+  const int i0 = ss_row0(), j0 = ss_col0();
+  auto each_result = [&](auto&& f) {                   // f(a result of this thread, where it goes)
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const int i = ss_row(i0, r);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const int p = c0 + ss_row(j0, c);
+        if (i < ck.n && p < dm.Dv) f(acc[r][c], out + ((size_t)(ck.t0 + i) * dm.H + h) * dm.Dv + p);
+      }
+    }
+  };
+  // ---- E^T q_i
+  for (int s = 0; s < e_steps; ++s) {
+    float* As = Ms + (s & 1) * 32 * 64;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {                      // q turned: a row of shared memory holds one dim of all tokens
+      float* ap = As + 4 * m * 64 + tid;
+      ap[0] = qv[m].x, ap[64] = qv[m].y, ap[128] = qv[m].z, ap[192] = qv[m].w;
+    }
+    ss_copy_wait<0>();
+    __syncthreads();                                   // (and every thread is done with the tiles of the step before)
+    copy_rows(s + 1);
+    if (s + 1 < e_steps) fetch_q((s + 1) * 32);
+    ss_product<2>(acc, As, 64, Bs[s & 1], 64, min(32, Dp - s * 32));      // (rows of E past D are zero)
+    if ((s + 1) * 32 == LA_FOLD && s + 1 < e_steps)    // the first LA_FOLD dims' sums wait where the result goes
+      each_result([](float& a, float* to) { *to = a, a = 0.f; });
+  }
+  if (dm.D > LA_FOLD) each_result([](float& a, float* to) { a += *to; });
+  __syncthreads();                                     // the turned q has been read: its place takes the masked matrix
+  {
+    // a thread a column j; what lies above the diagonal is zero
+    const float* cbj = cb + (((size_t)slot * dm.H + h) * 64 + tid) * 64;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float4 d[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) d[m] = 16 * q + 15 >= tid ? ss_load4(cbj + 16 * q + 4 * m) : zero;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        float o[4] = {d[m].x, d[m].y, d[m].z, d[m].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = 16 * q + 4 * m + e;
+          o[e] = i >= tid ? o[e] * power[i - tid] : 0.f;
+        }
+        ss_store4(Ms + tid * LA_LDM + 16 * q + 4 * m, make_float4(o[0], o[1], o[2], o[3]));
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const float ga = power[ss_row(i0, r) + 1];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[r][c] *= ga;
+  }
+  // ---- + sum over the chunk's own tokens
+  for (int s = e_steps; s < steps; ++s) {
+    ss_copy_wait<0>();
+    __syncthreads();
+    if (s + 1 < steps) copy_rows(s + 1);
+    const int jb = (s - e_steps) * 32;
+    if (jb == 0) ss_product<2>(acc, Ms, LA_LDM, Bs[s & 1], 64, min(32, ck.n));
+    else ss_product<2, false>(acc, Ms + jb * LA_LDM, LA_LDM, Bs[s & 1], 64, ck.n - jb);      // (they reach rows 32.. only)
+  }
+  const bool vec = (dm.Dv & 3) == 0 && ((uintptr_t)out & 15) == 0;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const int i = ss_row(i0, r);
+    if (i >= ck.n) continue;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int p = c0 + j0 + 32 * half;
+      if (p >= dm.Dv) continue;
+      const float* a = acc[r] + 4 * half;
+      float* dst = out + ((size_t)(ck.t0 + i) * dm.H + h) * dm.Dv + p;
+      if (vec) ss_store4(dst, make_float4(a[0], a[1], a[2], a[3]));
+      else
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (p + c < dm.Dv) dst[c] = a[c];
+    }
+  }
+}
+
 // One warp per (sequence, head) walks the step's tokens of the sequence in order: the gates' pre-activations are
 // columns i_off + h and f_off + h of the projected row (plus a bias), i = cap tanh(z_i / cap), f =
 // logsigmoid(cap tanh(z_f / cap)); m is read from and written back to the sequence's state (m_off floats into the
@@ -451,11 +781,18 @@ LLMX_API int llmx_gate_scan(const void* proj, int in_dtype, int n_split, long lo
   return LLMX_LAUNCH_STATUS();
 }
 
+// Whether prompts of more than one segment go by chunks: under a fixed decay, for states of at least 64 x 64 (v_size counts
+// the extra column), which fill a tile.  16 heads, four prompts of 700 to 1300 tokens, chunks against the recurrence in
+// segments: 291 / 586 us at 128 x 128, 139 / 212 at 64 x 64, 105 / 117 at 32 x 32, 87 / 81 at 16 x 16.  States below 64 have
+// little to gain and keep the recurrence, whose sums for a whole prompt and for its tokens one by one lie closer together.
+LLMX_API int llmx_decay_scan_by_chunks(int gated, int k_size, int v_size) { return !gated && k_size >= 64 && v_size >= 64; }
+
 // proj: [T, row_stride] (or split partials of it); prep: float32 scratch of T * H * (2 Dp + Dvp) elements, 16-byte
 // aligned; out: float32 [T, H*Dva]; state: float32 [slots, H, head_stride >= D*Dva], Dva = Dv + v_ones (v_ones:
 // the values get one more column that is 1 for every token).  max_new: most tokens of one sequence; seg_len:
-// tokens per segment (0: LA_SEG); partial: float32 scratch [n_seqs, H, ceil(max_new / seg_len), D, Dva], needed
-// when max_new > seg_len.  gates: null (the heads' fixed `decay`), or float32 [T, H, 4] as gate_scan leaves them
+// tokens per segment (0: LA_SEG); partial: float32 scratch, 16-byte aligned, needed when max_new > seg_len:
+// [n_seqs, H, ceil(max_new / seg_len), D, Dva], or where llmx_decay_scan_by_chunks says so C chunks, C = n_tokens / 64 +
+// n_seqs, of H (D Dvap + 4098) floats (Dvap: Dva rounded up to 4).  gates: null (the heads' fixed `decay`), or float32 [T, H, 4] as gate_scan leaves them
 // (made with the same seg_len).
 LLMX_API int llmx_decay_scan(const void* proj, int in_dtype, int n_split, long long split_stride, long long row_stride,
                              int q_off, int k_off, int v_off, float* prep, float* out, float* state, float* partial,
@@ -476,7 +813,8 @@ LLMX_API int llmx_decay_scan(const void* proj, int in_dtype, int n_split, long l
   if (seg_len <= 0) seg_len = LA_SEG;
   if (max_new <= 0 || max_new > n_tokens) max_new = n_tokens;
   const int n_seg = (max_new + seg_len - 1) / seg_len;
-  if (n_seg > 1 && !partial) return LLMX_REFUSED(4);
+  const bool by_chunks = n_seg > 1 && llmx_decay_scan_by_chunks(gates != nullptr, D, Dva);
+  if (n_seg > 1 && (!partial || (by_chunks && ((uintptr_t)partial & 15)))) return LLMX_REFUSED(4);
   const dim3 pgrid(n_tokens, H);
   if (in_dtype == LLMX_F32)
     launch_pdl(decay_prep_kernel<float>, pgrid, dim3(128), 0, stream, (const float*)proj, n_split, (size_t)split_stride,
@@ -491,16 +829,34 @@ LLMX_API int llmx_decay_scan(const void* proj, int in_dtype, int n_split, long l
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   Dv = Dva;                                        // from here on the extra column is a column like the others
+  if (by_chunks) {
+    // (a sequence of up to seg_len tokens goes through the plain recurrence below, as it does without long ones beside it)
+    const LaDims dm = {H, D, Dv, seg_len, (size_t)head_stride};
+    const int slots = n_tokens / SS_CHUNK + n_seqs, p_tiles = (dm.Dvp() + 63) / 64, d_tiles = (D + 63) / 64;
+    const long long per_state = (long long)H * D * (dm.Dvp() / 4), jobs = (long long)slots * H * (d_tiles * p_tiles + 1);
+    if (jobs > 0x7fffffff) return LLMX_REFUSED(3);
+    float* cb = partial + (size_t)slots * H * D * dm.Dvp();
+    float2* at = reinterpret_cast<float2*>(cb + (size_t)slots * H * 4096);
+    launch_pdl(decay_chunk_kernel, dim3((unsigned)jobs), dim3(SS_THREADS), 0, stream, (const float*)prep, decay, partial, at,
+               cb, seq_start, n_seqs, n_tokens, dm);
+    launch_pdl(decay_pass_kernel, dim3((unsigned)((per_state + 255) / 256), n_seqs), dim3(256), 0, stream, partial,
+               (const float2*)at, state, seq_start, seq_slot, dm);
+    launch_pdl(decay_out_kernel, dim3((unsigned)(slots * H * p_tiles)), dim3(SS_THREADS), 0, stream, (const float*)prep, decay,
+               (const float*)partial, (const float*)cb, out, seq_start, n_seqs, n_tokens, dm);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return (int)e;
+  }
+  const int scan_segs = by_chunks ? 1 : n_seg;
   // columns per CTA: as many as still give every SM a CTA or two (a CTA with more columns stages q and k fewer times)
   // and two a thread in prompts
   const int C = max_new >= 2 * LA_CHUNK ? 2 : 1;
   int cols = 32 * C;
-  while (cols > 8 * C && (long long)n_seqs * H * n_seg * ((Dv + cols - 1) / cols) < 2LL * n_sm) cols >>= 1;
+  while (cols > 8 * C && (long long)n_seqs * H * scan_segs * ((Dv + cols - 1) / cols) < 2LL * n_sm) cols >>= 1;
   while (cols > 4 * C && cols / 2 >= Dv) cols >>= 1;
   const int Dp = (D + 3) & ~3;
   const int col_blocks = (Dv + cols - 1) / cols;
-  if ((long long)col_blocks * n_seg > 0x7fffffff) return LLMX_REFUSED(3);
-  dim3 grid(col_blocks * n_seg, H, n_seqs), block(cols * 8 / C);
+  if ((long long)col_blocks * scan_segs > 0x7fffffff) return LLMX_REFUSED(3);
+  dim3 grid(col_blocks * scan_segs, H, n_seqs), block(cols * 8 / C);
   const size_t smem = (size_t)LA_STAGES * LA_CHUNK * (2 * Dp + cols + (gates ? 4 : 0)) * sizeof(float);
 #define GO2(DPT, PASS, GATED, C)                                                                                       \
   do {                                                                                                                 \
@@ -512,7 +868,8 @@ LLMX_API int llmx_decay_scan(const void* proj, int in_dtype, int n_split, long l
       attr_set = true;                                                                                                 \
     }                                                                                                                  \
     launch_pdl(decay_scan_kernel<DPT, PASS, GATED, C>, grid, block, smem, stream, (const float*)prep, out, state, partial, \
-               seq_start, seq_slot, decay, gates, (size_t)head_stride, H, D, Dv, cols, col_blocks, seg_len, n_seg);    \
+               seq_start, seq_slot, decay, gates, (size_t)head_stride, H, D, Dv, cols, col_blocks, seg_len, n_seg,     \
+               (int)by_chunks);                                                                                        \
   } while (0)
 #define GO1(DPT, PASS)              \
   do {                              \
@@ -524,7 +881,7 @@ LLMX_API int llmx_decay_scan(const void* proj, int in_dtype, int n_split, long l
 #define GO(DPT)                    \
   do {                             \
     GO1(DPT, 1);                   \
-    if (n_seg > 1) GO1(DPT, 2);    \
+    if (scan_segs > 1) GO1(DPT, 2); \
   } while (0)
   if (Dp <= 32) GO(4);
   else if (Dp <= 64) GO(8);

@@ -1251,8 +1251,9 @@ def decay_scan(proj, out, state, seq_start, token_pos, seq_slot, decay, cos, sin
     (``head_dim`` each) and v heads at ``v_off`` (``v_head_dim`` each); ``activation`` is applied to all three,
     then q and k are rotated (first ``n_rot`` dims, float32 tables, at ``token_pos``) and scaled.  ``out`` float32
     [T, H*Dv]; ``state`` float32 [slots, H, D, Dv], read and written in place for the step's slots.  A sequence
-    that brings more than ``seg_len`` tokens (0: 128) is walked in segments side by side; ``max_new`` is the most
-    tokens one sequence brings (0: not known, taken as all of them).
+    that brings more than ``seg_len`` tokens (0: 128) is walked in segments side by side, or where
+    ``llmx_decay_scan_by_chunks`` says so (long keys and values under a fixed decay) in chunks of 64; ``max_new`` is
+    the most tokens one sequence brings (0: not known, taken as all of them).
 
     With ``gates`` (float32 [T, H, 4] as ``gate_scan`` leaves them, same ``seg_len``) decay and input weight come
     per token: S_t = a_t S_(t-1) + b_t k_t v_t^T.  With ``ones_column`` the values get one more column that is 1
@@ -1278,9 +1279,14 @@ def decay_scan(proj, out, state, seq_start, token_pos, seq_slot, decay, cos, sin
     seg = seg_len or 128
     n_seg = (max_new + seg - 1) // seg
     partial = None
-    if n_seg > 1:
+    by_chunks = n_seg > 1 and _fn("linear_attention", "llmx_decay_scan_by_chunks", [c_int] * 3)(
+        int(gates is not None), head_dim, dva)
+    if n_seg > 1 and not by_chunks:
         partial = guard.scratch((n_seqs * n_heads * n_seg * head_dim * dva,), torch.float32, out.device,
                                 "last states of a prompt's segments")
+    elif n_seg > 1:
+        partial = guard.scratch(((T // 64 + n_seqs) * n_heads * (head_dim * pad4(dva) + 4098),), torch.float32, out.device,
+                                "states and products of a prompt's chunks")
     f = _fn("linear_attention", "llmx_decay_scan",
             [c_void_p, c_int, c_int, c_longlong, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
              c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_int, c_int, c_int,
@@ -1290,7 +1296,8 @@ def decay_scan(proj, out, state, seq_start, token_pos, seq_slot, decay, cos, sin
              _ptr(sin), n_rot, _ACTS[activation], k_scale, T, n_seqs, max_new, seg, n_heads, head_dim, v_head_dim,
              n_sm(out.device), _ptr(gates), head_stride, q_scale, int(ones_column), _stream()), "decay_scan")
     global launch_count
-    launch_count += 2 if n_seg > 1 else 1          # beside the preparation: the recurrence, and the segments' second pass
+    # beside the preparation: the recurrence, and the segments' second pass or the chunks' three kernels
+    launch_count += 1 if n_seg == 1 else 4 if by_chunks else 2
 
 
 def gate_scan(proj, i_off: int, f_off: int, bias_i, bias_f, cap: float, gates, state, m_off: int, seq_start, seq_slot,
