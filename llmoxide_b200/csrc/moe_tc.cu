@@ -14,6 +14,11 @@
 //   MODE 1 (gate|up): two accumulators, rows n and n + F of the expert's [2F, K]; act[row, n] = gated_act(gate, up) (common.cuh)
 //   MODE 0 (down):    y[dest[row]][n] = weight[row] * acc, float32 (dest = choice * tokens + token, from the sort)
 //   MODE 2 (up):      act[row, n] = the activation of an expert without a gate (plain_act)
+//   MODE 3 (gate|up, narrow row tiles): as MODE 1, from one tile of 64 gate rows above the 64 up rows of the same features;
+//                     the warps that hold up hand it over in shared memory.  A step of few tokens touches a few experts,
+//                     and 64 features a unit give twice as many CTAs something to stream.  Four tokens that pick
+//                     2 of 16 experts of 2 x 1024 x 2048: gate|up and down together 24.8 -> 20.8 us, 64 tokens
+//                     44.3 -> 39.2; bound by the length of a CTA's stream (32 blocks of K) up to about four tokens.
 //
 // Which expert a unit reads is decided on the device by the kernel before, so every thread waits for that
 // kernel first.  Every wait on an mbarrier is bounded; when one runs out the CTA records it in the library's
@@ -39,6 +44,7 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                       const GateAct act) {
   extern __shared__ uint8_t smem_raw[];
   constexpr int N_ACC = MODE == 1 ? 2 : 1;
+  constexpr int FEATURES = MODE == 3 ? MT_BM / 2 : MT_BM;                   // of a unit
   constexpr uint32_t A_BYTES = MT_BM * MT_BK * 2;
   constexpr uint32_t B_BYTES = BN * MT_BK * 2;
   constexpr uint32_t STAGE_BYTES = N_ACC * A_BYTES + B_BYTES;
@@ -57,6 +63,7 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
   int* tile_dest = reinterpret_cast<int*>(bars + 2 * n_stages + 6);          // [BN] MODE 0: the unit's output rows
   float* tile_weight = reinterpret_cast<float*>(tile_dest + BN);            // [BN] and their weights
   volatile int* gave_up = reinterpret_cast<volatile int*>(tile_weight + BN); // an epilogue warp's wait ran out: all four leave
+  float* up_rows = tile_weight + BN + 4;                                     // [2][BN][64] MODE 3: a unit's up rows
 
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
@@ -93,7 +100,7 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     e = __ldcg(tiles + 3 * tl);
     row0 = __ldcg(tiles + 3 * tl + 1);
     n_rows = __ldcg(tiles + 3 * tl + 2);
-    n0 = (u - tl * row_tiles) * MT_BM;
+    n0 = (u - tl * row_tiles) * FEATURES;
     return e >= 0;
   };
 
@@ -114,6 +121,7 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
           const int k = i * MT_BK;
           tma_load_2d(stage, &map_w, k, wrow, bar);
           if (MODE == 1) tma_load_2d(stage + A_BYTES, &map_w, k, wrow + N, bar);     // the up rows: N = F
+          if (MODE == 3) tma_load_2d(stage + A_BYTES / 2, &map_w, k, wrow + N, bar);
           tma_load_2d(stage + N_ACC * A_BYTES, &map_x, k, row0, bar);
         }
       }
@@ -174,19 +182,30 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         mt_report(3);
         *gave_up = 1;
       }
-      if (MODE == 0) {
-        asm volatile("bar.sync 1, 128;" ::: "memory");     // the rows' list is in place, and so is any warp's failure
+      const uint32_t acc_addr = tmem_base + (uint32_t)buf * ACC_COLS + ((uint32_t)(quad * 32) << 16);
+      float* up = up_rows + (size_t)(j & 1) * BN * 64;     // (a buffer is written again behind the next unit's barrier)
+      if (MODE == 3 && quad >= 2 && __shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) {
+        tc_fence_after();
+#pragma unroll 1
+        for (int c = 0; c < BN && c < n_rows; c += 16) {
+          float v[16];
+          tmem_ld16(acc_addr + (uint32_t)c, v);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) up[(c + i) * 64 + (quad - 2) * 32 + lane] = v[i];
+        }
+      }
+      if (MODE == 0 || MODE == 3) {
+        asm volatile("bar.sync 1, 128;" ::: "memory");     // the rows' list (the up rows) is in place, and so is any warp's failure
         failed = *gave_up != 0;
       } else {
         failed = __shfl_sync(0xffffffffu, ok ? 0 : 1, 0) != 0;
       }
       if (failed) break;
       tc_fence_after();
-      const uint32_t acc_addr = tmem_base + (uint32_t)buf * ACC_COLS + ((uint32_t)(quad * 32) << 16);
       const int n = n0 + quad * 32 + lane;                 // this lane's row of the expert's matrix = output feature
 #pragma unroll 1
       for (int c = 0; c < BN; c += 16) {
-        if (c >= n_rows) break;
+        if (c >= n_rows || (MODE == 3 && quad >= 2)) break;
         float v[16], g[16];
         tmem_ld16(acc_addr + (uint32_t)c, v);
         if (MODE == 1) tmem_ld16(acc_addr + (uint32_t)(BN + c), g);
@@ -196,8 +215,8 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
           for (int i = 0; i < 16; ++i) {
             const int r = c + i;
             if (r >= n_rows) break;
-            if (MODE == 1) {
-              Y[(size_t)(row0 + r) * N + n] = from_f32<TY>(gated_act_fast(act, v[i], g[i]));
+            if (MODE == 1 || MODE == 3) {
+              Y[(size_t)(row0 + r) * N + n] = from_f32<TY>(gated_act_fast(act, v[i], MODE == 3 ? up[r * 64 + quad * 32 + lane] : g[i]));
             } else if (MODE == 2) {
               Y[(size_t)(row0 + r) * N + n] = from_f32<TY>(v[i]);
             } else {
@@ -231,19 +250,23 @@ static int mt_sm_count() {
 
 template <int BN, int MODE, typename TY>
 static int mt_launch(const CUtensorMap& mw, const CUtensorMap& mx, void* Y, const int* tiles, int max_tiles, const int* dest,
-                     const float* sorted_weight, int N, int K, int w_rows, const GateAct act, cudaStream_t stream) {
+                     const float* sorted_weight, long long P, int N, int K, int w_rows, const GateAct act,
+                     cudaStream_t stream) {
   constexpr int N_ACC = MODE == 1 ? 2 : 1;
+  constexpr int FEATURES = MODE == 3 ? MT_BM / 2 : MT_BM;
   constexpr size_t STAGE = (size_t)N_ACC * MT_BM * MT_BK * 2 + (size_t)BN * MT_BK * 2;
-  const int row_tiles = (N + MT_BM - 1) / MT_BM;
+  constexpr size_t UP_ROWS = MODE == 3 ? 2 * BN * 64 * sizeof(float) : 0;
+  if (P < max_tiles) max_tiles = (int)P;              // (every tile holds a pair, and the used ones come first)
+  const int row_tiles = (N + FEATURES - 1) / FEATURES;
   const long long n_units = (long long)row_tiles * max_tiles;
   if (n_units > 0x7fffffff) return LLMX_REFUSED(3);
   // narrow row tiles stream weights: two CTAs per SM keep more loads in flight; wide ones take the whole SM
   const int ctas_per_sm = BN <= 64 ? 2 : 1;
-  const size_t budget = ctas_per_sm == 2 ? 108 * 1024 : 200 * 1024;
+  const size_t budget = (ctas_per_sm == 2 ? 108 * 1024 : 200 * 1024) - UP_ROWS;
   int stages = (int)(budget / STAGE);
   if (stages > 12) stages = 12;
   if (stages < 2) stages = 2;
-  const size_t smem = 1024 + (size_t)stages * STAGE + (2 * stages + 6) * 8 + (size_t)BN * 8 + 16;
+  const size_t smem = 1024 + (size_t)stages * STAGE + (2 * stages + 6) * 8 + (size_t)BN * 8 + 16 + UP_ROWS;
   auto kernel = moe_grouped_tc_kernel<BN, MODE, TY>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -275,19 +298,21 @@ LLMX_API int llmx_moe_grouped_tc(const void* X, long long ldx, long long P, cons
   if (gated < 0 || gated > 2) return LLMX_REFUSED(1);
   const int w_rows = gated == 1 ? 2 * N : N;
   CUtensorMap mw, mx;
-  if (make_map(&mw, W, (uint64_t)n_experts * w_rows, (uint64_t)K, (uint64_t)K, MT_BM, true)) return LLMX_REFUSED(4);
+  // gate and up rows of a narrow tile come by boxes of 64 rows
+  const uint32_t box = gated == 1 && tile_rows == 16 ? MT_BM / 2 : MT_BM;
+  if (make_map(&mw, W, (uint64_t)n_experts * w_rows, (uint64_t)K, (uint64_t)K, box, true)) return LLMX_REFUSED(4);
   if (make_map(&mx, X, (uint64_t)P, (uint64_t)K, (uint64_t)ldx, (uint32_t)tile_rows, false)) return LLMX_REFUSED(4);
-#define GO(BN)                                                                                                      \
-  return gated == 1 ? mt_launch<BN, 1, bf16>(mw, mx, Y, tiles, max_tiles, dest, sorted_weight, N, K, w_rows, act, stream) \
-       : gated == 2 ? mt_launch<BN, 2, bf16>(mw, mx, Y, tiles, max_tiles, dest, sorted_weight, N, K, w_rows, act, stream) \
-               : mt_launch<BN, 0, float>(mw, mx, Y, tiles, max_tiles, dest, sorted_weight, N, K, w_rows, act, stream)
+#define RUN(BN, MODE, TY) \
+  mt_launch<BN, MODE, TY>(mw, mx, Y, tiles, max_tiles, dest, sorted_weight, P, N, K, w_rows, act, stream)
+#define GO(BN, GATED) return gated == 1 ? RUN(BN, GATED, bf16) : gated == 2 ? RUN(BN, 2, bf16) : RUN(BN, 0, float)
   switch (tile_rows) {
-    case 16: GO(16);
-    case 64: GO(64);
-    case 128: GO(128);
+    case 16: GO(16, 3);
+    case 64: GO(64, 1);
+    case 128: GO(128, 1);
     default: return LLMX_REFUSED(1);
   }
 #undef GO
+#undef RUN
 }
 
 // Sorted rows of x: xs[place] = x[perm[place] / top] (bfloat16, 16 bytes per thread and step).
