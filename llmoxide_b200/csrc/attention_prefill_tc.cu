@@ -14,8 +14,9 @@
 //   warp 1     one lane issues  S = Q K^T  (both operands K-major) into one of
 //              two S buffers in tensor memory, and  O += P V  (P from tensor
 //              memory, V MN-major straight from its cache layout)
-//   warps 2-5  softmax, one thread per query row: tcgen05.ld the row of S,
-//              mask, running maximum, exp2, row sum, P as bfloat16 back into
+//   warps 2-9  softmax, two threads per query row, 32 keys each (warps w and
+//              w + 4 share 32 rows): tcgen05.ld half a row of S, mask, running
+//              maximum, exp2, half the row's sum, P as bfloat16 back into
 //              tensor memory over the scores it came from (tcgen05.st; two keys
 //              to a column), where the MMA takes it as its A operand: P never
 //              passes through shared memory, whose bandwidth is what a key tile
@@ -23,10 +24,20 @@
 //              written by the copies).  O stays in tensor memory;
 //              it is rescaled (load, multiply, store) only when a row's maximum
 //              has grown by more than 2^8 since the maximum its exponentials
-//              were taken against, which is rare after the first tiles.
+//              were taken against, which is rare after the first tiles: the two
+//              warps of 32 rows learn whether one of them wants it from a barrier
+//              that carries the answer, and only then exchange their maxima.
+//              One thread a row, with twice the chain of dependent instructions a
+//              tile, left the schedulers idle 62 % of the time (wait and
+//              scoreboard stalls at 2.6 warps each): 32 heads over 8, one prompt
+//              of 2048 tokens 60.6 -> 58.4 us (588 TFLOP/s), of 200 tokens 16.7
+//              -> 12.6, eight of 1200 to 2048 tokens 336 -> 316, sixty-four of 17
+//              to 250 tokens 144 -> 136.  A tile's 96 KB through shared memory
+//              (768 cycles) beside 512 cycles of exponentials and 520 of matrix
+//              products is the next bound.
 // S of tile j+1 is issued before P V of tile j, so the tensor core works on the
 // next scores while the softmax warps work on these.  A CTA takes half of an
-// SM (96 KB of shared memory, 256 columns of tensor memory, 168 registers),
+// SM (97 KB of shared memory, 256 columns of tensor memory, 96 registers),
 // so two CTAs share it: while one's softmax warps wait for a tensor-memory load
 // or the special-function unit, the other's run.  Every mbarrier wait is
 // bounded; a wait that runs out sets the status word and the CTA winds down.
@@ -34,21 +45,23 @@
 // Compiled a second time with LLMX_SCORE_CAP=1 (a library of its own) every scaled score is capped (common.cuh).
 // `sinks` (float32 [H]): exp(sinks[h]) joins head h's denominator once.
 // Compiled a third time with LLMX_SCORE_BIAS=1 a learned bias per distance and head joins every scaled score (common.cuh): a
-// softmax warp's 32 rows and a tile's 64 keys span 95 distances, which it copies to shared memory while it waits for the
-// tile's scores; lane r then reads entry r + 63 - e for key e, 32 neighbouring words a load.
+// softmax warp's 32 rows and 32 keys span 63 distances, which it copies to shared memory while it waits for the tile's
+// scores; lane r then reads entry r + 31 - e for its key e, 32 neighbouring words a load.
 #include "tc_ptx.cuh"
 
 #define AT_ROWS 128        // query rows per CTA = MMA M
 #define AT_KEYS 64         // keys per tile = MMA N of S = one cache page
 #define AT_D 128
-#define AT_THREADS 192        // warp 0 TMA, warp 1 MMA, warps 2..5 softmax
+#define AT_THREADS 320        // warp 0 TMA, warp 1 MMA, warps 2..9 softmax
+#define AT_HALF (AT_KEYS / 2) // keys of a tile that one softmax thread takes
 #define AT_PANEL (128 * 128)   // bytes of one [128 rows x 64 elements] panel of Q
 #define AT_TILE (2 * AT_PANEL) // bytes of the [128 x 128] query tile
 #define AT_KPANEL (AT_KEYS * 128)   // bytes of one [64 keys x 64 dims] panel of K or V
 #define AT_KTILE (2 * AT_KPANEL)    // bytes of a [64 keys x 128 dims] tile of K or V
-#define AT_BIAS 96                  // distances between a warp's rows and a tile's keys (95), padded
+#define AT_BIAS 64                  // distances between a warp's rows and its keys of a tile (63), padded
 #define AT_BARS (16 * 8 + 64)
-#define AT_SMEM (AT_TILE + 4 * AT_KTILE + AT_BARS + (LLMX_SCORE_BIAS ? 4 * AT_BIAS * 4 : 0))   // Q, K[2], V[2], barriers
+#define AT_PAIR (2 * AT_ROWS * 4)   // what the two threads of a row tell each other
+#define AT_SMEM (AT_TILE + 4 * AT_KTILE + AT_BARS + AT_PAIR + (LLMX_SCORE_BIAS ? 8 * AT_BIAS * 4 : 0))   // Q, K[2], V[2], barriers, ...
 
 __device__ int g_at_status = 0;    // 0, or which bounded wait ran out (1..10 below), 20: shared memory not 1024-byte aligned
 __device__ __forceinline__ void at_report(int code) {
@@ -61,6 +74,46 @@ __device__ __forceinline__ void at_report(int code) {
 __host__ __device__ constexpr uint32_t at_idesc(bool b_mn_major, uint32_t n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((n >> 3) << 17) |
          ((uint32_t)(128 >> 4) << 24);
+}
+
+// 16 columns of this warp's 32 lanes of tensor memory.
+__device__ __forceinline__ void at_tmem_st16(uint32_t taddr, const uint32_t* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// The two warps of 32 rows meet; true if any of their 64 threads says so.  (Barrier numbers as constants: a number in a
+// register would reserve all sixteen.)
+template <int ID>
+__device__ __forceinline__ bool at_meet_any(bool p) {
+  int any;
+  asm volatile(
+      "{\n.reg .pred p, q;\nsetp.ne.s32 p, %1, 0;\nbarrier.cta.red.or.aligned.pred q, %2, 64, p;\nselp.s32 %0, 1, 0, q;\n}"
+      : "=r"(any)
+      : "r"((int)p), "n"(ID)
+      : "memory");
+  return any != 0;
+}
+__device__ __forceinline__ bool at_pair_any(int quad, bool p) {
+  return quad == 0 ? at_meet_any<1>(p) : quad == 1 ? at_meet_any<2>(p) : quad == 2 ? at_meet_any<3>(p) : at_meet_any<4>(p);
+}
+__device__ __forceinline__ unsigned long long at_pack(float x, float y) {
+  return (unsigned long long)__float_as_uint(x) | ((unsigned long long)__float_as_uint(y) << 32);
+}
+__device__ __forceinline__ float at_lo(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float at_hi(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ unsigned long long at_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long at_add2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
 }
 
 __global__ void __launch_bounds__(AT_THREADS, 2)
@@ -133,7 +186,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       mbar_init(s_full0 + 8u * i, 1);
       mbar_init(pv_done0 + 8u * i, 1);
     }
-    for (int i = 0; i < 2; ++i) mbar_init(p_ready0 + 8u * i, 4);
+    for (int i = 0; i < 2; ++i) mbar_init(p_ready0 + 8u * i, 8);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
@@ -209,128 +262,152 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       if (ok) issue_pv(n_tiles - 1);
     }
   } else {
-    // ---------------- softmax, one thread per query row ----------------
-    const int quad = warp & 3;
+    // ---------------- softmax, two threads per query row ----------------
+    // Rule: the two warps of 32 rows leave the walk together, at a barrier of theirs.  A warp whose wait ran out remembers
+    // it, does nothing more of the tile, and says so at the next barrier.
+    const int quad = warp & 3, half = (warp - 2) >> 2;
     const int row = quad * 32 + lane;
     const int pos = past + i0 + row;                              // this row's position
     int first = (window > 0 && pos - (window - 1) > 0) ? pos - (window - 1) : 0;
     if (mask_chunk > 0) first = max(first, pos - pos % mask_chunk);
     const bool row_live = row < rows_here;
     const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
-    float m_used = -INFINITY;      // the maximum the exponentials are taken against (may lag the true one)
-    float l = 0.f;                 // row sum in units of 2^-m_used
-    bool ok = true;
+    float* told = reinterpret_cast<float*>(pV0 + 2 * AT_KTILE + AT_BARS);      // [2][AT_ROWS]
+    float m_used = -INFINITY;      // the maximum the exponentials are taken against (may lag the true one); of both threads
+    float l = 0.f;                 // this thread's share of the row sum in units of 2^-m_used
+    bool ok = true, left = false;
+    auto waited = [&](uint32_t bar, uint32_t parity, int code) {  // the warp agrees on whether a wait was met
+      const bool met = mbar_wait(bar, parity);
+      if (!met && lane == 0) at_report(code);
+      return __shfl_sync(0xffffffffu, met ? 1 : 0, 0) != 0;
+    };
 #if LLMX_SCORE_BIAS
-    float* wbias = reinterpret_cast<float*>(pV0 + 2 * AT_KTILE + AT_BARS) + (warp - 2) * AT_BIAS;
+    float* wbias = told + 2 * AT_ROWS + (warp - 2) * AT_BIAS;
     const float* brow = bias.table + (size_t)hq * bias.len;
 #endif
-    for (int j = 0; j < n_tiles && ok; ++j) {
+    for (int j = 0; j < n_tiles; ++j) {
       const int st = j & 1;
+      const int key0 = tile_at(j) * AT_KEYS, my_key0 = key0 + half * AT_HALF;
 #if LLMX_SCORE_BIAS
       __syncwarp();                 // (every lane has read the tile before's)
       {
-        const int d0 = past + i0 + quad * 32 - (tile_at(j) * AT_KEYS + AT_KEYS - 1);
+        const int d0 = past + i0 + quad * 32 - (my_key0 + AT_HALF - 1);
 #pragma unroll
         for (int i = 0; i < AT_BIAS; i += 32)
           wbias[i + lane] = brow[min(max(d0 + i + lane, 0), bias.len - 1)] * LLMX_LOG2E;
       }
       __syncwarp();
 #endif
-      ok = mbar_wait(s_full0 + 8u * st, (j >> 1) & 1);
-      if (!ok && lane == 0) at_report(7);
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      if (!ok) break;
-      tc_fence_after();
+      ok = ok && waited(s_full0 + 8u * st, (j >> 1) & 1, 7);
       const uint32_t tS = tS0 + (uint32_t)st * AT_KEYS + lane_off;
-      const int key0 = tile_at(j) * AT_KEYS;
-      // the row of S: four loads in flight, one wait
-      uint32_t sr[AT_KEYS];
-#pragma unroll
-      for (int c = 0; c < AT_KEYS; c += 32) tmem_ld32_nowait(tS + (uint32_t)c, sr + c);
-      tmem_ld_wait();
+      uint32_t sr[AT_HALF];
+      float mt = -INFINITY;
+      if (ok) {
+        tc_fence_after();
+        tmem_ld32_nowait(tS + (uint32_t)(half * AT_HALF), sr);
+        tmem_ld_wait();
 #if LLMX_SCORE_CAP
 #pragma unroll
-      for (int e = 0; e < AT_KEYS; ++e) sr[e] = __float_as_uint(capped_score_log2(cap, __uint_as_float(sr[e])));
+        for (int e = 0; e < AT_HALF; ++e) sr[e] = __float_as_uint(capped_score_log2(cap, __uint_as_float(sr[e])));
 #endif
 #if LLMX_SCORE_BIAS
-      {
-        const float* wb = wbias + lane + AT_KEYS - 1;
+        {
+          const float* wb = wbias + lane + AT_HALF - 1;
 #pragma unroll
-        for (int e = 0; e < AT_KEYS; ++e)
-          sr[e] = __float_as_uint(fmaf(__uint_as_float(sr[e]), scale_log2_arg, wb[-e]));
-      }
+          for (int e = 0; e < AT_HALF; ++e)
+            sr[e] = __float_as_uint(fmaf(__uint_as_float(sr[e]), scale_log2_arg, wb[-e]));
+        }
 #endif
-      // Tiles that some row of this CTA sees only in part (the diagonal, a window's edge, rows past the
-      // sequence's end) are masked; the others, which is most of them, skip the compares.
-      const bool edge = (key0 + AT_KEYS - 1 > pos_lo) || (window > 0 && key0 < pos_hi - (window - 1)) ||
-                        (mask_chunk > 0 && key0 < pos_hi - pos_hi % mask_chunk) || (rows_here < AT_ROWS);
-      if (edge) {
+        // Tiles that some row of this CTA sees only in part (the diagonal, a window's edge, rows past the
+        // sequence's end) are masked; the others, which is most of them, skip the compares.
+        const bool edge = (key0 + AT_KEYS - 1 > pos_lo) || (window > 0 && key0 < pos_hi - (window - 1)) ||
+                          (mask_chunk > 0 && key0 < pos_hi - pos_hi % mask_chunk) || (rows_here < AT_ROWS);
+        if (edge) {
 #pragma unroll
-        for (int e = 0; e < AT_KEYS; ++e) {
-          const int key = key0 + e;
-          if (!(row_live && (key >= first || key < keep_first) && key <= pos)) sr[e] = 0xff800000u;     // -inf
+          for (int e = 0; e < AT_HALF; ++e) {
+            const int key = my_key0 + e;
+            if (!(row_live && (key >= first || key < keep_first) && key <= pos)) sr[e] = 0xff800000u;     // -inf
+          }
         }
-      }
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // four chains, so the maxima overlap
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // four chains, so the maxima overlap
 #pragma unroll
-      for (int e = 0; e < AT_KEYS; e += 4) {
-        mx4[0] = fmaxf(mx4[0], __uint_as_float(sr[e]));
-        mx4[1] = fmaxf(mx4[1], __uint_as_float(sr[e + 1]));
-        mx4[2] = fmaxf(mx4[2], __uint_as_float(sr[e + 2]));
-        mx4[3] = fmaxf(mx4[3], __uint_as_float(sr[e + 3]));
+        for (int e = 0; e < AT_HALF; e += 4) {
+          mx4[0] = fmaxf(mx4[0], __uint_as_float(sr[e]));
+          mx4[1] = fmaxf(mx4[1], __uint_as_float(sr[e + 1]));
+          mx4[2] = fmaxf(mx4[2], __uint_as_float(sr[e + 2]));
+          mx4[3] = fmaxf(mx4[3], __uint_as_float(sr[e + 3]));
+        }
+        mt = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;   // scale_log2 > 0
+        tc_fence_before();         // (the other warp's P goes over scores that this one has read, and the other way round)
       }
-      const float mt = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;   // scale_log2 > 0
-      // the maximum to use: keep the old one unless the true maximum outgrew it by more than 2^8
-      float alpha = 1.0f;
-      if (mt > m_used + 8.0f) {                                   // also the first time (m_used = -inf)
-        alpha = (m_used == -INFINITY) ? 0.0f : exp2f(m_used - mt);
-        m_used = mt;
-      }
-      l *= alpha;
-      // probabilities (a masked score is -inf and gives exactly 0), their sum, and P as bfloat16 in the
-      // MMA's layout: [panel = key / 64][row][128 bytes], 16-byte chunk index XOR (row % 8)
-      const float neg_ref = (m_used == -INFINITY) ? 0.f : -m_used;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-      uint32_t packed[AT_KEYS / 2];
-#pragma unroll
-      for (int e = 0; e < AT_KEYS; e += 2) {
-        const float p0 = ex2_approx(fmaf(__uint_as_float(sr[e]), scale_log2, neg_ref));
-        const float p1 = ex2_approx(fmaf(__uint_as_float(sr[e + 1]), scale_log2, neg_ref));
-        sum4[(e >> 1) & 3] += p0 + p1;
-        __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);
-        packed[e >> 1] = *reinterpret_cast<uint32_t*>(&hh);
-      }
-      l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-      // O belongs to P V of the tile before until it is done.  It is rescaled only when some row of the warp
-      // needs it; otherwise P goes out first and the wait for that P V (every tile's is waited for, so that the
-      // barrier's phases are followed one by one) comes after, off the path to the next P V.
-      const bool rescale = j >= 1 && __any_sync(0xffffffffu, alpha != 1.0f);
-      if (rescale) {
-        ok = mbar_wait(pv_done0 + 8u * ((j - 1) & 1), ((j - 1) >> 1) & 1);
-        if (!ok && lane == 0) at_report(8);
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        if (!ok) break;
+      // the maximum to use: keep the old one unless the row's true maximum outgrew it by more than 2^8
+      bool rescale = false;
+      if (at_pair_any(quad, !ok || mt > m_used + 8.0f)) {           // also the first time (m_used = -inf)
+        told[half * AT_ROWS + row] = ok ? mt : __int_as_float(0x7fffffff);       // (a NaN: this warp leaves)
+        at_pair_any(quad, false);
+        const float other = told[(half ^ 1) * AT_ROWS + row];
+        if (!ok || __any_sync(0xffffffffu, __float_as_int(other) == 0x7fffffff)) {
+          ok = false;
+          left = true;
+          break;
+        }
         tc_fence_after();
-#pragma unroll 1
-        for (int c = 0; c < AT_D; c += 32) {
-          float o[32];
-          tmem_ld32(tO + lane_off + (uint32_t)c, o);
-#pragma unroll
-          for (int e = 0; e < 32; ++e) o[e] *= alpha;
-          tmem_st32(tO + lane_off + (uint32_t)c, o);
+        mt = fmaxf(mt, other);
+        float alpha = 1.0f;
+        if (mt > m_used + 8.0f) {
+          alpha = (m_used == -INFINITY) ? 0.0f : exp2f(m_used - mt);
+          m_used = mt;
         }
+        l *= alpha;
+        // O belongs to P V of the tile before until it is done.  It is rescaled only when some row of the warps needs
+        // it, each warp half of its columns; otherwise P goes out first and the wait for that P V (every tile's is
+        // waited for, so that the barrier's phases are followed one by one) comes after, off the path to the next P V.
+        rescale = j >= 1 && __any_sync(0xffffffffu, alpha != 1.0f);
+        if (rescale) {
+          ok = waited(pv_done0 + 8u * ((j - 1) & 1), ((j - 1) >> 1) & 1, 8);
+          if (ok) {
+            tc_fence_after();
+#pragma unroll 1
+            for (int c = 0; c < AT_D / 2; c += 16) {
+              float o[16];
+              const uint32_t at = tO + lane_off + (uint32_t)(half * (AT_D / 2) + c);
+              tmem_ld16(at, o);
+              uint32_t u[16];
+#pragma unroll
+              for (int e = 0; e < 16; ++e) u[e] = __float_as_uint(o[e] * alpha);
+              at_tmem_st16(at, u);
+            }
+          }
+        }
+      } else {
+        tc_fence_after();
       }
-      // P as bfloat16 over the scores it came from: this row's lane, two keys to a column
-      tmem_st32_u32(tS, packed);
+      if (!ok) continue;
+      // probabilities (a masked score is -inf and gives exactly 0), their sum, and P as bfloat16
+      {
+        const float neg_ref = (m_used == -INFINITY) ? 0.f : -m_used;
+        const unsigned long long scale2 = at_pack(scale_log2, scale_log2), ref2 = at_pack(neg_ref, neg_ref);
+        unsigned long long sum2[2] = {0ull, 0ull};
+        uint32_t packed[AT_HALF / 2];
+#pragma unroll
+        for (int e = 0; e < AT_HALF; e += 2) {
+          const unsigned long long x = at_fma2(at_pack(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), scale2, ref2);
+          const float p0 = ex2_approx(at_lo(x)), p1 = ex2_approx(at_hi(x));
+          sum2[(e >> 1) & 1] = at_add2(sum2[(e >> 1) & 1], at_pack(p0, p1));
+          __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);
+          packed[e >> 1] = *reinterpret_cast<uint32_t*>(&hh);
+        }
+        l += (at_lo(sum2[0]) + at_hi(sum2[0])) + (at_lo(sum2[1]) + at_hi(sum2[1]));
+        // over the scores it came from: this row's lane, two keys to a column
+        at_tmem_st16(tS + (uint32_t)(half * (AT_HALF / 2)), packed);
+      }
       // the last tile: rows of V past the newest key were never written (or belong to another owner of the page)
       if (key0 + AT_KEYS - 1 > pos_hi) {
-        ok = mbar_wait(v_full0 + 8u * st, (j >> 1) & 1);
-        if (!ok && lane == 0) at_report(9);
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        if (!ok) break;
+        ok = waited(v_full0 + 8u * st, (j >> 1) & 1, 9);
+        if (!ok) continue;
         const int valid = pos_hi - key0 + 1;
         uint8_t* vt = pV0 + st * AT_KTILE;
-        for (int idx = (warp - 2) * 32 + lane; idx < (AT_KEYS - valid) * 16; idx += 128) {
+        for (int idx = (warp - 2) * 32 + lane; idx < (AT_KEYS - valid) * 16; idx += 256) {
           const int r = valid + (idx >> 4), part = idx & 15;       // 16 x 16 bytes per row: 8 per panel
           *reinterpret_cast<uint4*>(vt + (part >> 3) * AT_KPANEL + r * 128 + ((part & 7) << 4)) = make_uint4(0u, 0u, 0u, 0u);
         }
@@ -339,28 +416,26 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_ready0 + 8u * st);
-      if (j >= 1 && !rescale) {
-        ok = mbar_wait(pv_done0 + 8u * ((j - 1) & 1), ((j - 1) >> 1) & 1);
-        if (!ok && lane == 0) at_report(8);
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      }
+      if (j >= 1 && !rescale) ok = waited(pv_done0 + 8u * ((j - 1) & 1), ((j - 1) >> 1) & 1, 8);
     }
-    // ---------------- normalise and store ----------------
-    if (ok) {
-      ok = mbar_wait(pv_done0 + 8u * ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1);
-      if (!ok && lane == 0) at_report(10);
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-    }
+    // ---------------- normalise and store, half of the dims a thread ----------------
+    ok = ok && waited(pv_done0 + 8u * ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, 10);
     if (ok) {
       tc_fence_after();
+      told[half * AT_ROWS + row] = l;
+    }
+    __syncwarp();
+    // (a pair that left the walk left it together and does not meet here; one whose last waits differ does)
+    if (!left && !at_pair_any(quad, !ok)) {
+      l = told[row] + told[AT_ROWS + row];
       // a sink: `sink` keys of score 0 without a value; they only add to the denominator (l is in units of 2^-m_used)
       if (sinks && row_live) l += exp2f(sinks[hq] * 1.4426950408889634f - m_used);
       const float inv = 1.0f / ((sink > 0.f && row_live) ? l + sink * exp2f(-m_used) : l);
-      bf16* orow = out + ((size_t)(tok0 + i0 + row) * H + hq) * AT_D;
+      bf16* orow = out + ((size_t)(tok0 + i0 + row) * H + hq) * AT_D + half * (AT_D / 2);
 #pragma unroll 1
-      for (int c = 0; c < AT_D; c += 32) {
+      for (int c = 0; c < AT_D / 2; c += 32) {
         float o[32];
-        tmem_ld32(tO + lane_off + (uint32_t)c, o);
+        tmem_ld32(tO + lane_off + (uint32_t)(half * (AT_D / 2) + c), o);
         if (row_live) {
 #pragma unroll
           for (int e = 0; e < 32; e += 8) {
