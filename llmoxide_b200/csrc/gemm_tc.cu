@@ -70,7 +70,8 @@ __host__ __device__ constexpr uint32_t umma_idesc(int n) {
 template <int BN, int MODE, typename TY>
 __device__ __forceinline__ void epilogue_tile(uint32_t acc_addr, bool have_acc, bool store, TY* __restrict__ out,
                                               int n0, int t0, int T, int n_limit, long long ldy, int quad, int lane,
-                                              const GateAct act, const float* row_scale = nullptr) {
+                                              const GateAct act, const float* row_scale = nullptr,
+                                              const float* parts = nullptr, int n_parts = 0) {
   const int row = quad * 32 + lane;
   const int n = MODE == 2 ? (n0 >> 1) + quad * 16 + (lane & 15) : n0 + row;
   const bool upper = lane >= 16;
@@ -86,6 +87,11 @@ __device__ __forceinline__ void epilogue_tile(uint32_t acc_addr, bool have_acc, 
     } else {
 #pragma unroll
       for (int e = 0; e < 16; ++e) v[e] = g[e] = 0.f;
+    }
+    for (int p = 0; p < n_parts; ++p) {        // what the cluster's other CTAs have of this tile, in their order
+      const float* other = parts + ((size_t)p * BN + c) * TC_BM + row;
+#pragma unroll
+      for (int e = 0; e < 16; ++e) v[e] += other[e * TC_BM];
     }
     if (row_scale) {            // column t of the accumulator times r[t] (tokens past T are never stored)
 #pragma unroll
@@ -187,12 +193,34 @@ __device__ __forceinline__ void epilogue_tile_staged(uint32_t acc_addr, const CU
 // MODE 0: Y (bf16 or f32) [T, N] or split partials f32 [n_split][T, N].
 // MODE 1: two accumulators, rows n and n + F of W; act[T, F] = silu(g) * u.
 // MODE 3: Y (bf16) [T, N] = act(product).
+//
+// PARTS: a step of few tokens against a matrix with few row tiles, whose result is not wanted as partial sums (an
+// activation follows, or bfloat16 goes out).  The CTAs of a cluster share a unit, each a part of K (n_parts of them,
+// k_blocks_per_split blocks each); all but the first leave their accumulators in the first one's shared memory, which
+// adds them in their order and finishes the unit.  Without it 16 to 32 CTAs stream the matrix: gate|up of 4096 rows,
+// K = 2048, four tokens 11.6 -> 7.6 us of a decode step's path (floor 2.6; what is left is the chain from the kernel
+// before, four blocks of K and the hand-over).
 // ---------------------------------------------------------------------------
-template <int BN, int MODE, typename TY>
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int BN, int MODE, typename TY, bool PARTS>
 __global__ void __launch_bounds__(TC_THREADS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                TY* __restrict__ Y, int T, int N, int K, long long ldy, int k_blocks_per_split,
-               long long split_stride, int F, int n_stages, int row_tiles, int token_tiles, int n_units,
+               long long split_stride, int F, int n_stages, int row_tiles, int token_tiles, int n_units, int n_parts,
                const TcScale sc, const GateAct act) {
   extern __shared__ uint8_t smem_raw[];
   constexpr int N_ACC = MODE == 1 ? 2 : 1;   // MODE 2 has one accumulator: gate and up rows share a tile
@@ -214,6 +242,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   const uint32_t acc_full0 = empty0 + 8u * n_stages, acc_empty0 = acc_full0 + 16u;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * n_stages + 4);
   float* row_scales = reinterpret_cast<float*>(bars + 2 * n_stages + 6);   // [64] r[t]
+  float* parts = row_scales + 64;                                          // PARTS: [n_parts - 1][BN][TC_BM]
+  const uint32_t part = PARTS ? cluster_ctarank() : 0u;
+  const int first_unit = PARTS ? (int)blockIdx.x / n_parts : (int)blockIdx.x;      // (PARTS: the only one)
 
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
@@ -236,7 +267,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
-  __syncthreads();
+  if (PARTS) __syncwarp();
+  if (PARTS) cluster_sync_all();           // (every CTA of the cluster runs: its shared memory may be written)
+  else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
 
@@ -248,17 +281,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     split = rest / row_tiles;
     n0 = rt * TC_BM;
     t0 = tt * BN;
-    kb_begin = split * k_blocks_per_split;
+    kb_begin = (PARTS ? (int)part : split) * k_blocks_per_split;
     const int kb_end = min(total_kb, kb_begin + k_blocks_per_split);
     n_kb = max(0, kb_end - kb_begin);
   };
 
+  bool done = false;                       // (PARTS) this warp has seen the accumulator complete
   if (warp == 0) {
     // ---------------- producer ----------------
     if (lane == 0) {
       RingPos pos{0, 0};          // where the next k-block goes
       bool waited = false, ok = true;
-      for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+      for (int u = first_unit; u < n_units && ok; u += gridDim.x) {
         int n0, t0, kb_begin, n_kb, split;
         unit_coords(u, n0, t0, kb_begin, n_kb, split);
         int i = 0;
@@ -303,7 +337,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       RingPos pos{0, 0};
       const uint32_t desc0 = umma_desc_lo(base);       // stage 0's W tile; every other tile is an offset from it
       bool ok = true;
-      for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++j) {
+      for (int u = first_unit; u < n_units && ok; u += gridDim.x, ++j) {
         int n0, t0, kb_begin, n_kb, split;
         unit_coords(u, n0, t0, kb_begin, n_kb, split);
         const int buf = j % ACC_BUFS, use = j / ACC_BUFS;
@@ -355,7 +389,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       row_scale = row_scales;
     }
     int j = 0;
-    for (int u = blockIdx.x; u < n_units; u += gridDim.x, ++j) {
+    for (int u = first_unit; u < n_units; u += gridDim.x, ++j) {
       int n0, t0, kb_begin, n_kb, split;
       unit_coords(u, n0, t0, kb_begin, n_kb, split);
       const int buf = j % ACC_BUFS, use = j / ACC_BUFS;
@@ -365,6 +399,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         failed = __shfl_sync(0xffffffffu, ok ? 0 : 1, 0) != 0;
       }
       if (failed) break;
+      done = true;
       tc_fence_after();
       if (n_kb == 0 && !waited) {       // no load ordered this unit after the kernel before: do it here
         pdl_wait();
@@ -372,11 +407,38 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       }
       TY* out = Y + (MODE == 0 ? (size_t)split * split_stride : 0);
       const uint32_t acc_addr = tmem_base + (uint32_t)buf * ACC_COLS + ((uint32_t)(quad * 32) << 16);
+      if (PARTS) {
+        if (part == 0) break;                    // finished below, once the others' accumulators are here
+        const uint32_t dst = map_to_cta(smem_u32(parts + (size_t)(part - 1) * BN * TC_BM + quad * 32 + lane), 0);
+#pragma unroll 1
+        for (int c = 0; c < BN && t0 + c < T; c += 16) {
+          float v[16];
+          tmem_ld16(acc_addr + (uint32_t)c, v);
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + (uint32_t)((c + e) * TC_BM * 4)), "f"(v[e]) : "memory");
+        }
+        break;
+      }
       epilogue_tile<BN, MODE, TY>(acc_addr, n_kb > 0, true, out, n0, t0, T, n_limit, ldy, quad, lane, act, row_scale);
       // hand the accumulator set back to the MMA warp
       tc_fence_before();
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty0 + 8u * buf) : "memory");
+    }
+  }
+  if (PARTS) {
+    __syncwarp();
+    cluster_sync_all();
+    const bool missing = __shfl_sync(0xffffffffu, done ? 0 : 1, 0) != 0;          // (a wait of this CTA ran out)
+    if (part == 0 && warp >= 2 && !missing) {
+      int n0, t0, kb_begin, n_kb, split;
+      unit_coords(first_unit, n0, t0, kb_begin, n_kb, split);
+      const int quad = warp & 3;
+      tc_fence_after();
+      epilogue_tile<BN, MODE, TY>(tmem_base + ((uint32_t)(quad * 32) << 16), true, true, Y, n0, t0, T,
+                                  MODE == 0 || MODE == 3 ? N : F, ldy, quad, lane, act, sc.sumsq ? row_scales : nullptr, parts,
+                                  n_parts - 1);
     }
   }
   tc_fence_before();
@@ -401,20 +463,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 // CTAs by one multicast tcgen05.commit; both CTAs' epilogue warps arrive on
 // the leader's `acc_empty`.  Every wait is bounded.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -733,7 +781,7 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, void* Y, int T, 
   if (stages < 2) stages = 2;
   const size_t smem = 1024 + (size_t)stages * STAGE + (2 * stages + 6) * 8 +
                       TC_FUSE_BYTES;
-  auto kernel = gemm_tc_kernel<BN, MODE, TY>;
+  auto kernel = gemm_tc_kernel<BN, MODE, TY, false>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -743,7 +791,44 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, void* Y, int T, 
   const int max_ctas = sm_count() * ctas_per_sm;
   const int grid = n_units < max_ctas ? (int)n_units : max_ctas;
   launch_pdl(kernel, dim3(grid), dim3(TC_THREADS), smem, stream, mw, mx, (TY*)Y, T, N, K, ldy, per_split,
-             split_stride, F, stages, row_tiles, token_tiles, (int)n_units, sc, t_gate_act);
+             split_stride, F, stages, row_tiles, token_tiles, (int)n_units, 1, sc, t_gate_act);
+  return LLMX_LAUNCH_STATUS();
+}
+
+// How many CTAs share the K of a tile in a step of few tokens whose result goes out whole: a power of two up to 8, no more
+// than one CTA per SM in all, at least four blocks of K each, and 96 KB at most for the accumulators that are handed over.
+static int choose_parts(int T, int N, int K) {
+  if (T > 64) return 1;
+  const int tiles = (N + TC_BM - 1) / TC_BM, blocks = (K + TC_BK - 1) / TC_BK, bn = T <= 16 ? 16 : T <= 32 ? 32 : 64;
+  int parts = 1;
+  while (parts < 8 && tiles * parts * 2 <= sm_count() && blocks >= parts * 2 * 4 &&
+         (parts * 2 - 1) * bn * TC_BM * 4 <= 96 * 1024)
+    parts *= 2;
+  while (parts > 1 && (blocks + parts - 1) / parts * (parts - 1) >= blocks) parts /= 2;      // (no part is empty)
+  return parts;
+}
+
+template <int BN, int MODE, typename TY>
+static int launch_parts(const CUtensorMap& mw, const CUtensorMap& mx, void* Y, int T, int N, int K, long long ldy, int n_parts,
+                        int F, const TcScale& sc, cudaStream_t stream) {
+  static_assert(MODE != 1 && BN <= 64, "one accumulator, few tokens");
+  constexpr size_t STAGE = (size_t)TC_BM * TC_BK * 2 + (size_t)BN * TC_BK * 2;
+  const size_t handed = (size_t)(n_parts - 1) * BN * TC_BM * 4;
+  const int blocks = (K + TC_BK - 1) / TC_BK, per_part = (blocks + n_parts - 1) / n_parts;
+  int stages = (int)((200 * 1024 - handed) / STAGE);
+  if (stages > 12) stages = 12;
+  if (stages > per_part) stages = per_part < 2 ? 2 : per_part;
+  const size_t smem = 1024 + (size_t)stages * STAGE + (2 * stages + 6) * 8 + TC_FUSE_BYTES + handed;
+  auto kernel = gemm_tc_kernel<BN, MODE, TY, true>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return (int)e;
+    attr_set = true;
+  }
+  const int row_tiles = (N + TC_BM - 1) / TC_BM;             // (MODE 2 walks all 2F interleaved rows; one tile of tokens)
+  launch_pdl_cluster(kernel, dim3(row_tiles * n_parts), dim3(TC_THREADS), smem, stream, (unsigned)n_parts, mw, mx, (TY*)Y, T,
+                     N, K, ldy, per_part, (long long)0, F, stages, row_tiles, 1, row_tiles, n_parts, sc, t_gate_act);
   return LLMX_LAUNCH_STATUS();
 }
 
@@ -786,6 +871,19 @@ LLMX_API int llmx_gemm_tc_scaled(const void* X, const void* W, void* Y, int y_dt
   CUtensorMap mw, mx;
   if (make_map(&mw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, TC_BM, true)) return LLMX_REFUSED(4);
   if (make_map(&mx, X, (uint64_t)T, (uint64_t)K, (uint64_t)ldx, (uint32_t)bn, false)) return LLMX_REFUSED(4);
+  const int parts = n_split == 1 && mode != 1 && y_dtype == LLMX_BF16 ? choose_parts(T, N, K) : 1;
+  if (parts > 1) {
+#define PARTS(MODE)                                                                                       \
+  switch (bn) {                                                                                           \
+    case 16: return launch_parts<16, MODE, bf16>(mw, mx, Y, T, N, K, ldy, parts, F, sc, stream);          \
+    case 32: return launch_parts<32, MODE, bf16>(mw, mx, Y, T, N, K, ldy, parts, F, sc, stream);          \
+    default: return launch_parts<64, MODE, bf16>(mw, mx, Y, T, N, K, ldy, parts, F, sc, stream);          \
+  }
+    if (mode == 0) PARTS(0)
+    if (mode == 2) PARTS(2)
+    PARTS(3)
+#undef PARTS
+  }
 #define GO(BN, MODE, TY) return launch<BN, MODE, TY>(mw, mx, Y, T, N, K, ldy, n_split, split_stride, F, sc, stream)
 #define BY_BN(MODE, TY)                    \
   switch (bn) {                            \
