@@ -255,6 +255,57 @@ add_rms_norm_kernel(float* __restrict__ h, const TD* __restrict__ delta, int n_s
   }
 }
 
+// The norm alone (no residual to add) of many rows: out[r,:] = rms(h[r,:]) * gain.  CTAs walk rows, the gain stays in
+// registers and a row is asked for while the one before is being reduced: with a CTA per row every row paid its own launch,
+// its gain and one memory round trip ahead of the reduction, at half of the HBM rate.  Thread by thread the same elements
+// and additions as add_rms_norm_kernel.  Rows of 4096 to bfloat16: 13182 rows 81.4 -> 53.4 us (6.1 TB/s), 2048 rows
+// 10.5 -> 9.0; 4000 rows of 2048 12.5 -> 10.3.  Bound by HBM.
+template <typename TO, int CH>
+__global__ void __launch_bounds__(512, 3)
+norm_rows_kernel(const float* __restrict__ h, const float* __restrict__ gain, float eps, TO* __restrict__ out, int d,
+                 int n_rows) {
+  __shared__ float red[32];
+  pdl_launch_dependents();
+  const int nthreads = blockDim.x;
+  float4 g[CH], v[CH];
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int i = (c * nthreads + threadIdx.x) * 4;
+    g[c] = i < d ? load4(gain + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  pdl_wait();
+  auto fetch = [&](int r) {
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const int i = (c * nthreads + threadIdx.x) * 4;
+      v[c] = i < d && r < n_rows ? load4(h + (size_t)r * d + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  fetch(blockIdx.x);
+  for (int r = blockIdx.x; r < n_rows; r += gridDim.x) {
+    float4 x[CH];
+    float ss = 0.f;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      x[c] = v[c];
+      ss += x[c].x * x[c].x;
+      ss += x[c].y * x[c].y;
+      ss += x[c].z * x[c].z;
+      ss += x[c].w * x[c].w;
+    }
+    fetch(r + gridDim.x);
+    const float total = block_sum(ss, red);
+    const float scale = 1.0f / sqrtf(total / (float)d + eps);
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const int i = (c * nthreads + threadIdx.x) * 4;
+      if (i < d)
+        store4(out + (size_t)r * d + i, make_float4((x[c].x * scale) * g[c].x, (x[c].y * scale) * g[c].y,
+                                                    (x[c].z * scale) * g[c].z, (x[c].w * scale) * g[c].w));
+    }
+  }
+}
+
 // (vectors per thread, threads) for a row of d elements; 0 vectors: the staged path
 static void norm_shape(int d, int& ch, int& threads) {
   const int vecs = (d + 3) / 4;
@@ -274,6 +325,14 @@ static int launch_add_rms_norm(float* h, const void* delta, int n_split, size_t 
   int ch, threads;
   norm_shape(d, ch, threads);
   const bool deep = delta && n_split > 1;
+  // Rule: rows without a residual to add, more of them than run at once with a CTA each (three to an SM at 512 threads);
+  // fewer gain nothing (1000 rows of 4096: 9.0 us either way)
+  const int at_once = 148 * (1536 / threads);
+  if (!delta && out && !rows && (ch == 1 || ch == 2) && n_rows > at_once) {
+    if (ch == 1) launch_pdl(norm_rows_kernel<TO, 1>, dim3(at_once), dim3(threads), 0, stream, (const float*)h, gain, eps, (TO*)out, d, n_rows);
+    else launch_pdl(norm_rows_kernel<TO, 2>, dim3(at_once), dim3(threads), 0, stream, (const float*)h, gain, eps, (TO*)out, d, n_rows);
+    return LLMX_LAUNCH_STATUS();
+  }
 #define GO(CH, SMEM)                                                                                              \
   do {                                                                                                            \
     if (deep)                                                                                                     \
