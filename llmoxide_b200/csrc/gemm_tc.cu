@@ -196,7 +196,7 @@ __device__ __forceinline__ void epilogue_tile_staged(uint32_t acc_addr, const CU
 //
 // PARTS: a step of few tokens against a matrix with few row tiles, whose result is not wanted as partial sums (an
 // activation follows, or bfloat16 goes out).  The CTAs of a cluster share a unit, each a part of K (n_parts of them,
-// k_blocks_per_split blocks each); all but the first leave their accumulators in the first one's shared memory, which
+// k_blocks_per_split blocks each; tiles_or_parts is their number, the token tiles' otherwise); all but the first leave their accumulators in the first one's shared memory, which
 // adds them in their order and finishes the unit.  Without it 16 to 32 CTAs stream the matrix: gate|up of 4096 rows,
 // K = 2048, four tokens 11.6 -> 7.6 us of a decode step's path (floor 2.6; what is left is the chain from the kernel
 // before, four blocks of K and the hand-over).
@@ -220,7 +220,7 @@ template <int BN, int MODE, typename TY, bool PARTS>
 __global__ void __launch_bounds__(TC_THREADS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                TY* __restrict__ Y, int T, int N, int K, long long ldy, int k_blocks_per_split,
-               long long split_stride, int F, int n_stages, int row_tiles, int token_tiles, int n_units, int n_parts,
+               long long split_stride, int F, int n_stages, int row_tiles, int tiles_or_parts, int n_units,
                const TcScale sc, const GateAct act) {
   extern __shared__ uint8_t smem_raw[];
   constexpr int N_ACC = MODE == 1 ? 2 : 1;   // MODE 2 has one accumulator: gate and up rows share a tile
@@ -243,6 +243,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * n_stages + 4);
   float* row_scales = reinterpret_cast<float*>(bars + 2 * n_stages + 6);   // [64] r[t]
   float* parts = row_scales + 64;                                          // PARTS: [n_parts - 1][BN][TC_BM]
+  const int token_tiles = PARTS ? 1 : tiles_or_parts, n_parts = PARTS ? tiles_or_parts : 1;
   const uint32_t part = PARTS ? cluster_ctarank() : 0u;
   const int first_unit = PARTS ? (int)blockIdx.x / n_parts : (int)blockIdx.x;      // (PARTS: the only one)
 
@@ -791,7 +792,7 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, void* Y, int T, 
   const int max_ctas = sm_count() * ctas_per_sm;
   const int grid = n_units < max_ctas ? (int)n_units : max_ctas;
   launch_pdl(kernel, dim3(grid), dim3(TC_THREADS), smem, stream, mw, mx, (TY*)Y, T, N, K, ldy, per_split,
-             split_stride, F, stages, row_tiles, token_tiles, (int)n_units, 1, sc, t_gate_act);
+             split_stride, F, stages, row_tiles, token_tiles, (int)n_units, sc, t_gate_act);
   return LLMX_LAUNCH_STATUS();
 }
 
@@ -828,7 +829,7 @@ static int launch_parts(const CUtensorMap& mw, const CUtensorMap& mx, void* Y, i
   }
   const int row_tiles = (N + TC_BM - 1) / TC_BM;             // (MODE 2 walks all 2F interleaved rows; one tile of tokens)
   launch_pdl_cluster(kernel, dim3(row_tiles * n_parts), dim3(TC_THREADS), smem, stream, (unsigned)n_parts, mw, mx, (TY*)Y, T,
-                     N, K, ldy, per_part, (long long)0, F, stages, row_tiles, 1, row_tiles, n_parts, sc, t_gate_act);
+                     N, K, ldy, per_part, (long long)0, F, stages, row_tiles, n_parts, row_tiles, sc, t_gate_act);
   return LLMX_LAUNCH_STATUS();
 }
 
