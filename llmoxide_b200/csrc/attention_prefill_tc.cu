@@ -343,14 +343,13 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       // the maximum to use: keep the old one unless the row's true maximum outgrew it by more than 2^8
       bool rescale = false;
       if (at_pair_any(quad, !ok || mt > m_used + 8.0f)) {           // also the first time (m_used = -inf)
-        told[half * AT_ROWS + row] = ok ? mt : __int_as_float(0x7fffffff);       // (a NaN: this warp leaves)
-        at_pair_any(quad, false);
-        const float other = told[(half ^ 1) * AT_ROWS + row];
-        if (!ok || __any_sync(0xffffffffu, __float_as_int(other) == 0x7fffffff)) {
+        told[half * AT_ROWS + row] = mt;
+        if (at_pair_any(quad, !ok)) {      // (the barrier itself says so to both: any maximum, a NaN too, is a maximum)
           ok = false;
           left = true;
           break;
         }
+        const float other = told[(half ^ 1) * AT_ROWS + row];
         tc_fence_after();
         mt = fmaxf(mt, other);
         float alpha = 1.0f;

@@ -157,6 +157,30 @@ def test_prompt_attention_whose_wait_runs_out_is_reported():
     assert kernels.attention_prefill_tc_status() == 0
 
 
+@pytest.mark.parametrize("scale", [0.0, math.nan])
+def test_prompt_attention_whose_maxima_are_nan_comes_back(scale):
+    """Under such a scale the maximum of a masked half tile is NaN.  The two warps that share a row have to leave or stay
+    together whatever their maxima are; what they write is not looked at."""
+    from llmoxide_b200 import kernels
+
+    H, G, D, T = 4, 2, 128, 200
+    g = torch.Generator().manual_seed(5)
+    kc, vc = (torch.randn(6, G, 64, D, generator=g).bfloat16().cuda() for _ in range(2))
+    table = torch.tensor([[1, 2, 3, 4]], dtype=torch.int32).cuda()
+    q = torch.randn(T, H * D, generator=g).bfloat16().cuda()
+    out, again = torch.empty_like(q), torch.empty_like(q)
+    start, past = torch.tensor([0, T], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda()
+    args = (kc, vc, table, start, past, 1, T, H, G, D, None)
+    kernels.attention_prefill_tc(q, out, *args, D ** -0.5)
+    kernels.attention_prefill_tc(q, again, *args, scale)
+    torch.cuda.synchronize()
+    kernels.check_status()
+    kernels.attention_prefill_tc(q, again, *args, D ** -0.5)
+    torch.cuda.synchronize()
+    kernels.check_status()
+    assert torch.equal(out, again) and kernels.attention_prefill_tc_status() == 0
+
+
 def test_the_engine_raises_where_it_has_waited(tmp_path):
     """Through the product path: the generation loop (reading a step's tokens) and trace replay (reading a
     step's logits) raise ``KernelError``; afterwards the same engine gives right logits again."""
