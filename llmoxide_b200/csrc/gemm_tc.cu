@@ -241,6 +241,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8u * n_stages;
   const uint32_t acc_full0 = empty0 + 8u * n_stages, acc_empty0 = acc_full0 + 16u;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * n_stages + 4);
+  uint32_t* lost = tmem_holder + 1;                                        // PARTS, the first CTA's: a part that will not come
   float* row_scales = reinterpret_cast<float*>(bars + 2 * n_stages + 6);   // [64] r[t]
   float* parts = row_scales + 64;                                          // PARTS: [n_parts - 1][BN][TC_BM]
   const int token_tiles = PARTS ? 1 : tiles_or_parts, n_parts = PARTS ? tiles_or_parts : 1;
@@ -257,6 +258,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       mbar_init(acc_full0 + 8u * i, 1);
       mbar_init(acc_empty0 + 8u * i, 4);      // one arrival per epilogue warp
     }
+    if (PARTS) *lost = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
@@ -361,8 +363,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           }
           umma_commit(empty0 + 8u * s);   // the stage is free once these MMAs have read it
         }
-        // (tests: with llmx_withhold the first unit's accumulator is never announced, and the epilogue's wait runs out)
-        if (!(j == 0 && llmx_withhold))
+        // (tests: with llmx_withhold the first unit's accumulator is never announced, and the epilogue's wait runs out; where
+        // CTAs share a unit, the last part's)
+        if (!(j == 0 && llmx_withhold && (!PARTS || (int)part == n_parts - 1)))
           umma_commit(acc_full0 + 8u * buf);  // this unit's accumulator is complete once every MMA has finished
       }
     }
@@ -429,9 +432,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
   }
   if (PARTS) {
+    if (part != 0 && warp >= 2 && lane == 0 && !done)                 // a wait of this CTA ran out: the tile is not finished
+      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(smem_u32(lost), 0)), "r"(1u) : "memory");
     __syncwarp();
     cluster_sync_all();
-    const bool missing = __shfl_sync(0xffffffffu, done ? 0 : 1, 0) != 0;          // (a wait of this CTA ran out)
+    const bool missing = __shfl_sync(0xffffffffu, done ? 0 : 1, 0) != 0 || *(volatile uint32_t*)lost != 0;
     if (part == 0 && warp >= 2 && !missing) {
       int n0, t0, kb_begin, n_kb, split;
       unit_coords(first_unit, n0, t0, kb_begin, n_kb, split);

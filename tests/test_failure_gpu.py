@@ -78,6 +78,32 @@ def test_a_matrix_product_whose_wait_runs_out_is_reported_and_the_library_goes_o
     assert kernels.gemm_tc_status() == 0
 
 
+@pytest.mark.parametrize("T", [3, 40])
+def test_a_part_of_k_that_never_comes_leaves_the_tile_unwritten(T):
+    """CTAs that share the K of a tile: the last part's accumulator is never announced, the first one's is."""
+    from llmoxide_b200 import kernels
+    from llmoxide_b200.errors import KernelError
+
+    torch.manual_seed(1)
+    x, w = torch.randn(T, 2048).bfloat16().cuda(), (torch.randn(384, 2048) * 2048 ** -0.5).bfloat16().cuda()
+    want = x.double() @ w.double().t()
+    out = torch.full((T, 384), 7.0, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    try:
+        kernels.test_waits("gemm_tc", SHORT, True)
+        kernels.gemm_tc(x, w, out)
+        torch.cuda.synchronize()
+        with pytest.raises(KernelError, match="gemm_tc"):
+            kernels.check_status()
+        assert kernels.gemm_tc_status() == 3 and (out == 7.0).all()
+    finally:
+        _reset("gemm_tc")
+    kernels.gemm_tc(x, w, out)
+    torch.cuda.synchronize()
+    kernels.check_status()
+    assert float((out.double() - want).abs().max() / want.abs().max()) < 6e-3 and kernels.gemm_tc_status() == 0
+
+
 def _decode_case(D, lengths, G=2, H=8):
     g = torch.Generator().manual_seed(3)
     n_pages = sum((n + 63) // 64 for n in lengths) + 1
