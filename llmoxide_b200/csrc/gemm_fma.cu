@@ -201,10 +201,15 @@ gemm_f32_rows_kernel(const float* __restrict__ X, const float* __restrict__ W, f
              ((i / PER_SEG) * G + q) * F32_SEG + (i % PER_SEG) * BK, K);
   };
   pdl_launch_dependents();
-  for (int s = 0; s < STAGES - 1 && s < n_steps; ++s) load_w(s);     // the weights do not wait for the kernel before
+  // W may be what the kernel before writes, so nothing of it is read ahead of that kernel's end; its lines are asked for as
+  // far as L2, where that kernel's stores arrive too
+  for (int i = threadIdx.x; i < (STAGES - 1) * G * BN; i += 128) {
+    const int k = (i / BN % G) * F32_SEG + (i / (G * BN)) * BK, n = n0 + i % BN;
+    if (n < N && k < K) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (size_t)n * ldw + k));
+  }
   pdl_wait();
   for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < n_steps) load_x(s);
+    if (s < n_steps) load_w(s), load_x(s);
     copy_commit();
   }
   unsigned long long acc[MT];

@@ -48,6 +48,21 @@ def test_gemm_f32_keeps_infinities_and_nan_in_their_rows():
     assert torch.equal(~torch.isfinite(out), bad)
 
 
+def test_gemm_f32_takes_a_matrix_that_the_kernel_before_writes():
+    """The product of a prompt becomes the matrix of a product of few tokens, launched right behind it."""
+    from llmoxide_b200 import kernels
+    torch.manual_seed(11)
+    a, b, x = torch.randn(700, 2048, device=DEV), torch.randn(2048, 2048, device=DEV) / 45, torch.randn(3, 2048, device=DEV)
+    want = x.double() @ (a.double() @ b.double().T).T
+    for M in (1, 3):
+        w, out = torch.full((700, 2048), 7.0, device=DEV), torch.empty(M, 700, device=DEV)
+        for _ in range(3):
+            w.fill_(7.0)
+            kernels.gemm_fma(a, b, w)
+            kernels.gemm_fma(x[:M], w, out)
+            assert rel(out, want[:M]) < 2e-6
+
+
 CASES = [   # H, G, D, Dv, lengths, window, keep_first, chunk, sink, softcap, sinks, bias entries, gate
     (6, 3, 48, 48, [1, 64, 130], None, 0, 0, 0.0, 0.0, False, 0, False),
     (16, 4, 128, 128, [300, 65], 70, 0, 0, 0.0, 0.0, False, 0, False),
