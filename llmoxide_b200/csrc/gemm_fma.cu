@@ -185,7 +185,8 @@ gemm_f32_rows_kernel(const float* __restrict__ X, const float* __restrict__ W, f
   const int f = threadIdx.x & 15, g = (threadIdx.x >> 4) & 3, h = threadIdx.x >> 6;
   const int n0 = (blockIdx.x % n_tiles) * BN, m0 = (blockIdx.x / n_tiles) * BM;
   const int n_seg = (K + F32_SEG - 1) / F32_SEG, n_rounds = (n_seg + G - 1) / G;
-  const int n_steps = n_rounds * PER_SEG;                  // step i: k block i % PER_SEG of the segments of round i / PER_SEG
+  // step i: k block i % PER_SEG of the segments of round i / PER_SEG; a last round of one segment ends where K does
+  const int n_steps = n_seg % G == 1 ? (n_rounds - 1) * PER_SEG + (K - (n_seg - 1) * F32_SEG + BK - 1) / BK : n_rounds * PER_SEG;
   const BlockCopy<BN, BK, VEC> copy_w(W, ldw, n0, N);
   const BlockCopy<BM, BK, VEC> copy_x(X, ldx, m0, M);
   auto load_w = [&](int i) {
@@ -216,6 +217,22 @@ gemm_f32_rows_kernel(const float* __restrict__ X, const float* __restrict__ W, f
   float total[MT];                                         // (group 0 keeps the totals of its feature)
 #pragma unroll
   for (int i = 0; i < MT; ++i) acc[i] = 0ull, total[i] = 0.f;
+  auto join = [&](int round) {                             // the round's segments join the totals in their order
+#pragma unroll
+    for (int i = 0; i < MT; ++i) sums[(g * BM + 2 * i + h) * BN + f] = both(acc[i]), acc[i] = 0ull;
+    __syncthreads();
+    if (g == 0) {
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        const float* t = sums + (2 * i + h) * BN + f;
+        total[i] = round == 0 ? *t : __fadd_rn(total[i], *t);
+        for (int q = 1; q < G && round * G + q < n_seg; ++q) total[i] = __fadd_rn(total[i], t[q * BM * BN]);
+      }
+    }
+    __syncthreads();
+  };
+  constexpr int UNROLL = MT == 2 ? 1 : 2;                  // (by measurement: 16 tokens 13.5 us at N = 256, K = 2048, 15.3 without; 4 tokens 7.5, 8.8 with)
+#pragma unroll UNROLL
   for (int step = 0; step < n_steps; ++step) {
     asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
     __syncthreads();
@@ -232,22 +249,9 @@ gemm_f32_rows_kernel(const float* __restrict__ X, const float* __restrict__ W, f
         fma2(acc[i], a.x, b.x), fma2(acc[i], a.y, b.y);
       }
     }
-    if ((step + 1) % PER_SEG == 0) {                       // the round's segments join the totals in their order
-      const int round = step / PER_SEG;
-#pragma unroll
-      for (int i = 0; i < MT; ++i) sums[(g * BM + 2 * i + h) * BN + f] = both(acc[i]), acc[i] = 0ull;
-      __syncthreads();
-      if (g == 0) {
-#pragma unroll
-        for (int i = 0; i < MT; ++i) {
-          const float* t = sums + (2 * i + h) * BN + f;
-          total[i] = round == 0 ? *t : __fadd_rn(total[i], *t);
-          for (int q = 1; q < G && round * G + q < n_seg; ++q) total[i] = __fadd_rn(total[i], t[q * BM * BN]);
-        }
-      }
-      __syncthreads();
-    }
+    if ((step + 1) % PER_SEG == 0) join(step / PER_SEG);
   }
+  if (n_steps % PER_SEG) join(n_rounds - 1);
   if (g == 0 && n0 + f < N) {
 #pragma unroll
     for (int i = 0; i < MT; ++i) {
@@ -282,20 +286,22 @@ LLMX_API int llmx_gemm_f32_form(int form, const float* X, const float* W, float*
   if (K <= 0 || ldx < K || ldw < K || ldy < N || form >= F32_N_FORMS) return LLMX_REFUSED(1);
   if ((M + 63) / 64 > 65535) return LLMX_REFUSED(3);
   if (form < 0) {
-    // Rule: up to 16 tokens in one CTA's rows.  Beyond that the cheapest of what was measured at K = 2048 (us; all three
-    // grow with K alike): a round of 296 CTAs of 16 x 16 elements takes 19, 148 tiles of 32 x 64 take 33 (52 at least,
-    // for one alone cannot hide its waits), 148 tiles of 64 x 128 take 112 (150 at least).
-    const auto rounds = [](long long n, int m) { return (n + m - 1) / m; };
-    const auto tiles = [&](int bm, int bn) { return rounds(M, bm) * rounds(N, bn); };
-    if (M <= 16) {
-      form = M <= 2 ? 0 : M <= 4 ? 1 : M <= 8 ? 2 : 3;
-    } else {
-      const long long rows = 19 * rounds(tiles(16, 16), 296);
-      long long small = 33 * rounds(tiles(32, 64), 148), large = 112 * rounds(tiles(64, 128), 148);
-      if (small < 52) small = 52;
-      if (large < 150) large = 150;
-      form = rows <= small && rows <= large ? 3 : small <= large ? 4 : 5;
-    }
+    // Rule: the cheapest by what was measured over K = 64 to 8192, N = 64 to 8192 and 1 to 2500 tokens (us beside a launch's
+    // 1.5).  A step of 32 k in four segments costs a round of 296 CTAs of rows 0.6, 0.65, 0.75 or 1.1 (2, 4, 8, 16 tokens);
+    // 16 k cost 148 tiles of 32 x 64 0.26 (0.41 at least, for a tile alone cannot hide its waits), 148 tiles of 64 x 128 0.88
+    // (1.17 at least).  Up to 512 k only one segment's threads work, so tiles win there from few tokens on:
+    // 16 tokens, N = 8192, K = 256: 18 us by rows, 9.3 by tiles; N = 2048, K = 2048: 19 and 50.
+    const auto rounds = [](long long n, int m) { return (double)((n + m - 1) / m); };
+    const auto tiles = [&](int bm, int bn) { return (long long)rounds(M, bm) * (long long)rounds(N, bn); };
+    const int n_seg = (K + F32_SEG - 1) / F32_SEG;
+    const double steps = (n_seg / 4) * 16 + (n_seg % 4 == 1 ? (K - (n_seg - 1) * F32_SEG + 31) / 32 : n_seg % 4 ? 16 : 0);
+    const double blocks = (K + 15) / 16;
+    const int few = M <= 2 ? 0 : M <= 4 ? 1 : M <= 8 ? 2 : 3;
+    const double a_step[4] = {0.6, 0.65, 0.75, 1.1};
+    const double rows = a_step[few] * steps * rounds(tiles(2 << few, 16), 296);
+    const double small = blocks * fmax(0.26 * rounds(tiles(32, 64), 148), 0.41);
+    const double large = blocks * fmax(0.88 * rounds(tiles(64, 128), 148), 1.17);
+    form = rows <= small && rows <= large ? few : small <= large ? 4 : 5;
   }
   // 16-byte copies where every row starts on a 16-byte boundary and K ends on one, else 4-byte copies
   const bool wide = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && !((uintptr_t)X & 15) && !((uintptr_t)W & 15);

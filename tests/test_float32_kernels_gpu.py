@@ -37,6 +37,12 @@ def test_gemm_f32_forms_agree(M, N, K, pad):
         assert torch.equal(y, out[:, :N]), form
 
 
+@pytest.mark.parametrize("M, N, K, pad", [(20, 40, 33, 0), (9, 100, 64, 0), (40, 70, 96, 1), (6, 50, 480, 0), (3, 20, 2049, 3),
+                                          (18, 33, 2080, 0), (2, 16, 4097, 0)])
+def test_gemm_f32_ends_where_a_single_last_segment_does(M, N, K, pad):
+    test_gemm_f32_forms_agree(M, N, K, pad)
+
+
 def test_gemm_f32_keeps_infinities_and_nan_in_their_rows():
     from llmoxide_b200 import kernels
     x, w = torch.randn(20, 70, device=DEV), torch.randn(40, 70, device=DEV)
