@@ -672,10 +672,27 @@ decay_out_kernel(const float* __restrict__ prep, const float* __restrict__ decay
   // ---- + sum over the chunk's own tokens
   for (int s = e_steps; s < steps; ++s) {
     ss_copy_wait<0>();
-    __syncthreads();
+    // A token's infinite or NaN value is not multiplied by the zeros above the diagonal: tokens before it do not see it.
+    float zero_if_finite = 0.f;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {                      // (what this thread copied)
+      const float4 v = ss_load4(Bs[s & 1] + (lr + 4 * m) * 64 + lc);
+      zero_if_finite = fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, fmaf(v.w, 0.f, zero_if_finite))));
+    }
+    const bool select = __syncthreads_or(!(zero_if_finite == 0.f));
     if (s + 1 < steps) copy_rows(s + 1);
     const int jb = (s - e_steps) * 32;
-    if (jb == 0) ss_product<2>(acc, Ms, LA_LDM, Bs[s & 1], 64, min(32, ck.n));
+    if (select) {
+      for (int k = 0; k < min(32, ck.n - jb); ++k)
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const int i = ss_row(i0, r);
+          if (jb + k > i) continue;
+          const float m = Ms[(jb + k) * LA_LDM + i];
+#pragma unroll
+          for (int c = 0; c < 8; ++c) acc[r][c] = fmaf(m, Bs[s & 1][k * 64 + ss_row(j0, c)], acc[r][c]);
+        }
+    } else if (jb == 0) ss_product<2>(acc, Ms, LA_LDM, Bs[s & 1], 64, min(32, ck.n));
     else ss_product<2, false>(acc, Ms + jb * LA_LDM, LA_LDM, Bs[s & 1], 64, ck.n - jb);      // (they reach rows 32.. only)
   }
   const bool vec = (dm.Dv & 3) == 0 && ((uintptr_t)out & 15) == 0;

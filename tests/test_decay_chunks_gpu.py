@@ -47,3 +47,23 @@ def test_chunks_against_64_bits(H, D, Dv):
         assert torch.equal(run(proj[t0 : t0 + n], [n], H, D, Dv, decay, alone, [slot]), out[t0 : t0 + n])
         assert torch.equal(alone[slot], state[slot])
         t0 += n
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("at", [64, 70, 100, 127, 130])
+def test_a_value_that_is_not_finite_changes_no_token_before_it(at, bad):
+    H, D, Dv, n = 2, 128, 65, 140
+    torch.manual_seed(at)
+    decay, proj = torch.tensor([0.9, 0.99], device=DEV), torch.randn(n, H * (2 * D + Dv), device=DEV)
+    start = torch.randn(1, H, D, Dv, device=DEV)
+    clean = run(proj, [n], H, D, Dv, decay, start.clone(), [0])
+    proj[at, 2 * H * D + 3] = bad                                  # head 0, column 3
+    state = start.clone()
+    out = run(proj, [n], H, D, Dv, decay, state, [0])
+    changed = torch.zeros(n, H * Dv, dtype=torch.bool, device=DEV)
+    changed[at:, 3] = True
+    assert torch.equal(~torch.isfinite(out), changed)
+    assert torch.equal(out[~changed], clean[~changed])
+    lost = torch.zeros(H, D, Dv, dtype=torch.bool, device=DEV)
+    lost[0, :, 3] = True
+    assert torch.equal(~torch.isfinite(state[0]), lost)
