@@ -134,12 +134,11 @@ __device__ __forceinline__ void la_cp_async_wait() {
 // GATED: decay and input weight per token from `gates` [T, H, 4] = (a, b, exp(-m), product of a over the segment
 // up to and including the token) instead of the head's fixed decay.  head_stride: floats from one head's state to
 // the next (a design may keep more than S there).
-// C: neighbouring columns a thread owns.  Prompts take two: q and k then cost half as many shared-memory reads a
-// multiply-add, which is what one column a thread waits for (the multiply-adds are packed in pairs of dims), and the
-// shares of a chunk's eight tokens are added so that each of the eight lanes ends with one token's sum (7 shuffles a
-// column instead of 24).  Steps of few tokens stream the state and want the threads: one column.  Both, and a chunk cut
-// short, make the same additions in the same order.  Prompts of 700 to 1300 tokens, 16 heads of 128 x 128: the first pass
-// took 383 us with one column, 292 with two.
+// C: neighbouring columns a thread owns.  Two (some prompts: the rule is at the launch): q and k then cost half as many
+// shared-memory reads a multiply-add, which is what one column a thread waits for (the multiply-adds are packed in pairs of
+// dims), and the shares of a chunk's eight tokens are added so that each of the eight lanes ends with one token's sum (7
+// shuffles a column instead of 24).  Steps of few tokens stream the state and want the threads: one column.  Both, and a
+// chunk cut short, make the same additions in the same order.
 __device__ __forceinline__ void la_fma2(unsigned long long& d, unsigned long long a, unsigned long long b, unsigned long long c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
 }
@@ -171,6 +170,7 @@ decay_scan_kernel(const float* __restrict__ prep, float* __restrict__ out, float
   const int cw = (warp * 4 + (lane >> 3)) * C;    // this thread's first column of the CTA's
   const int col = c0 + cw;                        // and of v
   const int r = lane & 7;                         // its share of D
+  const bool col_live = col < Dv;
   const int seq_t0 = seq_start[b], seq_new = seq_start[b + 1] - seq_t0;
   const int n_seg = (seq_new + seg_len - 1) / seg_len;        // this sequence's segments
   const float g = GATED ? 1.f : decay[h];
@@ -185,38 +185,60 @@ decay_scan_kernel(const float* __restrict__ prep, float* __restrict__ out, float
   pdl_wait();
 
   auto own = [&](int i) { return 4 * (r + 8 * (i >> 2)) + (i & 3); };        // dim of this thread's i-th state value
-  unsigned long long s2[C][DPT / 2];                                         // its values in pairs of neighbouring dims
-  if (PASS == 1) {
+  float s_reg[C == 1 ? DPT : 1];                                             // one column: its values
+  unsigned long long s2[C][C == 1 ? 1 : DPT / 2];                            // two: their values in pairs of neighbouring dims
+  if constexpr (C == 1) {
+    if (PASS == 1) {
 #pragma unroll
-    for (int c = 0; c < C; ++c)
+      for (int i = 0; i < DPT; ++i) s_reg[i] = (seg == 0 && col_live && own(i) < D) ? S[(size_t)own(i) * Dv + col] : 0.f;
+    } else {
+      // E_(seg-1): what the segments before left, each decayed over the segments after it
+      float g_seg = 1.f;
+      if (!GATED)
+        for (int i = 0; i < seg_len; ++i) g_seg *= g;
 #pragma unroll
-      for (int i = 0; i < DPT; i += 2) {
-        const bool live = seg == 0 && col + c < Dv;
-        s2[c][i >> 1] = la_pair(live && own(i) < D ? S[(size_t)own(i) * Dv + col + c] : 0.f,
-                                live && own(i + 1) < D ? S[(size_t)own(i + 1) * Dv + col + c] : 0.f);
+      for (int i = 0; i < DPT; ++i) s_reg[i] = 0.f;
+      for (int sp = 0; sp < seg; ++sp) {
+        const float* ps = part_seq + (size_t)sp * D * Dv;
+        if (GATED) g_seg = __ldcg(gates + ((size_t)(seq_t0 + (sp + 1) * seg_len - 1) * H + h) * 4 + 3);   // over all of segment sp
+#pragma unroll
+        for (int i = 0; i < DPT; ++i)
+          if (col_live && own(i) < D) s_reg[i] = fmaf(g_seg, s_reg[i], __ldcg(ps + (size_t)own(i) * Dv + col));
       }
+    }
   } else {
-    // E_(seg-1): what the segments before left, each decayed over the segments after it
-    float g_seg = 1.f;
-    if (!GATED)
-      for (int i = 0; i < seg_len; ++i) g_seg *= g;
+    if (PASS == 1) {
 #pragma unroll
-    for (int c = 0; c < C; ++c)
+      for (int c = 0; c < C; ++c)
 #pragma unroll
-      for (int i = 0; i < DPT / 2; ++i) s2[c][i] = 0ull;
-    for (int sp = 0; sp < seg; ++sp) {
-      const float* ps = part_seq + (size_t)sp * D * Dv;
-      if (GATED) g_seg = __ldcg(gates + ((size_t)(seq_t0 + (sp + 1) * seg_len - 1) * H + h) * 4 + 3);   // over all of segment sp
-      const unsigned long long gg = la_pair(g_seg, g_seg);
-#pragma unroll
-      for (int i = 0; i < DPT; i += 2)
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          const bool live = col + c < Dv;
-          la_fma2(s2[c][i >> 1], gg, s2[c][i >> 1],
-                  la_pair(live && own(i) < D ? __ldcg(ps + (size_t)own(i) * Dv + col + c) : 0.f,
-                          live && own(i + 1) < D ? __ldcg(ps + (size_t)own(i + 1) * Dv + col + c) : 0.f));
+        for (int i = 0; i < DPT; i += 2) {
+          const bool live = seg == 0 && col + c < Dv;
+          s2[c][i >> 1] = la_pair(live && own(i) < D ? S[(size_t)own(i) * Dv + col + c] : 0.f,
+                                  live && own(i + 1) < D ? S[(size_t)own(i + 1) * Dv + col + c] : 0.f);
         }
+    } else {
+      // E_(seg-1): what the segments before left, each decayed over the segments after it
+      float g_seg = 1.f;
+      if (!GATED)
+        for (int i = 0; i < seg_len; ++i) g_seg *= g;
+#pragma unroll
+      for (int c = 0; c < C; ++c)
+#pragma unroll
+        for (int i = 0; i < DPT / 2; ++i) s2[c][i] = 0ull;
+      for (int sp = 0; sp < seg; ++sp) {
+        const float* ps = part_seq + (size_t)sp * D * Dv;
+        if (GATED) g_seg = __ldcg(gates + ((size_t)(seq_t0 + (sp + 1) * seg_len - 1) * H + h) * 4 + 3);   // over all of segment sp
+        const unsigned long long gg = la_pair(g_seg, g_seg);
+#pragma unroll
+        for (int i = 0; i < DPT; i += 2)
+#pragma unroll
+          for (int c = 0; c < C; ++c) {
+            const bool live = col + c < Dv;
+            la_fma2(s2[c][i >> 1], gg, s2[c][i >> 1],
+                    la_pair(live && own(i) < D ? __ldcg(ps + (size_t)own(i) * Dv + col + c) : 0.f,
+                            live && own(i + 1) < D ? __ldcg(ps + (size_t)own(i + 1) * Dv + col + c) : 0.f));
+          }
+      }
     }
   }
 
@@ -263,102 +285,168 @@ decay_scan_kernel(const float* __restrict__ prep, float* __restrict__ out, float
     // one token.  PASS 1: S = g S + k v, then this thread's share of q . S.  PASS 2: its share of q . E.  The
     // shares are added and stored afterwards, so that in a full chunk (the loop below unrolls) one token's
     // shuffles overlap the next token's arithmetic.
-    auto one_token = [&](int tt, float (&share)[C]) {
-      const float* qrow = buf + tt * tok_len;
-      const float* krow = qrow + Dp;
-      unsigned long long vv[C], acc01[C], acc23[C];
-      const float gt = GATED && PASS == 1 ? qrow[2 * Dp + cols] : g;              // a_t
-      const unsigned long long gg = la_pair(gt, gt);
+    if constexpr (C == 1) {
+      auto one_token = [&](int tt) {
+        const float* qrow = buf + tt * tok_len;
+        const float* krow = qrow + Dp;
+        float v = (PASS == 1 && col_live) ? qrow[2 * Dp + warp * 4 + (lane >> 3)] : 0.f;
+        float gt = g;
+        if (GATED && PASS == 1) gt = qrow[2 * Dp + cols], v *= qrow[2 * Dp + cols + 1];      // a_t; b_t rides on v
+        float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f, acc3 = 0.f;
 #pragma unroll
-      for (int c = 0; c < C; ++c) {
-        float v = (PASS == 1 && col + c < Dv) ? qrow[2 * Dp + cw + c] : 0.f;
-        if (GATED && PASS == 1) v *= qrow[2 * Dp + cols + 1];                       // b_t rides on v
-        vv[c] = la_pair(v, v);
-        acc01[c] = acc23[c] = 0ull;
-      }
-#pragma unroll
-      for (int i4 = 0; i4 < DPT / 4; ++i4) {
-        const int d = 4 * (r + 8 * i4);
-        if (d < Dp) {
-          const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(qrow + d);
-          if (PASS == 1) {
-            const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(krow + d);
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-              la_fma2(s2[c][2 * i4], gg, s2[c][2 * i4], la_mul2(k4.x, vv[c]));
-              la_fma2(s2[c][2 * i4 + 1], gg, s2[c][2 * i4 + 1], la_mul2(k4.y, vv[c]));
+        for (int i4 = 0; i4 < DPT / 4; ++i4) {
+          const int d = 4 * (r + 8 * i4);
+          if (d < Dp) {
+            const float4 q4 = *reinterpret_cast<const float4*>(qrow + d);
+            float* s4 = s_reg + 4 * i4;
+            if (PASS == 1) {
+              const float4 k4 = *reinterpret_cast<const float4*>(krow + d);
+              s4[0] = fmaf(gt, s4[0], k4.x * v);
+              s4[1] = fmaf(gt, s4[1], k4.y * v);
+              s4[2] = fmaf(gt, s4[2], k4.z * v);
+              s4[3] = fmaf(gt, s4[3], k4.w * v);
             }
-          }
-#pragma unroll
-          for (int c = 0; c < C; ++c) {
-            la_fma2(acc01[c], s2[c][2 * i4], q4.x, acc01[c]);
-            la_fma2(acc23[c], s2[c][2 * i4 + 1], q4.y, acc23[c]);
+            acc0 = fmaf(s4[0], q4.x, acc0);
+            acc1 = fmaf(s4[1], q4.y, acc1);
+            acc2 = fmaf(s4[2], q4.z, acc2);
+            acc3 = fmaf(s4[3], q4.w, acc3);
           }
         }
-      }
-#pragma unroll
-      for (int c = 0; c < C; ++c) share[c] = (la_lo(acc01[c]) + la_hi(acc01[c])) + (la_lo(acc23[c]) + la_hi(acc23[c]));
-    };
-    float* out_chunk = out_col + (size_t)base * out_stride;
-    // what token tt's sum is worth (PASS 2: added to what the first pass left there)
-    auto result = [&](int tt, float acc, float before, float pow) {
-      if (PASS == 1) return acc;
-      return GATED ? before + buf[tt * tok_len + 2 * Dp + cols + 3] * acc : before + pow * acc;
-    };
-    if (n_tok == LA_CHUNK) {
-      static_assert(LA_CHUNK == 8, "a token for each of a column's lanes");
-      float part[LA_CHUNK][C], before[C], pow = 0.f;
-      float* mine = out_chunk + (size_t)r * out_stride;        // lane r finishes token r
-#pragma unroll
-      for (int c = 0; c < C; ++c) before[c] = (PASS == 2 && col + c < Dv) ? __ldcg(mine + c) : 0.f;
-#pragma unroll
-      for (int tt = 0; tt < LA_CHUNK; ++tt) one_token(tt, part[tt]);
-      if (PASS == 2 && !GATED) {
-#pragma unroll
-        for (int tt = 0; tt < LA_CHUNK; ++tt) {
-          if (tt == r) pow = g_pow;
+        return (acc0 + acc1) + (acc2 + acc3);
+      };
+      const bool writer = r == 0 && col_live;
+      float* out_chunk = out_col + (size_t)base * out_stride;
+      auto out_at = [&](int tt) { return out_chunk + (size_t)tt * out_stride; };
+      auto finish = [&](int tt, float acc, float before) {       // before: PASS 2, what the first pass left there
+        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+        if (PASS == 1) {
+          if (writer) *out_at(tt) = acc;
+        } else if (GATED) {
+          if (writer) *out_at(tt) = before + buf[tt * tok_len + 2 * Dp + cols + 3] * acc;
+        } else {
+          if (writer) *out_at(tt) = before + g_pow * acc;
           g_pow *= g;
         }
-      }
-      // lanes r and r ^ 1 add their shares and keep every other token, then r ^ 2, then r ^ 4
+      };
+      if (n_tok == LA_CHUNK) {
+        float part[LA_CHUNK], before[LA_CHUNK];
+        if (PASS == 2) {                       // the chunk's outputs of the first pass, fetched together
 #pragma unroll
-      for (int c = 0; c < C; ++c) {
-        float a4[4], a2[2];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {               // tokens 2 j (even lanes) and 2 j + 1 (odd lanes)
-          const float give = (r & 1) ? part[2 * j][c] : part[2 * j + 1][c], keep = (r & 1) ? part[2 * j + 1][c] : part[2 * j][c];
-          a4[j] = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+          for (int tt = 0; tt < LA_CHUNK; ++tt) before[tt] = writer ? __ldcg(out_at(tt)) : 0.f;
         }
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const float give = (r & 2) ? a4[2 * j] : a4[2 * j + 1], keep = (r & 2) ? a4[2 * j + 1] : a4[2 * j];
-          a2[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+        for (int tt = 0; tt < LA_CHUNK; ++tt) part[tt] = one_token(tt);
+#pragma unroll
+        for (int tt = 0; tt < LA_CHUNK; ++tt) finish(tt, part[tt], PASS == 2 ? before[tt] : 0.f);
+      } else {
+        for (int tt = 0; tt < n_tok; ++tt) {
+          const float before = (PASS == 2 && writer) ? __ldcg(out_at(tt)) : 0.f;
+          finish(tt, one_token(tt), before);
         }
-        const float give = (r & 4) ? a2[0] : a2[1], keep = (r & 4) ? a2[1] : a2[0];
-        const float acc = keep + __shfl_xor_sync(0xffffffffu, give, 4);
-        if (col + c < Dv) mine[c] = result(r, acc, before[c], pow);
       }
     } else {
-      for (int tt = 0; tt < n_tok; ++tt) {
-        float* at = out_chunk + (size_t)tt * out_stride;
-        float share[C];
-        one_token(tt, share);
+      auto one_token = [&](int tt, float (&share)[C]) {
+        const float* qrow = buf + tt * tok_len;
+        const float* krow = qrow + Dp;
+        unsigned long long vv[C], acc01[C], acc23[C];
+        const float gt = GATED && PASS == 1 ? qrow[2 * Dp + cols] : g;              // a_t
+        const unsigned long long gg = la_pair(gt, gt);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-          const bool writer = r == 0 && col + c < Dv;
-          const float before = (PASS == 2 && writer) ? __ldcg(at + c) : 0.f;
-          float acc = share[c];
-          acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-          acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-          acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-          if (writer) at[c] = result(tt, acc, before, g_pow);
+          float v = (PASS == 1 && col + c < Dv) ? qrow[2 * Dp + cw + c] : 0.f;
+          if (GATED && PASS == 1) v *= qrow[2 * Dp + cols + 1];                       // b_t rides on v
+          vv[c] = la_pair(v, v);
+          acc01[c] = acc23[c] = 0ull;
         }
-        if (PASS == 2 && !GATED) g_pow *= g;
+#pragma unroll
+        for (int i4 = 0; i4 < DPT / 4; ++i4) {
+          const int d = 4 * (r + 8 * i4);
+          if (d < Dp) {
+            const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(qrow + d);
+            if (PASS == 1) {
+              const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(krow + d);
+#pragma unroll
+              for (int c = 0; c < C; ++c) {
+                la_fma2(s2[c][2 * i4], gg, s2[c][2 * i4], la_mul2(k4.x, vv[c]));
+                la_fma2(s2[c][2 * i4 + 1], gg, s2[c][2 * i4 + 1], la_mul2(k4.y, vv[c]));
+              }
+            }
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+              la_fma2(acc01[c], s2[c][2 * i4], q4.x, acc01[c]);
+              la_fma2(acc23[c], s2[c][2 * i4 + 1], q4.y, acc23[c]);
+            }
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c) share[c] = (la_lo(acc01[c]) + la_hi(acc01[c])) + (la_lo(acc23[c]) + la_hi(acc23[c]));
+      };
+      float* out_chunk = out_col + (size_t)base * out_stride;
+      // what token tt's sum is worth (PASS 2: added to what the first pass left there)
+      auto result = [&](int tt, float acc, float before, float pow) {
+        if (PASS == 1) return acc;
+        return GATED ? before + buf[tt * tok_len + 2 * Dp + cols + 3] * acc : before + pow * acc;
+      };
+      if (n_tok == LA_CHUNK) {
+        static_assert(LA_CHUNK == 8, "a token for each of a column's lanes");
+        float part[LA_CHUNK][C], before[C], pow = 0.f;
+        float* mine = out_chunk + (size_t)r * out_stride;        // lane r finishes token r
+#pragma unroll
+        for (int c = 0; c < C; ++c) before[c] = (PASS == 2 && col + c < Dv) ? __ldcg(mine + c) : 0.f;
+#pragma unroll
+        for (int tt = 0; tt < LA_CHUNK; ++tt) one_token(tt, part[tt]);
+        if (PASS == 2 && !GATED) {
+#pragma unroll
+          for (int tt = 0; tt < LA_CHUNK; ++tt) {
+            if (tt == r) pow = g_pow;
+            g_pow *= g;
+          }
+        }
+        // lanes r and r ^ 1 add their shares and keep every other token, then r ^ 2, then r ^ 4
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          float a4[4], a2[2];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {               // tokens 2 j (even lanes) and 2 j + 1 (odd lanes)
+            const float give = (r & 1) ? part[2 * j][c] : part[2 * j + 1][c], keep = (r & 1) ? part[2 * j + 1][c] : part[2 * j][c];
+            a4[j] = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+          }
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const float give = (r & 2) ? a4[2 * j] : a4[2 * j + 1], keep = (r & 2) ? a4[2 * j + 1] : a4[2 * j];
+            a2[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+          }
+          const float give = (r & 4) ? a2[0] : a2[1], keep = (r & 4) ? a2[1] : a2[0];
+          const float acc = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+          if (col + c < Dv) mine[c] = result(r, acc, before[c], pow);
+        }
+      } else {
+        for (int tt = 0; tt < n_tok; ++tt) {
+          float* at = out_chunk + (size_t)tt * out_stride;
+          float share[C];
+          one_token(tt, share);
+#pragma unroll
+          for (int c = 0; c < C; ++c) {
+            const bool writer = r == 0 && col + c < Dv;
+            const float before = (PASS == 2 && writer) ? __ldcg(at + c) : 0.f;
+            float acc = share[c];
+            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+            acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+            acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+            if (writer) at[c] = result(tt, acc, before, g_pow);
+          }
+          if (PASS == 2 && !GATED) g_pow *= g;
+        }
       }
     }
     __syncthreads();                              // the buffer is refilled by the next round's copies
   }
-  auto value = [&](int c, int i) { return (i & 1) ? la_hi(s2[c][i >> 1]) : la_lo(s2[c][i >> 1]); };
+  auto value = [&](int c, int i) {
+    if constexpr (C == 1) return s_reg[i];
+    else return (i & 1) ? la_hi(s2[c][i >> 1]) : la_lo(s2[c][i >> 1]);
+  };
   if (PASS == 1) {
     float* dst = n_seg == 1 ? S : part_seq + (size_t)seg * D * Dv;
 #pragma unroll
@@ -864,9 +952,19 @@ LLMX_API int llmx_decay_scan(const void* proj, int in_dtype, int n_split, long l
     if (e != cudaSuccess) return (int)e;
   }
   const int scan_segs = by_chunks ? 1 : n_seg;
+  // Rule: two columns a thread where they were faster (H = 2 to 16, sizes of 16 to 256, 1 to 4000 tokens a sequence; one
+  // column / two, us): long gated prompts (four of 700 to 1300 tokens: 855 / 657 at 16 heads of 128 x 128, 216 / 196 at
+  // 64 x 64, 566 / 480 at 192 x 96), many prompts of up to a segment with keys of 65 to 128 (eight of 100, gated: 126 / 104),
+  // and small ungated states in prompts up to about 1000 tokens (300 tokens, 32 x 32: 50 / 40; 4000: 82 / 95).  Not short
+  // prompts with larger keys, whose registers halve the CTAs of an SM (100 tokens, 256 x 256, gated: 81 / 110), nor steps of
+  // mostly single tokens (32 of them, 128 x 128, gated: 10 / 16) unless the states are small (31 and a prompt of 200, 32 x 32,
+  // gated: 44 / 35).
+  const bool prompts = !by_chunks && (n_tokens >= 32 * n_seqs || (D <= 32 && n_seg > 1));
+  const bool two = prompts && ((gates && max_new > (D <= 32 ? 128 : D <= 128 ? 256 : 640)) ||
+                               (D > 64 && D <= 128 && n_tokens >= 512 && max_new >= 64 && max_new <= 128) ||
+                               (!gates && D <= 32 && max_new <= 1024));
+  const int C = two ? 2 : 1;
   // columns per CTA: as many as still give every SM a CTA or two (a CTA with more columns stages q and k fewer times)
-  // and two a thread in prompts
-  const int C = max_new >= 2 * LA_CHUNK ? 2 : 1;
   int cols = 32 * C;
   while (cols > 8 * C && (long long)n_seqs * H * scan_segs * ((Dv + cols - 1) / cols) < 2LL * n_sm) cols >>= 1;
   while (cols > 4 * C && cols / 2 >= Dv) cols >>= 1;
@@ -888,12 +986,13 @@ LLMX_API int llmx_decay_scan(const void* proj, int in_dtype, int n_split, long l
                seq_start, seq_slot, decay, gates, (size_t)head_stride, H, D, Dv, cols, col_blocks, seg_len, n_seg,     \
                (int)by_chunks);                                                                                        \
   } while (0)
-#define GO1(DPT, PASS)              \
-  do {                              \
-    if (gates && C == 2) GO2(DPT, PASS, true, 2);       \
-    else if (gates) GO2(DPT, PASS, true, 1);            \
-    else if (C == 2) GO2(DPT, PASS, false, 2);          \
-    else GO2(DPT, PASS, false, 1);                      \
+// (the instances that the rule reaches)
+#define GO1(DPT, PASS)                                                                       \
+  do {                                                                                       \
+    if (gates && C == 2) GO2(DPT, PASS, true, 2);                                            \
+    else if (gates) GO2(DPT, PASS, true, 1);                                                 \
+    else if (C == 2) GO2(DPT, PASS, false, (DPT == 4 || (DPT == 16 && PASS == 1) ? 2 : 1));  \
+    else GO2(DPT, PASS, false, 1);                                                           \
   } while (0)
 #define GO(DPT)                    \
   do {                             \

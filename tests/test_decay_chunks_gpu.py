@@ -67,3 +67,75 @@ def test_a_value_that_is_not_finite_changes_no_token_before_it(at, bad):
     lost = torch.zeros(H, D, Dv, dtype=torch.bool, device=DEV)
     lost[0, :, 3] = True
     assert torch.equal(~torch.isfinite(state[0]), lost)
+
+
+def recurrence(proj, lens, slots, state, a, b, H, D, Dv, ones):
+    """Token by token in 64 bits; a, b: [T, H]."""
+    outs, t0 = [], 0
+    after = state.double()
+    for n, slot in zip(lens, slots):
+        p = proj[t0 : t0 + n].double()
+        q, k, v = p[:, : H * D].view(n, H, D), p[:, H * D : 2 * H * D].view(n, H, D), p[:, 2 * H * D : 2 * H * D + H * Dv].view(n, H, Dv)
+        if ones:
+            v = torch.cat([v, torch.ones(n, H, 1, device=DEV, dtype=torch.float64)], 2)
+        S = after[slot].clone()
+        for t in range(n):
+            S = a[t0 + t, :, None, None] * S + b[t0 + t, :, None, None] * k[t, :, :, None] * v[t, :, None, :]
+            outs.append((q[t, :, :, None] * S).sum(1).reshape(-1))
+        after[slot] = S
+        t0 += n
+    return torch.stack(outs), after
+
+
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("H, D, Dv, lens", [
+    (2, 32, 30, [300, 40]), (1, 30, 31, [129, 127, 1]),            # small states: one pass or two of two columns
+    (2, 128, 65, [100] * 6), (1, 66, 40, [128] * 4 + [64]),         # many prompts of up to a segment
+    (1, 64, 33, [257, 300]), (2, 128, 64, [270]),                   # longer than two segments
+    (1, 130, 20, [300]), (1, 256, 16, [140, 3]), (1, 192, 20, [650])])    # keys above 128: one column, two in long prompts
+def test_one_and_two_columns_a_thread(H, D, Dv, lens, gated):
+    """Prompts by two columns a thread against 64 bits, and the same prompts one token a step, which one column takes:
+    up to a segment the same bits.  Tolerance as above (up to 256 multiply-adds a chain: 1e-6)."""
+    from llmoxide_b200 import kernels
+    torch.manual_seed(D + Dv)
+    T, B, slots, dva = sum(lens), len(lens), list(range(len(lens)))[::-1], Dv + int(gated)
+    proj = torch.randn(T, H * (2 * D + Dv), device=DEV)
+    decay = torch.tensor([0.9, 0.999][:H], device=DEV)
+    before = torch.randn(B, H, D, dva, device=DEV)
+    ab = torch.rand(2, T, H, device=DEV) * 0.3 + 0.69 if gated else None
+    seg_of = torch.cat([torch.arange(n) // 128 for n in lens])
+
+    def call(rows, n_of, state, seqs):
+        """``rows`` of every sequence in ``seqs``, n_of tokens each."""
+        starts = torch.tensor([sum(n_of[:i]) for i in range(len(seqs) + 1)], dtype=torch.int32, device=DEV)
+        out = torch.full((len(rows), H * dva), float("nan"), device=DEV)
+        gates = None
+        if gated:
+            gates = torch.empty(len(rows), H, 4, device=DEV)
+            gates[:, :, 0], gates[:, :, 1], gates[:, :, 2] = ab[0, rows], ab[1, rows], 1.0
+            t0 = 0
+            for n in n_of:                                          # the product of a over the token's segment so far
+                for s in range(0, n, 128):
+                    gates[t0 + s : t0 + min(n, s + 128), :, 3] = ab[0, rows][t0 + s : t0 + min(n, s + 128)].cumprod(0)
+                t0 += n
+        kernels.decay_scan(proj[rows], out, state, starts, torch.zeros(len(rows), dtype=torch.int32, device=DEV),
+                           torch.tensor([slots[b] for b in seqs], dtype=torch.int32, device=DEV), None if gated else decay,
+                           None, None, 0, "none", 1.0, H, D, Dv, 0, H * D, 2 * H * D, max_new=max(n_of), gates=gates,
+                           ones_column=gated)
+        return out
+
+    state = before.clone()
+    out = call(torch.arange(T, device=DEV), lens, state, list(range(B)))
+    a = ab[0].double() if gated else decay.double().expand(T, H)
+    b = ab[1].double() if gated else torch.ones(T, H, device=DEV, dtype=torch.float64)
+    want, after = recurrence(proj, lens, slots, before, a, b, H, D, Dv, gated)
+    assert ((out - want).norm() / want.norm()).item() < 1e-6
+    assert ((state - after).norm() / after.norm()).item() < 1e-6
+    if max(lens) <= 128:
+        alone = before.clone()
+        starts = [sum(lens[:b]) for b in range(B)]
+        for t in range(max(lens)):
+            seqs = [b for b in range(B) if t < lens[b]]
+            rows = torch.tensor([starts[b] + t for b in seqs], device=DEV)
+            assert torch.equal(call(rows, [1] * len(seqs), alone, seqs), out[rows])
+        assert torch.equal(alone, state)
