@@ -175,10 +175,12 @@ __device__ __forceinline__ void af_copy_rows(float* dst, int pitch, const float*
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
                        (uint32_t)__cvta_generic_to_shared(dst + r * pitch + c)), "l"(src + r * ld + c) : "memory");
 }
+// What exponentials are taken against: a maximum of -inf stands for scores that are all -inf, whose exponentials are 0.
+__device__ __forceinline__ float af_against(float m) { return m == -INFINITY ? 0.f : m; }
 // A partial result joins a running one: the maximum, and the factors of both.
 __device__ __forceinline__ float af_join(float m, float pm, float& c1, float& c2) {
-  const float mn = fmaxf(m, pm);
-  c1 = expf(m - mn), c2 = expf(pm - mn);
+  const float mn = fmaxf(m, pm), ref = af_against(mn);
+  c1 = expf(m - ref), c2 = expf(pm - ref);
   return mn;
 }
 __device__ __forceinline__ float af_remote(const float* local, unsigned rank) {      // the same word of another CTA of the cluster
@@ -353,7 +355,7 @@ __global__ void __launch_bounds__(AF_THREADS) attention_f32_kernel(const AfArgs 
           pl[i] = 0.f;
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const float e = live[c] ? expf(sv[c] - pm[i]) : -1.f;
+            const float e = live[c] ? expf(sv[c] - af_against(pm[i])) : -1.f;
             if (live[c]) pl[i] = __fadd_rn(pl[i], e);
             Ps[(i * 8 + tm) * PP + tn + 16 * c] = e;
           }

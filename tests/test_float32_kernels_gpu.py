@@ -154,3 +154,27 @@ def test_attention_f32_leaves_out_what_a_row_does_not_see():
         kernels.attention_paged(q, out, k, v, table, seq, pos, H, G, D, None, 0.125)
         outs.append(out)
     assert torch.equal(outs[0][:90], outs[1][:90]) and torch.isnan(outs[1][90:]).all()
+
+
+def test_attention_f32_tiles_whose_scores_are_all_minus_infinity():
+    """A bias of -inf at short distances: the newest tiles of a row hold no finite score, the older ones do."""
+    from llmoxide_b200 import kernels
+    H, G, D, L, near = 4, 2, 64, 300, 90
+    torch.manual_seed(3)
+    k, v = torch.randn(5, G, 64, D, device=DEV), torch.randn(5, G, 64, D, device=DEV)
+    table, q = torch.arange(5, dtype=torch.int32, device=DEV)[None], torch.randn(L, H * D, device=DEV)
+    seq, pos = torch.zeros(L, dtype=torch.int32, device=DEV), torch.arange(L, dtype=torch.int32, device=DEV)
+    bias = torch.randn(H, 128, device=DEV)
+    bias[:, :near] = -math.inf
+    K, V = (z.transpose(1, 2).reshape(-1, G, D)[:L].double() for z in (k, v))
+    i, j = torch.arange(L, device=DEV)[:, None], torch.arange(L, device=DEV)[None]
+    want = []
+    for h in range(H):
+        s = q.view(L, H, D)[:, h].double() @ K[:, h * G // H].T * 0.125 + bias[h].double()[(i - j).clamp(0, 127)]
+        want.append(torch.softmax(s.masked_fill(j > i, -math.inf), 1) @ V[:, h * G // H])
+    want = torch.stack(want, 1).reshape(L, H * D)
+    for single in (False, True):
+        out = torch.empty(L, H * D, device=DEV)
+        kernels.attention_paged(q, out, k, v, table, seq, pos, H, G, D, None, 0.125, score_bias=bias, single_tokens=single)
+        assert torch.isnan(out[:near]).all()                  # no finite score at all
+        assert rel(out[near:], want[near:]) < 2e-6
