@@ -137,13 +137,12 @@ __global__ void attention_paged_kernel(const TA* __restrict__ q, TA* __restrict_
 // butterfly over 16 lanes) and the weighted values key by key.  The tiles' (maximum, sum, values) then join a running
 // state in the order of the tiles.  That order depends on the query's position and mask alone, and both forms below
 // follow it step by step, so a position's result does not depend on how tokens were cut into steps or batched.
-//   prompts (SPLIT false)   a CTA owns 8 TR query rows (tokens x the heads that share a kv head) and walks the tiles
-//   few tokens (SPLIT true) a cluster of 8 CTAs owns one token's rows; CTA r takes tiles r, r + 8, ..., and after every
-//                           round of 8 tiles each CTA joins a slice of the dims out of the eight partial results
+//   SPLIT false   a CTA owns 8 TR query rows (tokens of one sequence x the heads that share a kv head) and walks the tiles
+//   SPLIT true    a cluster of 8 CTAs owns 8 such rows; CTA r takes tiles r, r + 8, ..., and after every round of 8 tiles
+//                 each CTA joins a slice of the dims out of the eight partial results
 // A key that a row must not see is left out, not multiplied by zero (its value may be anything).
-// 16 heads of 128 over 4 kv heads, a window of 1024: three prompts of 517, 323 and 130 tokens 235 us (the kernel above:
-// 2060), one more token each 27 us (656).  A few tokens are bound by the latency of a round of tiles (copy, scores,
-// values, join, one after the other), prompts by the shared-memory reads.
+// A few tokens are bound by the latency of a round of tiles (copy, scores, values, join, one after the other), prompts by
+// the shared-memory reads; measurements at the rule below.
 // ---------------------------------------------------------------------------
 #define AF_KEYS 64             // keys per tile = LLMX_PAGE
 #define AF_THREADS 128         // 8 (rows) x 16 (keys, then dims)
@@ -153,10 +152,12 @@ static_assert(AF_KEYS == LLMX_PAGE, "a tile is a page");
 struct AfArgs {
   const float *q, *k_cache, *v_cache, *gate, *sinks, *score_bias;
   float* out;
-  const int *block_table, *token_seq, *token_pos;
+  const int *block_table, *token_seq, *token_pos, *seq_start;
   size_t q_stride, gate_stride;
+  int n_seqs;
   int table_width, n_tokens, H, G, D, Dv, window, keep_first, chunk, bias_len;
   int heads_per_cta, tokens_per_cta, head_blocks;
+  bool q_vec;                    // rows of q are whole 16-byte pieces
   float scale, sink, softcap;
 };
 
@@ -223,29 +224,59 @@ __global__ void __launch_bounds__(AF_THREADS) attention_f32_kernel(const AfArgs 
   const int tn = lane & 15, tm = warp * 2 + (lane >> 4);     // a row's 16 threads are half a warp
   const int rank = SPLIT ? (int)(blockIdx.x % AF_SPLIT) : 0;
   const int R = a.H / a.G, g = blockIdx.y / a.head_blocks, h0 = (blockIdx.y % a.head_blocks) * a.heads_per_cta;
-  // prompts: the last tokens, which see most keys, start first
-  const int t0 = SPLIT ? (int)(blockIdx.x / AF_SPLIT) : ((int)gridDim.x - 1 - (int)blockIdx.x) * a.tokens_per_cta;
-  const int n_tok = SPLIT ? 1 : min(a.tokens_per_cta, a.n_tokens - t0);
+  // this CTA's tokens (prompts: the last ones, which see most keys, start first)
+  const int slot = SPLIT ? (int)(blockIdx.x / AF_SPLIT) : (int)gridDim.x - 1 - (int)blockIdx.x, per = a.tokens_per_cta;
+  int t0 = slot * per, n_tok = min(per, a.n_tokens - t0);
+  if (a.seq_start) {                       // of one sequence: its slots start at seq_start / per + its number
+    int b = 0;
+    for (int hi = a.n_seqs - 1; b < hi;) {
+      const int mid = (b + hi + 1) >> 1;
+      if (a.seq_start[mid] / per + mid <= slot) b = mid; else hi = mid - 1;
+    }
+    const int row0 = a.seq_start[b], row1 = min(a.seq_start[b + 1], a.n_tokens);
+    t0 = row0 + (slot - (row0 / per + b)) * per;
+    n_tok = min(per, row1 - t0);
+  }
+  // Without seq_start neighbouring tokens may be different sequences'; the z-th of gridDim.z CTAs takes every gridDim.z-th
+  // run of tokens of one sequence.
+  auto new_run = [&](int tok) { return a.token_seq[t0 + tok] != a.token_seq[t0 + tok - 1]; };
+  if (gridDim.z > 1) {
+    int n_runs = 1;
+    for (int i = 1; i < n_tok; ++i) n_runs += new_run(i);
+    if ((int)blockIdx.z >= n_runs) return;
+  }
+  if (n_tok <= 0) return;                  // (uniform over a cluster, as is the return above)
 
   for (int r = threadIdx.x; r < BR; r += AF_THREADS) {
     const int tok = r / a.heads_per_cta, h = h0 + r % a.heads_per_cta;
-    const bool here = tok < n_tok && h < R;
+    bool here = tok < n_tok && h < R;
+    if (here && gridDim.z > 1) {
+      int run = 0;
+      for (int i = 1; i <= tok; ++i) run += new_run(i);
+      here = run % (int)gridDim.z == (int)blockIdx.z;
+    }
     const int p = here ? a.token_pos[t0 + tok] : 0;
     int first = (a.window > 0 && p - (a.window - 1) > 0) ? p - (a.window - 1) : 0;
     if (a.chunk > 0) first = max(first, p - p % a.chunk);
     row_pos[r] = p, row_first[r] = first, row_seq[r] = here ? a.token_seq[t0 + tok] : -1;
   }
-  for (int i = threadIdx.x; i < AF_KEYS * VP; i += AF_THREADS) Vs[i] = 0.f;       // (dims past Dv)
-  for (int r = 0; r < BR; ++r) {
+  if (Dv < VP)                             // dims past Dv
+    for (int i = threadIdx.x; i < AF_KEYS * VP; i += AF_THREADS) Vs[i] = 0.f;
+  __syncthreads();
+  for (int r = warp; r < BR; r += AF_THREADS / 32) {
     const int tok = r / a.heads_per_cta, h = h0 + r % a.heads_per_cta;
-    if (tok >= n_tok || h >= R) {
-      for (int i = threadIdx.x; i < D; i += AF_THREADS) Qs[r * DP + i] = 0.f;
+    float* dst = Qs + r * DP;
+    const float* src = a.q + (size_t)(t0 + tok) * a.q_stride + (size_t)(g * R + h) * D;
+    if (row_seq[r] < 0) {
+      for (int i = lane; i < D; i += 32) dst[i] = 0.f;
+    } else if (a.q_vec) {                  // (they come with the first tile of keys)
+      for (int c = lane * 4; c < D; c += 128)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + c)), "l"(src + c)
+                     : "memory");
     } else {
-      const float* src = a.q + (size_t)(t0 + tok) * a.q_stride + (size_t)(g * R + h) * D;
-      for (int i = threadIdx.x; i < D; i += AF_THREADS) Qs[r * DP + i] = src[i];
+      for (int i = lane; i < D; i += 32) dst[i] = src[i];
     }
   }
-  __syncthreads();
 
   int pos[TR], first[TR], seq[TR];
   float m[TR], l[TR];
@@ -265,8 +296,13 @@ __global__ void __launch_bounds__(AF_THREADS) attention_f32_kernel(const AfArgs 
   for (int e = 0; e < OWN; ++e) om[e] = -INFINITY, ol[e] = 0.f, oa[e] = 0.f;
 
   // tokens of one sequence that follow one another share its tiles
+  int parity = 0;                               // SPLIT: of the rounds so far
   for (int run = 0; run < n_tok;) {
     const int s = row_seq[run * a.heads_per_cta];
+    if (s < 0) {                                // (another CTA's)
+      ++run;
+      continue;
+    }
     int lo = row_first[run * a.heads_per_cta], hi = row_pos[run * a.heads_per_cta], end = run + 1;
     for (; end < n_tok && row_seq[end * a.heads_per_cta] == s; ++end) {
       lo = min(lo, row_first[end * a.heads_per_cta]);
@@ -298,7 +334,7 @@ __global__ void __launch_bounds__(AF_THREADS) attention_f32_kernel(const AfArgs 
     constexpr int STEP = SPLIT ? AF_SPLIT : 1;
     __syncthreads();                            // (a run before is done with K and V)
     load_k(rank), load_v(rank);
-    for (int j = rank, round = 0; j - rank < n_tiles; j += STEP, ++round) {
+    for (int j = rank, round = 0; j - rank < n_tiles; j += STEP, ++round, parity ^= 1) {
       unsigned long long pacc[TR][2 * NC];
       float pm[TR], pl[TR];
       bool any[TR];
@@ -407,7 +443,7 @@ __global__ void __launch_bounds__(AF_THREADS) attention_f32_kernel(const AfArgs 
                                 __fmaf_rn(af_hi(pacc[i][c]), c2, __fmul_rn(af_hi(acc[i][c]), c1)));
         }
       } else {
-        float* mine_part = part + ((size_t)(round & 1) * 8 + tm) * PART;
+        float* mine_part = part + ((size_t)parity * 8 + tm) * PART;
         if (j < n_tiles) {
           if (tn == 0) mine_part[0] = pm[0], mine_part[1] = any[0] ? pl[0] : -1.f;
 #pragma unroll
@@ -422,7 +458,7 @@ __global__ void __launch_bounds__(AF_THREADS) attention_f32_kernel(const AfArgs 
         for (int e = 0; e < OWN; ++e) {
           const int idx = e * AF_THREADS + threadIdx.x, row = idx / slice, d = rank * slice + idx % slice;
           if (row >= 8 || d >= Dv) continue;
-          const float* src = part + ((size_t)(round & 1) * 8 + row) * PART;
+          const float* src = part + ((size_t)parity * 8 + row) * PART;
           for (int k = 0; k < here; ++k) {
             const float km = af_remote(src, k), kl = af_remote(src + 1, k), ka = af_remote(src + 2 + d, k);
             if (kl < 0.f) continue;
@@ -450,8 +486,8 @@ __global__ void __launch_bounds__(AF_THREADS) attention_f32_kernel(const AfArgs 
     for (int e = 0; e < OWN; ++e) {
       const int idx = e * AF_THREADS + threadIdx.x, row = idx / slice, d = rank * slice + idx % slice;
       if (row >= 8 || d >= Dv || row_seq[row] < 0) continue;
-      const int h = g * R + h0 + row;
-      a.out[((size_t)t0 * a.H + h) * Dv + d] = __fmul_rn(oa[e], inverse(om[e], ol[e], t0, h));
+      const int tok = t0 + row / a.heads_per_cta, h = g * R + h0 + row % a.heads_per_cta;
+      a.out[((size_t)tok * a.H + h) * Dv + d] = __fmul_rn(oa[e], inverse(om[e], ol[e], tok, h));
     }
     af_cluster_sync();                          // nobody leaves while its partial results may be read
   } else {
@@ -473,11 +509,15 @@ __global__ void __launch_bounds__(AF_THREADS) attention_f32_kernel(const AfArgs 
 }
 
 template <int TR, int NC, bool SPLIT>
-static int launch_f32(AfArgs a, cudaStream_t stream) {
+static int launch_f32(AfArgs a, bool single_tokens, cudaStream_t stream) {
   const int R = a.H / a.G, rows = 8 * TR;
   a.heads_per_cta = R < rows ? R : rows;
-  a.tokens_per_cta = SPLIT ? 1 : rows / a.heads_per_cta;
+  a.tokens_per_cta = single_tokens ? 1 : rows / a.heads_per_cta;
   a.head_blocks = (R + a.heads_per_cta - 1) / a.heads_per_cta;
+  if (a.tokens_per_cta == 1) a.seq_start = nullptr;             // (a token is a run by itself)
+  const unsigned slots = a.seq_start ? a.n_tokens / a.tokens_per_cta + a.n_seqs
+                                     : (a.n_tokens + a.tokens_per_cta - 1) / a.tokens_per_cta;
+  const unsigned runs = a.seq_start || a.tokens_per_cta == 1 ? 1 : a.tokens_per_cta < 8 ? a.tokens_per_cta : 8;
   auto kernel = attention_f32_kernel<TR, NC, SPLIT>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -487,20 +527,42 @@ static int launch_f32(AfArgs a, cudaStream_t stream) {
     attr_set = true;
   }
   const size_t smem = af_smem<TR, NC>(a.D, SPLIT);
+  const dim3 grid(slots * (SPLIT ? AF_SPLIT : 1), a.G * a.head_blocks, runs);
   if (SPLIT)
-    launch_pdl_cluster(kernel, dim3((unsigned)a.n_tokens * AF_SPLIT, a.G * a.head_blocks), dim3(AF_THREADS), smem, stream,
-                       AF_SPLIT, a);
+    launch_pdl_cluster(kernel, grid, dim3(AF_THREADS), smem, stream, AF_SPLIT, a);
   else
-    launch_pdl(kernel, dim3((a.n_tokens + a.tokens_per_cta - 1) / a.tokens_per_cta, a.G * a.head_blocks), dim3(AF_THREADS),
-               smem, stream, a);
+    launch_pdl(kernel, grid, dim3(AF_THREADS), smem, stream, a);
   return LLMX_LAUNCH_STATUS();
 }
 
-// Rule: a step of single tokens (each of a sequence of its own), or one of so few tokens that tiles of rows would leave
-// most SMs idle, gives every token a cluster; other steps share tiles among rows.
-static int attention_f32(const AfArgs& a, bool single_tokens, cudaStream_t stream) {
-  const bool split = single_tokens || a.n_tokens <= 32;
-#define GO(NC) return split ? launch_f32<1, NC, true>(a, stream) : launch_f32<4, NC, false>(a, stream)
+// launch: 0: rows of 8 in a cluster, 1: rows of 8, 2: rows of 32, -1: by the rule.
+// Rule: the cheapest by what 90 steps took (heads of 64, 128 and 256, 1 to 8 rows and more a kv head, single tokens, prompts,
+// portions of prompts and mixtures, depths of 17 to 4096).  The unit is what a CTA of 8 rows takes for a tile with an SM to
+// itself (5.6, 7.8 and 10.8 us by head size), a cluster's round costs 1.55 of it and a tile of 32 rows 1.75; where CTAs
+// share the SMs, a CTA-tile costs an SM what the table says.  us by cluster / 8 rows / 32 rows (heads of 128): one
+// token at depth 4096, 16 heads over 4: 97 / 502 / 849; 64 tokens at depth 300, 16 over 16: 486 / 165 / 327; three prompts
+// of 500, 16 over 4: 1575 / 376 / 262; 40 tokens at depth 2048 beside a prompt of 64, 16 over 16: 1273 / 667 / 1425.  The
+// kernel above takes 2655, 458, 3353 and 2981.
+static int attention_f32(const AfArgs& a, bool single_tokens, int launch, cudaStream_t stream) {
+  if (launch < 0) {
+    static const double share[3][3] = {{0.45, 0.38, 1.07}, {0.97, 0.55, 1.45}, {1.93, 1.2, 3.1}};     // [head size][launch]
+    const int size = a.D > a.Dv ? a.D : a.Dv, R = a.H / a.G;
+    const double* cost = share[size <= 64 ? 0 : size <= 128 ? 1 : 2];
+    double tiles = a.table_width;
+    if (a.window > 0) tiles = fmin(tiles, (a.window + a.keep_first) / AF_KEYS + 2.0);
+    const auto per_sm = [&](int rows) {                     // CTAs of that many rows
+      const int heads = R < rows ? R : rows, tokens = single_tokens ? 1 : rows / heads;
+      const double slots = a.n_tokens / tokens + (a.seq_start && tokens > 1 ? a.n_seqs : 0);
+      return fmax(slots, 1.0) * a.G * ((R + heads - 1) / heads) / llmx_sm_count();
+    };
+    const double by_cluster = 0.85 * ceil(tiles / AF_SPLIT) * fmax(1.55, per_sm(8) * AF_SPLIT * cost[0]);
+    const double by_8 = tiles * fmax(1.0, per_sm(8) * cost[1]), by_32 = tiles * fmax(1.75, per_sm(32) * cost[2]);
+    launch = by_cluster < by_8 && by_cluster < by_32 ? 0 : by_8 <= by_32 ? 1 : 2;
+  }
+#define GO(NC)                                                                  \
+  return launch == 0   ? launch_f32<1, NC, true>(a, single_tokens, stream)      \
+         : launch == 1 ? launch_f32<1, NC, false>(a, single_tokens, stream)     \
+                       : launch_f32<4, NC, false>(a, single_tokens, stream)
   switch ((a.Dv + 63) / 64) {
     case 1: GO(1);
     case 2: GO(2);
@@ -514,15 +576,18 @@ static int attention_f32(const AfArgs& a, bool single_tokens, cudaStream_t strea
 // pool_table (as wide as block_table); needs a window and no kept first keys.  gate: null, or float32 with
 // gate[t * gate_stride + head] the logit of head's output gate.
 // softcap <= 0: scores are not capped; sinks: null, or float32 [H]; score_bias: null, or float32 [H, bias_len].
-// single_tokens: every token is a sequence's only one in this step (a hint: it picks the launch, not the result).
+// Hints, which pick the launch and not the result: single_tokens: every token is a sequence's only one in this step;
+// seq_start: null, or [n_seqs + 1]: the tokens lie sequence after sequence from there; launch: see attention_f32.
 LLMX_API int llmx_attention_paged_biased(const void* q, void* out, int act_dtype, const void* k_cache,
                                   const void* v_cache, int cache_dtype, const int* block_table, int table_width,
                                   const int* token_seq, const int* token_pos, int n_tokens, int H, int G, int D,
                                   int Dv, long long q_stride, int window, int keep_first, float scale, float sink,
                                   int chunk, int pool, const void* pool_k, const void* pool_v, const int* pool_table,
                                   const float* gate, long long gate_stride, float softcap, const float* sinks,
-                                  const float* score_bias, int bias_len, int single_tokens, cudaStream_t stream) {
+                                  const float* score_bias, int bias_len, int single_tokens, const int* seq_start,
+                                  int n_seqs, int launch, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
+  if (launch > 2 || (seq_start && n_seqs <= 0)) return LLMX_REFUSED(1);
   if (score_bias && (bias_len <= 0 || pool > 0 || softcap > 0.f)) return LLMX_REFUSED(1);
   if (chunk < 0 || (chunk > 0 && keep_first > 0)) return LLMX_REFUSED(1);
   if (pool < 0 || (pool > 0 && (window <= 0 || keep_first > 0 || chunk > 0 || !pool_k || !pool_v || !pool_table)))
@@ -540,7 +605,8 @@ LLMX_API int llmx_attention_paged_biased(const void* q, void* out, int act_dtype
     a.token_seq = token_seq, a.token_pos = token_pos, a.q_stride = (size_t)q_stride, a.gate_stride = (size_t)gate_stride;
     a.table_width = table_width, a.n_tokens = n_tokens, a.H = H, a.G = G, a.D = D, a.Dv = Dv, a.window = window;
     a.keep_first = keep_first, a.chunk = chunk, a.bias_len = bias_len, a.scale = scale, a.sink = sink, a.softcap = softcap;
-    return attention_f32(a, single_tokens != 0, stream);
+    a.seq_start = seq_start, a.n_seqs = n_seqs, a.q_vec = aligned(q) && q_stride % 4 == 0;
+    return attention_f32(a, single_tokens != 0, launch, stream);
   }
   dim3 grid(n_tokens, (H + ATT_WARPS - 1) / ATT_WARPS);
   const size_t smem = (size_t)ATT_WARPS * D * sizeof(float);
@@ -568,7 +634,7 @@ LLMX_API int llmx_attention_paged_capped(const void* q, void* out, int act_dtype
   return llmx_attention_paged_biased(q, out, act_dtype, k_cache, v_cache, cache_dtype, block_table, table_width,
                                      token_seq, token_pos, n_tokens, H, G, D, Dv, q_stride, window, keep_first, scale,
                                      sink, chunk, pool, pool_k, pool_v, pool_table, gate, gate_stride, softcap, sinks,
-                                     nullptr, 0, 0, stream);
+                                     nullptr, 0, 0, nullptr, 0, -1, stream);
 }
 
 LLMX_API int llmx_attention_paged_pooled(const void* q, void* out, int act_dtype, const void* k_cache,

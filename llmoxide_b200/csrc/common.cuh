@@ -185,6 +185,19 @@ extern "C" __attribute__((visibility("default"))) int llmx_touch() {
 }
 #endif
 
+// SMs of the current device at the first call.
+static inline int llmx_sm_count() {
+  static int n = 0;
+  if (n == 0) {
+    int dev = 0, found = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&found, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || found <= 0)
+      found = 148;
+    n = found;
+  }
+  return n;
+}
+
 // Tokens per cache page.  A sequence's position p lives in its logical page
 // p / PAGE at row p % PAGE; the block table maps logical to physical pages.
 #define LLMX_PAGE 64

@@ -640,7 +640,8 @@ def _score_bias_args(score_bias) -> tuple:
 def attention_paged(q, out, k_cache, v_cache, block_table, token_seq, token_pos, n_heads: int,
                     n_kv_heads: int, head_dim: int, window, scale: float, v_head_dim=None, keep_first: int = 0,
                     sink: float = 0.0, chunk: int = 0, pool: int = 0, pool_k=None, pool_v=None, pool_table=None,
-                    gate=None, softcap: float = 0.0, sinks=None, score_bias=None, single_tokens: bool = False) -> None:
+                    gate=None, softcap: float = 0.0, sinks=None, score_bias=None, single_tokens: bool = False,
+                    seq_start=None, launch: int = -1) -> None:
     """General attention over the paged cache; q [T,H*D] (rows may be the first columns of wider rows), out
     [T,H*Dv].  Under a window the first ``keep_first`` keys of a sequence stay visible.  ``sink`` is added to the
     softmax's denominator (as many keys of score 0 that have no value).  With ``chunk`` n > 0 a query sees only the
@@ -650,9 +651,11 @@ def attention_paged(q, out, k_cache, v_cache, block_table, token_seq, token_pos,
     head h's output is multiplied by sigmoid(gate[t, h]).  ``softcap`` c > 0: every scaled score s becomes
     c * tanh(s / c).  ``sinks`` float32 [H]: exp(sinks[h]) joins head h's denominator (no key, no value, not capped).
     ``score_bias`` float32 [H, n]: score_bias[h, min(p - j, n - 1)] joins the scaled score of the key at j (the last entry
-    stands for every longer distance; not beside pooled blocks or a cap).  ``single_tokens``: no sequence brings two of the
-    tokens (a hint; results are the same without it)."""
-    _dev(q, out, k_cache, v_cache, block_table, token_seq, token_pos, pool_k, pool_v, pool_table, gate, sinks, score_bias)
+    stands for every longer distance; not beside pooled blocks or a cap).  Hints, with
+    which results are the same: ``single_tokens``: no sequence brings two of the tokens; ``seq_start`` int32 [sequences + 1]:
+    the tokens lie sequence after sequence from there.  ``launch`` (tests): a launch of the float32 tiles by number."""
+    _dev(q, out, k_cache, v_cache, block_table, token_seq, token_pos, pool_k, pool_v, pool_table, gate, sinks, score_bias,
+         seq_start)
     _check_score_bias(score_bias, n_heads)
     _check_sinks(sinks, n_heads)
     _contig("out", out), _contig("block_table", block_table)
@@ -667,16 +670,19 @@ def attention_paged(q, out, k_cache, v_cache, block_table, token_seq, token_pos,
         raise Unsupported(f"head_dim {head_dim}/{v_head_dim}: the general attention kernel takes sizes up to 256")
     if n_heads % n_kv_heads:
         raise Unsupported(f"{n_heads} heads are not a multiple of {n_kv_heads} kv heads")
+    assert seq_start is None or (seq_start.dtype == torch.int32 and seq_start.is_contiguous() and seq_start.numel() >= 2)
     f = _fn("attention", "llmx_attention_paged_biased",
             [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,
              c_int, c_int, c_int, c_int, c_int, c_longlong, c_int, c_int, c_float, c_float, c_int, c_int, c_void_p,
-             c_void_p, c_void_p, c_void_p, c_longlong, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p])
+             c_void_p, c_void_p, c_void_p, c_longlong, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
+             c_void_p])
     _check(f(_ptr(q), _ptr(out), _tag(q), _ptr(k_cache), _ptr(v_cache), _tag(k_cache), _ptr(block_table),
              block_table.shape[1], _ptr(token_seq), _ptr(token_pos), q.shape[0], n_heads, n_kv_heads, head_dim,
              v_head_dim, q.stride(0), int(window or 0), int(keep_first or 0), scale, float(sink or 0.0), int(chunk or 0),
              int(pool or 0), _ptr(pool_k), _ptr(pool_v), _ptr(pool_table), _ptr(gate),
              gate.stride(0) if gate is not None else 0, float(softcap or 0.0), _ptr(sinks), *_score_bias_args(score_bias),
-             int(single_tokens), _stream()), "attention_paged")
+             int(single_tokens), _ptr(seq_start), 0 if seq_start is None else seq_start.numel() - 1, launch, _stream()),
+           "attention_paged")
 
 
 def pool_blocks(k_cache, v_cache, block_table, pool_k, pool_v, pool_table, seq_start, seq_past, n_seqs: int,

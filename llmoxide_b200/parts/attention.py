@@ -357,4 +357,5 @@ class GQAttention:
         else:
             kernels.attention_paged(q, out, view.k, view.v, block_table, ctx.token_seq, ctx.token_pos,
                                     H, G, D, self.window, self.scale, v_head_dim=self.Dv, keep_first=self.keep_first,
-                                    sink=self.sink, chunk=self.chunk, single_tokens=ctx.is_decode, **extra)
+                                    sink=self.sink, chunk=self.chunk, single_tokens=ctx.is_decode,
+                                    seq_start=ctx.seq_start, **extra)

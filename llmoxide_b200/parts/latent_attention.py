@@ -247,7 +247,7 @@ class LatentAttention:
         else:
             kernels.attention_paged(q, out, view.k, view.v, block_table, ctx.token_seq, ctx.token_pos,
                                     H, H, E, self.window, self.scale, v_head_dim=self.Dv, gate=gate, sinks=self.sinks,
-                                    single_tokens=ctx.is_decode)
+                                    single_tokens=ctx.is_decode, seq_start=ctx.seq_start)
             return
         if gate is not None:
             kernels.head_gate(out, gate, H, self.Dv)

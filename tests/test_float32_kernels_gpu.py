@@ -178,3 +178,58 @@ def test_attention_f32_tiles_whose_scores_are_all_minus_infinity():
         kernels.attention_paged(q, out, k, v, table, seq, pos, H, G, D, None, 0.125, score_bias=bias, single_tokens=single)
         assert torch.isnan(out[:near]).all()                  # no finite score at all
         assert rel(out[near:], want[near:]) < 2e-6
+
+
+@pytest.mark.parametrize("H, G, D, Dv, window, keep, steps", [
+    # (tokens held, tokens brought) per sequence
+    (4, 4, 64, 64, None, 0, [(200, 1)] * 35 + [(0, 70)] + [(3, 1)]),       # 32 rows hold runs of 32 sequences
+    (8, 2, 128, 128, 100, 5, [(600, 1), (0, 1), (63, 2), (64, 9), (0, 130), (500, 3)]),
+    (12, 1, 48, 80, None, 0, [(70, 5), (10, 1), (0, 1), (129, 66)]),        # more heads a kv head than 8 rows
+    (3, 3, 256, 256, 70, 0, [(300, 7), (0, 20)]),
+    (5, 1, 20, 16, None, 0, [(1, 1), (0, 33)]),
+])
+def test_attention_f32_launches_agree(H, G, D, Dv, window, keep, steps):
+    """Every launch, told where the sequences start or not, gives the same bits, and rows of q that are no whole 16-byte
+    pieces too; against 64 bits as above."""
+    from llmoxide_b200 import kernels
+    torch.manual_seed(H * D)
+    lens, new = [a + b for a, b in steps], [b for _, b in steps]
+    width = max(-(-L // 64) for L in lens)
+    pages = torch.randperm(width * len(lens), dtype=torch.int32).view(len(lens), width)
+    k, v = (torch.full((pages.numel(), G, 64, n), math.nan, device=DEV) for n in (D, Dv))
+    ks, vs = [torch.randn(L, G, D, device=DEV) for L in lens], [torch.randn(L, G, Dv, device=DEV) for L in lens]
+    for b, L in enumerate(lens):
+        for i in range(-(-L // 64)):
+            n = min(64, L - 64 * i)
+            k[pages[b, i], :, :n], v[pages[b, i], :, :n] = (z[b][64 * i : 64 * i + n].transpose(0, 1) for z in (ks, vs))
+    T = sum(new)
+    wide = torch.randn(T, H * D + 3, device=DEV)
+    q = wide[:, : H * D].contiguous()
+    seq = torch.cat([torch.full((n,), b, dtype=torch.int32) for b, n in enumerate(new)]).to(DEV)
+    pos = torch.cat([torch.arange(a, a + n, dtype=torch.int32) for a, n in steps]).to(DEV)
+    starts = torch.tensor([sum(new[:b]) for b in range(len(new) + 1)], dtype=torch.int32, device=DEV)
+
+    def run(q, **hints):
+        out = torch.full((T, H * Dv), 7.0, device=DEV)
+        kernels.attention_paged(q, out, k, v, pages.to(DEV), seq, pos, H, G, D, window, D ** -0.5, v_head_dim=Dv,
+                                keep_first=keep, **hints)
+        return out
+
+    out = run(q)
+    for launch in (-1, 0, 1, 2):
+        for start in (None, starts):
+            assert torch.equal(run(q, launch=launch, seq_start=start), out), (launch, start is None)
+        assert torch.equal(run(q, launch=launch, single_tokens=True), out), launch      # (a token by itself)
+        assert torch.equal(run(wide[:, : H * D], launch=launch, seq_start=starts), out), launch
+    want, t0 = [], 0
+    for b, (past, n) in enumerate(steps):
+        i, j = torch.arange(past, past + n, device=DEV)[:, None], torch.arange(past + n, device=DEV)[None]
+        hidden = j > i
+        if window:
+            hidden = hidden | ((i - j >= window) & (j >= keep))
+        qs = q[t0 : t0 + n].double().view(n, H, D)
+        want.append(torch.stack([torch.softmax((qs[:, h] @ ks[b][:, h * G // H].double().T * D ** -0.5)
+                                               .masked_fill(hidden, -math.inf), 1) @ vs[b][:, h * G // H].double()
+                                 for h in range(H)], 1).reshape(n, H * Dv))
+        t0 += n
+    assert rel(out, torch.cat(want)) < 2e-6
