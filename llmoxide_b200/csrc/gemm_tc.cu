@@ -90,6 +90,7 @@ __device__ __forceinline__ void epilogue_tile(uint32_t acc_addr, bool have_acc, 
       for (int e = 0; e < 16; ++e) v[e] = g[e] = 0.f;
     }
     if constexpr (PARTS) {
+#pragma unroll 2
       for (int p = 0; p < n_parts; ++p) {
         const float* other = parts + ((size_t)p * BN + c) * TC_BM + row;
 #pragma unroll
@@ -904,17 +905,52 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, void* Y, int T, 
   return LLMX_LAUNCH_STATUS();
 }
 
-// How many CTAs share the K of a tile in a step of few tokens whose result goes out whole: a power of two up to 8, no more
-// than one CTA per SM in all, at least four blocks of K each, and 96 KB at most for the accumulators that are handed over.
+// Clusters of 2, 4 or 8 such CTAs that run at once with an SM each: not every SM can be part of one, so it is asked for,
+// once per size.
+static int parts_clusters(int parts) {
+  static int fits[9] = {};
+  if (!fits[parts]) {
+    auto kernel = gemm_tc_parts_kernel<16, 0, bf16>;
+    const int smem = 120 * 1024;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)parts;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sm_count() / parts * parts));
+    cfg.blockDim = dim3(TC_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0)
+      n = sm_count() / (2 * parts);
+    fits[parts] = n;
+  }
+  return fits[parts];
+}
+
+// How many CTAs share the K of a tile in a step of few tokens whose result goes out whole.  Rule: the cheapest by what 1440
+// products took (128 to 12288 rows, K = 256 to 8192, 1 to 64 tokens): 0.245 us for a block of K, and for a hand-over to one,
+// three or seven others what the table says, more where the clusters fill the GPU.  All clusters have to run at once: 36
+// tiles in fours take 10.2 us where they take 7.1 alone and 6.1 in pairs (bfloat16 out, K = 1024, 24 tokens).  us alone / in
+// 2 / 4 / 8, gated, 16 tokens, K = 2048: 12 tiles 11.0 / 7.8 / 6.3 / 6.4, 32 tiles 11.4 / 8.3 / 7.8 / 16.2; 64 tokens, 32
+// tiles: K = 1024 11.3 / 10.7 / 12.1, K = 512 8.9 / 9.6 / 11.9.  None of the 1440 is more than 1.1 % slower than alone.
 static int choose_parts(int T, int N, int K) {
   if (T > 64) return 1;
-  const int tiles = (N + TC_BM - 1) / TC_BM, blocks = (K + TC_BK - 1) / TC_BK, bn = T <= 16 ? 16 : T <= 32 ? 32 : 64;
-  int parts = 1;
-  while (parts < 8 && tiles * parts * 2 <= sm_count() && blocks >= parts * 2 * 4 &&
-         (parts * 2 - 1) * bn * TC_BM * 4 <= 96 * 1024)
-    parts *= 2;
-  while (parts > 1 && (blocks + parts - 1) / parts * (parts - 1) >= blocks) parts /= 2;      // (no part is empty)
-  return parts;
+  static const double hand_over[3][3] = {{0.85, 1.45, 2.4}, {1.4, 2.3, 4.2}, {1.9, 4.4, 1e9}};     // [tokens][2, 4, 8 parts]
+  const double* cost = hand_over[T <= 16 ? 0 : T <= 32 ? 1 : 2];
+  const int tiles = (N + TC_BM - 1) / TC_BM, blocks = (K + TC_BK - 1) / TC_BK;
+  int best = 1;
+  double least = 0.245 * blocks;
+  for (int i = 0, parts = 2; i < 3; ++i, parts *= 2) {
+    const int per_part = (blocks + parts - 1) / parts;
+    const double us = 0.245 * per_part + cost[i] + 0.02 * fmax(0.0, tiles * parts / 2 - 32);
+    // (no part is empty; the accumulators that are handed over take 112 KB at most)
+    if (us < least && per_part * (parts - 1) < blocks && tiles <= parts_clusters(parts)) best = parts, least = us;
+  }
+  return best;
 }
 
 template <int BN, int MODE, typename TY>
@@ -980,7 +1016,9 @@ LLMX_API int llmx_gemm_tc_scaled(const void* X, const void* W, void* Y, int y_dt
   CUtensorMap mw, mx;
   if (make_map(&mw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, TC_BM, true)) return LLMX_REFUSED(4);
   if (make_map(&mx, X, (uint64_t)T, (uint64_t)K, (uint64_t)ldx, (uint32_t)bn, false)) return LLMX_REFUSED(4);
-  const int parts = n_split == 1 && mode != 1 && y_dtype == LLMX_BF16 ? choose_parts(T, N, K) : 1;
+  // (an activation without a gate, mode 3: the split product and the activation behind it were faster, 5.5 us against 8.6 at
+  // 1024 rows, K = 2048, four tokens)
+  const int parts = n_split == 1 && (mode == 0 || mode == 2) && y_dtype == LLMX_BF16 ? choose_parts(T, N, K) : 1;
   if (parts > 1) {
 #define PARTS(MODE)                                                                                       \
   switch (bn) {                                                                                           \
@@ -989,8 +1027,7 @@ LLMX_API int llmx_gemm_tc_scaled(const void* X, const void* W, void* Y, int y_dt
     default: return launch_parts<64, MODE, bf16>(mw, mx, Y, T, N, K, ldy, parts, F, sc, stream);          \
   }
     if (mode == 0) PARTS(0)
-    if (mode == 2) PARTS(2)
-    PARTS(3)
+    PARTS(2)
 #undef PARTS
   }
 #define GO(BN, MODE, TY) return launch<BN, MODE, TY>(mw, mx, Y, T, N, K, ldy, n_split, split_stride, F, sc, stream)
