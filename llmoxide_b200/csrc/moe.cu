@@ -11,6 +11,8 @@
 // expert's segment is whatever the sort's atomics gave; no value depends on it.
 #include "common.cuh"
 
+#include <type_traits>
+
 #define MOE_TILE 64          // rows (and columns) per tile of the grouped products
 #define MOE_BK 16
 #define MOE_MAX_TOP 16
@@ -202,25 +204,26 @@ moe_router_kernel(const TX* __restrict__ x, long long ldx, const float* __restri
   const TX* xr[TOK];
 #pragma unroll
   for (int j = 0; j < TOK; ++j) xr[j] = x + (size_t)min(t0 + j, n_tokens - 1) * ldx;
-  for (int e = warp; e < n_rows; e += 16) {
-    const bool two = e + 8 < n_rows;
-    const float* wr[2] = {w + (size_t)e * K, w + (size_t)(two ? e + 8 : e) * K};
-    float acc[2][TOK];
+  // rows e and, of two, e + 8 (a warp that has one row left does not read it twice)
+  auto products = [&](int e, auto rows) {
+    constexpr int Q = decltype(rows)::value;
+    float acc[Q][TOK];
 #pragma unroll
-    for (int q = 0; q < 2; ++q)
+    for (int q = 0; q < Q; ++q)
 #pragma unroll
       for (int j = 0; j < TOK; ++j) acc[q][j] = 0.f;
+    const float* wr = w + (size_t)e * K;
     if (vec) {           // K a multiple of 8 and rows 16-byte aligned: 8 consecutive k per lane and step
-      constexpr int UNROLL = TOK == 1 ? 4 : 1;
+      constexpr int UNROLL = TOK == 1 ? 4 : Q == 1 ? 2 : 1;
 #pragma unroll UNROLL
       for (int k = lane * 8; k < K; k += 256) {
-        float wv[2][8], xv[TOK][8];
+        float wv[Q][8], xv[TOK][8];
 #pragma unroll
-        for (int q = 0; q < 2; ++q) moe_load8(wr[q] + k, wv[q]);
+        for (int q = 0; q < Q; ++q) moe_load8(wr + (size_t)q * 8 * K + k, wv[q]);
 #pragma unroll
         for (int j = 0; j < TOK; ++j) moe_load8(xr[j] + k, xv[j]);
 #pragma unroll
-        for (int q = 0; q < 2; ++q)
+        for (int q = 0; q < Q; ++q)
 #pragma unroll
           for (int j = 0; j < TOK; ++j)
 #pragma unroll
@@ -230,20 +233,24 @@ moe_router_kernel(const TX* __restrict__ x, long long ldx, const float* __restri
       for (int k0 = lane * 8; k0 < K; k0 += 256)
         for (int k = k0; k < k0 + 8 && k < K; ++k)
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const float wv = wr[q][k];
+          for (int q = 0; q < Q; ++q) {
+            const float wv = wr[(size_t)q * 8 * K + k];
 #pragma unroll
             for (int j = 0; j < TOK; ++j) acc[q][j] = fmaf(to_f32(xr[j][k]), wv, acc[q][j]);
           }
     }
 #pragma unroll
-    for (int q = 0; q < 2; ++q)
+    for (int q = 0; q < Q; ++q)
 #pragma unroll
       for (int j = 0; j < TOK; ++j) {
         const float v = warp_sum(acc[q][j]);
         const int row = e + 8 * q;
-        if (lane == 0 && (q == 0 || two)) route_smem[j * per_tok + row] = (logit_bias && row < E) ? v + logit_bias[row] : v;
+        if (lane == 0) route_smem[j * per_tok + row] = (logit_bias && row < E) ? v + logit_bias[row] : v;
       }
+  };
+  for (int e = warp; e < n_rows; e += 16) {
+    if (e + 8 < n_rows) products(e, std::integral_constant<int, 2>());
+    else products(e, std::integral_constant<int, 1>());
   }
   __syncthreads();
   const int t = t0 + warp;
