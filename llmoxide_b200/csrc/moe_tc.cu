@@ -16,9 +16,8 @@
 //   MODE 2 (up):      act[row, n] = the activation of an expert without a gate (plain_act)
 //   MODE 3 (gate|up, narrow row tiles): as MODE 1, from one tile of 64 gate rows above the 64 up rows of the same features;
 //                     the warps that hold up hand it over in shared memory.  A step of few tokens touches a few experts,
-//                     and 64 features a unit give twice as many CTAs something to stream.  Four tokens that pick
-//                     2 of 16 experts of 2 x 1024 x 2048: gate|up and down together 24.8 -> 20.8 us, 64 tokens
-//                     44.3 -> 39.2; bound by the length of a CTA's stream (32 blocks of K) up to about four tokens.
+//                     and 64 features a unit give twice as many CTAs something to stream (rule and measurements at
+//                     mt_narrow); bound by the length of a CTA's stream (32 blocks of K at 2048) up to about four tokens.
 //
 // Which expert a unit reads is decided on the device by the kernel before, so every thread waits for that
 // kernel first.  Every wait on an mbarrier is bounded; when one runs out the CTA records it in the library's
@@ -281,6 +280,20 @@ static int mt_launch(const CUtensorMap& mw, const CUtensorMap& mx, void* Y, cons
   return LLMX_LAUNCH_STATUS();
 }
 
+// Whether gate and up rows of 64 features share a tile (MODE 3) in row tiles of 16, or 128 of each have one of their own
+// (MODE 1).  Rule: by the units of 64 features that P pairs spread over the experts at random make, against the CTAs that
+// run at once (two an SM, 296), from 204 products (4 to 128 experts of 64 to 4096 features, 1 to 1000 tokens; us MODE 3 /
+// MODE 1): up to 0.95 of them the narrow units spread better (4 tokens, 2 of 16 experts of 1024: 11.2 / 14.8); just above
+// they need a second round where the wide ones do not (16 tokens, 4 of 64 experts of 512: 14.3 / 12.5); then they are even
+// or better again (16 tokens, 2 of 8 experts of 3000: 15.9 / 19.2) until the weights come at the HBM rate either way, with
+// fewer units to start (64 tokens, 4 of 64 experts of 512: 26.0 / 24.7).
+static bool mt_narrow(long long P, int n_experts, int N) {
+  const double per_expert = (double)P / n_experts;
+  const double tiles = n_experts * (1.0 - pow(1.0 - 1.0 / n_experts, (double)P)) * (1.0 + fmax(0.0, (per_expert - 10.0) / 12.0));
+  const double units = tiles * ((N + MT_BM / 2 - 1) / (MT_BM / 2)) / (2.0 * mt_sm_count());
+  return units <= 0.95 || (units > 1.165 && units <= 1.62 && per_expert <= 10.0);
+}
+
 // X: bf16 sorted rows [P, K] (row stride ldx); W: bf16 [E, w_rows, K] contiguous, w_rows = 2N when gated is 1 (gate rows,
 // then up rows) else N; tiles: int32 [max_tiles, 3] made with tile_rows rows per tile (16, 64 or 128).
 // gated 1: Y = act bf16 [P, N]; gated 2 (experts without a gate): W [E, N, K], Y = act(product) bf16 [P, N].  0: Y = float32 rows of N, row dest[place] = sorted_weight[place] * product
@@ -298,17 +311,20 @@ LLMX_API int llmx_moe_grouped_tc(const void* X, long long ldx, long long P, cons
   if (gated < 0 || gated > 2) return LLMX_REFUSED(1);
   const int w_rows = gated == 1 ? 2 * N : N;
   CUtensorMap mw, mx;
-  // gate and up rows of a narrow tile come by boxes of 64 rows
-  const uint32_t box = gated == 1 && tile_rows == 16 ? MT_BM / 2 : MT_BM;
+  // gate and up rows that share a tile come by boxes of 64 rows
+  const bool narrow = gated == 1 && tile_rows == 16 && mt_narrow(P, n_experts, N);
+  const uint32_t box = narrow ? MT_BM / 2 : MT_BM;
   if (make_map(&mw, W, (uint64_t)n_experts * w_rows, (uint64_t)K, (uint64_t)K, box, true)) return LLMX_REFUSED(4);
   if (make_map(&mx, X, (uint64_t)P, (uint64_t)K, (uint64_t)ldx, (uint32_t)tile_rows, false)) return LLMX_REFUSED(4);
 #define RUN(BN, MODE, TY) \
   mt_launch<BN, MODE, TY>(mw, mx, Y, tiles, max_tiles, dest, sorted_weight, P, N, K, w_rows, act, stream)
-#define GO(BN, GATED) return gated == 1 ? RUN(BN, GATED, bf16) : gated == 2 ? RUN(BN, 2, bf16) : RUN(BN, 0, float)
+#define GO(BN) return gated == 1 ? RUN(BN, 1, bf16) : gated == 2 ? RUN(BN, 2, bf16) : RUN(BN, 0, float)
   switch (tile_rows) {
-    case 16: GO(16, 3);
-    case 64: GO(64, 1);
-    case 128: GO(128, 1);
+    case 16:
+      if (narrow) return RUN(16, 3, bf16);
+      GO(16);
+    case 64: GO(64);
+    case 128: GO(128);
     default: return LLMX_REFUSED(1);
   }
 #undef GO
