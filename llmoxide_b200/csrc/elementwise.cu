@@ -325,10 +325,12 @@ static int launch_add_rms_norm(float* h, const void* delta, int n_split, size_t 
   int ch, threads;
   norm_shape(d, ch, threads);
   const bool deep = delta && n_split > 1;
-  // Rule: rows without a residual to add, more of them than run at once with a CTA each (three to an SM at 512 threads);
-  // fewer gain nothing (1000 rows of 4096: 9.0 us either way)
-  const int at_once = 148 * (1536 / threads);
-  if (!delta && out && !rows && (ch == 1 || ch == 2) && n_rows > at_once) {
+  // Rule: rows without a residual to add, more of them than run at once with a CTA each (three to an SM at 512 threads), and
+  // twice as many where a thread has two vectors or the threads are no even share of an SM (1000 rows of 2052: 3.5 us by a
+  // CTA each, 4.2 by walking; 2000: 5.8 and 5.6; 900 rows of 1536: 3.3 and 3.5; 1000 rows of 1024: 3.0 and 2.8)
+  const int at_once = llmx_sm_count() * (1536 / threads);
+  const bool walk = n_rows > at_once && ((ch == 1 && (threads == 512 || threads <= 256)) || n_rows >= 2 * at_once);
+  if (!delta && out && !rows && (ch == 1 || ch == 2) && walk) {
     if (ch == 1) launch_pdl(norm_rows_kernel<TO, 1>, dim3(at_once), dim3(threads), 0, stream, (const float*)h, gain, eps, (TO*)out, d, n_rows);
     else launch_pdl(norm_rows_kernel<TO, 2>, dim3(at_once), dim3(threads), 0, stream, (const float*)h, gain, eps, (TO*)out, d, n_rows);
     return LLMX_LAUNCH_STATUS();

@@ -9,9 +9,15 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("d, n", [(64, 3600), (1024, 889), (2048, 445), (2052, 444), (4096, 445), (4096, 1337)])
-def test_rows_in_one_launch_and_a_few_at_a_time(d, n, dtype):
+# multiples of the rows that run at once with a CTA each, and a few more: a vector a thread and two, last vectors of which
+# some threads have none
+@pytest.mark.parametrize("d, rounds", [(64, 1), (1024, 1), (1536, 2), (2048, 1), (2052, 1), (2052, 2), (2052, 4), (3072, 3),
+                                       (4096, 1), (4096, 2), (4096, 3)])
+def test_rows_in_one_launch_and_a_few_at_a_time(d, rounds, dtype):
     from llmoxide_b200 import kernels
+    vectors = 1 if d <= 2048 else 2
+    threads = max(64, -(-d // 4 // vectors // 32) * 32)
+    n = rounds * torch.cuda.get_device_properties(0).multi_processor_count * (1536 // threads) + 5
     torch.manual_seed(d + n)
     h, gain = torch.randn(n + 1, d, device=DEV), torch.randn(d, device=DEV)
     out = torch.full((n + 1, d), 7.0, device=DEV, dtype=dtype)
