@@ -139,3 +139,35 @@ def test_one_and_two_columns_a_thread(H, D, Dv, lens, gated):
             rows = torch.tensor([starts[b] + t for b in seqs], device=DEV)
             assert torch.equal(call(rows, [1] * len(seqs), alone, seqs), out[rows])
         assert torch.equal(alone, state)
+
+
+@pytest.mark.parametrize("H, D, Dv, n_rot, activation, ones", [
+    (2, 66, 65, 0, "none", False), (1, 131, 64, 0, "none", False),          # keys that are no multiple of four
+    (2, 128, 64, 128, "silu", False), (1, 70, 66, 32, "none", False),       # rotated, all of a key or its first dims
+    (2, 64, 64, 0, "none", True), (1, 67, 63, 10, "silu", True)])           # one more column, of ones
+def test_chunks_of_prepared_keys_and_values(H, D, Dv, n_rot, activation, ones):
+    """As above; an activation and a rotation add a few roundings of 2^-24 to every q, k and v: 7e-7 in the 2-norm."""
+    from llmoxide_b200 import kernels
+    torch.manual_seed(D + Dv)
+    lens, slots, dva = [150, 1, 193], [1, 3, 0], Dv + int(ones)
+    decay = torch.tensor([0.95, 0.999][:H], device=DEV)
+    T, before = sum(lens), torch.randn(4, H, D, dva, device=DEV)
+    proj = torch.randn(T, H * (2 * D + Dv), device=DEV)
+    starts = torch.tensor([sum(lens[:i]) for i in range(4)], dtype=torch.int32, device=DEV)
+    pos = torch.cat([torch.arange(7, 7 + n, dtype=torch.int32) for n in lens]).to(DEV)
+    angle = torch.rand(max(lens) + 7, n_rot // 2, device=DEV) * 6.28 if n_rot else None
+    cos, sin = (angle.cos(), angle.sin()) if n_rot else (None, None)
+    state, out = before.clone(), torch.full((T, H * dva), float("nan"), device=DEV)
+    kernels.decay_scan(proj, out, state, starts, pos, torch.tensor(slots, dtype=torch.int32, device=DEV), decay, cos, sin,
+                       n_rot, activation, 0.7, H, D, Dv, 0, H * D, 2 * H * D, max_new=max(lens), q_scale=1.3, ones_column=ones)
+    p = torch.nn.functional.silu(proj.double()) if activation == "silu" else proj.double()
+    q, k, v = p[:, : H * D].view(T, H, D), p[:, H * D : 2 * H * D].view(T, H, D), p[:, 2 * H * D :]
+    if n_rot:
+        half, c, s = n_rot // 2, cos.double()[pos.long()][:, None], sin.double()[pos.long()][:, None]
+        q, k = (torch.cat([z[..., :half] * c - z[..., half:n_rot] * s, z[..., half:n_rot] * c + z[..., :half] * s, z[..., n_rot:]], 2)
+                for z in (q, k))
+    prepared = torch.cat([q.reshape(T, -1) * 1.3, k.reshape(T, -1) * 0.7, v], 1)
+    one = torch.ones(T, H, device=DEV, dtype=torch.float64)
+    want, after = recurrence(prepared, lens, slots, before, one * decay.double(), one, H, D, Dv, ones)
+    assert ((out - want).norm() / want.norm()).item() < 7e-7
+    assert ((state - after).norm() / after.norm()).item() < 7e-7
