@@ -1,7 +1,9 @@
 // Attention over the paged cache, general form: any number of heads and
-// groups, any head size that is a multiple of 16 up to 256, a window or none,
-// whole prompts and single tokens alike.  It is the float32 path's kernel and
-// the bfloat16 path's fallback for the sizes the tiled kernels refuse.
+// groups, any head size up to 256, a window or none, whole prompts and single
+// tokens alike.  Two kernels: attention_f32_kernel (tiles of keys) for float32
+// without pooled blocks and with sizes that are multiples of 4, and
+// attention_paged_kernel for everything else: the bfloat16 path's sizes that
+// the tiled kernels of other files refuse, pooled blocks, odd sizes.
 //
 // For the query at position p of head hq (crates/model/src/qwen35/cpu.rs:325-355):
 // kv head g = hq / (H/G); keys first..p are visible, first = 0 or p-(w-1) under
@@ -24,7 +26,7 @@
 // With `score_bias` (float32 [H, bias_len]) the scaled score of the key at j has score_bias[hq, min(p - j, bias_len - 1)]
 // added: a learned number per distance and head (not beside pooled blocks or a cap).
 //
-// One warp per (token, head).  Keys are taken 32 at a time starting at the
+// attention_paged_kernel: one warp per (token, head).  Keys are taken 32 at a time starting at the
 // range's first key: lane j scores key lo + c*32 + j with a sequential dot over
 // D, the chunk's maximum and sum update a running softmax, and the lanes then
 // own dims (lane, lane+32, ...) of the output and add the chunk's values key

@@ -68,7 +68,7 @@ struct BlockCopy {
 // Prompts: 128 threads as 8 (tokens) x 16 (features), TM x TN elements each.  Rows in shared memory are 20 floats apart,
 // so eight rows read at the same k lie in different banks; 8 x 8 elements take 16 shared-memory reads per 128 packed
 // multiply-adds.  The sums of earlier segments wait in shared memory.  Bound by the FMA units and the reads that feed
-// them (4 x 4: fmaheavy 66 %, shared-memory wavefronts 72 % of the cycles).  970 tokens, N = K = 2048: 231 us (35 TFLOP/s;
+// them.  970 tokens, N = K = 2048: 231 us (35 TFLOP/s;
 // the one-chain 64 x 64 kernel that this replaced: 16 TFLOP/s); 2500 tokens, N = 4096: 971 us (43 TFLOP/s).
 template <int TM, int TN>
 struct F32Tile {
@@ -161,9 +161,9 @@ gemm_f32_tile_kernel(const float* __restrict__ X, const float* __restrict__ W, f
 // Few tokens (up to 2 MT a CTA): 16 features, four segments of K at a time.  Thread (feature f, segment g, token half h)
 // follows its feature's chain over segment g for MT tokens, so a value of W is read from shared memory once per token
 // half and the tokens' values are broadcasts; a quarter of the chain's length and four streams of each row are what a
-// row costs.  The first stages of W are asked for before the kernel before has ended.  Three tokens, K = 2048: 10 us at
-// N = 2048 (the 64 x 64 kernel, 32 CTAs with one chain of 2048 steps: 184 us a product), 65 us at N = 32768 (4.1 TB/s);
-// bound by the latency of a CTA's first tiles at the former, by HBM and the reads of X at the latter.
+// row costs.  The first lines of W travel to L2 before the kernel before has ended.  Four tokens, K = 2048: 10 us at
+// N = 2048 (the 64 x 64 kernel, 32 CTAs with one chain of 2048 steps: 184 us a product), 25 us at N = 8192 (2.7 TB/s);
+// bound by the latency of a CTA's first tiles at the former, by that and the reads of X at the latter.
 template <int MT>
 struct F32Rows {
   static constexpr int BM = 2 * MT, BN = 16, GROUPS = 4, BK = 32, PITCH = BK + 4;
@@ -298,9 +298,9 @@ LLMX_API int llmx_gemm_f32_form(int form, const float* X, const float* W, float*
     const double blocks = (K + 15) / 16;
     const int few = M <= 2 ? 0 : M <= 4 ? 1 : M <= 8 ? 2 : 3;
     const double a_step[4] = {0.6, 0.65, 0.75, 1.1};
-    const double rows = a_step[few] * steps * rounds(tiles(2 << few, 16), 296);
-    const double small = blocks * fmax(0.26 * rounds(tiles(32, 64), 148), 0.41);
-    const double large = blocks * fmax(0.88 * rounds(tiles(64, 128), 148), 1.17);
+    const double rows = a_step[few] * steps * rounds(tiles(2 << few, 16), 2 * llmx_sm_count());
+    const double small = blocks * fmax(0.26 * rounds(tiles(32, 64), llmx_sm_count()), 0.41);
+    const double large = blocks * fmax(0.88 * rounds(tiles(64, 128), llmx_sm_count()), 1.17);
     form = rows <= small && rows <= large ? few : small <= large ? 4 : 5;
   }
   // 16-byte copies where every row starts on a 16-byte boundary and K ends on one, else 4-byte copies

@@ -14,7 +14,9 @@
 // a column (or of two neighbouring ones) split D among them in blocks of 4 dims (lane r owns dims 4 (r + 8 i) + 0..3),
 // update their part of S and add up q . S by shuffles.  The order of every addition is fixed by (d, column) alone, and a
 // token's update is the same arithmetic whether it arrives in a prompt, in a later portion of one or alone, so
-// a position's result does not depend on how tokens were cut into steps or batched, to the last bit.
+// among steps that bring a sequence up to seg_len tokens a position's result does not depend on how tokens were cut into
+// steps or batched, to the last bit.  Longer prompts go in segments or by chunks (below), whose sums are ordered by where
+// those begin: the same for every batch, but rounded differently when a prompt is cut differently.
 //
 // The same kernels run a recurrence whose decay and input weight change from token to token (the matrix memory
 // of an mLSTM layer, GATED below):
@@ -32,8 +34,8 @@
 // state, one for the output), which is what the FMA units are for; the state is read and written once per
 // step, which is what bounds a decode step.
 //
-// A sequence that brings a long prompt under a fixed decay, with a state worth it, is walked in chunks of 64 tokens
-// instead.  With E the state a chunk starts from,
+// A sequence that brings more than seg_len tokens under a fixed decay, with a state of at least 64 x 64, is walked in
+// chunks of 64 tokens instead.  With E the state a chunk starts from,
 //   o_i = decay^(i+1) E^T q_i + sum_(j<=i) decay^(i-j) (q_i . k_j) v_j,   E' = decay^n E + sum_j decay^(n-1-j) k_j v_j^T
 // which is the recurrence written out as products of small matrices (chunk_products.cuh, as the state-space layers walk
 // theirs): as many multiply-adds, but 8 x 8 results a thread share what they read from shared memory.
