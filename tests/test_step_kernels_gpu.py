@@ -1,0 +1,46 @@
+"""Launches that a rule on sizes chooses, each against what it stands in for or against 64 bits, at the sizes where the rule
+or a remainder changes."""
+
+import pytest
+import torch
+
+DEV = "cuda:0"
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm()).item()
+
+
+@pytest.mark.parametrize("D, n_rot, H, G, T, n_split", [(64, 64, 3, 1, 5, 3), (64, 0, 16, 8, 1, 5), (64, 64, 5, 2, 70, 1),
+                                                        (128, 0, 16, 4, 70, 1), (128, 0, 3, 2, 4, 4), (64, 0, 2, 1, 9, 2)])
+@pytest.mark.parametrize("gains", [False, True])
+def test_heads_of_64_and_unrotated_heads(D, n_rot, H, G, T, n_split, gains):
+    """Against 64 bits; q, k and v are rounded to bfloat16 once (2^-9 of a value, 2^-8 after a rotation's sum)."""
+    from llmoxide_b200 import kernels
+    torch.manual_seed(D + T)
+    x = torch.randn(n_split, T, (H + 2 * G) * D, device=DEV)
+    x = x[0].bfloat16() if n_split == 1 else x
+    row = (x.double() if n_split == 1 else x.double().sum(0)).view(T, H + 2 * G, D)
+    pos = torch.arange(30, 30 + T, dtype=torch.int32, device=DEV)
+    angle = torch.rand(200, max(n_rot // 2, 1), device=DEV) * 6.28
+    gq, gk = (1 + 0.1 * torch.randn(2, D, device=DEV)) if gains else (None, None)
+    table = torch.tensor([[2, 0, 1]], dtype=torch.int32, device=DEV)
+    kc, vc = (torch.zeros(3, G, 64, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    q = torch.empty(T, H * D, dtype=torch.bfloat16, device=DEV)
+    kernels.qk_norm_rope_cache(x, q, kc, vc, table, torch.zeros(T, dtype=torch.int32, device=DEV), pos, gq, gk, 1e-6,
+                               angle.cos() if n_rot else None, angle.sin() if n_rot else None, n_rot, H, G, D, True)
+
+    def made(y, gain):
+        if gains:
+            y = y / (y.pow(2).mean(-1, keepdim=True) + 1e-6).sqrt() * gain.double()
+        if n_rot:
+            c, s = (f(angle.double())[pos.long()][:, None] for f in (torch.cos, torch.sin))
+            a, b = y[..., : D // 2], y[..., D // 2 :]
+            y = torch.cat([a * c - b * s, b * c + a * s], -1)
+        return y
+
+    where = [(int(table[0, int(p) // 64]), int(p) % 64) for p in pos]
+    assert rel(q.view(T, H, D), made(row[:, :H], gq)) < 2 ** -8
+    assert rel(torch.stack([kc[a, :, r] for a, r in where]), made(row[:, H : H + G], gk)) < 2 ** -8
+    assert torch.equal(torch.stack([vc[a, :, r] for a, r in where]), row[:, H + G :].float().bfloat16())
