@@ -57,13 +57,25 @@ struct PnGroup {
   size_t stride;
   float weight;
 };
-__device__ __forceinline__ float4 pn_group4(const PnGroup& g, size_t at) {
-  float4 y = g.is_bf16 ? pn_load4((const bf16*)g.p + at) : pn_load4((const float*)g.p + at);
-  for (int s = 1; s < g.n_split; ++s) {
-    const size_t o = at + (size_t)s * g.stride;
-    const float4 q = g.is_bf16 ? pn_load4((const bf16*)g.p + o) : pn_load4((const float*)g.p + o);
-    y.x += q.x, y.y += q.y, y.z += q.z, y.w += q.w;
+// J partials are asked for together (a decode step's row waits for one trip, not for one after another).
+template <int J, typename T>
+__device__ __forceinline__ float4 pn_sum4(const T* p, int n_split, size_t stride) {
+  float4 y = pn_load4(p);
+  for (int s0 = 1; s0 < n_split; s0 += J) {
+    float4 q[J];
+#pragma unroll
+    for (int s = 0; s < J; ++s)
+      if (s0 + s < n_split) q[s] = pn_load4(p + (size_t)(s0 + s) * stride);
+#pragma unroll
+    for (int s = 0; s < J; ++s)
+      if (s0 + s < n_split) y.x += q[s].x, y.y += q[s].y, y.z += q[s].z, y.w += q[s].w;
   }
+  return y;
+}
+template <int J = 1>
+__device__ __forceinline__ float4 pn_group4(const PnGroup& g, size_t at) {
+  const float4 y = g.is_bf16 ? pn_sum4<1>((const bf16*)g.p + at, g.n_split, g.stride)      // (partials are float32)
+                             : pn_sum4<J>((const float*)g.p + at, g.n_split, g.stride);
   return make_float4(y.x * g.weight, y.y * g.weight, y.z * g.weight, y.w * g.weight);
 }
 __device__ __forceinline__ float pn_group1(const PnGroup& g, size_t at) {
@@ -203,7 +215,10 @@ __device__ __forceinline__ void pn_stats_reg(const float4 (&v)[NV], const bool (
   rstd = 1.0f / sqrtf(block_sum(ss, red) / (float)d + eps);
 }
 
-template <typename TO, int NV>
+// DEEP: a step of few rows (a decode step): partials are asked for in batches and the gains ahead of the wait (four rows of
+// 2048 behind a product of up to nine partials: 5.6 us a launch in a chain, 4.5 like this); otherwise few registers, so that
+// several rows share an SM.
+template <typename TO, int NV, bool DEEP>
 __global__ void __launch_bounds__(512)
 post_norm_add_norm_reg_kernel(float* __restrict__ h, const PnGroup g0, const PnGroup g1, const PnGroup gz,
                               const float* __restrict__ zb, const float* __restrict__ bias, const float* __restrict__ post_gain, int post_center,
@@ -224,6 +239,15 @@ post_norm_add_norm_reg_kernel(float* __restrict__ h, const PnGroup g0, const PnG
     live[k] = j < n4;
     col[k] = j * 4;
   }
+  // (in a decode step the gains come from memory, a trip each on the row's path)
+  constexpr int J = DEEP ? NV == 1 ? 7 : 4 : 1;
+  float4 pg[NV], og[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+    if (DEEP && live[k]) {
+      if (post_gain) pg[k] = pn_load4(post_gain + col[k]);
+      if (gain) og[k] = pn_load4(gain + col[k]);
+    }
   pdl_wait();
   if (g0.p) {
     const size_t at0 = (size_t)t * d;
@@ -234,9 +258,9 @@ post_norm_add_norm_reg_kernel(float* __restrict__ h, const PnGroup g0, const PnG
     for (int k = 0; k < NV; ++k) {
       float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
       if (live[k]) {
-        y = pn_group4(g0, at0 + col[k]);
+        y = pn_group4<J>(g0, at0 + col[k]);
         if (g1.p) {
-          const float4 z = pn_group4(g1, at0 + col[k]);
+          const float4 z = pn_group4<J>(g1, at0 + col[k]);
           y.x += z.x, y.y += z.y, y.z += z.z, y.w += z.w;
         }
         if (bias) {
@@ -253,7 +277,7 @@ post_norm_add_norm_reg_kernel(float* __restrict__ h, const PnGroup g0, const PnG
 #pragma unroll
       for (int k = 0; k < NV; ++k)
         if (live[k]) {
-          const float4 g = pn_load4(post_gain + col[k]);
+          const float4 g = DEEP ? pg[k] : pn_load4(post_gain + col[k]);
           v[k].x = ((v[k].x - mean) * rstd) * g.x, v[k].y = ((v[k].y - mean) * rstd) * g.y;
           v[k].z = ((v[k].z - mean) * rstd) * g.z, v[k].w = ((v[k].w - mean) * rstd) * g.w;
         }
@@ -280,7 +304,7 @@ post_norm_add_norm_reg_kernel(float* __restrict__ h, const PnGroup g0, const PnG
 #pragma unroll
   for (int k = 0; k < NV; ++k)
     if (live[k]) {
-      const float4 g = pn_load4(gain + col[k]);
+      const float4 g = DEEP ? og[k] : pn_load4(gain + col[k]);
       pn_store4(orow + col[k], make_float4(((v[k].x - mean) * rstd) * g.x, ((v[k].y - mean) * rstd) * g.y,
                                            ((v[k].z - mean) * rstd) * g.z, ((v[k].w - mean) * rstd) * g.w));
     }
@@ -335,15 +359,21 @@ LLMX_API int llmx_post_norm_add_norm_gated(float* h, const void* delta0, int dty
   if (vec && n4 <= 2048) {                              // the row in registers
     const int nv = n4 > 1024 ? 4 : n4 > 128 ? 2 : 1;
     const int reg_threads = ((n4 + nv - 1) / nv + 31) / 32 * 32;
+#define GO_DEEP(TO, NV, DEEP)                                                                                            \
+    launch_pdl(post_norm_add_norm_reg_kernel<TO, NV, DEEP>, dim3(n_rows), dim3(reg_threads), 0, stream, h, g0, g1, gz, zb, \
+               bias, post_gain, post_center, post_eps, rows, gain, center, eps, (TO*)out, d, write_h)
 #define GO_REG(TO, NV)                                                                                                   \
-    launch_pdl(post_norm_add_norm_reg_kernel<TO, NV>, dim3(n_rows), dim3(reg_threads), 0, stream, h, g0, g1, gz, zb, bias, \
-               post_gain, post_center, post_eps, rows, gain, center, eps, (TO*)out, d, write_h)
+  do {                                                                                                                   \
+    if (n_rows <= 64 && NV <= 2) GO_DEEP(TO, NV, (NV <= 2));                                                             \
+    else GO_DEEP(TO, NV, false);                                                                                         \
+  } while (0)
     if (out_bf16) {
       if (nv == 4) GO_REG(bf16, 4); else if (nv == 2) GO_REG(bf16, 2); else GO_REG(bf16, 1);
     } else {
       if (nv == 4) GO_REG(float, 4); else if (nv == 2) GO_REG(float, 2); else GO_REG(float, 1);
     }
 #undef GO_REG
+#undef GO_DEEP
     return LLMX_LAUNCH_STATUS();
   }
   if (out_bf16) {
