@@ -84,8 +84,25 @@ dual_norm_kernel(float* __restrict__ h, const DnGroup ga, const DnGroup gb, cons
     if (g.is_bf16) dn_add_group<NC, J>(v, (const bf16*)g.p + at, g.n_split, g.stride, col, d);
     else dn_add_group<NC, J>(v, (const float*)g.p + at, g.n_split, g.stride, col, d);
   };
-  add(ga);
-  add(gb);
+  if (DEEP && NC == 1 && ga.p && gb.p && !ga.is_bf16 && !gb.is_bf16 && ga.n_split <= J && gb.n_split <= J) {
+    // a decode step's two groups in one trip
+    const float *a = (const float*)ga.p + at + col[0], *b = (const float*)gb.p + at + col[0];
+    float4 y[J], z[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      if (col[0] < d && j < ga.n_split) y[j] = dn_load4(a + (size_t)j * ga.stride);
+      if (col[0] < d && j < gb.n_split) z[j] = dn_load4(b + (size_t)j * gb.stride);
+    }
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+      if (col[0] < d && j < ga.n_split) dn_add4(v[0], y[j]);
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+      if (col[0] < d && j < gb.n_split) dn_add4(v[0], z[j]);
+  } else {
+    add(ga);
+    add(gb);
+  }
   float ss = 0.f;
 #pragma unroll
   for (int c = 0; c < NC; ++c) {

@@ -118,9 +118,9 @@ def build_block(spec, weights: dict, rt):
 
 @register_arrangement("parallel")
 class ParallelBlock:
-    """A single norm feeds mixer and feed-forward: x = norm(h); h += mixer(x) + feed_forward(x).  The mixer's
-    result joins the float32 stream at once (nothing else reads the stream before the next layer's norm, and the
-    feed-forward reads x); the feed-forward's is handed on as the pending delta, which the next norm adds.
+    """A single norm feeds mixer and feed-forward: x = norm(h); h += mixer(x) + feed_forward(x).  Nothing else reads the
+    stream before the next layer's norm, and the feed-forward reads x: both results are handed on together as the pending
+    delta, which the next norm adds (the mixer's first), save what the mixer's last product has added to the stream itself.
 
     With a norm for each sublayer (``mixer`` and ``feed_forward`` instead of ``shared``) one kernel adds what the block
     before owes and makes the rows of both norms; both results are owed to the next block together (``parts.norm.Joined``),
@@ -146,7 +146,7 @@ class ParallelBlock:
         return self.mixer.cache_need()
 
     def libraries(self) -> set:
-        libs = {"dual_norm"} if self.norm is None else set()
+        libs = {"dual_norm"}
         for part in (self.norm, self.mixer_norm, self.ff_norm, self.mixer, self.feed_forward):
             if part is not None:
                 libs |= getattr(part, "libraries", set)()
@@ -190,11 +190,8 @@ class ParallelBlock:
         out = self.feed_forward.forward(x, ctx)
         if probe and out is not None:
             probe("ffn_out", _summed(out))
-        if a is not None:
-            if out is None:
-                return a
-            self.norm.add(h, a)
-        return out
+        # (what the mixer has not added to the stream itself joins it with the feed-forward's result, in the next norm's kernel)
+        return out if a is None else a if out is None else Joined([a, out])
 
 
 @register_arrangement("hyper_connections")

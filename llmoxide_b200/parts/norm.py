@@ -98,6 +98,8 @@ def _general_add_norm(h, delta, gain, center: bool, eps: float, out, rows, write
     elif isinstance(delta, PostNormed):
         terms, bias, post_gain, post_center, post_eps = delta.terms, delta.bias, delta.gain, delta.center, delta.eps
         gate = delta.gate
+    elif isinstance(delta, Joined):
+        terms, bias, post_gain, post_center, post_eps = [(t, 1.0) for t in delta.terms], delta.bias, None, False, 0.0
     else:
         terms, bias, post_gain, post_center, post_eps = _terms(delta), None, None, False, 0.0
     kernels.post_norm_add_norm(h, terms, bias, post_gain, post_center, post_eps, gain, center, eps, out, rows=rows,
