@@ -221,10 +221,28 @@ __global__ void __launch_bounds__(AF_THREADS) attention_f32_kernel(const AfArgs 
   int* row_seq = row_first + BR;
   float* part = reinterpret_cast<float*>(row_seq + BR);      // SPLIT: [2][8][PART] = maximum, sum (-1: no key), values
   pdl_launch_dependents();
-  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tn = lane & 15, tm = warp * 2 + (lane >> 4);     // a row's 16 threads are half a warp
   const int rank = SPLIT ? (int)(blockIdx.x % AF_SPLIT) : 0;
+  // A decode step's keys and values come from memory: the first two tiles of the CTA's first token are on their way to L2
+  // while the kernel before runs (positions and block tables are the step's inputs).  Three tokens at depths of 138 to 525, 16
+  // heads over 4: 22.9 us of a step's chain, 21.0 with this and the partial results of a round asked for together.
+  if (SPLIT && !a.seq_start) {
+    const int t = (int)(blockIdx.x / AF_SPLIT) * a.tokens_per_cta;
+    if (t < a.n_tokens) {
+      const int p = a.token_pos[t], kv = blockIdx.y / a.head_blocks;
+      int first = a.window > 0 ? max(p - (a.window - 1), 0) : 0;
+      if (a.chunk > 0) first = max(first, p - p % a.chunk);
+      const int* pages = a.block_table + (size_t)a.token_seq[t] * a.table_width;
+      for (int tile = first / AF_KEYS + rank, i = 0; i < 2 && tile <= p / AF_KEYS; ++i, tile += AF_SPLIT) {
+        const float* k = a.k_cache + cache_row_offset(pages[tile], kv, 0, a.G, D);
+        const float* v = a.v_cache + cache_row_offset(pages[tile], kv, 0, a.G, Dv);
+        for (int at = threadIdx.x * 32; at < AF_KEYS * D; at += AF_THREADS * 32) prefetch_l2(k + at);
+        for (int at = threadIdx.x * 32; at < AF_KEYS * Dv; at += AF_THREADS * 32) prefetch_l2(v + at);
+      }
+    }
+  }
+  pdl_wait();
   const int R = a.H / a.G, g = blockIdx.y / a.head_blocks, h0 = (blockIdx.y % a.head_blocks) * a.heads_per_cta;
   // this CTA's tokens (prompts: the last ones, which see most keys, start first)
   const int slot = SPLIT ? (int)(blockIdx.x / AF_SPLIT) : (int)gridDim.x - 1 - (int)blockIdx.x, per = a.tokens_per_cta;
@@ -461,13 +479,17 @@ __global__ void __launch_bounds__(AF_THREADS) attention_f32_kernel(const AfArgs 
           const int idx = e * AF_THREADS + threadIdx.x, row = idx / slice, d = rank * slice + idx % slice;
           if (row >= 8 || d >= Dv) continue;
           const float* src = part + ((size_t)parity * 8 + row) * PART;
-          for (int k = 0; k < here; ++k) {
-            const float km = af_remote(src, k), kl = af_remote(src + 1, k), ka = af_remote(src + 2 + d, k);
-            if (kl < 0.f) continue;
+          float km[AF_SPLIT], kl[AF_SPLIT], ka[AF_SPLIT];    // (all on their way together: one trip, not one a tile)
+#pragma unroll
+          for (int k = 0; k < AF_SPLIT; ++k)
+            if (k < here) km[k] = af_remote(src, k), kl[k] = af_remote(src + 1, k), ka[k] = af_remote(src + 2 + d, k);
+#pragma unroll
+          for (int k = 0; k < AF_SPLIT; ++k) {
+            if (k >= here || kl[k] < 0.f) continue;
             float c1, c2;
-            om[e] = af_join(om[e], km, c1, c2);
-            ol[e] = __fmaf_rn(kl, c2, __fmul_rn(ol[e], c1));
-            oa[e] = __fmaf_rn(ka, c2, __fmul_rn(oa[e], c1));
+            om[e] = af_join(om[e], km[k], c1, c2);
+            ol[e] = __fmaf_rn(kl[k], c2, __fmul_rn(ol[e], c1));
+            oa[e] = __fmaf_rn(ka[k], c2, __fmul_rn(oa[e], c1));
           }
         }
       }

@@ -310,6 +310,11 @@ __device__ __forceinline__ void plain_act_fast(const GateAct a, float (&x)[N]) {
   }
 }
 
+// Asks for the line of `p` as far as L2.  Nothing is read into the SM, so a kernel may do it ahead of its dependency wait for
+// whatever it will read behind it, also for what the kernel before still writes: in a decode step weights and states come
+// from memory otherwise, a trip each behind the wait.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Butterfly reductions: every lane ends with the same value, and the order of
 // the additions is fixed by the lane numbers alone.
 __device__ __forceinline__ float warp_sum(float v) {

@@ -518,6 +518,15 @@ delta_decode_kernel(const TIN* __restrict__ proj, const DeltaIn in, float* __res
   float* so = part + 8 * 2 * 32 * V;                    // [Dv] the head's output
   float* sv = so + ((Dv + 3) & ~3);                     // [Dv]
   __shared__ float red[32];
+  // the head's state, its channels' ring rows and weights are on their way to L2 while the kernel before runs (four tokens, 16
+  // heads of 128 x 128: 12.4 -> 10.8 us of a step's chain)
+  for (int i = tid * 32; i < D * Dv; i += 256 * 32) prefetch_l2(S + i);
+  auto channel = [&](int e) { return e < D ? j * D + e : e < 2 * D ? G * D + j * D + (e - D) : 2 * G * D + h * Dv + (e - 2 * D); };
+  for (int e = tid; e < 2 * D + Dv; e += 256)
+    for (int m = 0; m < taps; ++m) prefetch_l2(in.conv_w + (size_t)m * C + channel(e)), prefetch_l2(ring + (size_t)m * C + channel(e));
+  if (gain && tid * 32 < Dv) prefetch_l2(gain + tid * 32);
+  float a_rate = 0.f, dt_off = 0.f;
+  if (tid == 255) a_rate = -expf(in.a_log[h]), dt_off = in.dt_bias[h];
   pdl_wait();
   const TIN* row = proj + (size_t)b * in.row_stride;
   // the first tile of S is asked for before anything else
@@ -546,12 +555,12 @@ delta_decode_kernel(const TIN* __restrict__ proj, const DeltaIn in, float* __res
   if (tid == 255) {
     sums[3] = dr_sigmoid(dr_value(row, in.b_off + h, in.n_split, in.split_stride));
     const float a = dr_value(row, in.a_off + h, in.n_split, in.split_stride);
-    sums[4] = expf(-expf(in.a_log[h]) * dr_softplus(a + in.dt_bias[h]));
+    sums[4] = expf(a_rate * dr_softplus(a + dt_off));
   }
   // ---- convolution, activation; the token's projected row joins the ring
   const int p_place = p % taps;
   for (int e = tid; e < 2 * D + Dv; e += 256) {
-    const int c = e < D ? j * D + e : e < 2 * D ? G * D + j * D + (e - D) : 2 * G * D + h * Dv + (e - 2 * D);
+    const int c = channel(e);
     const float own = dr_value(row, dr_column(in, c), in.n_split, in.split_stride);
     float acc = 0.f;
     int place = p_place;                                  // the row of position p - taps + 1: the one behind p's

@@ -172,6 +172,9 @@ head_product_mma_kernel(const bf16* __restrict__ x, size_t x_ld, const bf16* __r
     xr[j] = x + ((size_t)(x_live[j] ? t : 0) * H + h) * x_ld;
   }
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  // few tokens: the warp's rows are on their way to L2 while the kernel before runs (in a decode step they come from memory)
+  if (TN == 1)
+    for (int i = lane * 64; i < min(16, N - n0) * K; i += 32 * 64) prefetch_l2(w + ((size_t)h * N + n0) * K + i);
   pdl_wait();
 #pragma unroll(TN == 1 ? 8 : 4)
   for (int k0 = 0; k0 < K; k0 += 32) {

@@ -365,6 +365,14 @@ ss_out_kernel(const SsProj proj, const SsDims dm, const float* __restrict__ xs, 
   };
   copy_rows(0);
   fetch_c(0);
+  // the rest is on its way to L2 meanwhile: rows of E, z and the products C . B
+  for (int i = tid; i < 2 * dm.N; i += SS_THREADS)
+    if (c0 + (i & 1) * 32 < Pp) prefetch_l2(st + ((size_t)slot * dm.H + h) * dm.N * Pp + (size_t)(i >> 1) * Pp + c0 + (i & 1) * 32);
+  for (int i = tid; i < 128; i += SS_THREADS) {
+    prefetch_l2(cb + ((size_t)slot * dm.G + g) * 4096 + i * 32);
+    if ((i >> 1) < ck.n && c0 + (i & 1) * 32 < dm.P)
+      prefetch_l2(proj.p + (size_t)(ck.t0 + (i >> 1)) * proj.row_stride + h * dm.P + c0 + (i & 1) * 32);
+  }
   const float2 own = tid < ck.n ? da[(size_t)h * n_tokens + ck.t0 + tid] : make_float2(1.f, 0.f);    // this token's a and dt
   a_s[tid] = own.x;
   float acc[8][8];
@@ -452,7 +460,8 @@ ss_out_kernel(const SsProj proj, const SsDims dm, const float* __restrict__ xs, 
     for (int half = 0; half < 2; ++half) {
       const int p = c0 + j0 + 32 * half;
       if (p >= dm.P) continue;
-      const float4 x = ss_load4(xs + (t * dm.H + h) * Pp + p);
+      // (the chunk's x are what the last steps read: tokens from 32 on in the other buffer)
+      const float4 x = ss_load4(Bs[(e_steps + (i >> 5)) & 1] + (i & 31) * 64 + j0 + 32 * half);
       const float* ar = acc[r] + 4 * half;
       float v[4] = {fmaf(dsk, x.x, ar[0]), fmaf(dsk, x.y, ar[1]), fmaf(dsk, x.z, ar[2]), fmaf(dsk, x.w, ar[3])};
       float* dst = y + t * inner + (size_t)h * dm.P + p;
@@ -556,13 +565,23 @@ ss_decode_kernel(const SsProj proj, const SsDims dm, const float* __restrict__ c
   float* base = state + (size_t)sl * slot_stride;
   float* S = base + (size_t)h * N * P + pc;
   float* ring = base + ring_off;
+  // the head's state, its channels' ring rows and weights are on their way to L2 while the kernel before runs (four tokens, 64
+  // heads of 128 x 64: 12.5 -> 11.4 us of a step's chain)
+  for (int i = tid * 32; i < N * P; i += 256 * 32) prefetch_l2(base + (size_t)h * N * P + i);
+  auto channel = [&](int idx) { return idx < P ? h * P + idx : idx < P + N ? inner + g * N + idx - P : inner + dm.G * N + g * N + idx - P - N; };
+  for (int idx = tid; idx < P + 2 * N; idx += 256) {
+    const int c = channel(idx);
+    for (int j = 0; j < taps; ++j) prefetch_l2(conv_w + (size_t)j * C + c), prefetch_l2(ring + (size_t)j * C + c);
+    if (conv_b) prefetch_l2(conv_b + c);
+  }
+  const float a_rate = -expf(a_log[h]), dt_off = dt_bias[h], skip_h = skip[h];
   pdl_wait();
   float s[U][V];
 #pragma unroll
   for (int u = 0; u < U; ++u)
     if (live && nr + u * R < N) ss_loadv<V>(S + (size_t)(nr + u * R) * P, s[u]);
   for (int idx = tid; idx < P + 2 * N; idx += 256) {    // the head's x, its group's B and C
-    const int c = idx < P ? h * P + idx : idx < P + N ? inner + g * N + idx - P : inner + dm.G * N + g * N + idx - P - N;
+    const int c = channel(idx);
     const float u = proj.at(b, inner + c);
     float v = conv_b ? conv_b[c] : 0.f;
     for (int j = 0; j < taps - 1; ++j) {
@@ -576,8 +595,8 @@ ss_decode_kernel(const SsProj proj, const SsDims dm, const float* __restrict__ c
     else if (idx < P + N) b_s[idx - P] = v;
     else c_s[idx - P - N] = v;
   }
-  const float dt = ss_softplus(proj.at(b, inner + C + h) + dt_bias[h]);
-  const float a = expf(-expf(a_log[h]) * dt);
+  const float dt = ss_softplus(proj.at(b, inner + C + h) + dt_off);
+  const float a = expf(a_rate * dt);
   __syncthreads();
   if (live) {
     float xd[V], acc[V];
@@ -607,7 +626,7 @@ ss_decode_kernel(const SsProj proj, const SsDims dm, const float* __restrict__ c
   for (int p = tid; p < P; p += 256) {
     float v = 0.f;
     for (int r = 0; r < R; ++r) v += red[r * Pp + p];
-    v = fmaf(skip[h], x_s[p], v);
+    v = fmaf(skip_h, x_s[p], v);
     y[(size_t)b * inner + (size_t)h * P + p] = v * ss_silu(proj.at(b, h * P + p));
   }
 }
