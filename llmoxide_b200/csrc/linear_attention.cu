@@ -42,7 +42,7 @@
 //   decay_chunk   per (chunk, head): the chunk's own part of E', and the 64 x 64 products q_i . k_j
 //   decay_pass    walks a sequence's chunks in order: leaves every chunk its E and the sequence its new state
 //   decay_out     per (chunk, head, 64 columns): the outputs
-// Four prompts of 700 to 1300 tokens, 16 heads of 128 x 128: 291 us, where the recurrence in segments took 586 (two
+// Four prompts of 700 to 1300 tokens, 16 heads of 128 x 128: 255 us, where the recurrence in segments took 586 (two
 // passes); off the 64-bit result by 2.7e-7 (3.4e-7).
 #include "chunk_products.cuh"
 
@@ -108,6 +108,94 @@ decay_prep_kernel(const TIN* __restrict__ proj, int n_split, size_t split_stride
   }
   for (int c = threadIdx.x; c < Dvp; c += blockDim.x)
     out[2 * Dp + c] = c < Dv ? la_act(la_value(vrow, c, n_split, split_stride), act) : (c == Dv && v_ones) ? 1.f : 0.f;
+}
+
+// Four neighbouring elements, a vector a partial; partials are added in order, seven asked for together.
+__device__ __forceinline__ void la_load(const float* p, float (&v)[4]) {
+  const float4 f = *reinterpret_cast<const float4*>(p);
+  v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
+}
+__device__ __forceinline__ void la_load(const bf16* p, float (&v)[4]) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  v[0] = __uint_as_float(u.x << 16), v[1] = __uint_as_float(u.x & 0xffff0000u);
+  v[2] = __uint_as_float(u.y << 16), v[3] = __uint_as_float(u.y & 0xffff0000u);
+}
+template <typename TIN>
+__device__ __forceinline__ void la_values(const TIN* p, int n_split, size_t split_stride, float (&v)[4]) {
+  la_load(p, v);
+  for (int s0 = 1; s0 < n_split; s0 += 7) {
+    float t[7][4];
+#pragma unroll
+    for (int s = 0; s < 7; ++s)
+      if (s0 + s < n_split) la_load(p + (size_t)(s0 + s) * split_stride, t[s]);
+#pragma unroll
+    for (int s = 0; s < 7; ++s)
+      if (s0 + s < n_split)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] += t[s][i];
+  }
+}
+
+// The same by four neighbouring dims a thread (sizes, rotated dims halved, offsets and strides all multiples of 4, whole
+// vectors, no column of ones): what decay_prep_kernel read and wrote an element at a time.  A thread takes the same piece of
+// TOKS tokens (2 in prompts, whose loads are then under way together).  Bound by the rows it writes: 4100 tokens, 16 heads of
+// 128: 72 us an element a thread, 36 like this (150 MB, 23 us at the copy's rate); with four tokens a thread and room for
+// partials in the same instance 107 (registers).  Four tokens in a decode step: 4.4 -> 2.5 us.
+template <typename TIN, int TOKS, bool SPLIT>
+__global__ void __launch_bounds__(128)
+decay_prep_vec_kernel(const TIN* __restrict__ proj, int n_split, size_t split_stride, size_t row_stride, int q_off, int k_off,
+                      int v_off, float* __restrict__ prep, const int* __restrict__ token_pos, const float* __restrict__ cos_t,
+                      const float* __restrict__ sin_t, int n_rot, int act, float k_scale, float q_scale, int n_tokens, int H,
+                      int D, int Dv) {
+  pdl_launch_dependents();
+  // a head's pieces: of q and of k the pairs (i, i + half) of the rotated dims, then the other dims; then v
+  const unsigned half = n_rot >> 1, pairs = half >> 2, per = pairs + ((D - n_rot) >> 2), pieces = 2 * per + (Dv >> 2);
+  const unsigned idx = blockIdx.x * 128u + threadIdx.x, gh = idx / pieces, piece = idx - gh * pieces, t0 = gh / H * TOKS, h = gh % H;
+  pdl_wait();
+  if (t0 >= (unsigned)n_tokens) return;
+  // where the piece comes from and goes to, in its token's row and its head's
+  const bool is_v = piece >= 2 * per, is_k = !is_v && piece >= per;
+  const unsigned q = is_v ? piece - 2 * per : is_k ? piece - per : piece;
+  const bool rotated = !is_v && q < pairs;
+  const unsigned d = is_v || rotated ? q * 4 : n_rot + (q - pairs) * 4;
+  const TIN* src = proj + (is_v ? v_off + h * Dv : (is_k ? k_off : q_off) + h * D) + d;
+  float* dst = prep + (size_t)h * (2 * D + Dv) + (is_v ? 2 * D : is_k ? D : 0) + d;
+  const float scale = is_v ? 1.f : is_k ? k_scale : q_scale;
+  const size_t to_step = (size_t)H * (2 * D + Dv);
+  auto put = [](float* to, const float (&v)[4]) { *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]); };
+  float x[TOKS][4], y[TOKS][4], c[TOKS][4], sn[TOKS][4];
+#pragma unroll
+  for (int j = 0; j < TOKS; ++j) {
+    const unsigned t = min(t0 + j, (unsigned)n_tokens - 1);
+    const TIN* from = src + (size_t)t * row_stride;
+    if (SPLIT) la_values(from, n_split, split_stride, x[j]);
+    else la_load(from, x[j]);
+    if (rotated) {
+      if (SPLIT) la_values(from + half, n_split, split_stride, y[j]);
+      else la_load(from + half, y[j]);
+      const size_t at = (size_t)token_pos[t] * half + d;
+      la_load(cos_t + at, c[j]);
+      la_load(sin_t + at, sn[j]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < TOKS; ++j) {
+    if (t0 + j >= (unsigned)n_tokens) break;
+    float* to = dst + (size_t)(t0 + j) * to_step;
+    if (rotated) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float u = la_act(x[j][i], act), w = la_act(y[j][i], act);
+        x[j][i] = (u * c[j][i] - w * sn[j][i]) * scale;
+        y[j][i] = (w * c[j][i] + u * sn[j][i]) * scale;
+      }
+      put(to + half, y[j]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[j][i] = la_act(x[j][i], act) * scale;
+    }
+    put(to, x[j]);
+  }
 }
 
 __device__ __forceinline__ void la_cp_async16(float* dst, const float* src) {
@@ -184,6 +272,8 @@ decay_scan_kernel(const float* __restrict__ prep, float* __restrict__ out, float
   const int t0 = seq_t0 + seg * seg_len;                                      // the segment's first token
   const int n_new = min(seg_len, seq_new - seg * seg_len);
   float* part_seq = partial ? partial + ((size_t)b * H + h) * (size_t)n_seg_max * D * Dv : nullptr;
+  if (PASS == 1 && seg == 0)           // this CTA's columns of the state, on their way to L2 while the kernel before runs
+    for (int d = tid; d < D; d += blockDim.x) prefetch_l2(S + (size_t)d * Dv + c0);
   pdl_wait();
 
   auto own = [&](int i) { return 4 * (r + 8 * (i >> 2)) + (i & 3); };        // dim of this thread's i-th state value
@@ -696,6 +786,10 @@ decay_out_kernel(const float* __restrict__ prep, const float* __restrict__ decay
   };
   copy_rows(0);
   fetch_q(0);
+  // the rest is on its way to L2 meanwhile: rows of E and the products q . k
+  for (int i = tid; i < 2 * dm.D; i += SS_THREADS)
+    if (c0 + (i & 1) * 32 < Dvp) prefetch_l2(st + ((size_t)slot * dm.H + h) * dm.D * Dvp + (size_t)(i >> 1) * Dvp + c0 + (i & 1) * 32);
+  for (int i = tid; i < 128; i += SS_THREADS) prefetch_l2(cb + ((size_t)slot * dm.H + h) * 4096 + i * 32);
   power[tid] = (float)la_power(g, tid);
   if (tid == 0) power[SS_CHUNK] = (float)la_power(g, SS_CHUNK);
   float acc[8][8];
@@ -923,16 +1017,35 @@ LLMX_API int llmx_decay_scan(const void* proj, int in_dtype, int n_split, long l
   const bool by_chunks = n_seg > 1 && llmx_decay_scan_by_chunks(gates != nullptr, D, Dva);
   if (n_seg > 1 && (!partial || (by_chunks && ((uintptr_t)partial & 15)))) return LLMX_REFUSED(4);
   const dim3 pgrid(n_tokens, H);
-  if (in_dtype == LLMX_F32)
-    launch_pdl(decay_prep_kernel<float>, pgrid, dim3(128), 0, stream, (const float*)proj, n_split, (size_t)split_stride,
-               (size_t)row_stride, q_off, k_off, v_off, prep, token_pos, cos_t, sin_t, n_rot, act, k_scale, q_scale,
-               v_ones, H, D, Dv);
-  else if (in_dtype == LLMX_BF16)
-    launch_pdl(decay_prep_kernel<bf16>, pgrid, dim3(128), 0, stream, (const bf16*)proj, n_split, (size_t)split_stride,
-               (size_t)row_stride, q_off, k_off, v_off, prep, token_pos, cos_t, sin_t, n_rot, act, k_scale, q_scale,
-               v_ones, H, D, Dv);
-  else
+  const int esz = in_dtype == LLMX_F32 ? 4 : 2;
+  const bool vec = !v_ones && ((D | Dv | (n_rot >> 1) | q_off | k_off | v_off) & 3) == 0 && ((row_stride | split_stride) & 3) == 0 &&
+                   ((uintptr_t)proj & (4 * esz - 1)) == 0 &&
+                   (((uintptr_t)cos_t | (uintptr_t)sin_t) & 15) == 0;
+  const bool many = n_tokens > 64 && n_split == 1;
+  const long long pieces = (long long)(many ? (n_tokens + 1) / 2 : n_tokens) * H * ((n_rot >> 2) + ((D - n_rot) >> 1) + (Dv >> 2));
+  const dim3 vgrid((unsigned)((pieces + 127) / 128));
+#define PREP_VEC(TIN, TOKS, SPLIT)                                                                                                 \
+  launch_pdl(decay_prep_vec_kernel<TIN, TOKS, SPLIT>, vgrid, dim3(128), 0, stream, (const TIN*)proj, n_split, (size_t)split_stride, \
+             (size_t)row_stride, q_off, k_off, v_off, prep, token_pos, cos_t, sin_t, n_rot, act, k_scale, q_scale, n_tokens, \
+             H, D, Dv)
+#define PREP(TIN)                                                                                                           \
+  if (vec && many && pieces < (1ll << 32) - 128)                                                                            \
+    PREP_VEC(TIN, 2, false);                                                                                                       \
+  else if (vec && pieces < (1ll << 32) - 128)                                                                               \
+    PREP_VEC(TIN, 1, true);                                                                                                       \
+  else                                                                                                                      \
+    launch_pdl(decay_prep_kernel<TIN>, pgrid, dim3(128), 0, stream, (const TIN*)proj, n_split, (size_t)split_stride,        \
+               (size_t)row_stride, q_off, k_off, v_off, prep, token_pos, cos_t, sin_t, n_rot, act, k_scale, q_scale,        \
+               v_ones, H, D, Dv)
+  if (in_dtype == LLMX_F32) {
+    PREP(float);
+  } else if (in_dtype == LLMX_BF16) {
+    PREP(bf16);
+  } else {
     return LLMX_REFUSED(2);
+  }
+#undef PREP
+#undef PREP_VEC
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   Dv = Dva;                                        // from here on the extra column is a column like the others
@@ -1067,6 +1180,67 @@ gated_norm_row_kernel(const float* __restrict__ o, const TIN* __restrict__ proj,
   }
 }
 
+// The same by four neighbouring elements a thread, U times (sizes, offsets and strides multiples of 4, no gates), everything
+// asked for ahead of the reduction: an element at a time, first the squares and then again the outputs, a row of 2048 with
+// five partials took 11.5 us in a decode step, 2.8 like this; 4100 rows 34 -> 28 (bound by memory).  U 0: a warp per (token,
+// head) of up to 128 columns: 6.4 -> 1.9 us and 34 -> 27.
+template <typename TIN, typename TO, int U>
+__global__ void __launch_bounds__(U ? 512 : 128)
+gated_norm_vec_kernel(const float* __restrict__ o, const TIN* __restrict__ proj, int n_split, size_t split_stride,
+                      size_t row_stride, int g_off, const float* __restrict__ gain, float eps, int gate_act,
+                      TO* __restrict__ y, int n_rows, int n, int H) {
+  __shared__ float red[32];
+  constexpr int PARTS = U ? U : 1, LANES = U ? 512 : 32;
+  pdl_launch_dependents();
+  const int lane = U ? threadIdx.x : threadIdx.x & 31, r = U ? blockIdx.x : blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int t = U ? r : r / H, h = U ? 0 : r - t * H;                  // row r of n elements: a token, or a head of one
+  float w[PARTS][4];
+#pragma unroll
+  for (int u = 0; u < PARTS; ++u) {
+    const int i = (u * LANES + lane) * 4;
+    if (gain && i < n) la_load(gain + h * n + i, w[u]);
+  }
+  pdl_wait();
+  if (!U && r >= n_rows) return;                                       // (uniform over a warp)
+  const float* orow = o + (size_t)r * n;
+  const TIN* grow = proj + (size_t)t * row_stride + g_off + h * n;
+  float v[PARTS][4], z[PARTS][4], ss = 0.f;
+#pragma unroll
+  for (int u = 0; u < PARTS; ++u) {
+    const int i = (u * LANES + lane) * 4;
+    if (i < n) la_load(orow + i, v[u]);
+    else v[u][0] = v[u][1] = v[u][2] = v[u][3] = 0.f;
+  }
+#pragma unroll
+  for (int u = 0; u < PARTS; ++u) {
+    const int i = (u * LANES + lane) * 4;
+    if (i < n) la_values(grow + i, n_split, split_stride, z[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < PARTS; ++u) ss += (v[u][0] * v[u][0] + v[u][1] * v[u][1]) + (v[u][2] * v[u][2] + v[u][3] * v[u][3]);
+  ss = U ? block_sum(ss, red) : warp_sum(ss);
+  const float rs = 1.0f / sqrtf(ss / (float)n + eps);
+#pragma unroll
+  for (int u = 0; u < PARTS; ++u) {
+    const int i = (u * LANES + lane) * 4;
+    if (i >= n) continue;
+    float f[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      f[e] = v[u][e] * rs;
+      if (gain) f[e] *= w[u][e];
+      f[e] *= la_act(z[u][e], gate_act);
+    }
+    TO* dst = y + (size_t)r * n + i;
+    if constexpr (sizeof(TO) == 4) {
+      *reinterpret_cast<float4*>(dst) = make_float4(f[0], f[1], f[2], f[3]);
+    } else {
+      const __nv_bfloat162 a = __floats2bfloat162_rn(f[0], f[1]), b = __floats2bfloat162_rn(f[2], f[3]);
+      *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+    }
+  }
+}
+
 // per_head != 0: the mean of squares is a head's; else the token's.  gain: float32 [H*Dv] or null.  gates (per_head
 // only): see the kernel; o is then [T, H, Dv + 1].
 LLMX_API int llmx_gated_norm(const float* o, const void* proj, int in_dtype, int n_split, long long split_stride,
@@ -1077,9 +1251,23 @@ LLMX_API int llmx_gated_norm(const float* o, const void* proj, int in_dtype, int
   if (H <= 0 || Dv <= 0 || n_split < 1 || (gates && !per_head)) return LLMX_REFUSED(1);
   const int o_stride = gates ? Dv + 1 : Dv;
   if (gate_act != LA_ACT_SILU && gate_act != LA_ACT_SIGMOID && gate_act != LA_ACT_NONE) return LLMX_REFUSED(1);
+  // four elements a thread where every row, gate and gain is whole vectors, and a row fits a CTA (a head a warp)
+  const int n = per_head ? Dv : H * Dv, in_size = in_dtype == LLMX_F32 ? 4 : 2, out_size = out_dtype == LLMX_F32 ? 4 : 2;
+  const bool vec = !gates && n % 4 == 0 && g_off % 4 == 0 && row_stride % 4 == 0 && split_stride % 4 == 0 &&
+                   n <= (per_head ? 128 : 8192) && (long long)n_tokens * H < (1ll << 31) && !((uintptr_t)o & 15) &&
+                   !((uintptr_t)gain & 15) && !((uintptr_t)proj & (4 * in_size - 1)) && !((uintptr_t)y & (4 * out_size - 1));
+#define VEC(TIN, TO, U)                                                                                              \
+  launch_pdl(gated_norm_vec_kernel<TIN, TO, U>, dim3(U ? n_tokens : (n_tokens * H + 3) / 4), dim3(U ? 512 : 128), 0, \
+             stream, o, (const TIN*)proj, n_split, (size_t)split_stride, (size_t)row_stride, g_off, gain, eps, gate_act, \
+             (TO*)y, per_head ? n_tokens * H : n_tokens, n, H)
 #define GO(TIN, TO)                                                                                                  \
   do {                                                                                                               \
-    if (per_head)                                                                                                    \
+    if (vec) {                                                                                                       \
+      if (per_head) VEC(TIN, TO, 0);                                                                                 \
+      else if (n <= 2048) VEC(TIN, TO, 1);                                                                           \
+      else if (n <= 4096) VEC(TIN, TO, 2);                                                                           \
+      else VEC(TIN, TO, 4);                                                                                          \
+    } else if (per_head)                                                                                                    \
       launch_pdl(gated_norm_heads_kernel<TIN, TO>, dim3(n_tokens, (H + 3) / 4), dim3(128), 0, stream, o,             \
                  (const TIN*)proj, n_split, (size_t)split_stride, (size_t)row_stride, g_off, gain, eps, gate_act,    \
                  (TO*)y, H, Dv, o_stride, gates, den_eps);                                                                                  \
@@ -1096,5 +1284,6 @@ LLMX_API int llmx_gated_norm(const float* o, const void* proj, int in_dtype, int
     default: return LLMX_REFUSED(2);
   }
 #undef GO
+#undef VEC
   return LLMX_LAUNCH_STATUS();
 }

@@ -44,3 +44,22 @@ def test_heads_of_64_and_unrotated_heads(D, n_rot, H, G, T, n_split, gains):
     assert rel(q.view(T, H, D), made(row[:, :H], gq)) < 2 ** -8
     assert rel(torch.stack([kc[a, :, r] for a, r in where]), made(row[:, H : H + G], gk)) < 2 ** -8
     assert torch.equal(torch.stack([vc[a, :, r] for a, r in where]), row[:, H + G :].float().bfloat16())
+
+
+@pytest.mark.parametrize("dtype, n_split", [(torch.bfloat16, 1), (torch.float32, 1), (torch.float32, 9)])
+@pytest.mark.parametrize("per_head, H, Dv", [(True, 3, 128), (True, 5, 20), (False, 4, 128), (False, 3, 700), (False, 17, 300),
+                                             (True, 2, 132), (False, 1, 8196)])
+def test_gated_norm_by_vectors(dtype, n_split, per_head, H, Dv):
+    """A row or head of whole vectors, and the first size beyond, against 64 bits; float32 throughout: sums of up to 8196
+    squares in chains of at most 33 and trees, 1e-6."""
+    from llmoxide_b200 import kernels
+    torch.manual_seed(H * Dv)
+    T, n = 7, H * Dv
+    o, gain = torch.randn(T, n, device=DEV), 1 + 0.1 * torch.randn(n, device=DEV)
+    proj = torch.randn(n_split, T, n + 8, device=DEV).to(dtype)
+    z = proj.double().sum(0)[:, 8:]
+    y = torch.empty(T, n, device=DEV)
+    kernels.gated_norm(o, proj[0] if n_split == 1 else proj, 8, gain, 1e-5, "silu", per_head, y, H, Dv)
+    v = o.double().view(T, H, Dv) if per_head else o.double().view(T, 1, n)
+    v = (v / (v.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt()).view(T, n)
+    assert rel(y, v * gain.double() * z * torch.sigmoid(z)) < 1e-6
