@@ -29,19 +29,18 @@ enum { MOE_SCORE_SIGMOID = 0, MOE_SCORE_SOFTMAX = 1, MOE_SCORE_SOFTMAX_TOP = 2 }
 // With a correction (`bias`, one number per expert) the groups are ranked and the experts chosen by s + bias,
 // while the weights stay the chosen experts' s.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void warp_argmax(float& v, int& i) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float v2 = __shfl_xor_sync(0xffffffffu, v, o);
-    const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-    if (v2 > v || (v2 == v && i2 < i)) v = v2, i = i2;
-  }
+// The largest v of the warp above -inf and the lowest i that goes with it; none: i = 0x7fffffff.  (NaN is not above -inf.)
+// Two reductions over the warp by the hardware, on integers in the order of the floats, in place of five rounds of two shuffles.
+__device__ __forceinline__ int warp_argmax(float v, int i) {
+  const int bits = __float_as_int(v + 0.0f);                       // (-0 and +0 are equal)
+  const unsigned key = v > -INFINITY ? (unsigned)bits ^ (bits < 0 ? 0xffffffffu : 0x80000000u) : 0u;
+  const unsigned top = __reduce_max_sync(0xffffffffu, key);
+  return (int)__reduce_min_sync(0xffffffffu, top != 0u && key == top ? (unsigned)i : 0x7fffffffu);
 }
 
 // One token, by one warp: z its E logits (global or shared memory), s, c and gs scratch of E, E and n_groups
-// floats (c: the scores the choice goes by), ids and wts its `top` outputs.
-__device__ __forceinline__ void moe_route_token(const float* z, float* s, float* c, float* gs, int* __restrict__ ids,
-                                                float* __restrict__ wts, int lane, int E, int top, int n_groups,
+// floats (c: the scores the choice goes by).  Lane k < top returns the k-th choice and its weight.
+__device__ __forceinline__ void moe_route_token(const float* z, float* s, float* c, float* gs, int& id, float& weight, int lane, int E, int top, int n_groups,
                                                 int keep_groups, int group_top, int score_kind, int normalize,
                                                 float norm_eps, float scale, const float* __restrict__ bias) {
   if (score_kind == MOE_SCORE_SOFTMAX) {
@@ -91,8 +90,8 @@ __device__ __forceinline__ void moe_route_token(const float* z, float* s, float*
       int bi = 0x7fffffff;
       for (int g = lane; g < n_groups; g += 32)
         if (gs[g] > best) best = gs[g], bi = g;     // ascending g: the lower index wins a tie
-      warp_argmax(best, bi);
-      if (lane == 0) gs[bi] = -INFINITY;            // kept: marked
+      bi = warp_argmax(best, bi);
+      if (lane == 0 && bi < n_groups) gs[bi] = -INFINITY;            // kept: marked (no group: all their scores are NaN)
       __syncwarp();
     }
     for (int e = lane; e < E; e += 32)
@@ -106,15 +105,14 @@ __device__ __forceinline__ void moe_route_token(const float* z, float* s, float*
     int bi = 0x7fffffff;
     for (int e = lane; e < E; e += 32)
       if (c[e] > best) best = c[e], bi = e;
-    warp_argmax(best, bi);
+    bi = warp_argmax(best, bi);
     if (bi >= E) {
       // No score compares greater than -inf: the token's row holds a NaN (or every score is -inf).  That is
       // reported (code 1); the lowest expert not chosen yet stands in, so that no index leaves its array.
       bi = 0x7fffffff;
       for (int e = lane; e < E; e += 32)
         if (!(c[e] == -INFINITY) && e < bi) bi = e;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) bi = min(bi, __shfl_xor_sync(0xffffffffu, bi, o));
+      bi = (int)__reduce_min_sync(0xffffffffu, (unsigned)bi);
       if (bi >= E) bi = k % E;
       if (lane == 0) llmx_report(1);
     }
@@ -130,17 +128,11 @@ __device__ __forceinline__ void moe_route_token(const float* z, float* s, float*
     const float z_max = warp_max(zk);
     const float ek = lane < top ? expf(zk - z_max) : 0.f;
     const float total = warp_sum(ek);
-    if (lane < top) {
-      ids[lane] = my_id;
-      wts[lane] = (ek / total) * scale;
-    }
+    id = my_id, weight = (ek / total) * scale;
     return;
   }
-  if (lane < top) {
-    const float w = normalize ? mine / (sum + norm_eps) : mine;
-    ids[lane] = my_id;
-    wts[lane] = w * scale;
-  }
+  const float w = normalize ? mine / (sum + norm_eps) : mine;
+  id = my_id, weight = w * scale;
 }
 
 __global__ void moe_route_kernel(const float* __restrict__ logits, int* __restrict__ ids, float* __restrict__ wts,
@@ -154,20 +146,54 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, int* __restri
   const int t = blockIdx.x * 4 + warp;
   if (t >= n_tokens) return;
   float* s = route_smem + warp * (2 * E + n_groups);
-  moe_route_token(logits + (size_t)t * E, s, s + E, s + 2 * E, ids + (size_t)t * top, wts + (size_t)t * top, lane, E, top,
-                  n_groups, keep_groups, group_top, score_kind, normalize, norm_eps, scale, bias);
+  int id;
+  float weight;
+  moe_route_token(logits + (size_t)t * E, s, s + E, s + 2 * E, id, weight, lane, E, top, n_groups, keep_groups, group_top,
+                  score_kind, normalize, norm_eps, scale, bias);
+  if (lane < top) ids[(size_t)t * top + lane] = id, wts[(size_t)t * top + lane] = weight;
 }
 
-// The router's product and the routing in one kernel: a CTA of 8 warps takes TOK tokens (4 in a prompt step, so
-// that a row of the router's matrix is fetched once for four tokens; 1 in a step of few tokens, so that more SMs
-// take part); warp w computes the float32 logits of experts w, w + 8, ... two at a time (a lane adds its share of k in
-// ascending order, eight consecutive k at a time, then the lanes are added by a butterfly: the order depends on
-// nothing but K), then warp j routes token j.  The matrix may hold n_extra rows behind the experts' (a gate
-// that reads the same input): their logits are written to extra_out [T, n_extra] as they are.
-// A step of few tokens waits for nothing but loads: the matrix is brought to L2 while the kernel before still runs, and a
-// lane has eight blocks of it under way.  Prompts convert a token's values once for two experts.
-// 16 experts in 4 groups, K = 2048: 4 tokens 8.1 -> 5.9 us (of which 2 us are a launch's), 4100 tokens 28 -> 24;
-// 64 experts in 8 groups: 4 tokens 23.1 -> 15.7, 4000 tokens 96 -> 79.
+// The router's product and the routing in one kernel: a CTA takes TOK tokens; warp w of n computes the float32 logits of
+// experts w, w + n, ... two at a time (a lane adds its share of k in ascending order, eight consecutive k at a time, then
+// the lanes are added by a butterfly: the order depends on nothing but K), then warp j routes token j.  The matrix may
+// hold n_extra rows behind the experts' (a gate that reads the same input): their logits are written to extra_out
+// [T, n_extra] as they are.
+// Prompts: four tokens a CTA.  (Eight, and sixteen with their rows by asynchronous copies through shared memory, read
+// the matrix less often and took longer: 4100 tokens, 16 experts 23.5 us by four, 29 and 24.5 by eight and sixteen; 64 experts
+// 73, 87 and 77.)
+// Steps of few tokens wait for nothing but loads: the matrix is brought to L2 while the kernel before still runs, and sixteen
+// warps share the experts.
+// PLACE (steps of up to 8 tokens): the CTAs are one cluster, which knows every choice behind one barrier, so each CTA also
+// finds its own pairs' places in the order by experts (what moe_sort_kernel makes in a launch of its own, with the places
+// inside an expert in the order of the pairs), copies its token's row there, and the first one writes the list of tiles.
+// Four tokens, top 4, K = 2048, the three launches and this one: 16 experts 9.9 and 7.8 us, 64 experts 20.1 and 12.7.  (With
+// several tokens a CTA it took longer than the three from 12 tokens on: 9.7 and 9.2 us, 64 experts 17.1 and 9.3.)
+// Eight values as they lie in memory, asked for in the order of the source.
+template <typename T>
+struct Moe8;
+template <>
+struct Moe8<float> {
+  float4 a, b;
+  __device__ __forceinline__ void load(const float* p) {
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w) : "l"(p) : "memory");
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(p + 4) : "memory");
+  }
+  __device__ __forceinline__ void get(float (&v)[8]) const {
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+  }
+};
+template <>
+struct Moe8<bf16> {
+  uint32_t raw[4];
+  __device__ __forceinline__ void load(const bf16* p) {
+    asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(raw[0]), "=r"(raw[1]), "=r"(raw[2]), "=r"(raw[3]) : "l"(p) : "memory");
+  }
+  __device__ __forceinline__ void get(float (&v)[8]) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[2 * i] = __uint_as_float(raw[i] << 16), v[2 * i + 1] = __uint_as_float(raw[i] & 0xffff0000u);
+  }
+};
+
 __device__ __forceinline__ void moe_load8(const float* p, float* v) {
   const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
   v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
@@ -182,14 +208,95 @@ __device__ __forceinline__ void moe_load8(const bf16* p, float* v) {
   }
 }
 
-template <typename TX, int TOK>
-__global__ void __launch_bounds__(256)
+struct MoePlaces {             // what moe_sort_kernel writes, and the rows in that order (bfloat16 [P, K])
+  int *perm, *dest, *tiles;
+  float* sorted_weight;
+  bf16* xs;
+  int max_tiles, tile_rows, n_tiled;
+};
+#define MOE_PLACE_TOKENS 8     // a CTA each, in one cluster
+
+// Behind the routing: own_ids/own_wts hold the `top` pairs of token t, row its values (eight a thread, the first 8 THREADS).
+template <int THREADS>
+__device__ __forceinline__ void moe_place(const MoePlaces pl, const int* own_ids, const float* own_wts, int* all_ids, int* count,
+                                          int* place, const bf16* __restrict__ xr, uint4 row, int t, int n_tokens, int K, int E,
+                                          int top) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, P = n_tokens * top;
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  for (int i = tid; i < P; i += THREADS) {
+    const int cta = i / top;
+    uint32_t there;
+    int v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(there) : "r"((uint32_t)__cvta_generic_to_shared(own_ids + (i - cta * top))), "r"(cta));
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(there) : "memory");
+    all_ids[i] = v;
+  }
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");       // (waited for at the end: others may still read)
+  for (int p = warp; p < top; p += THREADS / 32) {
+    const int e = own_ids[p], r = t * top + p;
+    unsigned before = 0;
+    for (int i = lane; i < P; i += 32) before += all_ids[i] < e || (all_ids[i] == e && i < r);
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) {
+      place[p] = (int)before;
+      pl.perm[before] = r;
+      pl.dest[before] = p * n_tokens + t;
+      pl.sorted_weight[before] = own_wts[p];
+    }
+  }
+  __syncthreads();
+  for (int c = tid * 8; c < K; c += THREADS * 8) {
+    if (c != tid * 8) row = *reinterpret_cast<const uint4*>(xr + c);
+    for (int p = 0; p < top; ++p) *reinterpret_cast<uint4*>(pl.xs + (size_t)place[p] * K + c) = row;
+  }
+  if (t == 0) {                // the first CTA: rows and tiles of the experts, in one scan (rows below, tiles above 16 bits)
+    int carry = 0;
+    for (int e0 = 0; e0 < E; e0 += THREADS) {
+      const int e = e0 + tid;
+      int n = 0;
+      for (int i = 0; i < P; ++i) n += all_ids[i] == e;
+      const int mine = e < E ? n | ((e < pl.n_tiled ? (n + pl.tile_rows - 1) / pl.tile_rows : 0) << 16) : 0;
+      int sum = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+      }
+      if (lane == 31) count[warp] = sum;
+      __syncthreads();
+      sum += carry;
+      for (int w = 0; w < THREADS / 32; ++w) {
+        if (w < warp) sum += count[w];
+        carry += count[w];
+      }
+      int at = (sum - mine) & 0xffff, tl = (sum - mine) >> 16;
+      if (e < E && e < pl.n_tiled)
+        for (int k = 0; k < n; k += pl.tile_rows, ++tl) {
+          pl.tiles[3 * tl] = e;
+          pl.tiles[3 * tl + 1] = at + k;
+          pl.tiles[3 * tl + 2] = min(n - k, pl.tile_rows);
+        }
+      __syncthreads();
+    }
+    for (int tl = (carry >> 16) + tid; tl < pl.max_tiles; tl += THREADS) pl.tiles[3 * tl] = -1;
+  }
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename TX, int TOK, int THREADS, bool PLACE>
+__global__ void __launch_bounds__(THREADS)
 moe_router_kernel(const TX* __restrict__ x, long long ldx, const float* __restrict__ w, int* __restrict__ ids,
                   float* __restrict__ wts, int n_tokens, int K, int E, int top, int n_groups, int keep_groups,
                   int group_top, int score_kind, int normalize, float norm_eps, float scale, int vec,
                   const float* __restrict__ bias, int n_extra, float* __restrict__ extra_out,
-                  const float* __restrict__ logit_bias) {
-  extern __shared__ float route_smem[];            // per token: E + n_extra logits, E scores, n_groups group scores
+                  const float* __restrict__ logit_bias, const MoePlaces places) {
+  // per token: E + n_extra logits, E scores, n_groups group scores; PLACE: this CTA's choices and weights, all choices,
+  // sums of the warps, places
+  extern __shared__ float route_smem[];
+  constexpr int WARPS = THREADS / 32;
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t0 = blockIdx.x * TOK;
@@ -200,11 +307,10 @@ moe_router_kernel(const TX* __restrict__ x, long long ldx, const float* __restri
     for (size_t at = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 128; at < bytes; at += (size_t)gridDim.x * blockDim.x * 128)
       asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(w) + at));
   }
-  pdl_wait();
-  const TX* xr[TOK];
-#pragma unroll
-  for (int j = 0; j < TOK; ++j) xr[j] = x + (size_t)min(t0 + j, n_tokens - 1) * ldx;
-  // rows e and, of two, e + 8 (a warp that has one row left does not read it twice)
+  const TX* x0 = x + (size_t)t0 * ldx;
+  const int last = n_tokens - 1 - t0;              // (rows past the last token repeat it)
+  uint4 row = {};                                  // PLACE: this thread's piece of the token's row, for its places
+  // rows e and, of two, e + WARPS (a warp that has one row left does not read it twice)
   auto products = [&](int e, auto rows) {
     constexpr int Q = decltype(rows)::value;
     float acc[Q][TOK];
@@ -213,15 +319,15 @@ moe_router_kernel(const TX* __restrict__ x, long long ldx, const float* __restri
 #pragma unroll
       for (int j = 0; j < TOK; ++j) acc[q][j] = 0.f;
     const float* wr = w + (size_t)e * K;
-    if (vec) {           // K a multiple of 8 and rows 16-byte aligned: 8 consecutive k per lane and step
-      constexpr int UNROLL = TOK == 1 ? 4 : Q == 1 ? 2 : 1;
+    if (vec && TOK > 1) {           // K a multiple of 8 and rows 16-byte aligned: 8 consecutive k per lane and step
+      constexpr int UNROLL = Q == 1 ? 2 : 1;
 #pragma unroll UNROLL
       for (int k = lane * 8; k < K; k += 256) {
         float wv[Q][8], xv[TOK][8];
 #pragma unroll
-        for (int q = 0; q < Q; ++q) moe_load8(wr + (size_t)q * 8 * K + k, wv[q]);
+        for (int q = 0; q < Q; ++q) moe_load8(wr + (size_t)q * WARPS * K + k, wv[q]);
 #pragma unroll
-        for (int j = 0; j < TOK; ++j) moe_load8(xr[j] + k, xv[j]);
+        for (int j = 0; j < TOK; ++j) moe_load8(x0 + (size_t)min(j, last) * ldx + k, xv[j]);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
 #pragma unroll
@@ -229,14 +335,42 @@ moe_router_kernel(const TX* __restrict__ x, long long ldx, const float* __restri
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc[q][j] = fmaf(xv[j][i], wv[q][i], acc[q][j]);
       }
+    } else if (vec) {
+      // U steps at a time, all their loads asked for before the first is used
+      auto steps = [&](int k, auto count) {
+        constexpr int U = decltype(count)::value;
+        Moe8<float> wv[U][Q];
+        Moe8<TX> xv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+#pragma unroll
+          for (int q = 0; q < Q; ++q) wv[u][q].load(wr + (size_t)q * WARPS * K + k + u * 256);
+          xv[u].load(x0 + k + u * 256);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          float v[8], f[8];
+          xv[u].get(v);
+#pragma unroll
+          for (int q = 0; q < Q; ++q) {
+            wv[u][q].get(f);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[q][0] = fmaf(v[i], f[i], acc[q][0]);
+          }
+        }
+      };
+      constexpr int U = 8 / Q;
+      int k = lane * 8;
+      for (; k + (U - 1) * 256 < K; k += U * 256) steps(k, std::integral_constant<int, U>());
+      for (; k < K; k += 256) steps(k, std::integral_constant<int, 1>());
     } else {
       for (int k0 = lane * 8; k0 < K; k0 += 256)
         for (int k = k0; k < k0 + 8 && k < K; ++k)
 #pragma unroll
           for (int q = 0; q < Q; ++q) {
-            const float wv = wr[(size_t)q * 8 * K + k];
+            const float wv = wr[(size_t)q * WARPS * K + k];
 #pragma unroll
-            for (int j = 0; j < TOK; ++j) acc[q][j] = fmaf(to_f32(xr[j][k]), wv, acc[q][j]);
+            for (int j = 0; j < TOK; ++j) acc[q][j] = fmaf(to_f32(x0[(size_t)min(j, last) * ldx + k]), wv, acc[q][j]);
           }
     }
 #pragma unroll
@@ -244,30 +378,58 @@ moe_router_kernel(const TX* __restrict__ x, long long ldx, const float* __restri
 #pragma unroll
       for (int j = 0; j < TOK; ++j) {
         const float v = warp_sum(acc[q][j]);
-        const int row = e + 8 * q;
+        const int row = e + WARPS * q;
         if (lane == 0) route_smem[j * per_tok + row] = (logit_bias && row < E) ? v + logit_bias[row] : v;
       }
   };
-  for (int e = warp; e < n_rows; e += 16) {
-    if (e + 8 < n_rows) products(e, std::integral_constant<int, 2>());
-    else products(e, std::integral_constant<int, 1>());
+  int* own_ids = reinterpret_cast<int*>(route_smem + TOK * per_tok);
+  float* own_wts = reinterpret_cast<float*>(own_ids + TOK * top);
+  // One token a CTA: the routing is run once ahead of the wait, on zeros and for nothing, so that its instructions are in the
+  // SM when the step waits for them.
+#pragma unroll 1
+  for (int pass = TOK == 1 ? 0 : 1; pass < 2; ++pass) {
+    if (pass == 0) {
+      for (int i = threadIdx.x; i < per_tok; i += THREADS) route_smem[i] = 0.f;
+    } else {
+      __syncthreads();
+      pdl_wait();
+      if constexpr (PLACE)
+        if ((int)threadIdx.x * 8 < K) row = *reinterpret_cast<const uint4*>(x0 + threadIdx.x * 8);
+      for (int e = warp; e < n_rows; e += 2 * WARPS) {
+        if (e + WARPS < n_rows) products(e, std::integral_constant<int, 2>());
+        else products(e, std::integral_constant<int, 1>());
+      }
+    }
+    __syncthreads();
+    for (int j = warp; j < TOK && t0 + j < n_tokens; j += WARPS) {
+      const int t = t0 + j;
+      float* z = route_smem + j * per_tok;
+      if (pass && lane < n_extra) extra_out[(size_t)t * n_extra + lane] = z[E + lane];
+      // (the logits are not needed once the scores exist: their place holds the choice scores)
+      int id;
+      float weight;
+      moe_route_token(z, z + n_rows, z, z + n_rows + E, id, weight, lane, E, top, n_groups, keep_groups, group_top, score_kind,
+                      normalize, norm_eps, scale, bias);
+      if (pass && lane < top) {
+        ids[(size_t)t * top + lane] = id, wts[(size_t)t * top + lane] = weight;
+        if (PLACE) own_ids[j * top + lane] = id, own_wts[j * top + lane] = weight;
+      }
+    }
   }
-  __syncthreads();
-  const int t = t0 + warp;
-  if (warp >= TOK || t >= n_tokens) return;
-  float* z = route_smem + warp * per_tok;
-  if (lane < n_extra) extra_out[(size_t)t * n_extra + lane] = z[E + lane];
-  // (the logits are not needed once the scores exist: their place holds the choice scores)
-  moe_route_token(z, z + n_rows, z, z + n_rows + E, ids + (size_t)t * top, wts + (size_t)t * top, lane, E, top, n_groups,
-                  keep_groups, group_top, score_kind, normalize, norm_eps, scale, bias);
+  if constexpr (PLACE) {
+    int* all_ids = reinterpret_cast<int*>(own_wts + TOK * top);
+    int* count = all_ids + n_tokens * top;
+    moe_place<THREADS>(places, own_ids, own_wts, all_ids, count, count + WARPS, x0, row, t0, n_tokens, K, E, top);
+  }
 }
 
 // x [T, K] (float32 or bfloat16, row stride ldx), w float32 [E, K] -> ids int32 [T, top], wts float32 [T, top].
 // logit_bias: null, or float32 [E] added to the experts' logits before anything is made of them.
-LLMX_API int llmx_moe_router_biased(const void* x, int x_dtype, long long ldx, const float* w, int* ids, float* wts,
-                             int n_tokens, int K, int E, int top, int n_groups, int keep_groups, int group_top,
-                             int score_kind, int normalize, float norm_eps, float scale, const float* bias,
-                             int n_extra, float* extra_out, const float* logit_bias, cudaStream_t stream) {
+// places: null, or what to fill beside (bfloat16 rows of whole vectors, up to MOE_PLACE_TOKENS tokens).
+static int moe_router(const void* x, int x_dtype, long long ldx, const float* w, int* ids, float* wts, int n_tokens, int K, int E,
+                      int top, int n_groups, int keep_groups, int group_top, int score_kind, int normalize, float norm_eps,
+                      float scale, const float* bias, int n_extra, float* extra_out, const float* logit_bias,
+                      const MoePlaces* places, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (score_kind < MOE_SCORE_SIGMOID || score_kind > MOE_SCORE_SOFTMAX_TOP || top > 32) return LLMX_REFUSED(1);
   if (n_extra < 0 || n_extra > 32 || (n_extra > 0 && !extra_out)) return LLMX_REFUSED(1);
@@ -275,24 +437,60 @@ LLMX_API int llmx_moe_router_biased(const void* x, int x_dtype, long long ldx, c
       keep_groups <= 0 || keep_groups > n_groups || group_top <= 0 || group_top > 8 ||
       top > E / n_groups * keep_groups)
     return LLMX_REFUSED(1);
-  const int tok = n_tokens <= 64 ? 1 : 4;
-  const size_t smem = (size_t)tok * (2 * E + n_extra + n_groups) * sizeof(float);
-  const dim3 grid((n_tokens + tok - 1) / tok);
   const int esz = x_dtype == LLMX_F32 ? 4 : 2;
   const int vec = (K % 8 == 0) && ((ldx * esz) % 16 == 0) && !((uintptr_t)x & 15) && !((uintptr_t)w & 15);
-#define GO(TX, TOK)                                                                                                    \
-  launch_pdl(moe_router_kernel<TX, TOK>, grid, dim3(256), smem, stream, (const TX*)x, ldx, w, ids, wts, n_tokens, K, E, \
-             top, n_groups, keep_groups, group_top, score_kind, normalize, norm_eps, scale, vec, bias, n_extra, extra_out, \
-             logit_bias)
-  if (x_dtype == LLMX_F32) {
-    if (tok == 1) GO(float, 1); else GO(float, 4);
-  } else if (x_dtype == LLMX_BF16) {
-    if (tok == 1) GO(bf16, 1); else GO(bf16, 4);
-  } else {
-    return LLMX_REFUSED(2);
+  if (places && (x_dtype != LLMX_BF16 || !vec || n_tokens > MOE_PLACE_TOKENS || ((uintptr_t)places->xs & 15) ||
+                 places->tile_rows <= 0 || places->n_tiled < 0 || places->n_tiled > E ||
+                 places->max_tiles < (n_tokens * top + places->tile_rows - 1) / places->tile_rows + E))
+    return LLMX_REFUSED(1);
+  const size_t per_tok = (size_t)(2 * E + n_extra + n_groups) * sizeof(float);
+  const int tok = n_tokens <= 64 ? 1 : 4;
+  const MoePlaces none = {};
+#define GO(TX, TOK, THREADS, PLACE, SMEM)                                                                                 \
+  {                                                                                                                       \
+    auto kernel = moe_router_kernel<TX, TOK, THREADS, PLACE>;                                                             \
+    const dim3 grid((n_tokens + TOK - 1) / TOK);                                                                          \
+    if (PLACE)                                                                                                            \
+      launch_pdl_cluster(kernel, grid, dim3(THREADS), SMEM, stream, grid.x, (const TX*)x, ldx, w, ids, wts, n_tokens, K, E, \
+                         top, n_groups, keep_groups, group_top, score_kind, normalize, norm_eps, scale, vec, bias, n_extra, \
+                         extra_out, logit_bias, *places);                                                                 \
+    else                                                                                                                  \
+      launch_pdl(kernel, grid, dim3(THREADS), SMEM, stream, (const TX*)x, ldx, w, ids, wts, n_tokens, K, E, top, n_groups, \
+                 keep_groups, group_top, score_kind, normalize, norm_eps, scale, vec, bias, n_extra, extra_out, logit_bias, \
+                 none);                                                                                                   \
+    return LLMX_LAUNCH_STATUS();                                                                                          \
   }
+  if (places) {
+    const size_t smem = per_tok + (size_t)top * 12 + (size_t)n_tokens * top * 4 + 64;      // (16 KB at most)
+    GO(bf16, 1, 512, true, smem)
+  }
+  if (x_dtype != LLMX_F32 && x_dtype != LLMX_BF16) return LLMX_REFUSED(2);
+  if (tok == 1 && x_dtype == LLMX_F32) GO(float, 1, 512, false, per_tok)
+  if (tok == 1) GO(bf16, 1, 512, false, per_tok)
+  if (x_dtype == LLMX_F32) GO(float, 4, 256, false, 4 * per_tok)
+  GO(bf16, 4, 256, false, 4 * per_tok)
 #undef GO
-  return LLMX_LAUNCH_STATUS();
+}
+
+LLMX_API int llmx_moe_router_biased(const void* x, int x_dtype, long long ldx, const float* w, int* ids, float* wts,
+                             int n_tokens, int K, int E, int top, int n_groups, int keep_groups, int group_top,
+                             int score_kind, int normalize, float norm_eps, float scale, const float* bias,
+                             int n_extra, float* extra_out, const float* logit_bias, cudaStream_t stream) {
+  return moe_router(x, x_dtype, ldx, w, ids, wts, n_tokens, K, E, top, n_groups, keep_groups, group_top, score_kind, normalize,
+                    norm_eps, scale, bias, n_extra, extra_out, logit_bias, nullptr, stream);
+}
+
+// The router, the order of the pairs by expert (perm, dest, sorted_weight [P], tiles, as llmx_moe_sort makes them) and the
+// tokens' rows in that order (xs [P, K], as llmx_moe_gather_rows makes them) in one launch: bfloat16 rows, up to 8 tokens.
+LLMX_API int llmx_moe_router_placed(const void* x, long long ldx, const float* w, int* ids, float* wts, int n_tokens, int K,
+                                    int E, int top, int n_groups, int keep_groups, int group_top, int score_kind, int normalize,
+                                    float norm_eps, float scale, const float* bias, int n_extra, float* extra_out,
+                                    const float* logit_bias, int* perm, int* dest, float* sorted_weight, int* tiles,
+                                    int max_tiles, int tile_rows, int n_tiled, void* xs, cudaStream_t stream) {
+  if (!perm || !dest || !sorted_weight || !tiles || !xs) return LLMX_REFUSED(4);
+  const MoePlaces places = {perm, dest, tiles, sorted_weight, (bf16*)xs, max_tiles, tile_rows, n_tiled};
+  return moe_router(x, LLMX_BF16, ldx, w, ids, wts, n_tokens, K, E, top, n_groups, keep_groups, group_top, score_kind, normalize,
+                    norm_eps, scale, bias, n_extra, extra_out, logit_bias, &places, stream);
 }
 
 LLMX_API int llmx_moe_router(const void* x, int x_dtype, long long ldx, const float* w, int* ids, float* wts,

@@ -1600,13 +1600,17 @@ def moe_sort(ids, n_experts: int, perm, tiles, tile_rows: int = MOE_TILE, pair_w
              _ptr(tiles), tiles.shape[0], tile_rows, n_experts if n_tiled is None else n_tiled, _stream()), "moe_sort")
 
 
+MOE_PLACE_TOKENS = 8      # steps of up to this many tokens route, sort and gather in one launch (``places``)
+
+
 def moe_router(x, w, ids, weights, n_groups: int, keep_groups: int, group_top: int, score: str, normalize: bool,
-               norm_eps: float, scale: float, bias=None, extra_out=None, logit_bias=None) -> None:
+               norm_eps: float, scale: float, bias=None, extra_out=None, logit_bias=None, places=None) -> None:
     """The router's product (float32 ``w`` [E, K] times the rows of ``x``, float32 sums) and the routing of
     ``moe_route`` in one kernel.  With ``extra_out`` float32 [T, n], ``w`` holds n more rows behind the experts',
     whose products are written there as they are.  ``logit_bias`` float32 [E] joins the experts' logits before the
     scores are made.  ``score`` "softmax_top": the largest logits win, and the weights are the softmax over the
-    winners' logits only."""
+    winners' logits only.  ``places``: (perm, dest, sorted_weight, tiles, tile_rows, n_tiled, xs) to fill as ``moe_sort``
+    and ``moe_gather_rows`` do, in the same launch (bfloat16 ``x`` that ``moe_tc_supports``, up to MOE_PLACE_TOKENS)."""
     _dev(x, w, ids, weights, bias, extra_out, logit_bias)
     assert logit_bias is None or (logit_bias.dtype == torch.float32 and logit_bias.is_contiguous()
                                   and logit_bias.numel() == w.shape[0] - (0 if extra_out is None else extra_out.shape[1]))
@@ -1616,6 +1620,22 @@ def moe_router(x, w, ids, weights, n_groups: int, keep_groups: int, group_top: i
     _contig("w", w), _contig("ids", ids), _contig("weights", weights)
     assert w.dtype == torch.float32 and x.stride(1) == 1 and ids.dtype == torch.int32 and weights.dtype == torch.float32
     T, top = ids.shape
+    if places is not None:
+        perm, dest, sorted_weight, tiles, tile_rows, n_tiled, xs = places
+        _dev(x, perm, dest, sorted_weight, tiles, xs)
+        for name, t in (("perm", perm), ("dest", dest), ("sorted_weight", sorted_weight), ("tiles", tiles), ("xs", xs)):
+            _contig(name, t)
+        assert x.dtype == torch.bfloat16 and xs.dtype == torch.bfloat16 and xs.shape == (T * top, x.shape[1])
+        assert perm.numel() == dest.numel() == sorted_weight.numel() == T * top
+        f = _fn("moe", "llmx_moe_router_placed",
+                [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                 c_int, c_float, c_float, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
+                 c_int, c_int, c_void_p, c_void_p])
+        _check(f(_ptr(x), x.stride(0), _ptr(w), _ptr(ids), _ptr(weights), T, x.shape[1], w.shape[0] - n_extra, top, n_groups,
+                 keep_groups, group_top, _SCORES[score], int(normalize), norm_eps, scale, _ptr(bias), n_extra,
+                 _ptr(extra_out), _ptr(logit_bias), _ptr(perm), _ptr(dest), _ptr(sorted_weight), _ptr(tiles),
+                 tiles.shape[0], tile_rows, n_tiled, _ptr(xs), _stream()), "moe_router_placed")
+        return
     f = _fn("moe", "llmx_moe_router_biased",
             [c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
              c_int, c_int, c_float, c_float, c_void_p, c_int, c_void_p, c_void_p, c_void_p])

@@ -153,19 +153,26 @@ class RoutedExperts:
         ids = torch.empty((T, self.top), dtype=torch.int32, device=dev)
         pair_w = torch.empty((T, self.top), dtype=torch.float32, device=dev)
         shared_z = torch.empty((T, 1), dtype=torch.float32, device=dev) if self.shared and self.shared_gated else None
+        perm = torch.empty((P,), dtype=torch.int32, device=dev)
+        fast = self.tensor_cores and x.dtype == torch.bfloat16 and kernels.moe_tc_supports(x, self.gate_up)
+        rows = self.tile_rows(P) if fast else kernels.MOE_TILE
+        tiles = torch.empty((kernels.moe_max_tiles(P, self.E_all, rows), 3), dtype=torch.int32, device=dev)
+        places = None
+        if fast:
+            dest = torch.empty((P,), dtype=torch.int32, device=dev)
+            sorted_w = torch.empty((P,), dtype=torch.float32, device=dev)
+            xs = torch.empty((P, x.shape[1]), dtype=torch.bfloat16, device=dev)
+            if self.table is None and T <= kernels.MOE_PLACE_TOKENS:
+                places = (perm, dest, sorted_w, tiles, rows, self.E, xs)      # the router sorts and gathers too
         if self.table is not None:
             kernels.moe_table_route(ctx.tokens, self.table, self.E, self.table_weight, ids, pair_w)
         else:
             kernels.moe_router(x, self.router, ids, pair_w, self.n_groups, self.keep_groups, self.group_top, self.score,
                                self.normalize, self.norm_eps, self.scale, bias=self.correction, extra_out=shared_z,
-                               logit_bias=self.router_bias)
+                               logit_bias=self.router_bias, places=places)
         probe = getattr(ctx, "probe", None)
         if probe:
             probe("router_ids", ids), probe("router_weights", pair_w)
-        perm = torch.empty((P,), dtype=torch.int32, device=dev)
-        fast = self.tensor_cores and x.dtype == torch.bfloat16 and kernels.moe_tc_supports(x, self.gate_up)
-        rows = self.tile_rows(P) if fast else kernels.MOE_TILE
-        tiles = torch.empty((kernels.moe_max_tiles(P, self.E_all, rows), 3), dtype=torch.int32, device=dev)
         act = torch.empty((P, self.F), dtype=self.rt.act_dtype, device=dev)
         d = self.down.shape[1]
         extra, shared_act = (1 if self.shared else 0), None
@@ -179,11 +186,9 @@ class RoutedExperts:
         y = torch.empty((self.top + extra, T, d), dtype=torch.float32, device=dev)
         mode = 1 if self.gated else 2
         if fast:
-            dest = torch.empty((P,), dtype=torch.int32, device=dev)
-            sorted_w = torch.empty((P,), dtype=torch.float32, device=dev)
-            kernels.moe_sort(ids, self.E_all, perm, tiles, rows, pair_w, dest, sorted_w, n_tiled=self.E)
-            xs = torch.empty((P, x.shape[1]), dtype=torch.bfloat16, device=dev)
-            kernels.moe_gather_rows(x, perm, self.top, xs)
+            if places is None:
+                kernels.moe_sort(ids, self.E_all, perm, tiles, rows, pair_w, dest, sorted_w, n_tiled=self.E)
+                kernels.moe_gather_rows(x, perm, self.top, xs)
             kernels.moe_grouped_tc(xs, self.gate_up, act, tiles, rows, dest, sorted_w, gated=mode,
                                    activation=self.activation)
             kernels.moe_grouped_tc(act, self.down, y, tiles, rows, dest, sorted_w, gated=False)

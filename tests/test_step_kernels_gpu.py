@@ -12,6 +12,61 @@ def rel(a, b):
     return ((a.double() - b.double()).norm() / b.double().norm()).item()
 
 
+@pytest.mark.parametrize("T, E, top, K, groups, keep, rows, score, bias, real", [
+    (1, 16, 2, 2048, 4, 2, 16, "sigmoid", False, 16), (4, 16, 2, 2048, 1, 1, 16, "softmax", False, 16),
+    (8, 64, 6, 1024, 8, 4, 16, "softmax", True, 64),          # a token a CTA, the most of them
+    (7, 7, 3, 264, 1, 1, 16, "sigmoid", False, 7), (8, 1024, 16, 64, 1, 1, 16, "softmax_top", False, 1024),
+    (3, 40, 4, 4104, 1, 1, 64, "sigmoid", False, 36),         # experts without tiles; a row of more than the threads hold
+    (6, 16, 2, 2048, 4, 2, 16, "sigmoid", True, 16), (8, 513, 9, 520, 1, 1, 16, "sigmoid", False, 513), (5, 3, 1, 8, 1, 1, 16, "softmax", False, 3)])
+def test_router_that_sorts_and_gathers(T, E, top, K, groups, keep, rows, score, bias, real):
+    """The same choices and weights as the router alone, and the order, tiles and rows that follow from them, exactly."""
+    from llmoxide_b200 import kernels
+    torch.manual_seed(T * E)
+    x, w = torch.randn(T, K, device=DEV).bfloat16(), torch.randn(E, K, device=DEV) * 0.05
+    b = torch.randn(E, device=DEV) * 0.1 if bias else None
+    args = (groups, keep, 2, score, True, 1e-9, 1.5)
+    ids, wts = torch.empty(T, top, dtype=torch.int32, device=DEV), torch.empty(T, top, device=DEV)
+    kernels.moe_router(x, w, ids, wts, *args, bias=b)
+    ids2, wts2, P = torch.empty_like(ids), torch.empty_like(wts), T * top
+    perm, dest = (torch.full((P,), -7, dtype=torch.int32, device=DEV) for _ in range(2))
+    sorted_w, xs = torch.empty(P, device=DEV), torch.empty(P, K, dtype=torch.bfloat16, device=DEV)
+    tiles = torch.full((kernels.moe_max_tiles(P, E, rows), 3), -9, dtype=torch.int32, device=DEV)
+    kernels.moe_router(x, w, ids2, wts2, *args, bias=b, places=(perm, dest, sorted_w, tiles, rows, real, xs))
+    assert torch.equal(ids, ids2) and torch.equal(wts, wts2)
+    pairs = ids.reshape(-1).long()
+    order = torch.sort(pairs, stable=True)[1]
+    assert torch.equal(perm.long(), order) and torch.equal(dest.long(), (order % top) * T + order // top)
+    assert torch.equal(sorted_w, wts.reshape(-1)[order]) and torch.equal(xs, x[order // top])
+    want, at = [], 0
+    for e in range(E):
+        n = int((pairs == e).sum())
+        want += [[e, at + k, min(rows, n - k)] for k in range(0, n, rows)] if e < real else []
+        at += n
+    got = tiles.tolist()
+    assert got[: len(want)] == want and all(t[0] == -1 for t in got[len(want):])
+
+
+@pytest.mark.parametrize("T", [63, 64, 65, 16 * 148, 2500])
+@pytest.mark.parametrize("E, n_extra", [(16, 0), (33, 1)])
+def test_router_of_few_and_many_tokens(T, E, n_extra):
+    """1, 4 and 16 tokens a CTA add up in the same order: a token's choices and weights have the same bits in every step."""
+    from llmoxide_b200 import kernels
+    torch.manual_seed(T + E)
+    x, w = torch.randn(T, 520, device=DEV).bfloat16(), torch.randn(E + n_extra, 520, device=DEV) * 0.05
+
+    def run(x):
+        ids, wts = torch.empty(len(x), 3, dtype=torch.int32, device=DEV), torch.empty(len(x), 3, device=DEV)
+        extra = torch.empty(len(x), n_extra, device=DEV) if n_extra else None
+        kernels.moe_router(x, w, ids, wts, 1, 1, 1, "sigmoid", True, 0.0, 1.0, extra_out=extra)
+        return ids, wts, extra
+
+    all_of = run(x)
+    for part in (x[:1], x[-20:], x[: T // 2]):
+        at = 0 if part.data_ptr() == x.data_ptr() else T - 20
+        for a, b in zip(run(part), all_of):
+            assert a is None or torch.equal(a, b[at : at + len(part)])
+
+
 @pytest.mark.parametrize("D, n_rot, H, G, T, n_split", [(64, 64, 3, 1, 5, 3), (64, 0, 16, 8, 1, 5), (64, 64, 5, 2, 70, 1),
                                                         (128, 0, 16, 4, 70, 1), (128, 0, 3, 2, 4, 4), (64, 0, 2, 1, 9, 2)])
 @pytest.mark.parametrize("gains", [False, True])
