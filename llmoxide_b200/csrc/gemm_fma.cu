@@ -70,6 +70,9 @@ struct BlockCopy {
 // multiply-adds.  The sums of earlier segments wait in shared memory.  Bound by the FMA units and the reads that feed
 // them.  970 tokens, N = K = 2048: 231 us (35 TFLOP/s;
 // the one-chain 64 x 64 kernel that this replaced: 16 TFLOP/s); 2500 tokens, N = 4096: 971 us (43 TFLOP/s).
+// SHARED: where the tiles are too few for the SMs, a cluster's CTAs take a segment of K each and add the segments' sums in
+// their order through distributed shared memory, so the bits are those of one CTA.  N = K = 2048: 40 tokens 49.7 -> 34.8 us,
+// 100 tokens 96.8 -> 38.6, 256 tokens 126 -> 64.4; 970 tokens, N = 3072: 345 -> 327.
 template <int TM, int TN>
 struct F32Tile {
   static constexpr int BM = 8 * TM, BN = 16 * TN, BK = 16, STAGES = 4, PITCH = BK + 4;
@@ -78,10 +81,10 @@ struct F32Tile {
   static constexpr size_t SMEM = ((size_t)STAGES * STAGE + (size_t)BM * TOTAL_PITCH) * sizeof(float);
 };
 
-template <int TM, int TN, int VEC>
+template <int TM, int TN, int VEC, bool SHARED>
 __global__ void __launch_bounds__(128, TM * TN >= 64 ? 2 : 4)
 gemm_f32_tile_kernel(const float* __restrict__ X, const float* __restrict__ W, float* __restrict__ Y, int M, int N, int K,
-                     long long ldx, long long ldw, long long ldy, int n_tiles) {
+                     long long ldx, long long ldw, long long ldy, int n_tiles, int n_seg) {
   using Tile = F32Tile<TM, TN>;
   constexpr int BM = Tile::BM, BN = Tile::BN, BK = Tile::BK, STAGES = Tile::STAGES, PITCH = Tile::PITCH, STAGE = Tile::STAGE;
   extern __shared__ __align__(16) float tiles[];                      // per stage: W [BN][PITCH], X [BM][PITCH]; totals
@@ -89,14 +92,15 @@ gemm_f32_tile_kernel(const float* __restrict__ X, const float* __restrict__ W, f
   const uint32_t base = (uint32_t)__cvta_generic_to_shared(tiles);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tn = (warp & 1) * 8 + (lane & 7), tm = (warp >> 1) * 4 + (lane >> 3);      // 16 x 8
-  const int n0 = (blockIdx.x % n_tiles) * BN, m0 = (blockIdx.x / n_tiles) * BM;
-  const int n_kb = (K + BK - 1) / BK;
+  const int rank = SHARED ? (int)blockIdx.x % n_seg : 0, tile = SHARED ? (int)blockIdx.x / n_seg : (int)blockIdx.x;
+  const int n0 = (tile % n_tiles) * BN, m0 = (tile / n_tiles) * BM;
+  const int k_first = rank * F32_SEG, n_kb = ((SHARED ? min(K - k_first, F32_SEG) : K) + BK - 1) / BK;
   const BlockCopy<BN, BK, VEC> copy_w(W, ldw, n0, N);
   const BlockCopy<BM, BK, VEC> copy_x(X, ldx, m0, M);
   auto load = [&](int kb) {
     const uint32_t dst = base + (uint32_t)((kb % STAGES) * STAGE) * 4u;
-    copy_w(dst, kb * BK, K);
-    copy_x(dst + (uint32_t)(BN * PITCH) * 4u, kb * BK, K);
+    copy_w(dst, k_first + kb * BK, K);
+    copy_x(dst + (uint32_t)(BN * PITCH) * 4u, k_first + kb * BK, K);
   };
   pdl_launch_dependents();
   pdl_wait();
@@ -132,7 +136,7 @@ gemm_f32_tile_kernel(const float* __restrict__ X, const float* __restrict__ W, f
         for (int i = 0; i < TM; ++i) fma2(acc[i][j], a[i].y, b.y);
       }
     }
-    if ((kb + 1) % (F32_SEG / BK) == 0 && kb + 1 < n_kb) {           // a segment ends and another follows
+    if (!SHARED && (kb + 1) % (F32_SEG / BK) == 0 && kb + 1 < n_kb) {           // a segment ends and another follows
       const bool first = kb + 1 == F32_SEG / BK;
 #pragma unroll
       for (int i = 0; i < TM; ++i)
@@ -143,6 +147,35 @@ gemm_f32_tile_kernel(const float* __restrict__ X, const float* __restrict__ W, f
           acc[i][j] = 0ull;
         }
     }
+  }
+  if (SHARED) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) totals[(i * 8 + tm) * Tile::TOTAL_PITCH + j * 16 + tn] = both(acc[i][j]);
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const uint32_t own = (uint32_t)__cvta_generic_to_shared(totals);
+    uint32_t there[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there[q]) : "r"(own), "r"(min(q, n_seg - 1)));
+    for (int r = rank; r < BM && m0 + r < M; r += n_seg)              // rows of the tile, a row's segments in their order
+      for (int c = threadIdx.x; c < BN; c += 128) {
+        float v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (q < n_seg)
+            asm volatile("ld.shared::cluster.f32 %0, [%1];"
+                         : "=f"(v[q]) : "r"(there[q] + (uint32_t)(r * Tile::TOTAL_PITCH + c) * 4u) : "memory");
+#pragma unroll
+        for (int q = 1; q < 8; ++q)
+          if (q < n_seg) v[0] = __fadd_rn(v[0], v[q]);
+        if (n0 + c < N) Y[(size_t)(m0 + r) * ldy + n0 + c] = v[0];
+      }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");     // nobody leaves while its sums may be read
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return;
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -262,29 +295,36 @@ gemm_f32_rows_kernel(const float* __restrict__ X, const float* __restrict__ W, f
 }
 
 // One launch of a kernel whose CTAs own BM tokens x BN features.
-template <typename Shape, typename Kernel>
+template <typename Shape, typename Kernel, typename... More>
 static int launch_f32(Kernel kernel, bool& attr_set, const float* X, const float* W, float* Y, int M, int N, int K,
-                      long long ldx, long long ldw, long long ldy, cudaStream_t stream) {
+                      long long ldx, long long ldw, long long ldy, cudaStream_t stream, int cluster, More... more) {
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape::SMEM);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
   const long long n_tiles = (N + Shape::BN - 1) / Shape::BN, m_tiles = (M + Shape::BM - 1) / Shape::BM;
-  if (n_tiles * m_tiles > 0x7fffffff) return LLMX_REFUSED(3);
-  launch_pdl(kernel, dim3((unsigned)(n_tiles * m_tiles)), dim3(128), Shape::SMEM, stream, X, W, Y, M, N, K, ldx, ldw, ldy,
-             (int)n_tiles);
+  if (n_tiles * m_tiles * cluster > 0x7fffffff) return LLMX_REFUSED(3);
+  const dim3 grid((unsigned)(n_tiles * m_tiles * cluster));
+  if (cluster > 1)
+    launch_pdl_cluster(kernel, grid, dim3(128), Shape::SMEM, stream, (unsigned)cluster, X, W, Y, M, N, K, ldx, ldw, ldy,
+                       (int)n_tiles, more...);
+  else
+    launch_pdl(kernel, grid, dim3(128), Shape::SMEM, stream, X, W, Y, M, N, K, ldx, ldw, ldy, (int)n_tiles, more...);
   return LLMX_LAUNCH_STATUS();
 }
 
 // The float32 product by a launch of the caller's choice (tests: every one gives the same bits); -1: by the rule.
-// 0..3: rows kernel with 2, 4, 8, 16 tokens a CTA; 4: tiles of 32 x 64; 5: tiles of 64 x 128.
-#define F32_N_FORMS 6
+// 0..3: rows kernel with 2, 4, 8, 16 tokens a CTA; 4: tiles of 32 x 64; 5: tiles of 64 x 128; 6, 7: the same, a cluster's
+// CTAs with a segment of K each (2 to 8 segments).
+#define F32_N_FORMS 8
 LLMX_API int llmx_gemm_f32_form(int form, const float* X, const float* W, float* Y, int M, int N, int K, long long ldx,
                                 long long ldw, long long ldy, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || ldx < K || ldw < K || ldy < N || form >= F32_N_FORMS) return LLMX_REFUSED(1);
   if ((M + 63) / 64 > 65535) return LLMX_REFUSED(3);
+  const int n_seg = (K + F32_SEG - 1) / F32_SEG;
+  if (form >= 6 && (n_seg < 2 || n_seg > 8)) return LLMX_REFUSED(1);
   if (form < 0) {
     // Rule: the cheapest by what was measured over K = 64 to 8192, N = 64 to 8192 and 1 to 2500 tokens (us beside a launch's
     // 1.5).  A step of 32 k in four segments costs a round of 296 CTAs of rows 0.6, 0.65, 0.75 or 1.1 (2, 4, 8, 16 tokens);
@@ -293,7 +333,6 @@ LLMX_API int llmx_gemm_f32_form(int form, const float* X, const float* W, float*
     // 16 tokens, N = 8192, K = 256: 18 us by rows, 9.3 by tiles; N = 2048, K = 2048: 19 and 50.
     const auto rounds = [](long long n, int m) { return (double)((n + m - 1) / m); };
     const auto tiles = [&](int bm, int bn) { return (long long)rounds(M, bm) * (long long)rounds(N, bn); };
-    const int n_seg = (K + F32_SEG - 1) / F32_SEG;
     const double steps = (n_seg / 4) * 16 + (n_seg % 4 == 1 ? (K - (n_seg - 1) * F32_SEG + 31) / 32 : n_seg % 4 ? 16 : 0);
     const double blocks = (K + 15) / 16;
     const int few = M <= 2 ? 0 : M <= 4 ? 1 : M <= 8 ? 2 : 3;
@@ -301,27 +340,48 @@ LLMX_API int llmx_gemm_f32_form(int form, const float* X, const float* W, float*
     const double rows = a_step[few] * steps * rounds(tiles(2 << few, 16), 2 * llmx_sm_count());
     const double small = blocks * fmax(0.26 * rounds(tiles(32, 64), llmx_sm_count()), 0.41);
     const double large = blocks * fmax(0.88 * rounds(tiles(64, 128), llmx_sm_count()), 1.17);
-    form = rows <= small && rows <= large ? few : small <= large ? 4 : 5;
+    double best = rows;
+    form = few;
+    const auto take = [&](int f, double us) {
+      if (us < best) best = us, form = f;
+    };
+    take(4, small);
+    take(5, large);
+    if (n_seg >= 2 && n_seg <= 8) {
+      take(6, 1.03 * fmax(5.0 + 0.0595 * n_seg * (double)tiles(32, 64), 33.0));
+      take(7, 1.03 * fmax(12.0 + 0.207 * n_seg * (double)tiles(64, 128), 55.0));
+    }
   }
   // 16-byte copies where every row starts on a 16-byte boundary and K ends on one, else 4-byte copies
   const bool wide = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && !((uintptr_t)X & 15) && !((uintptr_t)W & 15);
-#define GO(SHAPE, KERNEL, ...)                                                                                      \
+#define GO(SHAPE, CLUSTER, KERNEL, ...)                                                                             \
   {                                                                                                                 \
-    static bool set4 = false, set1 = false;                                                                         \
-    return wide ? launch_f32<SHAPE>(KERNEL<__VA_ARGS__, 4>, set4, X, W, Y, M, N, K, ldx, ldw, ldy, stream)           \
-                : launch_f32<SHAPE>(KERNEL<__VA_ARGS__, 1>, set1, X, W, Y, M, N, K, ldx, ldw, ldy, stream);          \
+    static bool set = false;                                                                                        \
+    return launch_f32<SHAPE>(KERNEL, set, X, W, Y, M, N, K, ldx, ldw, ldy, stream, CLUSTER, ##__VA_ARGS__);          \
   }
-#define TILE(TM, TN) \
-  { using S = F32Tile<TM, TN>; GO(S, gemm_f32_tile_kernel, TM, TN) }
+#define ROWS(MT)                                                                                                    \
+  {                                                                                                                 \
+    using S = F32Rows<MT>;                                                                                          \
+    if (wide) GO(S, 1, (gemm_f32_rows_kernel<MT, 4>)) else GO(S, 1, (gemm_f32_rows_kernel<MT, 1>))                    \
+  }
+#define TILE(TM, TN, SHARED)                                                                                        \
+  {                                                                                                                 \
+    using S = F32Tile<TM, TN>;                                                                                      \
+    if (wide) GO(S, SHARED ? n_seg : 1, (gemm_f32_tile_kernel<TM, TN, 4, SHARED>), n_seg)                             \
+    else GO(S, SHARED ? n_seg : 1, (gemm_f32_tile_kernel<TM, TN, 1, SHARED>), n_seg)                                  \
+  }
   switch (form) {
-    case 0: GO(F32Rows<1>, gemm_f32_rows_kernel, 1)
-    case 1: GO(F32Rows<2>, gemm_f32_rows_kernel, 2)
-    case 2: GO(F32Rows<4>, gemm_f32_rows_kernel, 4)
-    case 3: GO(F32Rows<8>, gemm_f32_rows_kernel, 8)
-    case 4: TILE(4, 4)
-    case 5: TILE(8, 8)
+    case 0: ROWS(1)
+    case 1: ROWS(2)
+    case 2: ROWS(4)
+    case 3: ROWS(8)
+    case 4: TILE(4, 4, false)
+    case 5: TILE(8, 8, false)
+    case 6: TILE(4, 4, true)
+    case 7: TILE(8, 8, true)
   }
 #undef TILE
+#undef ROWS
 #undef GO
   return LLMX_REFUSED(1);
 }

@@ -67,6 +67,30 @@ def test_router_of_few_and_many_tokens(T, E, n_extra):
             assert a is None or torch.equal(a, b[at : at + len(part)])
 
 
+@pytest.mark.parametrize("M, N, K, pad", [(17, 64, 513, 3), (65, 130, 1028, 0), (33, 65, 2048, 0), (200, 129, 4096, 4)])
+def test_float32_tiles_that_share_k(M, N, K, pad):
+    """The same bits as the launches that do not share (2 to 8 segments of K); more or fewer segments are refused."""
+    from ctypes import c_int, c_longlong, c_void_p
+    from llmoxide_b200 import kernels
+    torch.manual_seed(M + K)
+    x, w = torch.randn(M, K + pad, device=DEV)[:, :K], torch.randn(N, K + pad, device=DEV)[:, :K]
+    f = kernels._fn("gemm_fma", "llmx_gemm_f32_form", [c_int] + [c_void_p] * 3 + [c_int] * 3 + [c_longlong] * 3 + [c_void_p])
+
+    def run(form, k=K):
+        y = torch.full((M, N + 1), 7.0, device=DEV)
+        status = f(form, x.data_ptr(), w.data_ptr(), y.data_ptr(), M, N, k, x.stride(0), w.stride(0), N + 1,
+                   torch.cuda.current_stream().cuda_stream)
+        assert (y[:, N] == 7.0).all()
+        return status, y[:, :N]
+
+    want = run(4)[1]
+    assert rel(want, x.double() @ w.double().T) < 1e-6
+    for form in (6, 7):
+        status, y = run(form)
+        assert status == 0 and torch.equal(y, want)
+        assert run(form, 512)[0] < 0
+
+
 @pytest.mark.parametrize("D, n_rot, H, G, T, n_split", [(64, 64, 3, 1, 5, 3), (64, 0, 16, 8, 1, 5), (64, 64, 5, 2, 70, 1),
                                                         (128, 0, 16, 4, 70, 1), (128, 0, 3, 2, 4, 4), (64, 0, 2, 1, 9, 2)])
 @pytest.mark.parametrize("gains", [False, True])
