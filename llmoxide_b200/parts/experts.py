@@ -39,6 +39,7 @@ import torch
 
 from .. import kernels
 from ..errors import ConfigError, Unsupported
+from . import branches
 from .registry import register_feed_forward
 
 
@@ -164,6 +165,12 @@ class RoutedExperts:
             xs = torch.empty((P, x.shape[1]), dtype=torch.bfloat16, device=dev)
             if self.table is None and T <= kernels.MOE_PLACE_TOKENS:
                 places = (perm, dest, sorted_w, tiles, rows, self.E, xs)      # the router sorts and gathers too
+        d = self.down.shape[1]
+        y = join_shared = None
+        if self.shared and not self.gated and branches.wanted(ctx, T):
+            # (a captured decode step: the shared expert beside the routed ones, its partials behind the choices')
+            y = torch.empty((self.top + self.shared.down.partials(T), T, d), dtype=torch.float32, device=dev)
+            _, join_shared = branches.fork(self.rt, "shared expert", lambda: self.shared.down.into(self.shared.activate(x), y[self.top :]))
         if self.table is not None:
             kernels.moe_table_route(ctx.tokens, self.table, self.E, self.table_weight, ids, pair_w)
         else:
@@ -174,16 +181,16 @@ class RoutedExperts:
         if probe:
             probe("router_ids", ids), probe("router_weights", pair_w)
         act = torch.empty((P, self.F), dtype=self.rt.act_dtype, device=dev)
-        d = self.down.shape[1]
         extra, shared_act = (1 if self.shared else 0), None
-        if self.shared and not self.gated:
+        if join_shared is None and self.shared and not self.gated:
             # added to the stream by its last product, or as partials behind the choices'
             shared_act = self.shared.activate(x)
             if residual is not None and self.shared.down.add_into(shared_act, residual):
                 extra, shared_act = 0, None
             else:
                 extra = self.shared.down.partials(T)
-        y = torch.empty((self.top + extra, T, d), dtype=torch.float32, device=dev)
+        if y is None:
+            y = torch.empty((self.top + extra, T, d), dtype=torch.float32, device=dev)
         mode = 1 if self.gated else 2
         if fast:
             if places is None:
@@ -197,7 +204,9 @@ class RoutedExperts:
             kernels.moe_grouped(x, self.gate_up, act, perm, tiles, pair_w, self.top, T, gated=mode,
                                 activation=self.activation)
             kernels.moe_grouped(act, self.down, y, perm, tiles, pair_w, self.top, T, gated=False)
-        if shared_act is not None:
+        if join_shared is not None:
+            join_shared()
+        elif shared_act is not None:
             self.shared.down.into(shared_act, y[self.top :])
         elif self.n_identity or (self.shared and self.gated):
             # an identity expert's output is the token's own row times the weight; the shared expert's result is

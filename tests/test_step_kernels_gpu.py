@@ -142,3 +142,27 @@ def test_gated_norm_by_vectors(dtype, n_split, per_head, H, Dv):
     v = o.double().view(T, H, Dv) if per_head else o.double().view(T, 1, n)
     v = (v / (v.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt()).view(T, n)
     assert rel(y, v * gain.double() * z * torch.sigmoid(z)) < 1e-6
+
+
+@pytest.mark.parametrize("design, name", [("tifapel", "C"), ("tifapel", "A"), ("gebasun", "C"), ("gebasun", "D")])
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("batch", [1, 9, 64, 65])
+def test_captured_decode_steps_in_two_branches(tmp_path, design, name, dtype, batch):
+    """Steps replayed as graphs, whose mixers and feed-forwards are branches up to 64 tokens, give the bits of steps launched
+    one after another; several steps, so that what the branches allocate is used again from layer to layer and step to step."""
+    import gebasun_configs
+    import tifapel_configs
+    from llmoxide_b200 import Engine, LoadOptions
+    folder = dict(gebasun=gebasun_configs, tifapel=tifapel_configs)[design].make_folder(tmp_path, name, dtype)
+    rng = torch.Generator().manual_seed(batch)
+    prompts = [torch.randint(0, 200, (1 + 3 * (b % 7),), generator=rng).tolist() for b in range(batch)]
+    steps = [[torch.randint(0, 200, (1,), generator=rng).tolist() for _ in range(batch)] for _ in range(4)]
+    runs = []
+    for graphs in (True, False):
+        engine = Engine.load(folder, LoadOptions(dtype=dtype, max_tokens=64 * batch, max_batch=batch, cuda_graphs=graphs))
+        slots = [engine.acquire() for _ in prompts]
+        engine.step(list(zip(slots, prompts)))
+        runs.append([engine.step(list(zip(slots, tokens))).clone() for tokens in steps])
+        assert engine.options.cuda_graphs == graphs
+    for a, b in zip(*runs):
+        assert torch.equal(a, b)
