@@ -98,8 +98,14 @@ __device__ __forceinline__ void dr_conv8(const DeltaIn& in, const TIN* proj, con
   };
   if (TAPS > 0) {
     float u[DR_CHUNK + (TAPS > 0 ? TAPS : 1) - 1];
+    if (in.n_split == 1 && n == DR_CHUNK && pos0 - (TAPS - 1) >= p0) {      // inside a prompt: plain rows, nothing to ask
+      const TIN* p = proj + (size_t)(row0 + pos0 - (TAPS - 1) - p0) * in.row_stride + col;
 #pragma unroll
-    for (int r = 0; r < DR_CHUNK + TAPS - 1; ++r) u[r] = r - (TAPS - 1) < n ? u_at(pos0 - (TAPS - 1) + r) : 0.f;
+      for (int r = 0; r < DR_CHUNK + TAPS - 1; ++r) u[r] = to_f32(p[(size_t)r * in.row_stride]);
+    } else {
+#pragma unroll
+      for (int r = 0; r < DR_CHUNK + TAPS - 1; ++r) u[r] = r - (TAPS - 1) < n ? u_at(pos0 - (TAPS - 1) + r) : 0.f;
+    }
 #pragma unroll
     for (int i = 0; i < DR_CHUNK; ++i) y[i] = 0.f;
 #pragma unroll
@@ -121,8 +127,11 @@ __device__ __forceinline__ void dr_conv8(const DeltaIn& in, const TIN* proj, con
 
 // prep buffers: qk [slots][G][2][8][DL] (keys, then queries; DL: the staged row of delta_scan, zeros beyond D), vv [slots][H][Dvp][8] (beta_i v_i, a column's tokens
 // together), co [slots][H][DR_COEF]
+// Bound by the chain in a CTA (its rows, norms, dot products) and by how many CTAs an SM holds: four with four taps, the
+// rows of a chunk inside a prompt read without a question between them.  4100 tokens, 8 key and 16 value heads of 128:
+// 70 us; three CTAs and a choice by row 96.
 template <typename TIN, int TAPS>
-__global__ void __launch_bounds__(256, 3)
+__global__ void __launch_bounds__(256, TAPS == 4 ? 4 : 3)
 delta_prep_kernel(const TIN* __restrict__ proj, const DeltaIn in, const float* __restrict__ state,
                   float* __restrict__ qk, float* __restrict__ vv, float* __restrict__ co,
                   const int* __restrict__ seq_start, const int* __restrict__ seq_past,
