@@ -287,7 +287,7 @@ __device__ __forceinline__ void moe_place(const MoePlaces pl, const int* own_ids
 }
 
 template <typename TX, int TOK, int THREADS, bool PLACE>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, TOK == 1 ? 1 : sizeof(TX) == 2 ? 4 : 3)
 moe_router_kernel(const TX* __restrict__ x, long long ldx, const float* __restrict__ w, int* __restrict__ ids,
                   float* __restrict__ wts, int n_tokens, int K, int E, int top, int n_groups, int keep_groups,
                   int group_top, int score_kind, int normalize, float norm_eps, float scale, int vec,
