@@ -161,6 +161,8 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, int* __restri
 // Prompts: four tokens a CTA.  (Eight, and sixteen with their rows by asynchronous copies through shared memory, read
 // the matrix less often and took longer: 4100 tokens, 16 experts 23.5 us by four, 29 and 24.5 by eight and sixteen; 64 experts
 // 73, 87 and 77.)
+// Four such CTAs an SM (three of float32 rows), where unbounded registers let two in and three leave another round: 64 experts,
+// 2000 tokens 44 us (56 by three), 4100 tokens 72 (74 and 87); inside a prompt of 4100 tokens, 16 experts, 32 -> 27.
 // Steps of few tokens wait for nothing but loads: the matrix is brought to L2 while the kernel before still runs, and sixteen
 // warps share the experts.
 // PLACE (steps of up to 8 tokens): the CTAs are one cluster, which knows every choice behind one barrier, so each CTA also
