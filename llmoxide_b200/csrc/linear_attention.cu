@@ -42,9 +42,8 @@
 //   decay_chunk   per (chunk, head): the chunk's own part of E', and the 64 x 64 products q_i . k_j
 //   decay_pass    walks a sequence's chunks in order: leaves every chunk its E and the sequence its new state
 //   decay_out     per (chunk, head, 64 columns): the outputs
-// Four prompts of 700 to 1300 tokens, 16 heads of 128 x 128: 229 us, where the products on the FMA units took 291 (decay_chunk
-// 105 -> 92, decay_out 92 -> 80, the preparation 72 -> 36) and the recurrence in segments 586 (two passes); off the 64-bit
-// result by 1.8e-7 (2.7e-7; 3.4e-7).  Bound by the latency of a step (copies, splitting, products) at 16 warps an SM.
+// Four prompts of 700 to 1300 tokens, 16 heads of 128 x 128: 255 us, where the recurrence in segments took 586 (two
+// passes); off the 64-bit result by 2.7e-7 (3.4e-7).
 #include "chunk_products.cuh"
 
 #define LA_CHUNK 8           // tokens per staged chunk
@@ -579,6 +578,7 @@ struct LaDims {
   __host__ __device__ int row() const { return 2 * Dp() + Dvp(); }
 };
 
+#define LA_FOLD 128              // dims whose products are added in one chain; more are added in two
 __device__ __forceinline__ double la_power(double g, int n) {       // g^n, 0 <= n <= 64
   double p = 1.0;
 #pragma unroll
@@ -593,8 +593,8 @@ __global__ void __launch_bounds__(SS_THREADS)
 decay_chunk_kernel(const float* __restrict__ prep, const float* __restrict__ decay, float* __restrict__ st,
                    float2* __restrict__ at, float* __restrict__ cb, const int* __restrict__ seq_start, int n_seqs,
                    int n_tokens, const LaDims dm) {
-  __shared__ __align__(16) float As[64 * SS_LD];
-  __shared__ __align__(16) float Bs[64 * SS_LD];
+  __shared__ __align__(16) float As[64 * 64];
+  __shared__ __align__(16) float Bs[64 * 64];
   __shared__ float ws[SS_CHUNK];
   pdl_launch_dependents();
   const int Dp = dm.Dp(), Dvp = dm.Dvp();
@@ -604,9 +604,9 @@ decay_chunk_kernel(const float* __restrict__ prep, const float* __restrict__ dec
   const SsChunk ck = ss_chunk_of(seq_start, n_seqs, n_tokens, slot, dm.short_new);
   pdl_wait();                                          // (ahead of any leaving: a kernel whose CTAs all leave must not end
   if (ck.n <= 0) return;                               // before the one ahead of it)
-  float acc[4][8];
+  float acc[8][8];
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+  for (int r = 0; r < 8; ++r)
 #pragma unroll
     for (int c = 0; c < 8; ++c) acc[r][c] = 0.f;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -621,69 +621,81 @@ decay_chunk_kernel(const float* __restrict__ prep, const float* __restrict__ dec
     const float* vrow = prep + (size_t)ck.t0 * step + (size_t)h * dm.row() + 2 * Dp + c0 + lc;
     const bool k_live = n0 + lc < Dp, v_live = c0 + lc < Dvp;
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const int j = lr + 8 * m;
+    for (int m = 0; m < 16; ++m) {
+      const int j = lr + 4 * m;
       const bool live = v_live && j < ck.n;
-      ss_copy16(Bs + j * SS_LD + lc, live ? vrow + (size_t)j * step : prep, live);
+      ss_copy16(Bs + j * 64 + lc, live ? vrow + (size_t)j * step : prep, live);
     }
     ss_copy_commit();
-    float4 kv[8];
+    float4 kv[16];
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const int j = lr + 8 * m;
+    for (int m = 0; m < 16; ++m) {
+      const int j = lr + 4 * m;
       kv[m] = k_live && j < ck.n ? ss_load4(krow + (size_t)j * step) : zero;
     }
-    if (tid < SS_CHUNK) ws[tid] = (float)la_power(g, max(ck.n - 1 - tid, 0));        // (k past the chunk's tokens is zero)
+    ws[tid] = (float)la_power(g, max(ck.n - 1 - tid, 0));        // (k past the chunk's tokens is zero)
     if (tid == 0 && tl == 0) {
       const double all = la_power(g, ck.n);
       at[(size_t)slot * dm.H + h] = make_float2((float)all, (float)(all - (double)(float)all));
     }
     __syncthreads();
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const int j = lr + 8 * m;
+    for (int m = 0; m < 16; ++m) {
+      const int j = lr + 4 * m;
       const float w = ws[j];
-      ss_store4(As + j * SS_LD + lc, make_float4(kv[m].x * w, kv[m].y * w, kv[m].z * w, kv[m].w * w));
+      ss_store4(As + j * 64 + lc, make_float4(kv[m].x * w, kv[m].y * w, kv[m].z * w, kv[m].w * w));
     }
     ss_copy_wait<0>();
     __syncthreads();
-    ss_product(acc, As, Bs, ck.n);                       // (rows past the chunk's tokens are zero)
+    ss_product<4>(acc, As, 64, Bs, 64, (ck.n + 3) & ~3);   // (rows past the chunk's tokens are zero)
     float* dst = st + ((size_t)slot * dm.H + h) * dm.D * Dvp + c0 + j0;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int n = n0 + i0 + r;
+    for (int r = 0; r < 8; ++r) {
+      const int n = n0 + ss_row(i0, r);
       if (n >= dm.D) continue;
       if (c0 + j0 < Dvp) ss_store4(dst + (size_t)n * Dvp, make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]));
-      if (c0 + j0 + 4 < Dvp) ss_store4(dst + (size_t)n * Dvp + 4, make_float4(acc[r][4], acc[r][5], acc[r][6], acc[r][7]));
+      if (c0 + j0 + 32 < Dvp) ss_store4(dst + (size_t)n * Dvp + 32, make_float4(acc[r][4], acc[r][5], acc[r][6], acc[r][7]));
     }
     return;
   }
   // ---- q_i . k_j: both operands are turned so that a row of shared memory holds one dim of all tokens
-  const int h = job - dm.H * tiles, tok = tid & 63, part = (tid >> 6) * 4;       // two threads a token, 16 dims of a block each
-  const float* qrow = prep + (size_t)(ck.t0 + tok) * step + (size_t)h * dm.row();
-  const bool live = tok < ck.n;
+  const int h = job - dm.H * tiles;
+  const float* qrow = prep + (size_t)(ck.t0 + tid) * step + (size_t)h * dm.row();
+  const bool live = tid < ck.n;
   for (int kb = 0; kb < Dp; kb += 32) {
-    float4 qv[4], kv[4];
+    float4 qv[8], kv[8];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const int k = kb + 4 * (part + m);
-      qv[m] = live && k < Dp ? ss_load4(qrow + k) : zero;
-      kv[m] = live && k < Dp ? ss_load4(qrow + Dp + k) : zero;
+    for (int m = 0; m < 8; ++m) {
+      qv[m] = live && kb + 4 * m < Dp ? ss_load4(qrow + kb + 4 * m) : zero;
+      kv[m] = live && kb + 4 * m < Dp ? ss_load4(qrow + Dp + kb + 4 * m) : zero;
     }
     __syncthreads();                                   // (the tiles of the block before have been read)
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      float* ap = As + 4 * (part + m) * SS_LD + tok;
-      float* bp = Bs + 4 * (part + m) * SS_LD + tok;
-      ap[0] = qv[m].x, ap[SS_LD] = qv[m].y, ap[2 * SS_LD] = qv[m].z, ap[3 * SS_LD] = qv[m].w;
-      bp[0] = kv[m].x, bp[SS_LD] = kv[m].y, bp[2 * SS_LD] = kv[m].z, bp[3 * SS_LD] = kv[m].w;
+    for (int m = 0; m < 8; ++m) {
+      float* ap = As + 4 * m * 64 + tid;
+      float* bp = Bs + 4 * m * 64 + tid;
+      ap[0] = qv[m].x, ap[64] = qv[m].y, ap[128] = qv[m].z, ap[192] = qv[m].w;
+      bp[0] = kv[m].x, bp[64] = kv[m].y, bp[128] = kv[m].z, bp[192] = kv[m].w;
     }
     __syncthreads();
-    ss_product(acc, As, Bs, min(32, Dp - kb));
-  }
-  float* dst = cb + ((size_t)slot * dm.H + h) * 4096;
+    ss_product<4>(acc, As, 64, Bs, 64, min(32, Dp - kb));
+    if (kb + 32 == LA_FOLD || kb + 32 >= Dp) {         // the first LA_FOLD dims' sums wait where the result goes
+      float* dst = cb + ((size_t)slot * dm.H + h) * 4096;
 #pragma unroll
-  for (int c = 0; c < 8; ++c) ss_store4(dst + (j0 + c) * 64 + i0, make_float4(acc[0][c], acc[1][c], acc[2][c], acc[3][c]));
+      for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          float* row = dst + ss_row(j0, c) * 64 + i0 + 32 * half;
+          float4 v = make_float4(acc[4 * half][c], acc[4 * half + 1][c], acc[4 * half + 2][c], acc[4 * half + 3][c]);
+          if (kb >= LA_FOLD) {
+            const float4 w = ss_load4(row);
+            v = make_float4(w.x + v.x, w.y + v.y, w.z + v.z, w.w + v.w);
+          }
+          ss_store4(row, v);
+          acc[4 * half][c] = acc[4 * half + 1][c] = acc[4 * half + 2][c] = acc[4 * half + 3][c] = 0.f;
+        }
+    }
+  }
 }
 
 // Every four elements of a sequence's state, one thread: E_0 is the stored state, E_(c+1) = at_c E_c + st_c; st_c becomes
@@ -732,12 +744,13 @@ decay_pass_kernel(float* __restrict__ st, const float2* __restrict__ at, float* 
   }
 }
 
-__global__ void __launch_bounds__(SS_THREADS, 4)
+#define LA_LDM 68                // row stride of the masked 64 x 64 matrix in shared memory: 16-byte stores meet no bank twice
+__global__ void __launch_bounds__(SS_THREADS)
 decay_out_kernel(const float* __restrict__ prep, const float* __restrict__ decay, const float* __restrict__ st,
                  const float* __restrict__ cb, float* __restrict__ out, const int* __restrict__ seq_start, int n_seqs,
                  int n_tokens, const LaDims dm) {
-  __shared__ __align__(16) float Ms[64 * SS_LD];      // row j: decay^(i-j) (q_i . k_j) over i; before that the turned q
-  __shared__ __align__(16) float Bs[2][32 * SS_LD];       // rows of E, then of v
+  __shared__ __align__(16) float Ms[64 * LA_LDM];      // row j: decay^(i-j) (q_i . k_j) over i; before that the turned q
+  __shared__ __align__(16) float Bs[2][32 * 64];       // rows of E, then of v
   __shared__ float power[SS_CHUNK + 1];                // of the decay
   pdl_launch_dependents();
   const int Dp = dm.Dp(), Dvp = dm.Dvp(), p_tiles = (Dvp + 63) >> 6;
@@ -750,100 +763,130 @@ decay_out_kernel(const float* __restrict__ prep, const float* __restrict__ decay
   const float g = decay[h];
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const int lr = tid >> 4, lc = (tid & 15) * 4;        // a row of E or v: 16 lanes
-  const int tok = tid & 63, part = tid >> 6;           // a token's q, a column of the masked matrix: two threads
   const bool col_live = c0 + lc < Dvp;
   const float* e_base = st + ((size_t)slot * dm.H + h) * dm.D * Dvp + c0 + lc;
   const float* v_base = prep + (size_t)ck.t0 * step + (size_t)h * dm.row() + 2 * Dp + c0 + lc;
-  const float* qrow = prep + (size_t)(ck.t0 + tok) * step + (size_t)h * dm.row();
+  const float* qrow = prep + (size_t)(ck.t0 + tid) * step + (size_t)h * dm.row();
   const int e_steps = (dm.D + 31) >> 5, steps = e_steps + ((ck.n + 31) >> 5);
   auto copy_rows = [&](int k0) {                        // step k0: 32 rows of E, then of v, into one of two buffers
     float* dst = Bs[k0 & 1] + lc;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const int r = lr + 8 * m, k = (k0 < e_steps ? k0 : k0 - e_steps) * 32 + r;
+    for (int m = 0; m < 8; ++m) {
+      const int r = lr + 4 * m, k = (k0 < e_steps ? k0 : k0 - e_steps) * 32 + r;
       const bool live = col_live && (k0 < e_steps ? k < dm.D : k < ck.n);
       const float* src = k0 < e_steps ? e_base + (size_t)k * Dvp : v_base + (size_t)k * step;
-      ss_copy16(dst + r * SS_LD, live ? src : prep, live);
+      ss_copy16(dst + r * 64, live ? src : prep, live);
     }
     ss_copy_commit();
   };
-  float4 qv[4];
+  float4 qv[8];
   auto fetch_q = [&](int kb) {
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const int k = kb + 16 * part + 4 * m;
-      qv[m] = tok < ck.n && k < Dp ? ss_load4(qrow + k) : zero;
-    }
+    for (int m = 0; m < 8; ++m) qv[m] = tid < ck.n && kb + 4 * m < Dp ? ss_load4(qrow + kb + 4 * m) : zero;
   };
   copy_rows(0);
   fetch_q(0);
   // the rest is on its way to L2 meanwhile: rows of E and the products q . k
   for (int i = tid; i < 2 * dm.D; i += SS_THREADS)
     if (c0 + (i & 1) * 32 < Dvp) prefetch_l2(st + ((size_t)slot * dm.H + h) * dm.D * Dvp + (size_t)(i >> 1) * Dvp + c0 + (i & 1) * 32);
-  prefetch_l2(cb + ((size_t)slot * dm.H + h) * 4096 + tid * 32);
-  if (tid <= SS_CHUNK) power[tid] = (float)la_power(g, tid);
-  float acc[4][8];
+  for (int i = tid; i < 128; i += SS_THREADS) prefetch_l2(cb + ((size_t)slot * dm.H + h) * 4096 + i * 32);
+  power[tid] = (float)la_power(g, tid);
+  if (tid == 0) power[SS_CHUNK] = (float)la_power(g, SS_CHUNK);
+  float acc[8][8];
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+  for (int r = 0; r < 8; ++r)
 #pragma unroll
     for (int c = 0; c < 8; ++c) acc[r][c] = 0.f;
   const int i0 = ss_row0(), j0 = ss_col0();
-  // steps of 32: E^T q_i, then the sum over the chunk's own tokens
-#pragma unroll 1
-  for (int s = 0; s < steps; ++s) {
-    const int jb = (s - e_steps) * 32;
-    const float* A = Ms + jb * SS_LD;
-    int K = min(32, ck.n - jb), first_row = jb;
-    if (s < e_steps) {
-      float* As = Ms + (s & 1) * 32 * SS_LD;
+  auto each_result = [&](auto&& f) {                   // f(a result of this thread, where it goes)
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {                    // q turned: a row of shared memory holds one dim of all tokens
-        float* ap = As + (16 * part + 4 * m) * SS_LD + tok;
-        ap[0] = qv[m].x, ap[SS_LD] = qv[m].y, ap[2 * SS_LD] = qv[m].z, ap[3 * SS_LD] = qv[m].w;
+    for (int r = 0; r < 8; ++r) {
+      const int i = ss_row(i0, r);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const int p = c0 + ss_row(j0, c);
+        if (i < ck.n && p < dm.Dv) f(acc[r][c], out + ((size_t)(ck.t0 + i) * dm.H + h) * dm.Dv + p);
       }
-      A = As, K = min(32, Dp - s * 32), first_row = -64;                  // (rows of E past D are zero)
-    } else if (jb == 0) {
-      __syncthreads();                                 // the turned q has been read: its place takes the masked matrix
-      // what lies above the diagonal is zero
-      const float* cbj = cb + (((size_t)slot * dm.H + h) * 64 + tok) * 64;
+    }
+  };
+  // ---- E^T q_i
+  for (int s = 0; s < e_steps; ++s) {
+    float* As = Ms + (s & 1) * 32 * 64;
 #pragma unroll
-      for (int q = 2 * part; q < 2 * part + 2; ++q) {
-        float4 d[4];
-#pragma unroll
-        for (int m = 0; m < 4; ++m) d[m] = 16 * q + 15 >= tok ? ss_load4(cbj + 16 * q + 4 * m) : zero;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          float o[4] = {d[m].x, d[m].y, d[m].z, d[m].w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = 16 * q + 4 * m + e;
-            o[e] = i >= tok ? o[e] * power[i - tok] : 0.f;
-          }
-          ss_store4(Ms + tok * SS_LD + 16 * q + 4 * m, make_float4(o[0], o[1], o[2], o[3]));
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const float ga = power[i0 + r + 1];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) acc[r][c] *= ga;
-      }
+    for (int m = 0; m < 8; ++m) {                      // q turned: a row of shared memory holds one dim of all tokens
+      float* ap = As + 4 * m * 64 + tid;
+      ap[0] = qv[m].x, ap[64] = qv[m].y, ap[128] = qv[m].z, ap[192] = qv[m].w;
     }
     ss_copy_wait<0>();
     __syncthreads();                                   // (and every thread is done with the tiles of the step before)
-    if (s + 1 < steps) copy_rows(s + 1);
+    copy_rows(s + 1);
     if (s + 1 < e_steps) fetch_q((s + 1) * 32);
-    // (a token's infinite or NaN value is not multiplied by the zeros above the diagonal: tokens before it do not see it)
-    ss_product(acc, A, Bs[s & 1], K, first_row);
+    ss_product<2>(acc, As, 64, Bs[s & 1], 64, min(32, Dp - s * 32));      // (rows of E past D are zero)
+    if ((s + 1) * 32 == LA_FOLD && s + 1 < e_steps)    // the first LA_FOLD dims' sums wait where the result goes
+      each_result([](float& a, float* to) { *to = a, a = 0.f; });
+  }
+  if (dm.D > LA_FOLD) each_result([](float& a, float* to) { a += *to; });
+  __syncthreads();                                     // the turned q has been read: its place takes the masked matrix
+  {
+    // a thread a column j; what lies above the diagonal is zero
+    const float* cbj = cb + (((size_t)slot * dm.H + h) * 64 + tid) * 64;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float4 d[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) d[m] = 16 * q + 15 >= tid ? ss_load4(cbj + 16 * q + 4 * m) : zero;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        float o[4] = {d[m].x, d[m].y, d[m].z, d[m].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = 16 * q + 4 * m + e;
+          o[e] = i >= tid ? o[e] * power[i - tid] : 0.f;
+        }
+        ss_store4(Ms + tid * LA_LDM + 16 * q + 4 * m, make_float4(o[0], o[1], o[2], o[3]));
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const float ga = power[ss_row(i0, r) + 1];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[r][c] *= ga;
+  }
+  // ---- + sum over the chunk's own tokens
+  for (int s = e_steps; s < steps; ++s) {
+    ss_copy_wait<0>();
+    // A token's infinite or NaN value is not multiplied by the zeros above the diagonal: tokens before it do not see it.
+    float zero_if_finite = 0.f;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {                      // (what this thread copied)
+      const float4 v = ss_load4(Bs[s & 1] + (lr + 4 * m) * 64 + lc);
+      zero_if_finite = fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, fmaf(v.w, 0.f, zero_if_finite))));
+    }
+    const bool select = __syncthreads_or(!(zero_if_finite == 0.f));
+    if (s + 1 < steps) copy_rows(s + 1);
+    const int jb = (s - e_steps) * 32;
+    if (select) {
+      for (int k = 0; k < min(32, ck.n - jb); ++k)
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const int i = ss_row(i0, r);
+          if (jb + k > i) continue;
+          const float m = Ms[(jb + k) * LA_LDM + i];
+#pragma unroll
+          for (int c = 0; c < 8; ++c) acc[r][c] = fmaf(m, Bs[s & 1][k * 64 + ss_row(j0, c)], acc[r][c]);
+        }
+    } else if (jb == 0) ss_product<2>(acc, Ms, LA_LDM, Bs[s & 1], 64, min(32, ck.n));
+    else ss_product<2, false>(acc, Ms + jb * LA_LDM, LA_LDM, Bs[s & 1], 64, ck.n - jb);      // (they reach rows 32.. only)
   }
   const bool vec = (dm.Dv & 3) == 0 && ((uintptr_t)out & 15) == 0;
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = i0 + r;
+  for (int r = 0; r < 8; ++r) {
+    const int i = ss_row(i0, r);
     if (i >= ck.n) continue;
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-      const int p = c0 + j0 + 4 * half;
+      const int p = c0 + j0 + 32 * half;
       if (p >= dm.Dv) continue;
       const float* a = acc[r] + 4 * half;
       float* dst = out + ((size_t)(ck.t0 + i) * dm.H + h) * dm.Dv + p;

@@ -23,7 +23,8 @@
 //   ss_pass    walks a sequence's chunks in order: leaves every chunk its E and the sequence its new state; moves the ring
 //   ss_out     per (chunk, head): the outputs, times silu(z)
 //   ss_norm    the norm
-// The outputs' products run on the tensor cores in float32 precision, the others on the FMA units (chunk_products.cuh).  Single tokens: ss_decode, one CTA per (sequence, head), S read and
+// The products run on the FMA units from tiles in shared memory, 8 x 8 results a thread: the recurrence is float32 by the
+// design, which the tensor cores' formats are not.  Single tokens: ss_decode, one CTA per (sequence, head), S read and
 // written once; then ss_norm.
 //
 // Everything is float32.  A prompt's sums are ordered by its chunks, so a position's result may differ in rounding between
@@ -32,6 +33,7 @@
 
 #define SS_RUN 16                // tokens a thread of ss_prep walks
 #define SS_MAX_TAPS 16
+#define SS_LDM 68                // row stride of the masked 64 x 64 matrix in shared memory: 16-byte stores meet no bank twice
 
 __device__ __forceinline__ float ss_silu(float x) { return __fdividef(x, 1.0f + expf(-x)); }   // (quotient within 2 ulp)
 __device__ __forceinline__ float ss_softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
@@ -148,7 +150,7 @@ ss_prep_kernel(const SsProj proj, const SsDims dm, const float* __restrict__ con
 
 // st [slots][H][N][Pp]: the chunk's own part of its last state; at [slots][H]: gamma of its last token; cb [slots][G][64][64]:
 // C_i . B_j at row j, column i.
-__global__ void __launch_bounds__(SS_FMA_THREADS)
+__global__ void __launch_bounds__(SS_THREADS)
 ss_chunk_kernel(const float* __restrict__ xs, const float* __restrict__ bs, const float* __restrict__ cs,
                 const float2* __restrict__ da, float* __restrict__ st, float* __restrict__ at, float* __restrict__ cb,
                 const int* __restrict__ seq_start, int n_seqs, int n_tokens, const SsDims dm) {
@@ -167,7 +169,7 @@ ss_chunk_kernel(const float* __restrict__ xs, const float* __restrict__ bs, cons
 #pragma unroll
     for (int c = 0; c < 8; ++c) acc[r][c] = 0.f;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  const int i0 = ss_fma_row0(), j0 = ss_fma_col0();
+  const int i0 = ss_row0(), j0 = ss_col0();
   pdl_wait();
   if ((int)blockIdx.y < dm.H * tiles) {
     const int h = blockIdx.y / tiles, tl = blockIdx.y - h * tiles;
@@ -217,11 +219,11 @@ ss_chunk_kernel(const float* __restrict__ xs, const float* __restrict__ bs, cons
     }
     ss_copy_wait<0>();
     __syncthreads();
-    ss_product_fma<4>(acc, As, 64, Bs, 64, (ck.n + 3) & ~3);   // (rows past the chunk's tokens are zero)
+    ss_product<4>(acc, As, 64, Bs, 64, (ck.n + 3) & ~3);   // (rows past the chunk's tokens are zero)
     float* dst = st + ((size_t)slot * dm.H + h) * dm.N * Pp + c0 + j0;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
-      const int n = n0 + ss_fma_row(i0, r);
+      const int n = n0 + ss_row(i0, r);
       if (n >= dm.N) continue;
       if (c0 + j0 < Pp) ss_store4(dst + (size_t)n * Pp, make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]));
       if (c0 + j0 + 32 < Pp) ss_store4(dst + (size_t)n * Pp + 32, make_float4(acc[r][4], acc[r][5], acc[r][6], acc[r][7]));
@@ -249,12 +251,12 @@ ss_chunk_kernel(const float* __restrict__ xs, const float* __restrict__ bs, cons
       bp[0] = bv[m].x, bp[64] = bv[m].y, bp[128] = bv[m].z, bp[192] = bv[m].w;
     }
     __syncthreads();
-    ss_product_fma<4>(acc, As, 64, Bs, 64, min(32, Np - kb));
+    ss_product<4>(acc, As, 64, Bs, 64, min(32, Np - kb));
   }
   float* dst = cb + ((size_t)slot * dm.G + g) * 4096;
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
-    float* row = dst + ss_fma_row(j0, c) * 64 + i0;
+    float* row = dst + ss_row(j0, c) * 64 + i0;
     ss_store4(row, make_float4(acc[0][c], acc[1][c], acc[2][c], acc[3][c]));
     ss_store4(row + 32, make_float4(acc[4][c], acc[5][c], acc[6][c], acc[7][c]));
   }
@@ -321,16 +323,14 @@ ss_pass_kernel(const SsProj proj, const SsDims dm, float* __restrict__ st, const
   }
 }
 
-// y [T][inner] = (recurrence's output + D x) silu(z), 64 tokens x 64 columns of a head per CTA.  4100 tokens, 64 heads of
-// 128 x 64: 183 us (200 with the products on the FMA units); bound by the latency of its steps at 16 warps an SM.  Off the
-// 64-bit result by 1.6e-7 (1.9e-7).
-__global__ void __launch_bounds__(SS_THREADS, 4)
+// y [T][inner] = (recurrence's output + D x) silu(z), 64 tokens x 64 columns of a head per CTA.
+__global__ void __launch_bounds__(SS_THREADS)
 ss_out_kernel(const SsProj proj, const SsDims dm, const float* __restrict__ xs, const float* __restrict__ cs,
               const float2* __restrict__ da, const float* __restrict__ st, const float* __restrict__ cb,
               const float* __restrict__ skip, float* __restrict__ y, const int* __restrict__ seq_start, int n_seqs,
               int n_tokens) {
-  __shared__ __align__(16) float Ms[64 * SS_LD];      // row j: L_ij (C_i . B_j) dt_j over i; before that the turned C
-  __shared__ __align__(16) float Bs[2][32 * SS_LD];      // rows of E, then of x
+  __shared__ __align__(16) float Ms[64 * SS_LDM];      // row j: L_ij (C_i . B_j) dt_j over i; before that the turned C
+  __shared__ __align__(16) float Bs[2][32 * 64];       // rows of E, then of x
   __shared__ float a_s[SS_CHUNK], gamma[SS_CHUNK];
   pdl_launch_dependents();
   const int tid = threadIdx.x, slot = blockIdx.x;
@@ -342,128 +342,126 @@ ss_out_kernel(const SsProj proj, const SsDims dm, const float* __restrict__ xs, 
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   pdl_wait();
   const int lr = tid >> 4, lc = (tid & 15) * 4;        // a row of E or x: 16 lanes
-  const int tok = tid & 63, part = tid >> 6;           // a token's C, a column of the masked matrix: two threads
   const bool col_live = c0 + lc < Pp;
   const float* e_base = st + ((size_t)slot * dm.H + h) * dm.N * Pp + c0 + lc;
   const float* x_base = xs + ((size_t)ck.t0 * dm.H + h) * Pp + c0 + lc;
-  const float* crow = cs + ((size_t)(ck.t0 + tok) * dm.G + g) * Np;
+  const float* crow = cs + ((size_t)(ck.t0 + tid) * dm.G + g) * Np;
   const int e_steps = (dm.N + 31) >> 5, steps = e_steps + ((ck.n + 31) >> 5);
   auto copy_rows = [&](int step) {                      // 32 rows of E, then of x, into one of two buffers
     float* dst = Bs[step & 1] + lc;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const int r = lr + 8 * m, k = (step < e_steps ? step : step - e_steps) * 32 + r;
+    for (int m = 0; m < 8; ++m) {
+      const int r = lr + 4 * m, k = (step < e_steps ? step : step - e_steps) * 32 + r;
       const bool live = col_live && (step < e_steps ? k < dm.N : k < ck.n);
       const float* src = step < e_steps ? e_base + (size_t)k * Pp : x_base + (size_t)k * dm.H * Pp;
-      ss_copy16(dst + r * SS_LD, live ? src : xs, live);
+      ss_copy16(dst + r * 64, live ? src : xs, live);
     }
     ss_copy_commit();
   };
-  float4 cv[4];
+  float4 cv[8];
   auto fetch_c = [&](int kb) {
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const int k = kb + 16 * part + 4 * m;
-      cv[m] = tok < ck.n && k < Np ? ss_load4(crow + k) : zero;
-    }
+    for (int m = 0; m < 8; ++m) cv[m] = tid < ck.n && kb + 4 * m < Np ? ss_load4(crow + kb + 4 * m) : zero;
   };
   copy_rows(0);
   fetch_c(0);
   // the rest is on its way to L2 meanwhile: rows of E, z and the products C . B
   for (int i = tid; i < 2 * dm.N; i += SS_THREADS)
     if (c0 + (i & 1) * 32 < Pp) prefetch_l2(st + ((size_t)slot * dm.H + h) * dm.N * Pp + (size_t)(i >> 1) * Pp + c0 + (i & 1) * 32);
-  if (tok < ck.n && c0 + part * 32 < dm.P) prefetch_l2(proj.p + (size_t)(ck.t0 + tok) * proj.row_stride + h * dm.P + c0 + part * 32);
-  prefetch_l2(cb + ((size_t)slot * dm.G + g) * 4096 + tid * 32);
-  const float2 own = tok < ck.n ? da[(size_t)h * n_tokens + ck.t0 + tok] : make_float2(1.f, 0.f);    // this token's a and dt
-  a_s[tok] = own.x;
-  float acc[4][8];
+  for (int i = tid; i < 128; i += SS_THREADS) {
+    prefetch_l2(cb + ((size_t)slot * dm.G + g) * 4096 + i * 32);
+    if ((i >> 1) < ck.n && c0 + (i & 1) * 32 < dm.P)
+      prefetch_l2(proj.p + (size_t)(ck.t0 + (i >> 1)) * proj.row_stride + h * dm.P + c0 + (i & 1) * 32);
+  }
+  const float2 own = tid < ck.n ? da[(size_t)h * n_tokens + ck.t0 + tid] : make_float2(1.f, 0.f);    // this token's a and dt
+  a_s[tid] = own.x;
+  float acc[8][8];
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+  for (int r = 0; r < 8; ++r)
 #pragma unroll
     for (int c = 0; c < 8; ++c) acc[r][c] = 0.f;
   const int i0 = ss_row0(), j0 = ss_col0();
-  // steps of 32: E^T C_i, then the sum over the chunk's own tokens
-#pragma unroll 1
-  for (int s = 0; s < steps; ++s) {
-    const int jb = (s - e_steps) * 32;
-    const float* A = Ms + jb * SS_LD;
-    int K = min(32, ck.n - jb), first_row = jb;
-    if (s < e_steps) {
-      float* As = Ms + (s & 1) * 32 * SS_LD;
+  // ---- E^T C_i
+  for (int s = 0; s < e_steps; ++s) {
+    float* As = Ms + (s & 1) * 32 * 64;
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {                    // C turned: a row of shared memory holds one dim of all tokens
-        float* ap = As + (16 * part + 4 * m) * SS_LD + tok;
-        ap[0] = cv[m].x, ap[SS_LD] = cv[m].y, ap[2 * SS_LD] = cv[m].z, ap[3 * SS_LD] = cv[m].w;
-      }
-      A = As, K = min(32, Np - s * 32), first_row = -64;                  // (rows of E past N are zero)
-    } else if (jb == 0) {
-      if (tid < 32) {                                  // gamma, two tokens a lane, by a prefix product over the warp
-        const float a0 = a_s[2 * tid], a1 = a_s[2 * tid + 1];
-        float v = a0 * a1;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const float u = __shfl_up_sync(0xffffffffu, v, o);
-          if (tid >= o) v *= u;
-        }
-        float before = __shfl_up_sync(0xffffffffu, v, 1);
-        if (tid == 0) before = 1.f;
-        gamma[2 * tid] = before * a0;
-        gamma[2 * tid + 1] = before * a0 * a1;
-      }
-      __syncthreads();                                 // the turned C has been read: its place takes the masked matrix
-      // L_ij by multiplying a along i from the diagonal on; what lies above it is zero
-      const float* cbj = cb + (((size_t)slot * dm.G + g) * 64 + tok) * 64;
-      float L = own.y;                                 // (dt_j rides on it)
-      if (part == 1)
-#pragma unroll
-        for (int i = 1; i < 32; ++i)
-          if (i > tok) L *= a_s[i];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int i1 = 32 * part + 16 * q;
-        float4 d[4];
-#pragma unroll
-        for (int m = 0; m < 4; ++m) d[m] = i1 + 15 >= tok ? ss_load4(cbj + i1 + 4 * m) : zero;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          float o[4] = {d[m].x, d[m].y, d[m].z, d[m].w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = i1 + 4 * m + e;
-            if (i > tok) L *= a_s[i];
-            o[e] = i >= tok ? o[e] * L : 0.f;
-          }
-          ss_store4(Ms + tok * SS_LD + i1 + 4 * m, make_float4(o[0], o[1], o[2], o[3]));
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const float ga = gamma[i0 + r];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) acc[r][c] *= ga;
-      }
+    for (int m = 0; m < 8; ++m) {                      // C turned: a row of shared memory holds one dim of all tokens
+      float* ap = As + 4 * m * 64 + tid;
+      ap[0] = cv[m].x, ap[64] = cv[m].y, ap[128] = cv[m].z, ap[192] = cv[m].w;
     }
     ss_copy_wait<0>();
     __syncthreads();                                   // (and every thread is done with the tiles of the step before)
-    if (s + 1 < steps) copy_rows(s + 1);
+    copy_rows(s + 1);
     if (s + 1 < e_steps) fetch_c((s + 1) * 32);
-    ss_product(acc, A, Bs[s & 1], K, first_row);
+    ss_product<2>(acc, As, 64, Bs[s & 1], 64, min(32, Np - s * 32));
+  }
+  __syncthreads();                                     // the turned C has been read: its place takes the masked matrix
+  if (tid < 32) {                                      // gamma, two tokens a lane, by a prefix product over the warp
+    const float a0 = a_s[2 * tid], a1 = a_s[2 * tid + 1];
+    float v = a0 * a1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float u = __shfl_up_sync(0xffffffffu, v, o);
+      if (tid >= o) v *= u;
+    }
+    float before = __shfl_up_sync(0xffffffffu, v, 1);
+    if (tid == 0) before = 1.f;
+    gamma[2 * tid] = before * a0;
+    gamma[2 * tid + 1] = before * a0 * a1;
+  }
+  {
+    // L_ij by multiplying a along i, a thread a column j; what lies above the diagonal is zero
+    const float* cbj = cb + (((size_t)slot * dm.G + g) * 64 + tid) * 64;
+    float L = own.y;                                   // (dt_j rides on it)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float4 d[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) d[m] = 16 * q + 15 >= tid ? ss_load4(cbj + 16 * q + 4 * m) : zero;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        float o[4] = {d[m].x, d[m].y, d[m].z, d[m].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = 16 * q + 4 * m + e;
+          if (i > tid) L *= a_s[i];
+          o[e] = i >= tid ? o[e] * L : 0.f;
+        }
+        ss_store4(Ms + tid * SS_LDM + 16 * q + 4 * m, make_float4(o[0], o[1], o[2], o[3]));
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const float ga = gamma[ss_row(i0, r)];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[r][c] *= ga;
+  }
+  // ---- + sum over the chunk's own tokens
+  for (int s = e_steps; s < steps; ++s) {
+    ss_copy_wait<0>();
+    __syncthreads();
+    if (s + 1 < steps) copy_rows(s + 1);
+    const int jb = (s - e_steps) * 32;
+    if (jb == 0) ss_product<2>(acc, Ms, SS_LDM, Bs[s & 1], 64, min(32, ck.n));
+    else ss_product<2, false>(acc, Ms + jb * SS_LDM, SS_LDM, Bs[s & 1], 64, ck.n - jb);      // (they reach rows 32.. only)
   }
   // ---- + D x, times silu(z)
   const int inner = dm.inner();
   const float dsk = skip[h];
   const bool vec = (dm.P & 3) == 0 && (proj.row_stride & 3) == 0 && (proj.split_stride & 3) == 0;
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = i0 + r;
+  for (int r = 0; r < 8; ++r) {
+    const int i = ss_row(i0, r);
     if (i >= ck.n) continue;
     const size_t t = (size_t)(ck.t0 + i);
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-      const int p = c0 + j0 + 4 * half;
+      const int p = c0 + j0 + 32 * half;
       if (p >= dm.P) continue;
       // (the chunk's x are what the last steps read: tokens from 32 on in the other buffer)
-      const float4 x = ss_load4(Bs[(e_steps + (i >> 5)) & 1] + (i & 31) * SS_LD + j0 + 4 * half);
+      const float4 x = ss_load4(Bs[(e_steps + (i >> 5)) & 1] + (i & 31) * 64 + j0 + 32 * half);
       const float* ar = acc[r] + 4 * half;
       float v[4] = {fmaf(dsk, x.x, ar[0]), fmaf(dsk, x.y, ar[1]), fmaf(dsk, x.z, ar[2]), fmaf(dsk, x.w, ar[3])};
       float* dst = y + t * inner + (size_t)h * dm.P + p;
@@ -681,7 +679,7 @@ LLMX_API int llmx_ss_prompt(const float* proj, int n_split, long long split_stri
   }
 #undef PREP
 #undef PREP2
-  launch_pdl(ss_chunk_kernel, dim3(chunks, H * p_tiles * n_tiles + G), dim3(SS_FMA_THREADS), 0, stream, (const float*)xs,
+  launch_pdl(ss_chunk_kernel, dim3(chunks, H * p_tiles * n_tiles + G), dim3(SS_THREADS), 0, stream, (const float*)xs,
              (const float*)bs, (const float*)cs, (const float2*)da, st, at, cb, seq_start, n_seqs, n_tokens, dm);
   const long long quads = (long long)H * N * (dm.Pp() / 4);
   const int state_blocks = (int)((quads + 255) / 256), ring_blocks = taps > 1 ? (C + 255) / 256 : 0;

@@ -69,6 +69,39 @@ def test_a_value_that_is_not_finite_changes_no_token_before_it(at, bad):
     assert torch.equal(~torch.isfinite(state[0]), lost)
 
 
+@pytest.mark.parametrize("at", [64, 70, 100, 127, 130])
+def test_a_value_at_the_end_of_the_range_reaches_its_own_column_only(at):
+    """The largest finite values are values like others: finite results, and the tokens before one keep their bits."""
+    H, D, Dv, n = 2, 128, 65, 140
+    torch.manual_seed(at)
+    decay, proj = torch.tensor([0.9, 0.99], device=DEV), torch.randn(n, H * (2 * D + Dv), device=DEV)
+    proj[at, H * D : 2 * H * D] *= 0.01                            # (keys below 1: sums of the products stay in range)
+    start = torch.randn(1, H, D, Dv, device=DEV)
+    clean = run(proj, [n], H, D, Dv, decay, start.clone(), [0])
+    proj[at, 2 * H * D + 3] = 3.4025e38                            # head 0, column 3
+    state = start.clone()
+    out = run(proj, [n], H, D, Dv, decay, state, [0])
+    changed = torch.zeros(n, H * Dv, dtype=torch.bool, device=DEV)
+    changed[at:, 3] = True
+    assert torch.equal(out[~changed], clean[~changed])
+    assert torch.isfinite(out).all() and torch.isfinite(state).all()
+
+
+def test_products_of_equal_operands():
+    """Operands that are all (1 + 2^-11 - 2^-23) or its negative, whose products lose the same way every time where an
+    operand is cut in parts that do not hold all its bits.  Tolerance as above."""
+    H, D, Dv, n, e = 1, 128, 128, 192, 1 + 2.0 ** -11 - 2.0 ** -23
+    torch.manual_seed(0)
+    proj = torch.where(torch.rand(n, H * (2 * D + Dv), device=DEV) < 0.5, -e, e)
+    decay, before = torch.tensor([1.0], device=DEV), torch.zeros(1, H, D, Dv, device=DEV)
+    state = before.clone()
+    out = run(proj, [n], H, D, Dv, decay, state, [0])
+    one = torch.ones(n, H, device=DEV, dtype=torch.float64)
+    want, after = recurrence(proj, [n], [0], before, one, one, H, D, Dv, False)
+    assert ((out - want).norm() / want.norm()).item() < 5e-7
+    assert ((state - after).norm() / after.norm()).item() < 5e-7
+
+
 def recurrence(proj, lens, slots, state, a, b, H, D, Dv, ones):
     """Token by token in 64 bits; a, b: [T, H]."""
     outs, t0 = [], 0
