@@ -453,6 +453,33 @@ LLMX_API int llmx_add_gain_sumsq(float* h, const void* delta, int delta_dtype, i
 // table entry, gains and rotation rows are fetched once for all of them, and their loads go out together.
 #define QKV_SPW 4
 
+// Sum of squares of a head, V neighbouring dims a lane and LPH lanes a head, in the order of the kernel that owns dims lane,
+// lane + 32, ..: 32 chains, which meet by a butterfly.  Every path to a result has its bits.
+template <int V, int LPH>
+__device__ __forceinline__ float head_sumsq(const float (&x)[V], unsigned mask) {
+  constexpr int STEP = 32 / V;                      // lanes from a dim to the next of its chain
+  const int l = threadIdx.x % STEP;
+  float c[V];
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+    c[e] = 0.f;
+#pragma unroll
+    for (int k = 0; k < LPH / STEP; ++k) {
+      const float v = __shfl_sync(mask, x[e], l + k * STEP, LPH);
+      c[e] = fmaf(v, v, c[e]);
+    }
+  }
+#pragma unroll
+  for (int o = STEP / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int e = 0; e < V; ++e) c[e] += __shfl_xor_sync(mask, c[e], o);
+#pragma unroll
+  for (int o = V / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int e = 0; e < o; ++e) c[e] += c[e + o];
+  return c[0];
+}
+
 template <typename TIN, typename TA, typename TC, bool DEEP, int LPH>
 __global__ void qk_norm_rope_cache_kernel(const TIN* __restrict__ qkv, int n_split, size_t split_stride,
                                           TA* __restrict__ q_out,
@@ -487,7 +514,8 @@ __global__ void qk_norm_rope_cache_kernel(const TIN* __restrict__ qkv, int n_spl
   if constexpr (LPH > 0) {
     // Head size 4 LPH with full rotation or none: a lane owns four neighbouring dims, read and written as one vector, and
     // 32 / LPH heads share a warp; the rotation partner (half a head away) lives in lane +-LPH/2 and comes by shuffle.  Bound
-    // by two trips to L2; a decode step's launch with heads of 64, one token: 4.4 us an element a lane, 2.1 like this.
+    // by two trips to L2.  16 + 2 * 8 heads of 64, an element a lane and like this: one token of five partials 3.0 and 1.8 us,
+    // 23 tokens 6.0 and 2.9, 4000 tokens 33.8 and 13.9; unrotated heads of 128 with gains, 64 tokens: 6.1 and 2.9.
     constexpr int HD = 4 * LPH;
     const int l = lane % LPH, d0 = 4 * l, dh = d0 & (HD / 2 - 1), sub = lane / LPH;
     const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
@@ -516,9 +544,13 @@ __global__ void qk_norm_rope_cache_kernel(const TIN* __restrict__ qkv, int n_spl
       const int slot = slot0 + j * HPW + sub;
       float4 x = xs[j];
       const bool is_q = slot < H, is_k = !is_q && slot < H + G;
-      float ssq = x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
-#pragma unroll
-      for (int o = LPH / 2; o > 0; o >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
+      float ssq = 0.f;
+      if (LPH == 32 && n_rot) {
+        ssq = warp_sum(x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w);
+      } else if (q_gain || k_gain) {
+        const float v[4] = {x.x, x.y, x.z, x.w};
+        ssq = head_sumsq<4, LPH>(v, 0xffffffffu);
+      }
       if ((is_q && q_gain) || (is_k && k_gain)) {
         const float4 gn = is_q ? gq : gk;
         const float scale = 1.0f / sqrtf(ssq / (float)HD + eps);
@@ -530,11 +562,13 @@ __global__ void qk_norm_rope_cache_kernel(const TIN* __restrict__ qkv, int n_spl
       p.z = __shfl_xor_sync(0xffffffffu, x.z, LPH / 2);
       p.w = __shfl_xor_sync(0xffffffffu, x.w, LPH / 2);
       if (n_rot && (is_q || is_k)) {
-        if (l < LPH / 2) {   // dims i of the first half: x_i cos - x_(i+half) sin
-          r = make_float4(x.x * cs.x - p.x * sn.x, x.y * cs.y - p.y * sn.y, x.z * cs.z - p.z * sn.z, x.w * cs.w - p.w * sn.w);
-        } else {             // dims i + half: x_i sin + x_(i+half) cos
-          r = make_float4(p.x * sn.x + x.x * cs.x, p.y * sn.y + x.y * cs.y, p.z * sn.z + x.z * cs.z, p.w * sn.w + x.w * cs.w);
-        }
+        // dims i of the first half: x_i cos - x_(i+half) sin; dims i + half: x_i sin + x_(i+half) cos.  Which product is rounded
+        // by itself is what the kernels of these head sizes have always done.
+        auto turn = [&](float x, float p, float c, float s) {
+          if (l < LPH / 2) return fmaf(x, c, -__fmul_rn(p, s));
+          return LPH == 32 ? fmaf(x, c, __fmul_rn(p, s)) : fmaf(p, s, __fmul_rn(x, c));
+        };
+        r = make_float4(turn(x.x, p.x, cs.x, sn.x), turn(x.y, p.y, cs.y, sn.y), turn(x.z, p.z, cs.z, sn.z), turn(x.w, p.w, cs.w, sn.w));
       }
       if (slot >= n_slots) continue;
       if (is_q) store4(q_out + (size_t)t * H * HD + (size_t)slot * HD + d0, r);
@@ -593,7 +627,8 @@ __global__ void qk_norm_rope_cache_kernel(const TIN* __restrict__ qkv, int n_spl
 
 // The same for prompts when everything is bfloat16, the head size is 128 and the rotation is full or none: half a
 // warp per head, a lane owns eight consecutive dims (one 16-byte load, one 16-byte store); the rotation
-// partner (dim +-64) lives eight lanes away.  A warp takes eight heads of its token, two at a time.
+// partner (dim +-64) lives eight lanes away.  A warp takes eight heads of its token, two at a time.  4100 tokens of 16 + 2 * 4
+// heads: rotated 13.8 us, unrotated with gains 20.6 (their squares' chains cross lanes; an element a lane 32.2).
 #define QKV8_PER_WARP 8
 
 __global__ void qk_norm_rope_cache_bf16_d128_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ q_out,
@@ -670,10 +705,14 @@ __global__ void qk_norm_rope_cache_bf16_d128_kernel(const bf16* __restrict__ qkv
     const float* gain = is_q ? gq : gk;
     if (is_q ? q_gain != nullptr : k_gain != nullptr) {
       float ss = 0.f;
+      if (n_rot) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) ss += x[i] * x[i];
+        for (int i = 0; i < 8; ++i) ss += x[i] * x[i];
 #pragma unroll
-      for (int sh = 8; sh > 0; sh >>= 1) ss += __shfl_xor_sync(mask, ss, sh);
+        for (int sh = 8; sh > 0; sh >>= 1) ss += __shfl_xor_sync(mask, ss, sh);
+      } else {
+        ss = head_sumsq<8, 16>(x, mask);
+      }
       const float scale = 1.0f / sqrtf(ss / 128.0f + eps);
 #pragma unroll
       for (int i = 0; i < 8; ++i) x[i] = (x[i] * scale) * gain[i];

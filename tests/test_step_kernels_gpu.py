@@ -125,6 +125,30 @@ def test_heads_of_64_and_unrotated_heads(D, n_rot, H, G, T, n_split, gains):
     assert torch.equal(torch.stack([vc[a, :, r] for a, r in where]), row[:, H + G :].float().bfloat16())
 
 
+@pytest.mark.parametrize("D, n_rot, T, n_split", [(64, 64, 3, 1), (64, 64, 5, 3), (64, 0, 70, 1), (64, 64, 70, 2), (128, 0, 4, 4),
+                                                  (128, 0, 5, 1), (128, 0, 64, 1), (128, 0, 70, 1)])
+@pytest.mark.parametrize("act", [torch.float32, torch.bfloat16])
+def test_heads_by_vectors_add_squares_as_an_element_a_lane_does(D, n_rot, T, n_split, act):
+    """q and k have the same bits whether the heads go by vectors or, for values of another size, an element a lane."""
+    from llmoxide_b200 import kernels
+    torch.manual_seed(D + T)
+    H, G = 5, 2
+    qk, v = torch.randn(n_split, T, (H + G) * D, device=DEV), torch.randn(n_split, T, G * D, device=DEV)
+    gq, gk = 1 + 0.1 * torch.randn(2, D, device=DEV)
+    pos, seq = torch.arange(30, 30 + T, dtype=torch.int32, device=DEV), torch.zeros(T, dtype=torch.int32, device=DEV)
+    angle = torch.rand(200, max(n_rot // 2, 1), device=DEV) * 6.28
+    cos, sin = (angle.cos(), angle.sin()) if n_rot else (None, None)
+    table, made = torch.tensor([[2, 0, 1]], dtype=torch.int32, device=DEV), []
+    for Dv in (D, D - 4):
+        x = torch.cat([qk, v[:, :, : G * Dv]], 2)
+        x = x[0].to(act) if n_split == 1 else x
+        k_cache, v_cache = (torch.zeros(3, G, 64, n, dtype=act, device=DEV) for n in (D, Dv))
+        q = torch.empty(T, H * D, dtype=act, device=DEV)
+        kernels.qk_norm_rope_cache(x, q, k_cache, v_cache, table, seq, pos, gq, gk, 1e-6, cos, sin, n_rot, H, G, D, True, Dv)
+        made.append((q, k_cache))
+    assert torch.equal(made[0][0], made[1][0]) and torch.equal(made[0][1], made[1][1])
+
+
 @pytest.mark.parametrize("dtype, n_split", [(torch.bfloat16, 1), (torch.float32, 1), (torch.float32, 9)])
 @pytest.mark.parametrize("per_head, H, Dv", [(True, 3, 128), (True, 5, 20), (False, 4, 128), (False, 3, 700), (False, 17, 300),
                                              (True, 2, 132), (False, 1, 8196)])
