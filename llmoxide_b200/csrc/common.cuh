@@ -322,6 +322,32 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+// Sum of squares of a head, V neighbouring dims a lane and LPH lanes a head, in the order of the kernel that owns dims lane,
+// lane + 32, ..: 32 chains, which meet by a butterfly.  Every path to a result has its bits.
+template <int V, int LPH>
+__device__ __forceinline__ float head_sumsq(const float (&x)[V], unsigned mask) {
+  constexpr int STEP = 32 / V;                      // lanes from a dim to the next of its chain
+  const int l = threadIdx.x % STEP;
+  float c[V];
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+    c[e] = 0.f;
+#pragma unroll
+    for (int k = 0; k < LPH / STEP; ++k) {
+      const float v = __shfl_sync(mask, x[e], l + k * STEP, LPH);
+      c[e] = fmaf(v, v, c[e]);
+    }
+  }
+#pragma unroll
+  for (int o = STEP / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int e = 0; e < V; ++e) c[e] += __shfl_xor_sync(mask, c[e], o);
+#pragma unroll
+  for (int o = V / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int e = 0; e < o; ++e) c[e] += c[e + o];
+  return c[0];
+}
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

@@ -1181,9 +1181,10 @@ gated_norm_row_kernel(const float* __restrict__ o, const TIN* __restrict__ proj,
 }
 
 // The same by four neighbouring elements a thread, U times (sizes, offsets and strides multiples of 4, no gates), everything
-// asked for ahead of the reduction: an element at a time, first the squares and then again the outputs, a row of 2048 with
-// five partials took 11.5 us in a decode step, 2.8 like this; 4100 rows 34 -> 28 (bound by memory).  U 0: a warp per (token,
-// head) of up to 128 columns: 6.4 -> 1.9 us and 34 -> 27.
+// asked for ahead of the reduction.  The squares are added in the chains of the kernels above, a row's by way of shared memory,
+// so that the bits are theirs.  By elements and like this: four rows of 2048 with five partials (a decode step) 6.8 and 2.2 us,
+// of 8192 23.6 and 5.0; 4100 rows of 2048 24 both (bound by memory), of 8192 140 and 93.  U 0: a warp per (token, head) of up
+// to 128 columns: 4 and 4100 tokens of 16 heads 3.7 and 1.7, 28.8 and 23.8.
 template <typename TIN, typename TO, int U>
 __global__ void __launch_bounds__(U ? 512 : 128)
 gated_norm_vec_kernel(const float* __restrict__ o, const TIN* __restrict__ proj, int n_split, size_t split_stride,
@@ -1216,9 +1217,18 @@ gated_norm_vec_kernel(const float* __restrict__ o, const TIN* __restrict__ proj,
     const int i = (u * LANES + lane) * 4;
     if (i < n) la_values(grow + i, n_split, split_stride, z[u]);
   }
+  if constexpr (U == 0) {
+    ss = head_sumsq<4, 32>(v[0], 0xffffffffu);
+  } else {                                                             // a thread's squares are columns 256 apart
+    __shared__ __align__(16) float squared[U * 2048];
 #pragma unroll
-  for (int u = 0; u < PARTS; ++u) ss += (v[u][0] * v[u][0] + v[u][1] * v[u][1]) + (v[u][2] * v[u][2] + v[u][3] * v[u][3]);
-  ss = U ? block_sum(ss, red) : warp_sum(ss);
+    for (int u = 0; u < U; ++u) *reinterpret_cast<float4*>(squared + (u * 512 + lane) * 4) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+    __syncthreads();
+    if (lane < 256)
+#pragma unroll
+      for (int k = 0; k < 8 * U; ++k) ss = fmaf(squared[k * 256 + lane], squared[k * 256 + lane], ss);
+    ss = block_sum(ss, red);
+  }
   const float rs = 1.0f / sqrtf(ss / (float)n + eps);
 #pragma unroll
   for (int u = 0; u < PARTS; ++u) {

@@ -149,6 +149,25 @@ def test_heads_by_vectors_add_squares_as_an_element_a_lane_does(D, n_rot, T, n_s
     assert torch.equal(made[0][0], made[1][0]) and torch.equal(made[0][1], made[1][1])
 
 
+@pytest.mark.parametrize("dtype, n_split", [(torch.bfloat16, 1), (torch.float32, 3)])
+@pytest.mark.parametrize("per_head, H, Dv", [(True, 3, 128), (True, 5, 20), (True, 2, 96), (False, 4, 128), (False, 3, 700),
+                                             (False, 16, 128), (False, 17, 300), (False, 1, 8192), (False, 3, 4)])
+def test_gated_norm_by_vectors_adds_squares_as_by_elements(dtype, n_split, per_head, H, Dv):
+    """The same bits by vectors and, from a column that is no vector's first, by elements."""
+    from llmoxide_b200 import kernels
+    torch.manual_seed(H * Dv)
+    T, n = 5, H * Dv
+    o, gain = torch.randn(T, n, device=DEV), 1 + 0.1 * torch.randn(n, device=DEV)
+    z, made = torch.randn(n_split, T, n, device=DEV).to(dtype), []
+    for g_off in (8, 9):
+        proj = torch.zeros(n_split, T, n + 12, dtype=dtype, device=DEV)
+        proj[:, :, g_off : g_off + n] = z
+        y = torch.empty(T, n, device=DEV)
+        kernels.gated_norm(o, proj[0] if n_split == 1 else proj, g_off, gain, 1e-5, "silu", per_head, y, H, Dv)
+        made.append(y)
+    assert torch.equal(*made)
+
+
 @pytest.mark.parametrize("dtype, n_split", [(torch.bfloat16, 1), (torch.float32, 1), (torch.float32, 9)])
 @pytest.mark.parametrize("per_head, H, Dv", [(True, 3, 128), (True, 5, 20), (False, 4, 128), (False, 3, 700), (False, 17, 300),
                                              (True, 2, 132), (False, 1, 8196)])
