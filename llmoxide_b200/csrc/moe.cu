@@ -39,10 +39,11 @@ __device__ __forceinline__ int warp_argmax(float v, int i) {
 }
 
 // One token, by one warp: z its E logits (global or shared memory), s, c and gs scratch of E, E and n_groups
-// floats (c: the scores the choice goes by).  Lane k < top returns the k-th choice and its weight.
+// floats (c: the scores the choice goes by).  Lane k < top returns the k-th choice and its weight.  report: whether a choice
+// that cannot be made is one.
 __device__ __forceinline__ void moe_route_token(const float* z, float* s, float* c, float* gs, int& id, float& weight, int lane, int E, int top, int n_groups,
                                                 int keep_groups, int group_top, int score_kind, int normalize,
-                                                float norm_eps, float scale, const float* __restrict__ bias) {
+                                                float norm_eps, float scale, const float* __restrict__ bias, bool report = true) {
   if (score_kind == MOE_SCORE_SOFTMAX) {
     float m = -INFINITY;
     for (int e = lane; e < E; e += 32) m = fmaxf(m, z[e]);
@@ -114,7 +115,7 @@ __device__ __forceinline__ void moe_route_token(const float* z, float* s, float*
         if (!(c[e] == -INFINITY) && e < bi) bi = e;
       bi = (int)__reduce_min_sync(0xffffffffu, (unsigned)bi);
       if (bi >= E) bi = k % E;
-      if (lane == 0) llmx_report(1);
+      if (lane == 0 && report) llmx_report(1);
     }
     if (lane == 0) c[bi] = -INFINITY;               // chosen: out of the running
     __syncwarp();
@@ -411,7 +412,7 @@ moe_router_kernel(const TX* __restrict__ x, long long ldx, const float* __restri
       int id;
       float weight;
       moe_route_token(z, z + n_rows, z, z + n_rows + E, id, weight, lane, E, top, n_groups, keep_groups, group_top, score_kind,
-                      normalize, norm_eps, scale, bias);
+                      normalize, norm_eps, scale, bias, pass != 0);
       if (pass && lane < top) {
         ids[(size_t)t * top + lane] = id, wts[(size_t)t * top + lane] = weight;
         if (PLACE) own_ids[j * top + lane] = id, own_wts[j * top + lane] = weight;

@@ -168,6 +168,28 @@ def test_gated_norm_by_vectors_adds_squares_as_by_elements(dtype, n_split, per_h
     assert torch.equal(*made)
 
 
+def test_routing_ahead_of_the_wait_reports_nothing():
+    """A correction leaves the first group one expert that can be chosen; the scores keep the second group, and the run of the
+    routing on zeros ahead of them, which would keep the first, is nobody's failure.  Where the scores keep the first, it is."""
+    from llmoxide_b200 import kernels
+    from llmoxide_b200.errors import KernelError
+    kernels.check_status()
+    x = torch.ones(2, 8, device=DEV).bfloat16()
+    correction = torch.tensor([0.0] + [-float("inf")] * 3 + [-0.2] * 4, device=DEV)
+    for scores, fails in ((5.0, False), (-5.0, True)):
+        w = torch.zeros(8, 8, device=DEV)
+        w[4:, 0] = scores * torch.tensor([1.0, 0.9, 0.8, 0.7], device=DEV)
+        ids, weights = torch.empty(2, 2, dtype=torch.int32, device=DEV), torch.empty(2, 2, device=DEV)
+        kernels.moe_router(x, w, ids, weights, 2, 1, 1, "sigmoid", True, 0.0, 1.0, bias=correction)
+        torch.cuda.synchronize()
+        if fails:
+            with pytest.raises(KernelError):
+                kernels.check_status()
+        else:
+            assert ids.tolist() == [[4, 5]] * 2
+            kernels.check_status()
+
+
 @pytest.mark.parametrize("dtype, n_split", [(torch.bfloat16, 1), (torch.float32, 1), (torch.float32, 9)])
 @pytest.mark.parametrize("per_head, H, Dv", [(True, 3, 128), (True, 5, 20), (False, 4, 128), (False, 3, 700), (False, 17, 300),
                                              (True, 2, 132), (False, 1, 8196)])
