@@ -1610,7 +1610,8 @@ def moe_router(x, w, ids, weights, n_groups: int, keep_groups: int, group_top: i
     whose products are written there as they are.  ``logit_bias`` float32 [E] joins the experts' logits before the
     scores are made.  ``score`` "softmax_top": the largest logits win, and the weights are the softmax over the
     winners' logits only.  ``places``: (perm, dest, sorted_weight, tiles, tile_rows, n_tiled, xs) to fill as ``moe_sort``
-    and ``moe_gather_rows`` do, in the same launch (bfloat16 ``x`` that ``moe_tc_supports``, up to MOE_PLACE_TOKENS)."""
+    and ``moe_gather_rows`` do, in the same launch (bfloat16 ``x`` that ``moe_tc_supports``, up to MOE_PLACE_TOKENS, and a
+    ``w`` that starts on 16 bytes)."""
     _dev(x, w, ids, weights, bias, extra_out, logit_bias)
     assert logit_bias is None or (logit_bias.dtype == torch.float32 and logit_bias.is_contiguous()
                                   and logit_bias.numel() == w.shape[0] - (0 if extra_out is None else extra_out.shape[1]))

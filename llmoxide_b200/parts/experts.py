@@ -163,7 +163,7 @@ class RoutedExperts:
             dest = torch.empty((P,), dtype=torch.int32, device=dev)
             sorted_w = torch.empty((P,), dtype=torch.float32, device=dev)
             xs = torch.empty((P, x.shape[1]), dtype=torch.bfloat16, device=dev)
-            if self.table is None and T <= kernels.MOE_PLACE_TOKENS:
+            if self.table is None and T <= kernels.MOE_PLACE_TOKENS and self.router.data_ptr() % 16 == 0:
                 places = (perm, dest, sorted_w, tiles, rows, self.E, xs)      # the router sorts and gathers too
         d = self.down.shape[1]
         y = join_shared = None

@@ -46,6 +46,27 @@ def test_router_that_sorts_and_gathers(T, E, top, K, groups, keep, rows, score, 
     assert got[: len(want)] == want and all(t[0] == -1 for t in got[len(want):])
 
 
+@pytest.mark.parametrize("T", [1, 8, 9])
+def test_experts_whose_router_starts_between_vectors(T):
+    """A float32 router that lies at no vector's start (a view of a larger buffer) chooses as the same numbers elsewhere do."""
+    from types import SimpleNamespace
+    from llmoxide_b200.config.spec import PartSpec, TensorSpec
+    from llmoxide_b200.parts import Runtime
+    from llmoxide_b200.parts.experts import RoutedExperts
+    torch.manual_seed(T)
+    E, d, ff = 4, 64, 32
+    x, numbers = torch.randn(T, d, device=DEV).bfloat16(), torch.randn(E * d + 1, device=DEV)
+    sizes = dict(gate=(ff, d), up=(ff, d), down=(d, ff))
+    tensors = dict(router=TensorSpec("router", (E, d)), **{f"{k}{e}": TensorSpec(f"{k}{e}", n) for k, n in sizes.items() for e in range(E)})
+    w = {f"{k}{e}": (torch.randn(n, device=DEV) * 0.1).bfloat16() for k, n in sizes.items() for e in range(E)}
+    made = []
+    for router in (numbers[1:].view(E, d), numbers[1:].view(E, d).clone()):
+        part = RoutedExperts(PartSpec("routed_experts", dict(hidden_size=d, intermediate_size=ff, n_experts=E, top=2), tensors),
+                             dict(w, router=router), Runtime(dtype="bfloat16", device=torch.device(DEV), max_positions=64))
+        made.append(part.forward(x, SimpleNamespace(probe=None)))
+    assert torch.equal(*made)
+
+
 @pytest.mark.parametrize("T", [63, 64, 65, 16 * 148, 2500])
 @pytest.mark.parametrize("E, n_extra", [(16, 0), (33, 1)])
 def test_router_of_few_and_many_tokens(T, E, n_extra):
