@@ -16,7 +16,7 @@ from .. import kernels
 from ..cache import Cache
 from ..config.spec import ModelSpec
 from ..parts import Runtime, build_block
-from ..parts.block import build_part
+from ..parts.block import build_part, join_results
 from ..parts.registry import EMBEDDINGS, HEADS, NORMS
 
 
@@ -31,6 +31,7 @@ class DecoderModel:
         for t in spec.embedding.tensors.values():       # the embedding left its tensors in for a tied head
             weights.pop(t.name, None)
         self._check_schedule()
+        join_results(self.blocks, spec.schedule, self.final_norm, int(getattr(spec, "residual_streams", 1) or 1))
         # A part that reads device data on the host during its forward (it says
         # so with ``graph_safe = False``) keeps decode steps out of CUDA graphs.
         self.graph_safe = (all(getattr(p, "graph_safe", True) for b in self.blocks for p in vars(b).values())

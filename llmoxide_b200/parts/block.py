@@ -121,11 +121,14 @@ def build_block(spec, weights: dict, rt):
 class ParallelBlock:
     """A single norm feeds mixer and feed-forward: x = norm(h); h += mixer(x) + feed_forward(x).  Nothing else reads the
     stream before the next layer's norm, and the feed-forward reads x: both results are handed on together as the pending
-    delta, which the next norm adds (the mixer's first), save what the mixer's last product has added to the stream itself.
+    delta, which the next norm adds (the mixer's first), where that norm takes them so (``join_results``).  Otherwise the
+    mixer's result, in any form that a norm adds, joins the stream at once, and the feed-forward's is the pending delta.
 
     With a norm for each sublayer (``mixer`` and ``feed_forward`` instead of ``shared``) one kernel adds what the block
     before owes and makes the rows of both norms; both results are owed to the next block together (``parts.norm.Joined``),
     save what a sublayer's last product has added to the stream itself."""
+
+    joins_results = False          # whether whoever follows takes both results as one ``Joined`` (``join_results``)
 
     def __init__(self, spec, weights: dict, rt):
         self.rt, position = rt, None
@@ -143,11 +146,15 @@ class ParallelBlock:
         if self.norm is None and getattr(self.mixer, "out_bias", None) is not None:
             self.mixer.defer_out_bias = True         # joins with the results, in the next block's norm kernel
 
+    @property
+    def takes_joined(self) -> bool:
+        return getattr(self.mixer_norm if self.norm is None else self.norm, "takes_joined", False)
+
     def cache_need(self):
         return self.mixer.cache_need()
 
     def libraries(self) -> set:
-        libs = {"dual_norm"}
+        libs = {"dual_norm"} if self.norm is None or self.joins_results else set()
         for part in (self.norm, self.mixer_norm, self.ff_norm, self.mixer, self.feed_forward):
             if part is not None:
                 libs |= getattr(part, "libraries", set)()
@@ -200,8 +207,22 @@ class ParallelBlock:
                             lambda a: probe("attn_output", _summed(a)) if probe else None)
         if probe and out is not None:
             probe("ffn_out", _summed(out))
-        # (what the mixer has not added to the stream itself joins it with the feed-forward's result, in the next norm's kernel)
-        return out if a is None else a if out is None else Joined([a, out])
+        if a is None or out is None:                 # (the mixer may have added its result to the stream itself)
+            return out if a is None else a
+        if self.joins_results and isinstance(a, torch.Tensor) and isinstance(out, torch.Tensor):
+            return Joined([a, out])
+        self.norm.add(h, a)
+        return out
+
+
+def join_results(blocks, schedule, final_norm, streams: int) -> None:
+    """Tells the parallel blocks with one norm whether every call that follows one of theirs (the model's last norm behind
+    the last) takes both results together: a norm of its own kind and size, and one copy of the stream."""
+    for i, block in enumerate(blocks):
+        if isinstance(block, ParallelBlock) and block.norm is not None:
+            after = [blocks[schedule[k + 1].layer] if k + 1 < len(schedule) else final_norm
+                     for k, call in enumerate(schedule) if call.layer == i]
+            block.joins_results = streams == 1 and all(getattr(part, "takes_joined", False) for part in after)
 
 
 @register_arrangement("hyper_connections")

@@ -204,6 +204,12 @@ class RMSNorm:
 
     ROW_SCALE_MAX_TOKENS = 64      # what the products' epilogues take
 
+    @property
+    def takes_joined(self) -> bool:
+        """Two results handed over as a ``Joined`` have the bits of one added after the other: both kernels then add up a
+        row by the same threads and vectors."""
+        return self.size % 4 == 0 and self.size <= 8192
+
     def add(self, h, delta) -> None:
         """h += delta (``delta`` [T,d] or split partials [S,T,d], added in order); nothing is normed."""
         if isinstance(delta, (PostNormed, WeightedSum)):

@@ -189,6 +189,25 @@ def test_gated_norm_by_vectors_adds_squares_as_by_elements(dtype, n_split, per_h
     assert torch.equal(*made)
 
 
+@pytest.mark.parametrize("d", [4, 60, 2048, 2052, 4096, 8192])
+@pytest.mark.parametrize("T, n_a, n_b", [(1, 1, 3), (3, 9, 5), (64, 2, 2), (65, 1, 1), (90, 3, 8)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_two_results_joined_as_one_after_the_other(d, T, n_a, n_b, dtype):
+    """A stream that gets two results and is normed in one kernel has the bits of one that gets them one by one."""
+    from llmoxide_b200 import kernels
+    torch.manual_seed(d + T)
+    a, b = (torch.randn(n, T, d, device=DEV) for n in (n_a, n_b))
+    a, b = a.to(dtype) if n_a == 1 else a, b.to(dtype) if n_b == 1 else b
+    gain, h, rows = 1 + 0.1 * torch.randn(d, device=DEV), torch.randn(T, d, device=DEV), torch.tensor([T - 1, 0], dtype=torch.int32, device=DEV)
+    for at in (None, rows):
+        one, two = h.clone(), h.clone()
+        out, joined = (torch.empty(T if at is None else 2, d, dtype=dtype, device=DEV) for _ in range(2))
+        kernels.add_rms_norm(one, a, gain, 1e-6, None)
+        kernels.add_rms_norm(one, b, gain, 1e-6, out, rows=at, write_h=at is None)
+        kernels.dual_norm(two, [a, b], None, gain, 1e-6, joined, rows=at, write_h=at is None)
+        assert torch.equal(out, joined) and (at is not None or torch.equal(one, two))
+
+
 def test_routing_ahead_of_the_wait_reports_nothing():
     """A correction leaves the first group one expert that can be chosen; the scores keep the second group, and the run of the
     routing on zeros ahead of them, which would keep the first, is nobody's failure.  Where the scores keep the first, it is."""
