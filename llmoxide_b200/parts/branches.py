@@ -12,8 +12,9 @@ from __future__ import annotations
 
 import torch
 
-# Steps of more tokens are bound by their products, not by the chain of launches (and a product of more than
-# ``kernels.PAIR_MIN_TOKENS`` may add to the residual stream itself, which two branches must not do at once).
+# The most tokens of a step that is cut up.  Two designs' steps (parallel blocks, most with routed experts; prompts of 200
+# tokens behind them) as one chain and in branches, us: 1 token 415 and 343, 516 and 378; 8: 544 and 511, 588 and 503; 16: 610
+# and 571, 677 and 583; 32: 689 and 652, 828 and 704; 64: 874 and 831, 1036 and 887.  Longer steps were not tried.
 MAX_TOKENS = 64
 
 

@@ -51,6 +51,21 @@ def test_results_are_joined_where_both_are_tensors_and_the_follower_takes_them()
             assert pending is out and block.norm.added == ([] if mixed is None else [mixed])
 
 
+def test_a_branch_leaves_the_stream_to_the_mixer(monkeypatch):
+    """Parts that add to the stream where they are given it: one after the other both are, side by side one is."""
+    from llmoxide_b200 import kernels
+    from llmoxide_b200.parts import branches
+    assert branches.MAX_TOKENS <= kernels.PAIR_MIN_TOKENS         # (products of more tokens add to the stream themselves)
+    h, a, out = torch.zeros(2, 8), torch.ones(2, 8), torch.ones(2, 8)
+    monkeypatch.setattr(branches, "fork", lambda rt, name, work: (work(), lambda: None))
+    for side_by_side in (False, True):
+        monkeypatch.setattr(branches, "wanted", lambda ctx, n: side_by_side)
+        block = block_of(a, out, norms="two", adds=True)
+        pending = block.forward(h, None, SimpleNamespace(probe=None), None)
+        assert pending.terms == [a, out] and block.mixer.residuals == [h]
+        assert block.feed_forward.residuals == ([None] if side_by_side else [h])
+
+
 def rms_norm(size):
     norm = RMSNorm.__new__(RMSNorm)
     norm.size = size
