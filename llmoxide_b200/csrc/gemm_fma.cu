@@ -327,25 +327,30 @@ LLMX_API int llmx_gemm_f32_form(int form, const float* X, const float* W, float*
   if (form >= 6 && (n_seg < 2 || n_seg > 8)) return LLMX_REFUSED(1);
   if (form < 0) {
     // Rule: the cheapest by what was measured over K = 64 to 8192, N = 64 to 8192 and 1 to 2500 tokens (us beside a launch's
-    // 1.5).  A step of 32 k in four segments costs a round of 296 CTAs of rows 0.6, 0.65, 0.75 or 1.1 (2, 4, 8, 16 tokens);
-    // 16 k cost 148 tiles of 32 x 64 0.26 (few tiles an SM cannot hide their waits: 0.41, 0.6, 1.01 and 1.1 at one to four),
-    // 148 tiles of 64 x 128 0.88 (1.17 at least).  Up to 512 k only one segment's threads work in the rows kernel, so tiles win
-    // there from few tokens on: 16 tokens, N = 8192, K = 256: 18 us by rows, 9.3 by tiles; N = 2048, K = 2048: 19 and 50.
-    // Tiles that share K cost by the CTA.  32 x 64: 14 + 0.0595, 20 at least (a round of rows that the rule puts at 17.6 takes 13,
-    // such tiles 16 to 18) and 40 beyond 296.  64 x 128: 57 and 69 while up to 148 and 256 run at once, then 32 + 0.222, and for many
-    // clusters of four, which fill the GPU better than three, six and eight do, 15 + 0.207.  Up to 16 tokens rows are cheaper than
-    // the rule thinks (9 tokens, N = 2048, K = 4096: 28 us, 35 by the rule, 31 shared).  64 tokens, N = 2048, K = 1024: 18.9 us
-    // shared, 26.6 not; 33 tokens, N = 8192, K = 2048: 64 and 91; 400 tokens, N = 8192, K = 3000: 613 and 574.
+    // 1.5, on 148 SMs; CTAs are counted by the SM).  A step of 32 k in four segments costs a round of two CTAs of rows an SM 0.6,
+    // 0.65, 0.75 or 1.1 (2, 4, 8, 16 tokens); 16 k cost a round of one tile of 32 x 64 an SM 0.26 (few tiles an SM cannot hide
+    // their waits: 0.41, 0.6, 1.01 and 1.1 at one to four), one of 64 x 128 0.88 (1.17 at least).  Up to 512 k only one
+    // segment's threads work in the rows kernel, so tiles win there from few tokens on: 16 tokens, N = 8192, K = 256: 18 us by
+    // rows, 9.3 by tiles; N = 2048, K = 2048: 19 and 50.
+    // Tiles that share K cost by the CTA, not by the round: their clusters are of all sizes.  32 x 64: 14 and 8.8 for every CTA an
+    // SM, 20 at least (a round of rows that the rule puts at 17.6 takes 13, such tiles 16 to 18) and 40 beyond two an SM.  64 x 128:
+    // 57 up to one an SM, 69 up to the 1.73 that run at once (clusters do not fill every GPC), then 32 and 32.9 for every
+    // one; many clusters of four, which fill the GPCs better than three, six and eight do, 15 and 30.6.  What the fit puts less
+    // than 3 % below another form is within its error and stays with that form (many clusters of four are taken as fitted).
+    // Up to 16 tokens rows are cheaper than the rule thinks (9 tokens, N = 2048, K = 4096: 28 us, 35 by the rule, 31
+    // shared).  64 tokens, N = 2048, K = 1024: 18.9 us shared, 26.6 not; 33 tokens, N = 8192, K = 2048: 64 and 91; 400 tokens,
+    // N = 8192, K = 3000: 613 and 574.  Over 621 shapes the rule's choice took 1.007 times the best form's time.
     const auto rounds = [](long long n, int m) { return (double)((n + m - 1) / m); };
     const auto tiles = [&](int bm, int bn) { return (long long)rounds(M, bm) * (long long)rounds(N, bn); };
+    const int sms = llmx_sm_count();
     const double steps = (n_seg / 4) * 16 + (n_seg % 4 == 1 ? (K - (n_seg - 1) * F32_SEG + 31) / 32 : n_seg % 4 ? 16 : 0);
     const double blocks = (K + 15) / 16;
     const int few = M <= 2 ? 0 : M <= 4 ? 1 : M <= 8 ? 2 : 3;
     const double a_step[4] = {0.6, 0.65, 0.75, 1.1};
-    const double rows = a_step[few] * steps * rounds(tiles(2 << few, 16), 2 * llmx_sm_count());
-    const double r = rounds(tiles(32, 64), llmx_sm_count());
+    const double rows = a_step[few] * steps * rounds(tiles(2 << few, 16), 2 * sms);
+    const double r = rounds(tiles(32, 64), sms);
     const double small = blocks * (r <= 1 ? 0.41 : r <= 2 ? 0.6 : fmax(0.26 * r, fmin(0.11 + 0.3 * r, 1.1)));
-    const double large = blocks * fmax(0.88 * rounds(tiles(64, 128), llmx_sm_count()), 1.17);
+    const double large = blocks * fmax(0.88 * rounds(tiles(64, 128), sms), 1.17);
     double best = rows;
     form = few;
     const auto take = [&](int f, double us) {
@@ -354,9 +359,9 @@ LLMX_API int llmx_gemm_f32_form(int form, const float* X, const float* W, float*
     take(4, small);
     take(5, large);
     if (M > 16 && n_seg >= 2 && n_seg <= 8) {
-      const double c6 = (double)n_seg * (double)tiles(32, 64), c7 = (double)n_seg * (double)tiles(64, 128);
-      take(6, 1.03 * fmax(14.0 + 0.0595 * c6, c6 > 296 ? 40.0 : 20.0));
-      take(7, c7 > 1000 && n_seg == 4 ? 15.0 + 0.207 * c7 : 1.03 * (c7 <= 148 ? 57.0 : c7 <= 256 ? 69.0 : 32.0 + 0.222 * c7));
+      const double fit = 1.03, c6 = (double)n_seg * (double)tiles(32, 64) / sms, c7 = (double)n_seg * (double)tiles(64, 128) / sms;
+      take(6, fit * fmax(14.0 + 8.8 * c6, c6 > 2.0 ? 40.0 : 20.0));
+      take(7, c7 > 6.76 && n_seg == 4 ? 15.0 + 30.6 * c7 : fit * (c7 <= 1.0 ? 57.0 : c7 <= 1.73 ? 69.0 : 32.0 + 32.9 * c7));
     }
   }
   // 16-byte copies where every row starts on a 16-byte boundary and K ends on one, else 4-byte copies

@@ -88,7 +88,8 @@ def test_router_of_few_and_many_tokens(T, E, n_extra):
             assert a is None or torch.equal(a, b[at : at + len(part)])
 
 
-@pytest.mark.parametrize("M, N, K, pad", [(17, 64, 513, 3), (65, 130, 1028, 0), (33, 65, 2048, 0), (200, 129, 4096, 4)])
+@pytest.mark.parametrize("M, N, K, pad", [(17, 64, 513, 3), (65, 130, 1028, 0), (33, 65, 2048, 0), (70, 66, 2049, 1),
+                                          (34, 130, 3072, 0), (129, 65, 3500, 0), (200, 129, 4096, 4)])
 def test_float32_tiles_that_share_k(M, N, K, pad):
     """The same bits as the launches that do not share (2 to 8 segments of K); more or fewer segments are refused."""
     from ctypes import c_int, c_longlong, c_void_p
