@@ -74,8 +74,17 @@ __device__ __forceinline__ float4 pn_sum4(const T* p, int n_split, size_t stride
 }
 template <int J = 1>
 __device__ __forceinline__ float4 pn_group4(const PnGroup& g, size_t at) {
-  const float4 y = g.is_bf16 ? pn_sum4<1>((const bf16*)g.p + at, g.n_split, g.stride)      // (partials are float32)
-                             : pn_sum4<J>((const float*)g.p + at, g.n_split, g.stride);
+  float4 y;
+  if (J > 1 && !g.is_bf16) {
+    y = pn_sum4<J>((const float*)g.p + at, g.n_split, g.stride);
+  } else {
+    y = g.is_bf16 ? pn_load4((const bf16*)g.p + at) : pn_load4((const float*)g.p + at);
+    for (int s = 1; s < g.n_split; ++s) {
+      const size_t o = at + (size_t)s * g.stride;
+      const float4 q = g.is_bf16 ? pn_load4((const bf16*)g.p + o) : pn_load4((const float*)g.p + o);
+      y.x += q.x, y.y += q.y, y.z += q.z, y.w += q.w;
+    }
+  }
   return make_float4(y.x * g.weight, y.y * g.weight, y.z * g.weight, y.w * g.weight);
 }
 __device__ __forceinline__ float pn_group1(const PnGroup& g, size_t at) {
