@@ -55,7 +55,10 @@ __device__ __forceinline__ void dn_add_group(float4 (&v)[NC], const TD* p, int n
 
 // DEEP: a step of few rows and many partials (a decode step): their loads are batched and the gains fetched ahead of the
 // wait; otherwise few registers, so that several rows share an SM.
-template <typename TO, int NC, bool DEEP>
+// TWO (DEEP, one vector a thread): both groups are up to eight float32 partials, asked for in one trip.  Eight rows of 2048, five
+// partials each: 2.6 us one group after the other, 2.5 like this.  An instance of its own: with the choice inside one, the other
+// calls took longer (three partials 1.9 -> 2.2 us, nine and nine 3.3 -> 4.0).
+template <typename TO, int NC, bool DEEP, bool TWO>
 __global__ void __launch_bounds__(512)
 dual_norm_kernel(float* __restrict__ h, const DnGroup ga, const DnGroup gb, const float* __restrict__ bias,
                  const int* __restrict__ rows, const float* __restrict__ gain0, const float* __restrict__ gain1, float eps,
@@ -84,8 +87,7 @@ dual_norm_kernel(float* __restrict__ h, const DnGroup ga, const DnGroup gb, cons
     if (g.is_bf16) dn_add_group<NC, J>(v, (const bf16*)g.p + at, g.n_split, g.stride, col, d);
     else dn_add_group<NC, J>(v, (const float*)g.p + at, g.n_split, g.stride, col, d);
   };
-  if (DEEP && NC == 1 && ga.p && gb.p && !ga.is_bf16 && !gb.is_bf16 && ga.n_split <= J && gb.n_split <= J) {
-    // a decode step's two groups in one trip
+  if (TWO) {
     const float *a = (const float*)ga.p + at + col[0], *b = (const float*)gb.p + at + col[0];
     float4 y[J], z[J];
 #pragma unroll
@@ -194,10 +196,14 @@ LLMX_API int llmx_dual_norm(float* h, const void* a, int dtype_a, int n_a, long 
     const int nc = vecs <= 512 ? 1 : vecs <= 1024 ? 2 : 4;
     int threads = ((vecs + nc - 1) / nc + 31) / 32 * 32;
     if (threads < 64) threads = 64;
-#define GO(TO, NC)                                                                                                \
-  do {                                                                                                            \
-    if (n_rows <= 64) launch_pdl(dual_norm_kernel<TO, NC, true>, dim3(n_rows), dim3(threads), 0, stream, ARGS(TO)); \
-    else launch_pdl(dual_norm_kernel<TO, NC, false>, dim3(n_rows), dim3(threads), 0, stream, ARGS(TO));           \
+    const bool two = nc == 1 && a && b && !ga.is_bf16 && !gb.is_bf16 && n_a <= 8 && n_b <= 8;
+#define RUN(TO, NC, DEEP, TWO) \
+  launch_pdl(dual_norm_kernel<TO, NC, DEEP, TWO>, dim3(n_rows), dim3(threads), 0, stream, ARGS(TO))
+#define GO(TO, NC)                                       \
+  do {                                                   \
+    if (n_rows > 64) RUN(TO, NC, false, false);          \
+    else if (two) RUN(TO, NC, true, NC == 1);            \
+    else RUN(TO, NC, true, false);                       \
   } while (0)
     if (out_bf16) {
       if (nc == 1) GO(bf16, 1); else if (nc == 2) GO(bf16, 2); else GO(bf16, 4);
@@ -205,6 +211,7 @@ LLMX_API int llmx_dual_norm(float* h, const void* a, int dtype_a, int n_a, long 
       if (nc == 1) GO(float, 1); else if (nc == 2) GO(float, 2); else GO(float, 4);
     }
 #undef GO
+#undef RUN
     return LLMX_LAUNCH_STATUS();
   }
   const size_t smem = (size_t)d * sizeof(float);
