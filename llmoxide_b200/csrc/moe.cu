@@ -154,23 +154,6 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, int* __restri
   if (lane < top) ids[(size_t)t * top + lane] = id, wts[(size_t)t * top + lane] = weight;
 }
 
-// The router's product and the routing in one kernel: a CTA takes TOK tokens; warp w of n computes the float32 logits of
-// experts w, w + n, ... two at a time (a lane adds its share of k in ascending order, eight consecutive k at a time, then
-// the lanes are added by a butterfly: the order depends on nothing but K), then warp j routes token j.  The matrix may
-// hold n_extra rows behind the experts' (a gate that reads the same input): their logits are written to extra_out
-// [T, n_extra] as they are.
-// Prompts: four tokens a CTA.  (Eight, and sixteen with their rows by asynchronous copies through shared memory, read
-// the matrix less often and took longer: 4100 tokens, 16 experts 23.5 us by four, 29 and 24.5 by eight and sixteen; 64 experts
-// 73, 87 and 77.)
-// Four such CTAs an SM (three of float32 rows), where unbounded registers let two in and three leave another round: 64 experts,
-// 2000 tokens 44 us (56 by three), 4100 tokens 72 (74 and 87); inside a prompt of 4100 tokens, 16 experts, 32 -> 27.
-// Steps of few tokens wait for nothing but loads: the matrix is brought to L2 while the kernel before still runs, and sixteen
-// warps share the experts.
-// PLACE (steps of up to 8 tokens): the CTAs are one cluster, which knows every choice behind one barrier, so each CTA also
-// finds its own pairs' places in the order by experts (what moe_sort_kernel makes in a launch of its own, with the places
-// inside an expert in the order of the pairs), copies its token's row there, and the first one writes the list of tiles.
-// Four tokens, top 4, K = 2048, the three launches and this one: 16 experts 9.9 and 7.8 us, 64 experts 20.1 and 12.7.  (With
-// several tokens a CTA it took longer than the three from 12 tokens on: 9.7 and 9.2 us, 64 experts 17.1 and 9.3.)
 // Eight values as they lie in memory, asked for in the order of the source.
 template <typename T>
 struct Moe8;
@@ -289,6 +272,23 @@ __device__ __forceinline__ void moe_place(const MoePlaces pl, const int* own_ids
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// The router's product and the routing in one kernel: a CTA takes TOK tokens; warp w of n computes the float32 logits of
+// experts w, w + n, ... two at a time (a lane adds its share of k in ascending order, eight consecutive k at a time, then
+// the lanes are added by a butterfly: the order depends on nothing but K), then warp j routes token j.  The matrix may
+// hold n_extra rows behind the experts' (a gate that reads the same input): their logits are written to extra_out
+// [T, n_extra] as they are.
+// Prompts: four tokens a CTA.  (Eight, and sixteen with their rows by asynchronous copies through shared memory, read
+// the matrix less often and took longer: 4100 tokens, 16 experts 23.5 us by four, 29 and 24.5 by eight and sixteen; 64 experts
+// 73, 87 and 77.)
+// Four such CTAs an SM (three of float32 rows), where unbounded registers let two in and three leave another round: 64 experts,
+// 2000 tokens 44 us (56 by three), 4100 tokens 72 (74 and 87); inside a prompt of 4100 tokens, 16 experts, 32 -> 27.
+// Steps of few tokens wait for nothing but loads: the matrix is brought to L2 while the kernel before still runs, and sixteen
+// warps share the experts.
+// PLACE (steps of up to 8 tokens): the CTAs are one cluster, which knows every choice behind one barrier, so each CTA also
+// finds its own pairs' places in the order by experts (what moe_sort_kernel makes in a launch of its own, with the places
+// inside an expert in the order of the pairs), copies its token's row there, and the first one writes the list of tiles.
+// Four tokens, top 4, K = 2048, the three launches and this one: 16 experts 9.9 and 7.8 us, 64 experts 20.1 and 12.7.  (With
+// several tokens a CTA it took longer than the three from 12 tokens on: 9.7 and 9.2 us, 64 experts 17.1 and 9.3.)
 template <typename TX, int TOK, int THREADS, bool PLACE>
 __global__ void __launch_bounds__(THREADS, TOK == 1 ? 1 : sizeof(TX) == 2 ? 4 : 3)
 moe_router_kernel(const TX* __restrict__ x, long long ldx, const float* __restrict__ w, int* __restrict__ ids,
