@@ -280,8 +280,8 @@ __device__ __forceinline__ void moe_place(const MoePlaces pl, const int* own_ids
 // Prompts: four tokens a CTA.  (Eight, and sixteen with their rows by asynchronous copies through shared memory, read
 // the matrix less often and took longer: 4100 tokens, 16 experts 23.5 us by four, 29 and 24.5 by eight and sixteen; 64 experts
 // 73, 87 and 77.)
-// Four such CTAs an SM (three of float32 rows), where unbounded registers let two in and three leave another round: 64 experts,
-// 2000 tokens 44 us (56 by three), 4100 tokens 72 (74 and 87); inside a prompt of 4100 tokens, 16 experts, 32 -> 27.
+// Four such CTAs an SM, where unbounded registers let two in and three leave another round: 64 experts, 2000 tokens 44 us (56 by
+// three), 4100 tokens 72 (74 and 87); inside a prompt of 4100 tokens, 16 experts, 32 -> 27; float32 rows, 2000 tokens 65 (79 by three).
 // Steps of few tokens wait for nothing but loads: the matrix is brought to L2 while the kernel before still runs, and sixteen
 // warps share the experts.
 // PLACE (steps of up to 8 tokens): the CTAs are one cluster, which knows every choice behind one barrier, so each CTA also
@@ -290,7 +290,7 @@ __device__ __forceinline__ void moe_place(const MoePlaces pl, const int* own_ids
 // Four tokens, top 4, K = 2048, the three launches and this one: 16 experts 9.9 and 7.8 us, 64 experts 20.1 and 12.7.  (With
 // several tokens a CTA it took longer than the three from 12 tokens on: 9.7 and 9.2 us, 64 experts 17.1 and 9.3.)
 template <typename TX, int TOK, int THREADS, bool PLACE>
-__global__ void __launch_bounds__(THREADS, TOK == 1 ? 1 : sizeof(TX) == 2 ? 4 : 3)
+__global__ void __launch_bounds__(THREADS, TOK == 1 ? 1 : 4)
 moe_router_kernel(const TX* __restrict__ x, long long ldx, const float* __restrict__ w, int* __restrict__ ids,
                   float* __restrict__ wts, int n_tokens, int K, int E, int top, int n_groups, int keep_groups,
                   int group_top, int score_kind, int normalize, float norm_eps, float scale, int vec,
