@@ -1183,8 +1183,8 @@ gated_norm_row_kernel(const float* __restrict__ o, const TIN* __restrict__ proj,
 // The same by four neighbouring elements a thread, U times (sizes, offsets and strides multiples of 4, no gates), everything
 // asked for ahead of the reduction.  The squares are added in the chains of the kernels above, a row's by way of shared memory,
 // so that the bits are theirs.  By elements and like this: four rows of 2048 with five partials (a decode step) 6.8 and 2.2 us,
-// of 8192 23.6 and 5.0; 4100 rows of 2048 24 both (bound by memory), of 8192 140 and 93.  U 0: a warp per (token, head) of up
-// to 128 columns: 4 and 4100 tokens of 16 heads 3.7 and 1.7, 28.8 and 23.8.
+// of 8192 23.6 and 5.0; 4100 rows of 8192 140 and 93.  U 0: a warp per (token, head) of up to 128 columns: 4 and 4100 tokens
+// of 16 heads 3.7 and 1.7, 28.8 and 23.8.
 template <typename TIN, typename TO, int U>
 __global__ void __launch_bounds__(U ? 512 : 128)
 gated_norm_vec_kernel(const float* __restrict__ o, const TIN* __restrict__ proj, int n_split, size_t split_stride,
@@ -1263,7 +1263,14 @@ LLMX_API int llmx_gated_norm(const float* o, const void* proj, int in_dtype, int
   if (gate_act != LA_ACT_SILU && gate_act != LA_ACT_SIGMOID && gate_act != LA_ACT_NONE) return LLMX_REFUSED(1);
   // four elements a thread where every row, gate and gain is whole vectors, and a row fits a CTA (a head a warp)
   const int n = per_head ? Dv : H * Dv, in_size = in_dtype == LLMX_F32 ? 4 : 2, out_size = out_dtype == LLMX_F32 ? 4 : 2;
-  const bool vec = !gates && n % 4 == 0 && g_off % 4 == 0 && row_stride % 4 == 0 && split_stride % 4 == 0 &&
+  // Where that is faster.  Heads: a warp needs more than half its lanes, or all warps run at once (seven CTAs of four an SM):
+  // 4800 and 3200 heads of 64, by vectors and by elements 3.5 and 3.3, 2.7 and 2.8 us; of 32 the line is two heads an SM.  Rows: a
+  // CTA is 512 threads whatever n is, and one or two share an SM: 64 rows of 512 2.2 and 2.5 us, of 256 2.1 and 2.0 (with partials
+  // 2.3 and 2.4); 300 rows of 2048 4.9 and 5.2, 1200 12.8 and 9.5, 1200 of 8192 29.7 and 44.
+  const long long rows = per_head ? (long long)n_tokens * H : n_tokens, sms = llmx_sm_count();
+  const bool fits = per_head ? n > 64 || rows <= (n == 64 ? 28 : 2) * sms
+                             : rows <= sms ? n >= 512 || n_split > 1 : n > 6144 || (n >= 2048 && rows <= 2 * sms);
+  const bool vec = fits && !gates && n % 4 == 0 && g_off % 4 == 0 && row_stride % 4 == 0 && split_stride % 4 == 0 &&
                    n <= (per_head ? 128 : 8192) && (long long)n_tokens * H < (1ll << 31) && !((uintptr_t)o & 15) &&
                    !((uintptr_t)gain & 15) && !((uintptr_t)proj & (4 * in_size - 1)) && !((uintptr_t)y & (4 * out_size - 1));
 #define VEC(TIN, TO, U)                                                                                              \
