@@ -453,7 +453,7 @@ LLMX_API int llmx_add_gain_sumsq(float* h, const void* delta, int delta_dtype, i
 // table entry, gains and rotation rows are fetched once for all of them, and their loads go out together.
 #define QKV_SPW 4
 
-template <typename TIN, typename TA, typename TC, bool DEEP, int LPH>
+template <typename TIN, typename TA, typename TC, bool DEEP>
 __global__ void qk_norm_rope_cache_kernel(const TIN* __restrict__ qkv, int n_split, size_t split_stride,
                                           TA* __restrict__ q_out,
                                           TC* __restrict__ k_cache, TC* __restrict__ v_cache,
@@ -462,89 +462,77 @@ __global__ void qk_norm_rope_cache_kernel(const TIN* __restrict__ qkv, int n_spl
                                           const float* __restrict__ q_gain, const float* __restrict__ k_gain,
                                           float eps, const float* __restrict__ cos_t,
                                           const float* __restrict__ sin_t, int n_rot, int H, int G, int D,
-                                          int Dv, int write_cache, const float* __restrict__ bias) {
-  constexpr int SPW = DEEP ? 1 : QKV_SPW, HPW = LPH > 0 ? 32 / LPH : 1;      // heads one after another, and side by side
+                                          int Dv, int write_cache, const float* __restrict__ bias, int by_vectors) {
+  constexpr int SPW = DEEP ? 1 : QKV_SPW;
   extern __shared__ float head_buf[];
   pdl_launch_dependents();
   // Positions, block table, gains and rotation tables are step inputs or weights, not results of the kernel
   // before: they are fetched ahead of the dependency wait, which only the qkv values need.
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = blockIdx.x;                        // tokens on x: a step may bring more than 65535
-  const int slot0 = (blockIdx.y * QKV_WARPS + warp) * SPW * HPW;   // the warp's first head of the fused row
+  const int slot0 = (blockIdx.y * QKV_WARPS + warp) * SPW;   // the warp's first head of the fused row
   const int n_slots = write_cache ? H + 2 * G : H;
   if (slot0 >= n_slots) return;
   float* buf = head_buf + warp * D;
   const TIN* tok = qkv + (size_t)t * ((size_t)(H + G) * D + (size_t)G * Dv);   // q heads, k heads (D each), v heads (Dv each)
   const int pos = token_pos[t];
   int page = 0;
-  if (slot0 + SPW * HPW > H) page = block_table[(size_t)token_seq[t] * table_width + pos / LLMX_PAGE];
+  if (slot0 + SPW > H) page = block_table[(size_t)token_seq[t] * table_width + pos / LLMX_PAGE];
   auto cache_row_of = [&](int slot) -> TC* {        // slot >= H: a k head, then the v heads
     const bool is_k = slot < H + G;
     return is_k ? k_cache + cache_row_offset(page, slot - H, pos % LLMX_PAGE, G, D)
                 : v_cache + cache_row_offset(page, slot - H - G, pos % LLMX_PAGE, G, Dv);
   };
 
-  if constexpr (LPH > 0) {
-    // Head size 4 LPH with full rotation or none: a lane owns four neighbouring dims, read and written as one vector, and
-    // 32 / LPH heads share a warp; the rotation partner (half a head away) lives in lane +-LPH/2 and comes by shuffle.  Bound
-    // by two trips to L2.  16 + 2 * 8 heads of 64, an element a lane and like this: one token of five partials 3.0 and 1.8 us,
-    // 23 tokens 6.0 and 2.9, 4000 tokens 33.8 and 13.9; unrotated heads of 128 with gains, 64 tokens: 6.1 and 2.9.
-    constexpr int HD = 4 * LPH;
-    const int l = lane % LPH, d0 = 4 * l, dh = d0 & (HD / 2 - 1), sub = lane / LPH;
+  if (by_vectors && D == 128 && n_rot == 128 && Dv == 128) {
+    // Head size 128 with full rotation: a lane owns dims 4*lane..4*lane+3, read and written as one
+    // vector; the rotation partner (dim +-64) lives in lane +-16 and comes by shuffle.
+    const int d0 = 4 * lane;
     const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
     const float4 gq = q_gain ? load4(q_gain + d0) : one, gk = k_gain ? load4(k_gain + d0) : one;
-    float4 cs = one, sn = one;
-    if (n_rot) cs = load4(cos_t + (size_t)pos * (HD / 2) + dh), sn = load4(sin_t + (size_t)pos * (HD / 2) + dh);
+    const float4 cs = load4(cos_t + (size_t)pos * 64 + (d0 & 63)), sn = load4(sin_t + (size_t)pos * 64 + (d0 & 63));
     pdl_wait();
     float4 xs[SPW];
 #pragma unroll
     for (int j = 0; j < SPW; ++j) {
-      const int slot = slot0 + j * HPW + sub;
-      xs[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (slot < n_slots) {
-        const TIN* src = tok + (size_t)slot * HD;
+      if (slot0 + j < n_slots) {
+        const TIN* src = tok + (size_t)(slot0 + j) * D;
         xs[j] = load4(src + d0);
         add_partials4<DEEP ? 8 : 1>(xs[j], src + split_stride + d0, n_split - 1, split_stride);
         if (bias) {
-          const float4 bv = load4(bias + (size_t)slot * HD + d0);
+          const float4 bv = load4(bias + (size_t)(slot0 + j) * D + d0);
           xs[j].x += bv.x, xs[j].y += bv.y, xs[j].z += bv.z, xs[j].w += bv.w;
         }
       }
     }
 #pragma unroll
     for (int j = 0; j < SPW; ++j) {
-      if (slot0 + j * HPW >= n_slots) break;
-      const int slot = slot0 + j * HPW + sub;
+      const int slot = slot0 + j;
+      if (slot >= n_slots) break;
       float4 x = xs[j];
       const bool is_q = slot < H, is_k = !is_q && slot < H + G;
-      float ssq = 0.f;
-      if (LPH == 32 && n_rot) {
-        ssq = warp_sum(x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w);
-      } else if (q_gain || k_gain) {
-        const float v[4] = {x.x, x.y, x.z, x.w};
-        ssq = head_sumsq<4, LPH>(v, 0xffffffffu);
+      if (!is_q && !is_k) {  // v: stored as it is
+        store4(cache_row_of(slot) + d0, x);
+        continue;
       }
-      if ((is_q && q_gain) || (is_k && k_gain)) {
+      if (is_q ? q_gain != nullptr : k_gain != nullptr) {
         const float4 gn = is_q ? gq : gk;
-        const float scale = 1.0f / sqrtf(ssq / (float)HD + eps);
+        const float ssq = warp_sum(x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w);
+        const float scale = 1.0f / sqrtf(ssq / 128.0f + eps);
         x.x = (x.x * scale) * gn.x; x.y = (x.y * scale) * gn.y; x.z = (x.z * scale) * gn.z; x.w = (x.w * scale) * gn.w;
       }
-      float4 r = x, p;
-      p.x = __shfl_xor_sync(0xffffffffu, x.x, LPH / 2);
-      p.y = __shfl_xor_sync(0xffffffffu, x.y, LPH / 2);
-      p.z = __shfl_xor_sync(0xffffffffu, x.z, LPH / 2);
-      p.w = __shfl_xor_sync(0xffffffffu, x.w, LPH / 2);
-      if (n_rot && (is_q || is_k)) {
-        // dims i of the first half: x_i cos - x_(i+half) sin; dims i + half: x_i sin + x_(i+half) cos.  Which product is rounded
-        // by itself is what the kernels of these head sizes have always done.
-        auto turn = [&](float x, float p, float c, float s) {
-          if (l < LPH / 2) return fmaf(x, c, -__fmul_rn(p, s));
-          return LPH == 32 ? fmaf(x, c, __fmul_rn(p, s)) : fmaf(p, s, __fmul_rn(x, c));
-        };
-        r = make_float4(turn(x.x, p.x, cs.x, sn.x), turn(x.y, p.y, cs.y, sn.y), turn(x.z, p.z, cs.z, sn.z), turn(x.w, p.w, cs.w, sn.w));
+      float4 p;
+      p.x = __shfl_xor_sync(0xffffffffu, x.x, 16);
+      p.y = __shfl_xor_sync(0xffffffffu, x.y, 16);
+      p.z = __shfl_xor_sync(0xffffffffu, x.z, 16);
+      p.w = __shfl_xor_sync(0xffffffffu, x.w, 16);
+      float4 r;
+      if (lane < 16) {   // dims i < 64: x_i cos - x_{i+64} sin
+        r = make_float4(x.x * cs.x - p.x * sn.x, x.y * cs.y - p.y * sn.y, x.z * cs.z - p.z * sn.z, x.w * cs.w - p.w * sn.w);
+      } else {           // dims i + 64: x_i sin + x_{i+64} cos
+        r = make_float4(p.x * sn.x + x.x * cs.x, p.y * sn.y + x.y * cs.y, p.z * sn.z + x.z * cs.z, p.w * sn.w + x.w * cs.w);
       }
-      if (slot >= n_slots) continue;
-      if (is_q) store4(q_out + (size_t)t * H * HD + (size_t)slot * HD + d0, r);
+      if (is_q) store4(q_out + (size_t)t * H * D + (size_t)slot * D + d0, r);
       else store4(cache_row_of(slot) + d0, r);
     }
     return;
@@ -598,12 +586,108 @@ __global__ void qk_norm_rope_cache_kernel(const TIN* __restrict__ qkv, int n_spl
   }
 }
 
+// The same for heads of 64 with full rotation or none and unrotated heads of 128, by vectors: a lane owns four neighbouring dims,
+// and 32 / LPH heads of 4 LPH share a warp; the rotation partner (half a head away) lives in lane +-LPH/2 and comes by shuffle.
+// Squares and rotations have the bits of the kernel above, which took these heads an element a lane.  Bound by two trips to L2.
+// 16 + 2 * 8 heads of 64, an element a lane and like this: one token of five partials 3.0 and 1.8 us, 23 tokens 6.0 and 2.9,
+// 4000 tokens 33.8 and 13.9; unrotated heads of 128 with gains, 64 tokens: 6.1 and 2.9.  (A kernel of its own: as one with that
+// above, rotated heads of 128 took 1.5 to 1.7 us in a decode step in place of 1.3.)
+template <typename TIN, typename TA, typename TC, bool DEEP, int LPH, bool ROT>
+__global__ void qk_norm_rope_cache_vec_kernel(const TIN* __restrict__ qkv, int n_split, size_t split_stride,
+                                          TA* __restrict__ q_out,
+                                          TC* __restrict__ k_cache, TC* __restrict__ v_cache,
+                                          const int* __restrict__ block_table, int table_width,
+                                          const int* __restrict__ token_seq, const int* __restrict__ token_pos,
+                                          const float* __restrict__ q_gain, const float* __restrict__ k_gain,
+                                          float eps, const float* __restrict__ cos_t,
+                                          const float* __restrict__ sin_t, int H, int G, int write_cache, const float* __restrict__ bias) {
+  constexpr int SPW = DEEP ? 1 : QKV_SPW, HPW = 32 / LPH, D = 4 * LPH;      // heads one after another, and side by side
+  pdl_launch_dependents();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int t = blockIdx.x;                        // tokens on x: a step may bring more than 65535
+  const int slot0 = (blockIdx.y * QKV_WARPS + warp) * SPW * HPW;   // the warp's first head of the fused row
+  const int n_slots = write_cache ? H + 2 * G : H;
+  if (slot0 >= n_slots) return;
+  const TIN* tok = qkv + (size_t)t * (H + 2 * G) * D;
+  const int pos = token_pos[t];
+  int page = 0;
+  if (slot0 + SPW * HPW > H) page = block_table[(size_t)token_seq[t] * table_width + pos / LLMX_PAGE];
+  auto cache_row_of = [&](int slot) -> TC* {        // slot >= H: a k head, then the v heads
+    const bool is_k = slot < H + G;
+    return is_k ? k_cache + cache_row_offset(page, slot - H, pos % LLMX_PAGE, G, D)
+                : v_cache + cache_row_offset(page, slot - H - G, pos % LLMX_PAGE, G, D);
+  };
+
+  const int l = lane % LPH, d0 = 4 * l, dh = d0 & (D / 2 - 1), sub = lane / LPH;
+  const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
+  const float4 gq = q_gain ? load4(q_gain + d0) : one, gk = k_gain ? load4(k_gain + d0) : one;
+  float4 cs = one, sn = one;
+  if (ROT) cs = load4(cos_t + (size_t)pos * (D / 2) + dh), sn = load4(sin_t + (size_t)pos * (D / 2) + dh);
+  pdl_wait();
+  float4 xs[SPW];
+#pragma unroll
+  for (int j = 0; j < SPW; ++j) {
+    const int slot = slot0 + j * HPW + sub;
+    if (HPW > 1) xs[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (slot < n_slots) {
+      const TIN* src = tok + (size_t)slot * D;
+      xs[j] = load4(src + d0);
+      add_partials4<DEEP ? 8 : 1>(xs[j], src + split_stride + d0, n_split - 1, split_stride);
+      if (bias) {
+        const float4 bv = load4(bias + (size_t)slot * D + d0);
+        xs[j].x += bv.x, xs[j].y += bv.y, xs[j].z += bv.z, xs[j].w += bv.w;
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < SPW; ++j) {
+    if (slot0 + j * HPW >= n_slots) break;
+    const int slot = slot0 + j * HPW + sub;
+    float4 x = xs[j];
+    const bool is_q = slot < H, is_k = !is_q && slot < H + G;
+    if (HPW == 1 && !is_q && !is_k) {                // v: stored as it is
+      store4(cache_row_of(slot) + d0, x);
+      continue;
+    }
+    if (q_gain || k_gain) {
+      const float v[4] = {x.x, x.y, x.z, x.w}, ssq = head_sumsq<4, LPH>(v, 0xffffffffu);
+      if ((is_q && q_gain) || (is_k && k_gain)) {
+        const float4 gn = is_q ? gq : gk;
+        const float scale = 1.0f / sqrtf(ssq / (float)D + eps);
+        x.x = (x.x * scale) * gn.x; x.y = (x.y * scale) * gn.y; x.z = (x.z * scale) * gn.z; x.w = (x.w * scale) * gn.w;
+      }
+    }
+    float4 r = x;
+    if (ROT) {
+      float4 p;
+      p.x = __shfl_xor_sync(0xffffffffu, x.x, LPH / 2);
+      p.y = __shfl_xor_sync(0xffffffffu, x.y, LPH / 2);
+      p.z = __shfl_xor_sync(0xffffffffu, x.z, LPH / 2);
+      p.w = __shfl_xor_sync(0xffffffffu, x.w, LPH / 2);
+      // dims i of the first half: x_i cos - x_(i+half) sin; dims i + half: x_i sin + x_(i+half) cos.  Which product is rounded
+      // by itself is what the kernel above does.
+      auto down = [](float x, float p, float c, float s) { return fmaf(x, c, -__fmul_rn(p, s)); };
+      auto up = [](float x, float p, float c, float s) { return fmaf(p, s, __fmul_rn(x, c)); };
+      if (!is_q && !is_k) {
+      } else if (l < LPH / 2) {
+        r = make_float4(down(x.x, p.x, cs.x, sn.x), down(x.y, p.y, cs.y, sn.y), down(x.z, p.z, cs.z, sn.z), down(x.w, p.w, cs.w, sn.w));
+      } else {
+        r = make_float4(up(x.x, p.x, cs.x, sn.x), up(x.y, p.y, cs.y, sn.y), up(x.z, p.z, cs.z, sn.z), up(x.w, p.w, cs.w, sn.w));
+      }
+    }
+    if (slot >= n_slots) continue;
+    if (is_q) store4(q_out + (size_t)t * H * D + (size_t)slot * D + d0, r);
+    else store4(cache_row_of(slot) + d0, r);
+  }
+}
+
 // The same for prompts when everything is bfloat16, the head size is 128 and the rotation is full or none: half a
 // warp per head, a lane owns eight consecutive dims (one 16-byte load, one 16-byte store); the rotation
 // partner (dim +-64) lives eight lanes away.  A warp takes eight heads of its token, two at a time.  4100 tokens of 16 + 2 * 4
 // heads: rotated 13.8 us, unrotated with gains 20.6 (their squares' chains cross lanes; an element a lane 32.2).
 #define QKV8_PER_WARP 8
 
+template <bool ROT>
 __global__ void qk_norm_rope_cache_bf16_d128_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ q_out,
                                                     bf16* __restrict__ k_cache, bf16* __restrict__ v_cache,
                                                     const int* __restrict__ block_table, int table_width,
@@ -612,7 +696,7 @@ __global__ void qk_norm_rope_cache_bf16_d128_kernel(const bf16* __restrict__ qkv
                                                     const float* __restrict__ q_gain,
                                                     const float* __restrict__ k_gain, float eps,
                                                     const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                                                    int n_rot, int H, int G, int write_cache) {
+                                                    int H, int G, int write_cache) {
   constexpr int D = 128;
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -632,7 +716,7 @@ __global__ void qk_norm_rope_cache_bf16_d128_kernel(const bf16* __restrict__ qkv
     const float4 a0 = q_gain ? load4(q_gain + d0) : one, a1 = q_gain ? load4(q_gain + d0 + 4) : one;
     const float4 b0 = k_gain ? load4(k_gain + d0) : one, b1 = k_gain ? load4(k_gain + d0 + 4) : one;
     float4 c0 = one, c1 = one, s0 = one, s1 = one;
-    if (n_rot) {
+    if (ROT) {
       const float *ct = cos_t + (size_t)pos * 64 + (d0 & 63), *st = sin_t + (size_t)pos * 64 + (d0 & 63);
       c0 = load4(ct), c1 = load4(ct + 4), s0 = load4(st), s1 = load4(st + 4);
     }
@@ -678,7 +762,7 @@ __global__ void qk_norm_rope_cache_bf16_d128_kernel(const bf16* __restrict__ qkv
     const float* gain = is_q ? gq : gk;
     if (is_q ? q_gain != nullptr : k_gain != nullptr) {
       float ss = 0.f;
-      if (n_rot) {
+      if (ROT) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) ss += x[i] * x[i];
 #pragma unroll
@@ -693,15 +777,16 @@ __global__ void qk_norm_rope_cache_bf16_d128_kernel(const bf16* __restrict__ qkv
     uint32_t packed[4];
 #pragma unroll
     for (int i = 0; i < 8; i += 2) {
-      const float p0 = __shfl_xor_sync(mask, x[i], 8), p1 = __shfl_xor_sync(mask, x[i + 1], 8);
       float r0 = x[i], r1 = x[i + 1];
-      if (!n_rot) {
-      } else if (l16 < 8) {   // dims i < 64: x_i cos - x_{i+64} sin
-        r0 = x[i] * cs[i] - p0 * sn[i];
-        r1 = x[i + 1] * cs[i + 1] - p1 * sn[i + 1];
-      } else {         // dims i + 64: x_i sin + x_{i+64} cos
-        r0 = p0 * sn[i] + x[i] * cs[i];
-        r1 = p1 * sn[i + 1] + x[i + 1] * cs[i + 1];
+      if (ROT) {
+        const float p0 = __shfl_xor_sync(mask, x[i], 8), p1 = __shfl_xor_sync(mask, x[i + 1], 8);
+        if (l16 < 8) {   // dims i < 64: x_i cos - x_{i+64} sin
+          r0 = x[i] * cs[i] - p0 * sn[i];
+          r1 = x[i + 1] * cs[i + 1] - p1 * sn[i + 1];
+        } else {         // dims i + 64: x_i sin + x_{i+64} cos
+          r0 = p0 * sn[i] + x[i] * cs[i];
+          r1 = p1 * sn[i + 1] + x[i + 1] * cs[i + 1];
+        }
       }
       __nv_bfloat162 h = __floats2bfloat162_rn(r0, r1);
       packed[i >> 1] = *reinterpret_cast<uint32_t*>(&h);
@@ -724,9 +809,9 @@ LLMX_API int llmx_qk_norm_rope_cache_biased(const void* qkv, int in_dtype, int n
   if (!bias && n_split == 1 && in_dtype == LLMX_BF16 && act_dtype == LLMX_BF16 && cache_dtype == LLMX_BF16 && D == 128 &&
       Dv == 128 && (n_rot == 128 || n_rot == 0) && n_tokens > 64 && !(((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15)) {
     const int per_cta = QKV_WARPS * QKV8_PER_WARP;
-    launch_pdl(qk_norm_rope_cache_bf16_d128_kernel, dim3(n_tokens, (n_slots + per_cta - 1) / per_cta),
+    launch_pdl(n_rot ? qk_norm_rope_cache_bf16_d128_kernel<true> : qk_norm_rope_cache_bf16_d128_kernel<false>, dim3(n_tokens, (n_slots + per_cta - 1) / per_cta),
                dim3(QKV_WARPS * 32), 0, stream, (const bf16*)qkv, (bf16*)q_out, (bf16*)k_cache, (bf16*)v_cache,
-               block_table, table_width, token_seq, token_pos, q_gain, k_gain, eps, cos_t, sin_t, n_rot, H, G, write_cache);
+               block_table, table_width, token_seq, token_pos, q_gain, k_gain, eps, cos_t, sin_t, H, G, write_cache);
     return LLMX_LAUNCH_STATUS();
   }
   // Lanes a head: four dims each for heads of 64 and 128 with full rotation or none (vectors in every dtype), else any size.
@@ -741,21 +826,23 @@ LLMX_API int llmx_qk_norm_rope_cache_biased(const void* qkv, int in_dtype, int n
   const size_t smem = lph ? 0 : (size_t)QKV_WARPS * D * sizeof(float);
   if (smem > 48 * 1024) return LLMX_REFUSED(3);
   // many partials (a decode step): their loads batched; one tensor (a prompt): few registers, many warps per SM
-#define RUN(TIN, TA, TC, DEEP, LPH)                                                                                \
-  launch_pdl(qk_norm_rope_cache_kernel<TIN, TA, TC, DEEP, LPH>, grid, dim3(QKV_WARPS * 32), smem, stream,          \
-        (const TIN*)qkv, n_split, (size_t)split_stride, (TA*)q_out, (TC*)k_cache, (TC*)v_cache, block_table,        \
-        table_width, token_seq, token_pos, q_gain, k_gain, eps, cos_t, sin_t, n_rot, H, G, D, Dv, write_cache, bias)
+#define ARGS(TIN, TA, TC)                                                                                          \
+  grid, dim3(QKV_WARPS * 32), smem, stream, (const TIN*)qkv, n_split, (size_t)split_stride, (TA*)q_out, (TC*)k_cache, \
+      (TC*)v_cache, block_table, table_width, token_seq, token_pos, q_gain, k_gain, eps, cos_t, sin_t
+#define VEC(TIN, TA, TC, DEEP, LPH, ROT) \
+  launch_pdl(qk_norm_rope_cache_vec_kernel<TIN, TA, TC, DEEP, LPH, ROT>, ARGS(TIN, TA, TC), H, G, write_cache, bias)
+#define BY_HEAD(TIN, TA, TC, DEEP)                                                                                 \
+  do {                                                                                                             \
+    if (lph == 16 && n_rot) VEC(TIN, TA, TC, DEEP, 16, true);                                                      \
+    else if (lph == 16) VEC(TIN, TA, TC, DEEP, 16, false);                                                         \
+    else if (lph == 32 && !n_rot) VEC(TIN, TA, TC, DEEP, 32, false);                                               \
+    else                                                                                                           \
+      launch_pdl(qk_norm_rope_cache_kernel<TIN, TA, TC, DEEP>, ARGS(TIN, TA, TC), n_rot, H, G, D, Dv, write_cache, bias, lph); \
+  } while (0)
 #define CASE(TIN, TA, TC)                                                                                          \
   do {                                                                                                             \
-    if (deep) {                                                                                                    \
-      if (lph == 32) RUN(TIN, TA, TC, true, 32);                                                                   \
-      else if (lph == 16) RUN(TIN, TA, TC, true, 16);                                                              \
-      else RUN(TIN, TA, TC, true, 0);                                                                              \
-    } else {                                                                                                       \
-      if (lph == 32) RUN(TIN, TA, TC, false, 32);                                                                  \
-      else if (lph == 16) RUN(TIN, TA, TC, false, 16);                                                             \
-      else RUN(TIN, TA, TC, false, 0);                                                                             \
-    }                                                                                                              \
+    if (deep) BY_HEAD(TIN, TA, TC, true);                                                                          \
+    else BY_HEAD(TIN, TA, TC, false);                                                                              \
   } while (0)
   const int key = in_dtype * 4 + act_dtype * 2 + cache_dtype;
   switch (key) {
@@ -768,7 +855,9 @@ LLMX_API int llmx_qk_norm_rope_cache_biased(const void* qkv, int in_dtype, int n
     default: return LLMX_REFUSED(2);
   }
 #undef CASE
-#undef RUN
+#undef BY_HEAD
+#undef VEC
+#undef ARGS
   return LLMX_LAUNCH_STATUS();
 }
 
