@@ -806,7 +806,11 @@ LLMX_API int llmx_qk_norm_rope_cache_biased(const void* qkv, int in_dtype, int n
   if (H <= 0 || G <= 0 || D <= 0 || Dv <= 0 || n_rot < 0 || n_rot > D || (n_rot & 1) || n_split < 1) return LLMX_REFUSED(1);
   if (n_rot > 0 && (!cos_t || !sin_t)) return LLMX_REFUSED(4);
   const int n_slots = write_cache ? H + 2 * G : H;
-  if (!bias && n_split == 1 && in_dtype == LLMX_BF16 && act_dtype == LLMX_BF16 && cache_dtype == LLMX_BF16 && D == 128 &&
+  const int sizes[3] = {in_dtype == LLMX_F32 ? 16 : 8, act_dtype == LLMX_F32 ? 16 : 8, cache_dtype == LLMX_F32 ? 16 : 8};
+  const bool vec = !((uintptr_t)qkv & (sizes[0] - 1)) && !(split_stride & 3) && !((uintptr_t)q_out & (sizes[1] - 1)) &&
+                   !(((uintptr_t)k_cache | (uintptr_t)v_cache) & (sizes[2] - 1)) &&
+                   !(((uintptr_t)q_gain | (uintptr_t)k_gain | (uintptr_t)cos_t | (uintptr_t)sin_t | (uintptr_t)bias) & 15);
+  if (vec && !bias && n_split == 1 && in_dtype == LLMX_BF16 && act_dtype == LLMX_BF16 && cache_dtype == LLMX_BF16 && D == 128 &&
       Dv == 128 && (n_rot == 128 || n_rot == 0) && n_tokens > 64 && !(((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15)) {
     const int per_cta = QKV_WARPS * QKV8_PER_WARP;
     launch_pdl(n_rot ? qk_norm_rope_cache_bf16_d128_kernel<true> : qk_norm_rope_cache_bf16_d128_kernel<false>, dim3(n_tokens, (n_slots + per_cta - 1) / per_cta),
@@ -815,10 +819,6 @@ LLMX_API int llmx_qk_norm_rope_cache_biased(const void* qkv, int in_dtype, int n
     return LLMX_LAUNCH_STATUS();
   }
   // Lanes a head: four dims each for heads of 64 and 128 with full rotation or none (vectors in every dtype), else any size.
-  const int sizes[3] = {in_dtype == LLMX_F32 ? 16 : 8, act_dtype == LLMX_F32 ? 16 : 8, cache_dtype == LLMX_F32 ? 16 : 8};
-  const bool vec = !((uintptr_t)qkv & (sizes[0] - 1)) && !(split_stride & 3) && !((uintptr_t)q_out & (sizes[1] - 1)) &&
-                   !(((uintptr_t)k_cache | (uintptr_t)v_cache) & (sizes[2] - 1)) &&
-                   !(((uintptr_t)q_gain | (uintptr_t)k_gain | (uintptr_t)cos_t | (uintptr_t)sin_t | (uintptr_t)bias) & 15);
   const int lph = vec && D == Dv && (n_rot == D || n_rot == 0) && (D == 64 || D == 128) ? D / 4 : 0;
   const bool deep = n_split > 2;
   const int per_cta = QKV_WARPS * (deep ? 1 : QKV_SPW) * (lph ? 32 / lph : 1);

@@ -171,6 +171,26 @@ def test_heads_by_vectors_add_squares_as_an_element_a_lane_does(D, n_rot, T, n_s
     assert torch.equal(made[0][0], made[1][0]) and torch.equal(made[0][1], made[1][1])
 
 
+@pytest.mark.parametrize("T", [64, 65, 70])
+@pytest.mark.parametrize("which", ["q", "k"])
+def test_gains_that_start_between_vectors(T, which):
+    """Unrotated heads whose gains lie at no vector's start (a view of a larger tensor): the bits of the same gains elsewhere."""
+    from llmoxide_b200 import kernels
+    torch.manual_seed(T)
+    H, G, D = 3, 2, 128
+    x, numbers = torch.randn(T, (H + 2 * G) * D, device=DEV).bfloat16(), 1 + 0.1 * torch.randn(2, D + 1, device=DEV)
+    pos, seq = torch.arange(T, dtype=torch.int32, device=DEV), torch.zeros(T, dtype=torch.int32, device=DEV)
+    table, made = torch.tensor([[1, 0]], dtype=torch.int32, device=DEV), []
+    for aligned in (True, False):
+        gains = dict(q=numbers[0, :D].clone(), k=numbers[0, :D].clone())
+        gains[which] = numbers.flatten()[1 : D + 1].clone() if aligned else numbers.flatten()[1 : D + 1]
+        k_cache, v_cache = (torch.zeros(2, G, 64, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        q = torch.empty(T, H * D, dtype=torch.bfloat16, device=DEV)
+        kernels.qk_norm_rope_cache(x, q, k_cache, v_cache, table, seq, pos, gains["q"], gains["k"], 1e-6, None, None, 0, H, G, D, True, D)
+        made.append((q, k_cache, v_cache))
+    assert all(torch.equal(a, b) for a, b in zip(*made))
+
+
 @pytest.mark.parametrize("dtype, n_split", [(torch.bfloat16, 1), (torch.float32, 3)])
 @pytest.mark.parametrize("per_head, H, Dv", [(True, 3, 128), (True, 5, 20), (True, 2, 96), (False, 4, 128), (False, 3, 700),
                                              (False, 16, 128), (False, 17, 300), (False, 1, 8192), (False, 3, 4)])
