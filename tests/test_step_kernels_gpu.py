@@ -88,6 +88,21 @@ def test_router_of_few_and_many_tokens(T, E, n_extra):
             assert a is None or torch.equal(a, b[at : at + len(part)])
 
 
+@pytest.mark.parametrize("E", [8, 9, 15, 16, 17])
+@pytest.mark.parametrize("K", [520, 517])
+def test_router_of_float32_rows(E, K):
+    """Rows of few experts are shared out to the warps in several ways: the same bits as in a prompt, which has one."""
+    from llmoxide_b200 import kernels
+    torch.manual_seed(E + K)
+    x, w, made = torch.randn(70, K, device=DEV), torch.randn(E, K, device=DEV) * 0.05, []
+    for part in (x, x[:64], x[:1]):
+        ids, weights = torch.empty(len(part), 3, dtype=torch.int32, device=DEV), torch.empty(len(part), 3, device=DEV)
+        kernels.moe_router(part, w, ids, weights, 1, 1, 1, "softmax", True, 0.0, 1.0)
+        made.append((ids, weights))
+    for ids, weights in made[1:]:
+        assert torch.equal(ids, made[0][0][: len(ids)]) and torch.equal(weights, made[0][1][: len(ids)])
+
+
 @pytest.mark.parametrize("M, N, K, pad", [(17, 64, 513, 3), (65, 130, 1028, 0), (33, 65, 2048, 0), (70, 66, 2049, 1),
                                           (34, 130, 3072, 0), (129, 65, 3500, 0), (200, 129, 4096, 4)])
 def test_float32_tiles_that_share_k(M, N, K, pad):
@@ -292,3 +307,20 @@ def test_captured_decode_steps_in_two_branches(tmp_path, design, name, dtype, ba
         assert engine.options.cuda_graphs == graphs
     for a, b in zip(*runs):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("batch, branched", [(1, True), (64, True), (65, False)])
+def test_steps_that_are_captured_in_branches(tmp_path, monkeypatch, batch, branched):
+    """Decode steps are cut up where they are captured and have up to 64 tokens, and nowhere else."""
+    import tifapel_configs
+    from llmoxide_b200 import Engine, LoadOptions
+    from llmoxide_b200.parts import branches
+    folder, forked, fork = tifapel_configs.make_folder(tmp_path, "C", "bfloat16"), [], branches.fork
+    monkeypatch.setattr(branches, "fork", lambda rt, name, work: forked.append(name) or fork(rt, name, work))
+    for graphs in (True, False):
+        engine = Engine.load(folder, LoadOptions(dtype="bfloat16", max_tokens=64 * batch, max_batch=batch, cuda_graphs=graphs))
+        slots = [engine.acquire() for _ in range(batch)]
+        for _ in range(4):
+            engine.step([(slot, [5]) for slot in slots])
+        assert bool(forked) == (graphs and branched)
+        forked.clear()
