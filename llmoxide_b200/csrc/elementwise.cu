@@ -589,8 +589,8 @@ __global__ void qk_norm_rope_cache_kernel(const TIN* __restrict__ qkv, int n_spl
 // The same for heads of 64 with full rotation or none and unrotated heads of 128, by vectors: a lane owns four neighbouring dims,
 // and 32 / LPH heads of 4 LPH share a warp; the rotation partner (half a head away) lives in lane +-LPH/2 and comes by shuffle.
 // Squares and rotations have the bits of the kernel above, which took these heads an element a lane.  Bound by two trips to L2.
-// 16 + 2 * 8 heads of 64, an element a lane and like this: one token of five partials 3.0 and 1.8 us, 23 tokens 6.0 and 2.9,
-// 4000 tokens 33.8 and 13.9; unrotated heads of 128 with gains, 64 tokens: 6.1 and 2.9.  (A kernel of its own: as one with that
+// 16 + 2 * 8 heads of 64 with gains, an element a lane and like this: one token of five partials 2.6 and 1.8 us, 4100 tokens 42.2
+// and 13.9; unrotated heads of 128 with gains, 64 tokens: 6.1 and 2.7.  (A kernel of its own: as one with that
 // above, rotated heads of 128 took 1.5 to 1.7 us in a decode step in place of 1.3.)
 template <typename TIN, typename TA, typename TC, bool DEEP, int LPH, bool ROT>
 __global__ void qk_norm_rope_cache_vec_kernel(const TIN* __restrict__ qkv, int n_split, size_t split_stride,
@@ -684,7 +684,7 @@ __global__ void qk_norm_rope_cache_vec_kernel(const TIN* __restrict__ qkv, int n
 // The same for prompts when everything is bfloat16, the head size is 128 and the rotation is full or none: half a
 // warp per head, a lane owns eight consecutive dims (one 16-byte load, one 16-byte store); the rotation
 // partner (dim +-64) lives eight lanes away.  A warp takes eight heads of its token, two at a time.  4100 tokens of 16 + 2 * 4
-// heads: rotated 13.8 us, unrotated with gains 20.6 (their squares' chains cross lanes; an element a lane 32.2).
+// heads with gains: rotated 12.9 us, unrotated 14.4 (their squares' chains cross lanes; an element a lane 38.3).
 #define QKV8_PER_WARP 8
 
 template <bool ROT>
