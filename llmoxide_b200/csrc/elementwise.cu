@@ -586,13 +586,16 @@ __global__ void qk_norm_rope_cache_kernel(const TIN* __restrict__ qkv, int n_spl
   }
 }
 
-// The same for heads of 64 with full rotation or none and unrotated heads of 128, by vectors: a lane owns four neighbouring dims,
-// and 32 / LPH heads of 4 LPH share a warp; the rotation partner (half a head away) lives in lane +-LPH/2 and comes by shuffle.
-// Squares and rotations have the bits of the kernel above, which took these heads an element a lane.  Bound by two trips to L2.
-// 16 + 2 * 8 heads of 64 with gains, an element a lane and like this: one token of five partials 2.6 and 1.8 us, 4100 tokens 42.2
-// and 13.9; unrotated heads of 128 with gains, 64 tokens: 6.1 and 2.7.  (A kernel of its own: as one with that
-// above, rotated heads of 128 took 1.5 to 1.7 us in a decode step in place of 1.3.)
-template <typename TIN, typename TA, typename TC, bool DEEP, int LPH, bool ROT>
+// The same for heads of 64 and 128 with full rotation or none, by vectors: a lane owns four neighbouring dims, and 32 / LPH heads
+// of 4 LPH share a warp; the rotation partner (half a head away) lives in lane +-LPH/2 and comes by shuffle.  Squares and
+// rotations have the bits of the kernel above, which took all but rotated heads of 128 an element a lane.  Bound by two trips to
+// L2.  16 + 2 * 8 heads of 64 with gains, an element a lane and like this: one token of five partials 2.6 and 1.8 us, 4100 tokens
+// 42.2 and 13.9; unrotated heads of 128 with gains, 64 tokens: 6.1 and 2.7.
+// Rotated heads of 128 come here where launches overlap (decode steps): a step of eight tokens through 36 layers takes 3301 us so
+// and 3397 with the kernel above, although launches of the same kernel in a row take 1.8 us here and 1.4 there: the step
+// decides; why it differs was not found.  Launched in order (prompts) the kernel above is the faster one: 400 tokens 2.9 us, 3.3
+// here.
+template <typename TIN, typename TA, typename TC, bool DEEP, int LPH>
 __global__ void qk_norm_rope_cache_vec_kernel(const TIN* __restrict__ qkv, int n_split, size_t split_stride,
                                           TA* __restrict__ q_out,
                                           TC* __restrict__ k_cache, TC* __restrict__ v_cache,
@@ -600,41 +603,43 @@ __global__ void qk_norm_rope_cache_vec_kernel(const TIN* __restrict__ qkv, int n
                                           const int* __restrict__ token_seq, const int* __restrict__ token_pos,
                                           const float* __restrict__ q_gain, const float* __restrict__ k_gain,
                                           float eps, const float* __restrict__ cos_t,
-                                          const float* __restrict__ sin_t, int H, int G, int write_cache, const float* __restrict__ bias) {
-  constexpr int SPW = DEEP ? 1 : QKV_SPW, HPW = 32 / LPH, D = 4 * LPH;      // heads one after another, and side by side
+                                          const float* __restrict__ sin_t, int n_rot, int H, int G, int D,
+                                          int Dv, int write_cache, const float* __restrict__ bias) {
+  constexpr int SPW = DEEP ? 1 : QKV_SPW, HPW = 32 / LPH;      // heads one after another, and side by side
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = blockIdx.x;                        // tokens on x: a step may bring more than 65535
   const int slot0 = (blockIdx.y * QKV_WARPS + warp) * SPW * HPW;   // the warp's first head of the fused row
   const int n_slots = write_cache ? H + 2 * G : H;
   if (slot0 >= n_slots) return;
-  const TIN* tok = qkv + (size_t)t * (H + 2 * G) * D;
+  const TIN* tok = qkv + (size_t)t * ((size_t)(H + G) * D + (size_t)G * Dv);
   const int pos = token_pos[t];
   int page = 0;
   if (slot0 + SPW * HPW > H) page = block_table[(size_t)token_seq[t] * table_width + pos / LLMX_PAGE];
   auto cache_row_of = [&](int slot) -> TC* {        // slot >= H: a k head, then the v heads
     const bool is_k = slot < H + G;
     return is_k ? k_cache + cache_row_offset(page, slot - H, pos % LLMX_PAGE, G, D)
-                : v_cache + cache_row_offset(page, slot - H - G, pos % LLMX_PAGE, G, D);
+                : v_cache + cache_row_offset(page, slot - H - G, pos % LLMX_PAGE, G, Dv);
   };
 
-  const int l = lane % LPH, d0 = 4 * l, dh = d0 & (D / 2 - 1), sub = lane / LPH;
+  constexpr int HD = 4 * LPH;
+  const int l = lane % LPH, d0 = 4 * l, dh = d0 & (HD / 2 - 1), sub = lane / LPH;
   const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
   const float4 gq = q_gain ? load4(q_gain + d0) : one, gk = k_gain ? load4(k_gain + d0) : one;
   float4 cs = one, sn = one;
-  if (ROT) cs = load4(cos_t + (size_t)pos * (D / 2) + dh), sn = load4(sin_t + (size_t)pos * (D / 2) + dh);
+  if (n_rot) cs = load4(cos_t + (size_t)pos * (HD / 2) + dh), sn = load4(sin_t + (size_t)pos * (HD / 2) + dh);
   pdl_wait();
   float4 xs[SPW];
 #pragma unroll
   for (int j = 0; j < SPW; ++j) {
     const int slot = slot0 + j * HPW + sub;
-    if (HPW > 1) xs[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    xs[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (slot < n_slots) {
-      const TIN* src = tok + (size_t)slot * D;
+      const TIN* src = tok + (size_t)slot * HD;
       xs[j] = load4(src + d0);
       add_partials4<DEEP ? 8 : 1>(xs[j], src + split_stride + d0, n_split - 1, split_stride);
       if (bias) {
-        const float4 bv = load4(bias + (size_t)slot * D + d0);
+        const float4 bv = load4(bias + (size_t)slot * HD + d0);
         xs[j].x += bv.x, xs[j].y += bv.y, xs[j].z += bv.z, xs[j].w += bv.w;
       }
     }
@@ -645,38 +650,34 @@ __global__ void qk_norm_rope_cache_vec_kernel(const TIN* __restrict__ qkv, int n
     const int slot = slot0 + j * HPW + sub;
     float4 x = xs[j];
     const bool is_q = slot < H, is_k = !is_q && slot < H + G;
-    if (HPW == 1 && !is_q && !is_k) {                // v: stored as it is
-      store4(cache_row_of(slot) + d0, x);
-      continue;
+    float ssq = 0.f;
+    if (LPH == 32 && n_rot) {
+      ssq = warp_sum(x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w);
+    } else if (q_gain || k_gain) {
+      const float v[4] = {x.x, x.y, x.z, x.w};
+      ssq = head_sumsq<4, LPH>(v, 0xffffffffu);
     }
-    if (q_gain || k_gain) {
-      const float v[4] = {x.x, x.y, x.z, x.w}, ssq = head_sumsq<4, LPH>(v, 0xffffffffu);
-      if ((is_q && q_gain) || (is_k && k_gain)) {
-        const float4 gn = is_q ? gq : gk;
-        const float scale = 1.0f / sqrtf(ssq / (float)D + eps);
-        x.x = (x.x * scale) * gn.x; x.y = (x.y * scale) * gn.y; x.z = (x.z * scale) * gn.z; x.w = (x.w * scale) * gn.w;
-      }
+    if ((is_q && q_gain) || (is_k && k_gain)) {
+      const float4 gn = is_q ? gq : gk;
+      const float scale = 1.0f / sqrtf(ssq / (float)HD + eps);
+      x.x = (x.x * scale) * gn.x; x.y = (x.y * scale) * gn.y; x.z = (x.z * scale) * gn.z; x.w = (x.w * scale) * gn.w;
     }
-    float4 r = x;
-    if (ROT) {
-      float4 p;
-      p.x = __shfl_xor_sync(0xffffffffu, x.x, LPH / 2);
-      p.y = __shfl_xor_sync(0xffffffffu, x.y, LPH / 2);
-      p.z = __shfl_xor_sync(0xffffffffu, x.z, LPH / 2);
-      p.w = __shfl_xor_sync(0xffffffffu, x.w, LPH / 2);
+    float4 r = x, p;
+    p.x = __shfl_xor_sync(0xffffffffu, x.x, LPH / 2);
+    p.y = __shfl_xor_sync(0xffffffffu, x.y, LPH / 2);
+    p.z = __shfl_xor_sync(0xffffffffu, x.z, LPH / 2);
+    p.w = __shfl_xor_sync(0xffffffffu, x.w, LPH / 2);
+    if (n_rot && (is_q || is_k)) {
       // dims i of the first half: x_i cos - x_(i+half) sin; dims i + half: x_i sin + x_(i+half) cos.  Which product is rounded
       // by itself is what the kernel above does.
-      auto down = [](float x, float p, float c, float s) { return fmaf(x, c, -__fmul_rn(p, s)); };
-      auto up = [](float x, float p, float c, float s) { return fmaf(p, s, __fmul_rn(x, c)); };
-      if (!is_q && !is_k) {
-      } else if (l < LPH / 2) {
-        r = make_float4(down(x.x, p.x, cs.x, sn.x), down(x.y, p.y, cs.y, sn.y), down(x.z, p.z, cs.z, sn.z), down(x.w, p.w, cs.w, sn.w));
-      } else {
-        r = make_float4(up(x.x, p.x, cs.x, sn.x), up(x.y, p.y, cs.y, sn.y), up(x.z, p.z, cs.z, sn.z), up(x.w, p.w, cs.w, sn.w));
-      }
+      auto turn = [&](float x, float p, float c, float s) {
+        if (l < LPH / 2) return fmaf(x, c, -__fmul_rn(p, s));
+        return LPH == 32 ? fmaf(x, c, __fmul_rn(p, s)) : fmaf(p, s, __fmul_rn(x, c));
+      };
+      r = make_float4(turn(x.x, p.x, cs.x, sn.x), turn(x.y, p.y, cs.y, sn.y), turn(x.z, p.z, cs.z, sn.z), turn(x.w, p.w, cs.w, sn.w));
     }
     if (slot >= n_slots) continue;
-    if (is_q) store4(q_out + (size_t)t * H * D + (size_t)slot * D + d0, r);
+    if (is_q) store4(q_out + (size_t)t * H * HD + (size_t)slot * HD + d0, r);
     else store4(cache_row_of(slot) + d0, r);
   }
 }
@@ -829,13 +830,12 @@ LLMX_API int llmx_qk_norm_rope_cache_biased(const void* qkv, int in_dtype, int n
 #define ARGS(TIN, TA, TC)                                                                                          \
   grid, dim3(QKV_WARPS * 32), smem, stream, (const TIN*)qkv, n_split, (size_t)split_stride, (TA*)q_out, (TC*)k_cache, \
       (TC*)v_cache, block_table, table_width, token_seq, token_pos, q_gain, k_gain, eps, cos_t, sin_t
-#define VEC(TIN, TA, TC, DEEP, LPH, ROT) \
-  launch_pdl(qk_norm_rope_cache_vec_kernel<TIN, TA, TC, DEEP, LPH, ROT>, ARGS(TIN, TA, TC), H, G, write_cache, bias)
+#define VEC(TIN, TA, TC, DEEP, LPH)                                                                                \
+  launch_pdl(qk_norm_rope_cache_vec_kernel<TIN, TA, TC, DEEP, LPH>, ARGS(TIN, TA, TC), n_rot, H, G, D, Dv, write_cache, bias)
 #define BY_HEAD(TIN, TA, TC, DEEP)                                                                                 \
   do {                                                                                                             \
-    if (lph == 16 && n_rot) VEC(TIN, TA, TC, DEEP, 16, true);                                                      \
-    else if (lph == 16) VEC(TIN, TA, TC, DEEP, 16, false);                                                         \
-    else if (lph == 32 && !n_rot) VEC(TIN, TA, TC, DEEP, 32, false);                                               \
+    if (lph == 16) VEC(TIN, TA, TC, DEEP, 16);                                                                     \
+    else if (lph == 32 && (!n_rot || llmx_pdl_allowed())) VEC(TIN, TA, TC, DEEP, 32);                              \
     else                                                                                                           \
       launch_pdl(qk_norm_rope_cache_kernel<TIN, TA, TC, DEEP>, ARGS(TIN, TA, TC), n_rot, H, G, D, Dv, write_cache, bias, lph); \
   } while (0)
